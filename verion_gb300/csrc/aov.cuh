@@ -146,8 +146,7 @@ static __global__ void __launch_bounds__(128) aov_main(const __grid_constant__ C
         V3 sd = normalize(sdir);
         float seen = 0.0f, through = 1.0f;
         for (uint32_t layer = 0; layer < 8 && through > 0.0f; layer++) {
-            vgt::TRay r = vgt::make_ray(so, sd);
-            vgt::TraceHit q = vgt::trace_bvh<false>(c.s.nodes, c.s.tris, r, 1.0e30f, c.err);
+            vgt::TraceHit q = vgt::trace_bvh<false>(c.s.nodes, c.s.tris, so, sd, 1.0e30f, c.err);
             if (!q.hit)
                 break;
             float op = opacityAt(c, q.inst, q.prim, q.b1, q.b2);

@@ -15,8 +15,10 @@
 // 8-bit integers and 2^e a power of two, q * 2^e is exact and the decoded plane is one rounded
 // add, which the builder reproduces to make every decoded box contain its child.
 // imask bit s: slot s is an internal node, stored at child_base + popc(imask & ((1 << s) - 1)).
-// meta[s] for a leaf slot: (count << 5) | offset, 1 <= count <= 3 triangles at tri_base + offset
-// (offset < 24); 0 for internal and empty slots.
+// meta[s]: bits 5-7 as many ones as the slot has bits in the traversal's hit word, bits 0-4 where they
+// start there. A leaf slot: 1 to 3 ones for its triangles at tri_base + offset (offset < 24); an
+// internal slot: one, at 24 + s (META_INNER | s); 0 for an empty slot. (The layout of Ylitie et al.:
+// a hit child's bits enter the hit word with one shift, whatever the child is.)
 // Slots are assigned so that a ray whose direction has sign octant o (bit k set when component k
 // is negative) meets the child in slot o first; traversal visits hit children in order of
 // (slot XOR o), a front-to-back order without sorting (the ordering idea of Ylitie, Karras and
@@ -34,6 +36,7 @@ constexpr uint32_t NODE_VEC4 = 5;        // 16-byte words per node
 constexpr uint32_t TRI_FLOATS = 12;      // f32 words per triangle record
 constexpr uint32_t TRI_VEC4 = 3;
 constexpr uint32_t MAX_LEAF_TRIS = 3;
+constexpr uint32_t META_INNER = 0x38u;   // one bit at 24 + slot
 constexpr uint32_t STACK_SIZE = 32;      // traversal stack entries (node groups)
 constexpr uint32_t MAX_WIDE_DEPTH = 30;  // the builder rejects trees deeper than this
 constexpr uint32_t ERR_STACK = 1u;       // error-status bit: a traversal stack overflowed

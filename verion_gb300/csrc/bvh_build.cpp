@@ -383,8 +383,9 @@ bool build_bvh8(const float* verts, const uint32_t* inst, const uint32_t* prim, 
             }
             if (c.count == 0) {
                 imask |= 1u << s;
+                meta[s] = (uint8_t)(bvh8::META_INNER | s);
             } else {
-                meta[s] = (uint8_t)((c.count << 5) | tri_off);
+                meta[s] = (uint8_t)((((1u << c.count) - 1u) << 5) | tri_off);
                 for (uint32_t i = 0; i < c.count; i++) {
                     uint32_t t = b.order[c.a + i];
                     const float* v = &verts[9 * (size_t)t];
@@ -449,14 +450,15 @@ bool build_bvh8(const float* verts, const uint32_t* inst, const uint32_t* prim, 
         }
         for (int s = 0; s < 8; s++) {
             if ((imask >> s) & 1u) {
-                if (meta[s] != 0) {
+                if (meta[s] != (bvh8::META_INNER | (uint32_t)s)) {
                     err = "BVH internal slot with leaf data";
                     return false;
                 }
                 continue;
             }
-            uint32_t cnt = meta[s] >> 5, off = meta[s] & 31u;
-            if (cnt > bvh8::MAX_LEAF_TRIS || (uint64_t)w[5] + off + cnt > tri_count) {
+            uint32_t cnt = (uint32_t)__builtin_popcount(meta[s] >> 5), off = meta[s] & 31u;
+            if ((meta[s] >> 5) != (1u << cnt) - 1u || cnt > bvh8::MAX_LEAF_TRIS || off >= 24u ||
+                (uint64_t)w[5] + off + cnt > tri_count) {
                 err = "BVH triangle range out of range";
                 return false;
             }

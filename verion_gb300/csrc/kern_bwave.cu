@@ -114,7 +114,7 @@ static __device__ __forceinline__ bool take_items(const WaveBatch& b, const Wave
 
 // The first wave's queue: slot i takes work item i. Also sets the request counters, the item
 // counter, the loop counter and the start time.
-__global__ void __launch_bounds__(256) bw_start(WaveBatch b, Wave w)
+__global__ void __launch_bounds__(256) bw_start(const __grid_constant__ WaveBatch b, const __grid_constant__ Wave w)
 {
     __shared__ uint32_t slot[8];
     uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
@@ -135,7 +135,7 @@ __global__ void __launch_bounds__(256) bw_start(WaveBatch b, Wave w)
 }
 
 // Closest hits of the wave's rays, each in its request's scene (wf_stream_extend_dyn).
-__global__ void __launch_bounds__(128, VG_TRACE_MIN_BLOCKS) bw_extend(WaveBatch b, Wave w, uint32_t wave)
+__global__ void __launch_bounds__(128, VG_TRACE_MIN_BLOCKS) bw_extend(const __grid_constant__ WaveBatch b, const __grid_constant__ Wave w, uint32_t wave)
 {
     uint32_t in = wave & 1u, out = in ^ 1u;
     if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -173,7 +173,7 @@ __global__ void __launch_bounds__(128, VG_TRACE_MIN_BLOCKS) bw_extend(WaveBatch 
 
 // Material classes of the wave's slots (wf_stream_classify), each from its request's scene; a
 // cached request's slots in classes SHADE_CLASSES and up.
-__global__ void __launch_bounds__(256) bw_classify(WaveBatch b, Wave w, uint32_t wave)
+__global__ void __launch_bounds__(256) bw_classify(const __grid_constant__ WaveBatch b, const __grid_constant__ Wave w, uint32_t wave)
 {
     uint32_t in = wave & 1u, out = in ^ 1u;
     if (blockIdx.x == 0 && threadIdx.x < BW_CLASSES)
@@ -200,7 +200,7 @@ __global__ void __launch_bounds__(256) bw_classify(WaveBatch b, Wave w, uint32_t
 // cached requests' slots, whose paths may end at the cache (a query record for the wave's answer
 // stage) or, on a training pixel, record their vertices.
 template <bool CACHE>
-__global__ void __launch_bounds__(128, VG_SHADE_MIN_BLOCKS) bw_shade(WaveBatch b, Wave w, uint32_t wave)
+__global__ void __launch_bounds__(128, VG_SHADE_MIN_BLOCKS) bw_shade(const __grid_constant__ WaveBatch b, const __grid_constant__ Wave w, uint32_t wave)
 {
     uint32_t in = wave & 1u;
     uint32_t n = w.n;
@@ -295,7 +295,7 @@ __global__ void __launch_bounds__(128, VG_SHADE_MIN_BLOCKS) bw_shade(WaveBatch b
 
 // Shadow rays of the wave's light samples, any hit, each in its request's scene. A scene with
 // translucent surfaces leaves its rays to the finish stage (occluded(): layers with opacity).
-__global__ void __launch_bounds__(128, VG_TRACE_MIN_BLOCKS) bw_shadow_trace(WaveBatch b, Wave w, uint32_t wave)
+__global__ void __launch_bounds__(128, VG_TRACE_MIN_BLOCKS) bw_shadow_trace(const __grid_constant__ WaveBatch b, const __grid_constant__ Wave w, uint32_t wave)
 {
     uint32_t in = wave & 1u;
     uint32_t count = w.counts[in];
@@ -408,7 +408,7 @@ static __device__ __forceinline__ bool finish_slot(const WaveBatch& b, const Wav
     return false;
 }
 
-__global__ void __launch_bounds__(128, 8) bw_finish(WaveBatch b, Wave w, uint32_t wave)
+__global__ void __launch_bounds__(128, 8) bw_finish(const __grid_constant__ WaveBatch b, const __grid_constant__ Wave w, uint32_t wave)
 {
     uint32_t in = wave & 1u, out = in ^ 1u;
     if (blockIdx.x == 0 && threadIdx.x == 0)
@@ -551,7 +551,7 @@ __global__ void __launch_bounds__(128) bw_answer(WaveBatch b)
 
 // The loop's condition after each body (two waves, so the next wave reads queue 0): go on while
 // more than b.tail slots are live, at most b.max_iter times.
-__global__ void bw_condition(WaveBatch b, Wave w, cudaGraphConditionalHandle loop)
+__global__ void bw_condition(const __grid_constant__ WaveBatch b, const __grid_constant__ Wave w, cudaGraphConditionalHandle loop)
 {
     uint32_t it = ++b.loop[0];
     cudaGraphSetConditional(loop, (w.counts[0] > b.tail && it < b.max_iter) ? 1u : 0u);
@@ -560,7 +560,7 @@ __global__ void bw_condition(WaveBatch b, Wave w, cudaGraphConditionalHandle loo
 // The tail: one thread per live slot (a grid-stride loop over queue 0) runs its path, the rest of
 // its pixel's samples and then further work items to the end, trace and shade in a loop as the
 // megakernel does.
-__global__ void __launch_bounds__(128, VG_TAIL_MIN_BLOCKS) bw_tail(WaveBatch b, Wave w)
+__global__ void __launch_bounds__(128, VG_TAIL_MIN_BLOCKS) bw_tail(const __grid_constant__ WaveBatch b, const __grid_constant__ Wave w)
 {
     uint32_t count = w.counts[0];
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) {

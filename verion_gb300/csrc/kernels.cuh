@@ -300,7 +300,7 @@ __global__ void VG_MK_BOUNDS mk_pathtrace(const __grid_constant__ Ctx c, uint32_
 
 // wf_args.slang:9-24 at depth 0: starts a sample. Every pixel's path is live unless adaptive
 // sampling fills the depth-0 queue (wf_select); the later queues and all work counters restart.
-static __global__ void wf_begin(const __grid_constant__ Ctx c, Wave w)
+static __global__ void wf_begin(const __grid_constant__ Ctx c, const __grid_constant__ Wave w)
 {
     uint32_t i = threadIdx.x;
     for (uint32_t k = i; k <= w.depth; k += blockDim.x) {
@@ -313,7 +313,7 @@ static __global__ void wf_begin(const __grid_constant__ Ctx c, Wave w)
 // wf_select.slang:7-18: queues the pixels that still take samples; one atomic per block of 256
 // (the reference takes one per pixel).
 template <typename A>
-__global__ void __launch_bounds__(256) wf_select(const __grid_constant__ Ctx c, Wave w)
+__global__ void __launch_bounds__(256) wf_select(const __grid_constant__ Ctx c, const __grid_constant__ Wave w)
 {
     __shared__ uint32_t slot[8];
     uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
@@ -334,7 +334,7 @@ static __device__ __forceinline__ void warp_count(unsigned long long* dst, uint3
 // wf_extend.slang:6-30: closest hit for every live path of depth d. STATS also counts rays,
 // BVH nodes visited and triangles tested into w.tstats[0..2] (rays at depth > 0 into [3]).
 template <bool STATS>
-__global__ void __launch_bounds__(128, 8) wf_extend(const __grid_constant__ Ctx c, Wave w, uint32_t d)
+__global__ void __launch_bounds__(128, 8) wf_extend(const __grid_constant__ Ctx c, const __grid_constant__ Wave w, uint32_t d)
 {
     uint32_t count = w.counts[d];
     const uint32_t* qin = w.queue[d & 1u];
@@ -358,8 +358,7 @@ __global__ void __launch_bounds__(128, 8) wf_extend(const __grid_constant__ Ctx 
                 org = v3(a.x, a.y, a.z);
                 dir = v3(b.x, b.y, b.z);
             }
-            vgt::TRay r = vgt::make_ray(org, dir);
-            vgt::TraceHit q = vgt::trace_bvh<false>(c.s.nodes, c.s.tris, r, 1.0e30f, c.err);
+            vgt::TraceHit q = vgt::trace_bvh<false>(c.s.nodes, c.s.tris, org, dir, 1.0e30f, c.err);
             w.hits[p] = make_uint4(q.hit ? 1u : 0u, q.hit ? q.inst : 0u, q.hit ? q.prim : 0u,
                                    __float_as_uint(q.hit ? q.t : 0.0f));
             if (STATS) {
@@ -380,7 +379,7 @@ __global__ void __launch_bounds__(128, 8) wf_extend(const __grid_constant__ Ctx 
 
 // wf_shade.slang:7-29: shade each live path of depth d, then queue it for d + 1 or finish it.
 template <bool LIGHT, bool RESTIR, typename A>
-__global__ void __launch_bounds__(128, VG_SHADE_MIN_BLOCKS) wf_shade(const __grid_constant__ Ctx c, Wave w, uint32_t d)
+__global__ void __launch_bounds__(128, VG_SHADE_MIN_BLOCKS) wf_shade(const __grid_constant__ Ctx c, const __grid_constant__ Wave w, uint32_t d)
 {
     uint32_t count = w.counts[d];
     const uint32_t* qin = w.queue[d & 1u];
@@ -467,7 +466,7 @@ __device__ __forceinline__ PathState<LIGHT> loadState(const Wave& w, uint32_t p)
 // Starts the batch: every pixel that takes a sample (wf_select's test) begins sample params[6].
 // With CACHE the training pixels of the frame are left out (a kernel of their own traces them).
 template <bool LIGHT, typename A, bool CACHE = false>
-__global__ void __launch_bounds__(256) wf_stream_start(const __grid_constant__ Ctx c, Wave w, CacheWave q)
+__global__ void __launch_bounds__(256) wf_stream_start(const __grid_constant__ Ctx c, const __grid_constant__ Wave w, CacheWave q)
 {
     __shared__ uint32_t slot[8];
     uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
@@ -483,7 +482,7 @@ __global__ void __launch_bounds__(256) wf_stream_start(const __grid_constant__ C
 }
 
 template <bool STATS>
-__global__ void __launch_bounds__(128, 8) wf_stream_extend(const __grid_constant__ Ctx c, Wave w, uint32_t wave)
+__global__ void __launch_bounds__(128, 8) wf_stream_extend(const __grid_constant__ Ctx c, const __grid_constant__ Wave w, uint32_t wave)
 {
     uint32_t in = wave & 1u, out = in ^ 1u;
     if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -503,8 +502,8 @@ __global__ void __launch_bounds__(128, 8) wf_stream_extend(const __grid_constant
             uint32_t p = qin[i];
             float4 a = w.state[p];
             float4 b = w.state[w.n + p];
-            vgt::TRay r = vgt::make_ray(v3(a.x, a.y, a.z), v3(b.x, b.y, b.z));
-            vgt::TraceHit q = vgt::trace_bvh<false>(c.s.nodes, c.s.tris, r, 1.0e30f, c.err);
+            vgt::TraceHit q = vgt::trace_bvh<false>(c.s.nodes, c.s.tris, v3(a.x, a.y, a.z), v3(b.x, b.y, b.z), 1.0e30f,
+                                                    c.err);
             w.hits[p] = make_uint4(q.hit ? 1u : 0u, q.hit ? q.inst : 0u, q.hit ? q.prim : 0u,
                                    __float_as_uint(q.hit ? q.t : 0.0f));
             if (STATS) {
@@ -525,7 +524,7 @@ __global__ void __launch_bounds__(128, 8) wf_stream_extend(const __grid_constant
 }
 
 template <bool LIGHT, typename A, bool RESTIR = false>
-__global__ void __launch_bounds__(128, VG_SHADE_MIN_BLOCKS) wf_stream_shade(const __grid_constant__ Ctx c, Wave w, uint32_t wave)
+__global__ void __launch_bounds__(128, VG_SHADE_MIN_BLOCKS) wf_stream_shade(const __grid_constant__ Ctx c, const __grid_constant__ Wave w, uint32_t wave)
 {
     uint32_t in = wave & 1u, out = in ^ 1u;
     if (blockIdx.x == 0 && threadIdx.x == 0)
@@ -590,7 +589,7 @@ static __device__ __forceinline__ uint32_t shadeClass(const Ctx& c, uint4 hr)
 // (one atomic per class present in a warp), so the deferred shade stage's warps mostly run one
 // BSDF's code. Clears the other parity's class counts for the next wave (the shade stage of the
 // previous wave, their last reader, has finished).
-static __global__ void __launch_bounds__(256) wf_stream_classify(const __grid_constant__ Ctx c, Wave w, uint32_t wave)
+static __global__ void __launch_bounds__(256) wf_stream_classify(const __grid_constant__ Ctx c, const __grid_constant__ Wave w, uint32_t wave)
 {
     uint32_t in = wave & 1u, out = in ^ 1u;
     if (blockIdx.x == 0 && threadIdx.x < SHADE_CLASSES)
@@ -618,7 +617,7 @@ static __global__ void __launch_bounds__(256) wf_stream_classify(const __grid_co
 // With SORTED the wave's slots are taken class by class from the classify stage's queues.
 template <typename A, bool CACHE = false, bool RESTIR = false, bool SORTED = false>
 __global__ void __launch_bounds__(128, RESTIR ? VG_RESTIR_SHADE_MIN_BLOCKS : VG_SHADE_MIN_BLOCKS) wf_stream_shade_deferred(const __grid_constant__ Ctx c,
-                                                                                    Wave w, uint32_t wave,
+                                                                                    const __grid_constant__ Wave w, uint32_t wave,
                                                                                     CacheWave q)
 {
     uint32_t in = wave & 1u;
@@ -738,7 +737,7 @@ __device__ __forceinline__ bool finishSlot(const Ctx& c, const Wave& w, uint32_t
 }
 
 template <typename A, bool RESTIR = false>
-__global__ void __launch_bounds__(128, 8) wf_stream_shadow(const __grid_constant__ Ctx c, Wave w, uint32_t wave)
+__global__ void __launch_bounds__(128, 8) wf_stream_shadow(const __grid_constant__ Ctx c, const __grid_constant__ Wave w, uint32_t wave)
 {
     uint32_t in = wave & 1u, out = in ^ 1u;
     if (blockIdx.x == 0 && threadIdx.x == 0)
@@ -798,7 +797,7 @@ __device__ __forceinline__ void trace_queue_any(const Ctx& c, uint32_t* fetch, u
 #endif
 
 template <bool STATS, bool COOP>
-__global__ void __launch_bounds__(128, VG_TRACE_MIN_BLOCKS) wf_stream_extend_dyn(const __grid_constant__ Ctx c, Wave w, uint32_t wave)
+__global__ void __launch_bounds__(128, VG_TRACE_MIN_BLOCKS) wf_stream_extend_dyn(const __grid_constant__ Ctx c, const __grid_constant__ Wave w, uint32_t wave)
 {
     uint32_t in = wave & 1u, out = in ^ 1u;
     if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -850,7 +849,7 @@ __global__ void __launch_bounds__(128, VG_TRACE_MIN_BLOCKS) wf_stream_extend_dyn
 #endif
 
 template <bool STATS, bool COOP>
-__global__ void __launch_bounds__(128, VG_SHADOW_MIN_BLOCKS) wf_stream_shadow_trace(const __grid_constant__ Ctx c, Wave w, uint32_t wave)
+__global__ void __launch_bounds__(128, VG_SHADOW_MIN_BLOCKS) wf_stream_shadow_trace(const __grid_constant__ Ctx c, const __grid_constant__ Wave w, uint32_t wave)
 {
     uint32_t in = wave & 1u;
     uint32_t count = w.counts[in];
@@ -888,7 +887,7 @@ __global__ void __launch_bounds__(128, VG_SHADOW_MIN_BLOCKS) wf_stream_shadow_tr
 #endif
 
 template <typename A, bool RESTIR = false>
-__global__ void __launch_bounds__(128, VG_FINISH_MIN_BLOCKS) wf_stream_finish(const __grid_constant__ Ctx c, Wave w, uint32_t wave)
+__global__ void __launch_bounds__(128, VG_FINISH_MIN_BLOCKS) wf_stream_finish(const __grid_constant__ Ctx c, const __grid_constant__ Wave w, uint32_t wave)
 {
     uint32_t in = wave & 1u, out = in ^ 1u;
     if (blockIdx.x == 0 && threadIdx.x == 0)
@@ -917,7 +916,7 @@ __global__ void __launch_bounds__(128, VG_FINISH_MIN_BLOCKS) wf_stream_finish(co
 // instead of one half-empty wave per bounce. Same functions, same order per pixel, same sums.
 // With CACHE (lighting split off) paths end at the cache as in wf_stream_shade_deferred.
 template <bool LIGHT, typename A, bool CACHE = false, bool RESTIR = false>
-__global__ void __launch_bounds__(128, VG_TAIL_MIN_BLOCKS) wf_stream_tail(const __grid_constant__ Ctx c, Wave w,
+__global__ void __launch_bounds__(128, VG_TAIL_MIN_BLOCKS) wf_stream_tail(const __grid_constant__ Ctx c, const __grid_constant__ Wave w,
                                                                           uint32_t wave, CacheWave q)
 {
     static_assert(!(CACHE && LIGHT), "the cache runs with the lighting split off");

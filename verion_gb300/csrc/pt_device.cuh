@@ -519,10 +519,9 @@ static __device__ __noinline__ float opacityAt(const Ctx& c, uint32_t instIdx, u
 
 static __device__ __forceinline__ vgt::TraceHit traceShadow(const Ctx& c, V3 o, V3 d, float tmax)
 {
-    vgt::TRay r = vgt::make_ray(o, d);
     if (c.s.shadow_any)
-        return vgt::trace_bvh<true>(c.s.nodes, c.s.tris, r, tmax, c.err);
-    return vgt::trace_bvh<false>(c.s.nodes, c.s.tris, r, tmax, c.err);
+        return vgt::trace_bvh<true>(c.s.nodes, c.s.tris, o, d, tmax, c.err);
+    return vgt::trace_bvh<false>(c.s.nodes, c.s.tris, o, d, tmax, c.err);
 }
 
 // pt_core.slang:580-613. A scene with translucent surfaces takes the closest occluder of each
@@ -622,8 +621,7 @@ __device__ PathState<LIGHT> generatePathFor(const Ctx& c, uint32_t px, uint32_t 
 // pt_core.slang:684-700
 static __device__ __forceinline__ Hit traceClosest(const Ctx& c, V3 org, V3 dir)
 {
-    vgt::TRay r = vgt::make_ray(org, dir);
-    vgt::TraceHit q = vgt::trace_bvh<false>(c.s.nodes, c.s.tris, r, 1.0e30f, c.err);
+    vgt::TraceHit q = vgt::trace_bvh<false>(c.s.nodes, c.s.tris, org, dir, 1.0e30f, c.err);
     Hit h;
     h.hit = q.hit;
     h.inst = q.hit ? q.inst : 0;

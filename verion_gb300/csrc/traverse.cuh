@@ -109,7 +109,7 @@ __device__ __forceinline__ bool tri_test(const TRay& r, V3 v0, V3 v1, V3 v2, flo
 
 struct TraceHit {
     bool hit;
-    uint32_t inst, prim, gid;
+    uint32_t inst, prim;
     float t;
     float b1, b2;           // barycentric weights of vertices 1 and 2
     uint32_t nodes, tests;  // nodes visited and triangles tested (dropped by the compiler unless read)
@@ -121,29 +121,51 @@ __device__ __forceinline__ uint32_t byte_of(uint32_t lo, uint32_t hi, int i)
     return (w >> ((i & 3) * 8)) & 0xffu;
 }
 
-// The byte as a float, exactly: the byte placed in the mantissa of 2^23 (one byte permute), minus
-// 2^23; equal to (float)byte_of(lo, hi, i) without an integer-to-float conversion.
-__device__ __forceinline__ float byte_f(uint32_t lo, uint32_t hi, int i)
+// The byte as a float plus 2^15, exactly: the byte placed in bits 8-15 of the mantissa of 2^15 (one
+// byte permute; the last place of the float there is 2^-8). The node test folds the 2^15 into the
+// constant of its FMA, so a plane costs a permute and an FMA, with no subtraction.
+__device__ __forceinline__ float byte_f15(uint32_t lo, uint32_t hi, int i)
 {
     uint32_t w = i < 4 ? lo : hi;
-    return __uint_as_float(__byte_perm(w, 0x4B000000u, 0x7650u + (uint32_t)(i & 3))) - 8388608.0f;
+    return __uint_as_float(__byte_perm(w, 0x47000000u, 0x7604u + ((uint32_t)(i & 3) << 4)));
 }
 
+__device__ __forceinline__ float max3(float a, float b, float c)
+{
+    float d;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+    return d;
+}
 
-// Child-box tests of one BVH8 node (words w0..w4, bvh8.h) for ray r with the closest hit so far at
-// best_t: the hit internal children as bits (slot XOR octant, the visiting order) and the triangles
-// of the hit leaf slots as bits from the node's triangle base.
+__device__ __forceinline__ float min3(float a, float b, float c)
+{
+    float d;
+    asm("min.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+    return d;
+}
+
+// Index of the highest set bit (x != 0).
+__device__ __forceinline__ uint32_t high_bit(uint32_t x) { return 31u - (uint32_t)__clz((int)x); }
+
+// x << (s mod 32): the shift count's upper bits are ignored, so a packed byte needs no mask.
+__device__ __forceinline__ uint32_t shl_wrap(uint32_t x, uint32_t s) { return __funnelshift_l(0u, x, s); }
+
+// Child-box tests of one BVH8 node (words w0, w1.zw = meta, w2..w4, bvh8.h) for ray r with the
+// closest hit so far at best_t. Returns the hit children in one word: bits 24-31 the internal ones
+// (bit 24 + (slot XOR octant XOR 7): the highest set bit is the child to visit first), bits 0-23 the
+// triangles of the hit leaf slots, from the node's triangle base.
 //
-// Node-local ray (Ylitie et al. 2017): t(q) = A + q S per axis with A = (p - o) / d and
-// S = 2^e / d, one FMA per plane. The plane p + q 2^e is exact; A and S carry at most a few
-// roundings, so every t is moved outwards by err = 2^-21 (|A| + 255 |S|), a bound on that error:
-// the test never rejects a box the ray enters, and the hits stay those of brute force.
-// (Tried: each axis's near and far planes through one packed f32x2 add and FMA, with three-input
-// max / min for the slab bounds. Same values, 0.408 against 0.407 ms per extend launch on the
-// 1M-triangle workload: the traversal is not limited by these instructions' count.)
-__device__ __forceinline__ void node_test(const TRay& r, uint4 w0, uint4 w2, uint4 w3, uint4 w4, uint32_t imask,
-                                          uint32_t meta_lo, uint32_t meta_hi, float best_t, uint32_t& inner_hits,
-                                          uint32_t& tri_bits)
+// Node-local ray (Ylitie et al. 2017): t(q) = A + q S per axis with A = (p - o) / d and S = 2^e / d,
+// one FMA per plane. The plane p + q 2^e is exact; A and S carry at most a few roundings, a
+// relative 2^-21 at most. The FMA takes 2^15 + q (byte_f15) and the constant A - 2^15 S, whose
+// rounding is at most 2^-9 |S| + 2^-24 |A|. So every t is moved outwards by
+// err = 2^-21 |A| + 2^-8 |S|, a bound on all of it: the test never rejects a box the ray enters, and
+// the hits stay those of brute force. The margin of 1/256 of a quantisation step adds no measurable
+// node visits; the byte's exact value (a subtraction per plane, 48 per node) needed 2^-13 of a step.
+//
+// Each child ends in one predicated OR of its meta byte's bits: no branch, whatever the lanes hit.
+__device__ __forceinline__ uint32_t node_test(const TRay& r, uint4 w0, uint32_t meta_lo, uint32_t meta_hi, uint4 w2,
+                                              uint4 w3, uint4 w4, float best_t)
 {
     float px = __uint_as_float(w0.x), py = __uint_as_float(w0.y), pz = __uint_as_float(w0.z);
     uint32_t em = w0.w;
@@ -161,110 +183,192 @@ __device__ __forceinline__ void node_test(const TRay& r, uint4 w0, uint4 w2, uin
     float ax = (px - r.o.x) * r.ix, sx = scx * r.ix;
     float ay = (py - r.o.y) * r.iy, sy = scy * r.iy;
     float az = (pz - r.o.z) * r.iz, sz = scz * r.iz;
-    float ex = 4.76837158e-7f * (fabsf(ax) + 255.0f * fabsf(sx));
-    float ey = 4.76837158e-7f * (fabsf(ay) + 255.0f * fabsf(sy));
-    float ez = 4.76837158e-7f * (fabsf(az) + 255.0f * fabsf(sz));
-    float anx = ax - ex, afx = ax + ex, any_ = ay - ey, afy = ay + ey, anz = az - ez, afz = az + ez;
-    inner_hits = 0;
-    tri_bits = 0;
+    constexpr float EA = 4.76837158e-7f, ES = 3.90625e-3f; // 2^-21, 2^-8
+    float ex = fmaf(EA, fabsf(ax), ES * fabsf(sx));
+    float ey = fmaf(EA, fabsf(ay), ES * fabsf(sy));
+    float ez = fmaf(EA, fabsf(az), ES * fabsf(sz));
+    float anx = fmaf(-32768.0f, sx, ax - ex), afx = fmaf(-32768.0f, sx, ax + ex);
+    float any_ = fmaf(-32768.0f, sy, ay - ey), afy = fmaf(-32768.0f, sy, ay + ey);
+    float anz = fmaf(-32768.0f, sz, az - ez), afz = fmaf(-32768.0f, sz, az + ez);
+    uint32_t flip = (r.oct ^ 7u) * 0x01010101u;
+    uint32_t found = 0;
 #pragma unroll
-    for (int i = 0; i < 8; i++) {
-        float tnx = fmaf(byte_f(nxl, nxh, i), sx, anx);
-        float tny = fmaf(byte_f(nyl, nyh, i), sy, any_);
-        float tnz = fmaf(byte_f(nzl, nzh, i), sz, anz);
-        float tfx = fmaf(byte_f(fxl, fxh, i), sx, afx);
-        float tfy = fmaf(byte_f(fyl, fyh, i), sy, afy);
-        float tfz = fmaf(byte_f(fzl, fzh, i), sz, afz);
-        float tn = fmaxf(fmaxf(tnx, tny), fmaxf(tnz, 0.0f));
-        float tf = fminf(fminf(tfx, tfy), fminf(tfz, best_t));
-        if (tn <= tf) {
-            if ((imask >> i) & 1u) {
-                inner_hits |= 1u << (i ^ r.oct);
-            } else {
-                uint32_t m = byte_of(meta_lo, meta_hi, i);
-                tri_bits |= ((1u << (m >> 5)) - 1u) << (m & 31u);
-            }
+    for (int half = 0; half < 2; half++) {
+        uint32_t meta = half ? meta_hi : meta_lo;
+        // Bytes of internal slots have bits 3 and 4 set (bit index 24 + slot): flip their slot.
+        uint32_t inner = (meta & (meta << 1)) & 0x10101010u;
+        uint32_t at = meta ^ (((inner >> 4) * 7u) & flip);
+        uint32_t bits = (meta >> 5) & 0x07070707u;
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            int i = 4 * half + j;
+            float tnx = fmaf(byte_f15(nxl, nxh, i), sx, anx);
+            float tny = fmaf(byte_f15(nyl, nyh, i), sy, any_);
+            float tnz = fmaf(byte_f15(nzl, nzh, i), sz, anz);
+            float tfx = fmaf(byte_f15(fxl, fxh, i), sx, afx);
+            float tfy = fmaf(byte_f15(fyl, fyh, i), sy, afy);
+            float tfz = fmaf(byte_f15(fzl, fzh, i), sz, afz);
+            float tn = fmaxf(max3(tnx, tny, tnz), 0.0f);
+            float tf = fminf(min3(tfx, tfy, tfz), best_t);
+            uint32_t b = shl_wrap((bits >> (8 * j)) & 0xffu, at >> (8 * j));
+            found |= tn <= tf ? b : 0u;
         }
     }
+    return found;
+}
+
+// A ray's way through the tree. group: the node group being visited, .x its first child's index,
+// .y its internal-child mask (bits 0-7) and the children still to visit (bits 24-31, node_test's
+// order). tri_base, tri_bits: the triangles of the last visited node still to test. hit_tri: the
+// closest hit's triangle record (NO_TRI: none).
+constexpr uint32_t NO_TRI = 0xffffffffu;
+
+struct Walk {
+    TRay r;
+    float tmax;             // the closest hit so far, or the ray's end
+    uint32_t hit_tri;
+    uint32_t item;          // queue traversal: the ray's queue entry
+    uint32_t node;          // the next node to visit
+    uint2 group;
+    uint32_t tri_base, tri_bits;
+    int sp;
+    float b1, b2;           // barycentric weights of vertices 1 and 2 at the hit (dropped unless read)
+    uint32_t nodes, tests;  // nodes visited and triangles tested (dropped unless read)
+};
+
+__device__ __forceinline__ void walk_begin(Walk& w, V3 o, V3 d, float tmax)
+{
+    w.r = make_ray(o, d);
+    w.tmax = tmax;
+    w.hit_tri = NO_TRI;
+    w.node = 0;
+    w.group = make_uint2(0u, 0u);
+    w.tri_base = w.tri_bits = 0;
+    w.sp = 0;
+    w.b1 = w.b2 = 0.0f;
+    w.nodes = w.tests = 0;
+}
+
+// Visits w.node: its hit internal children become the walk's node group, what the group before it
+// had left goes to the stack (next_node), its hit leaf slots' triangles become the pending ones.
+__device__ __forceinline__ void node_visit(const uint4* __restrict__ nodes, Walk& w)
+{
+    const uint4* np = nodes + (size_t)w.node * bvh8::NODE_VEC4;
+    uint4 w0 = __ldg(np), w1 = __ldg(np + 1), w2 = __ldg(np + 2), w3 = __ldg(np + 3), w4 = __ldg(np + 4);
+    w.nodes++;
+    uint32_t found = node_test(w.r, w0, w1.z, w1.w, w2, w3, w4, w.tmax);
+    w.group = make_uint2(w1.x, (found & 0xff000000u) | (w0.w >> 24));
+    w.tri_base = w1.y;
+    w.tri_bits = found & 0x00ffffffu;
+}
+
+// Tests one pending triangle. Returns true when an any-hit walk has its hit.
+template <bool ANY>
+__device__ __forceinline__ bool test_one(const float4* __restrict__ tris, Walk& w)
+{
+    uint32_t j = high_bit(w.tri_bits);
+    w.tri_bits ^= 1u << j;
+    uint32_t k = w.tri_base + j;
+    const float4* tp = tris + (size_t)k * bvh8::TRI_VEC4;
+    float4 a = __ldg(tp), b = __ldg(tp + 1), c = __ldg(tp + 2);
+    float t, U, V, W, det;
+    w.tests++;
+    if (tri_test(w.r, v3(a.x, a.y, a.z), v3(b.x, b.y, b.z), v3(c.x, c.y, c.z), t, U, V, W, det)) {
+        bool take = t < w.tmax;
+        if (!ANY && t == w.tmax && w.hit_tri != NO_TRI)
+            take = __float_as_uint(c.w) < __float_as_uint(__ldg(&tris[(size_t)w.hit_tri * bvh8::TRI_VEC4 + 2].w));
+        if (take) {
+            w.hit_tri = k;
+            w.tmax = t;
+            w.b1 = V / det;
+            w.b2 = W / det;
+            return ANY;
+        }
+    }
+    return false;
+}
+
+// Picks the next node: the first child left in the walk's group, else in the top group of the stack;
+// what the group has left then goes (back) to the stack. Returns true when the walk has finished
+// (nothing left, or the stack overflowed: the error flag is then set).
+__device__ __forceinline__ bool next_node(Walk& w, uint2* stack, uint32_t* err)
+{
+    uint2 g = w.group;
+    if (g.y < 0x01000000u) {
+        if (w.sp == 0)
+            return true;
+        g = stack[--w.sp];
+    }
+    uint32_t b = high_bit(g.y);
+    g.y ^= 1u << b;
+    uint32_t slot = (b ^ w.r.oct ^ 7u) & 7u;
+    w.node = g.x + __popc(g.y & ((1u << slot) - 1u));
+    if (g.y >= 0x01000000u) {
+        if (w.sp >= (int)bvh8::STACK_SIZE) {
+            atomicOr(err, bvh8::ERR_STACK);
+            return true;
+        }
+        stack[w.sp++] = g;
+    }
+    return false;
+}
+
+// One node visit: box tests, the node's triangles, then the next node. Returns true when the walk has
+// finished (nothing left, or an any-hit walk has its hit). (Tried: one triangle a step, a lane with
+// more of them skipping the node test of the steps that follow, so that the triangle test runs once
+// a step instead of as often as the warp's busiest lane needs: 7% slower on the 1M-triangle workload.)
+template <bool ANY>
+__device__ __forceinline__ bool walk_step(const uint4* __restrict__ nodes, const float4* __restrict__ tris, Walk& w,
+                                          uint2* stack, uint32_t* err)
+{
+    node_visit(nodes, w);
+    while (w.tri_bits)
+        if (test_one<ANY>(tris, w))
+            return true;
+    return next_node(w, stack, err);
+}
+
+__device__ __forceinline__ TraceHit walk_hit(const float4* __restrict__ tris, const Walk& w)
+{
+    TraceHit h;
+    h.hit = w.hit_tri != NO_TRI;
+    h.inst = h.prim = 0;
+    if (h.hit) {
+        const float4* tp = tris + (size_t)w.hit_tri * bvh8::TRI_VEC4;
+        h.inst = __float_as_uint(__ldg(&tp[0].w));
+        h.prim = __float_as_uint(__ldg(&tp[1].w));
+    }
+    h.t = w.tmax;
+    h.b1 = w.b1;
+    h.b2 = w.b2;
+    h.nodes = w.nodes;
+    h.tests = w.tests;
+    return h;
 }
 
 // Closest hit (ANY = false) or any hit (ANY = true) with 0 < t < tmax.
-template <bool ANY>
-__device__ __forceinline__ TraceHit trace_bvh(const uint4* __restrict__ nodes, const float4* __restrict__ tris,
-                                              const TRay& r, float tmax, uint32_t* err)
+// The answer of a queue item without a ray.
+__device__ __forceinline__ TraceHit no_hit(float tmax)
 {
     TraceHit h;
     h.hit = false;
     h.inst = h.prim = 0;
-    h.gid = 0xffffffffu;
     h.t = tmax;
     h.b1 = h.b2 = 0.0f;
     h.nodes = h.tests = 0;
-    float best_t = tmax;
-    uint2 stack[bvh8::STACK_SIZE];
-    int sp = 0;
-    uint32_t node = 0;
-    for (;;) {
-        const uint4* np = nodes + (size_t)node * bvh8::NODE_VEC4;
-        h.nodes++;
-        uint4 w0 = __ldg(np);
-        uint4 w1 = __ldg(np + 1);
-        uint4 w2 = __ldg(np + 2);
-        uint4 w3 = __ldg(np + 3);
-        uint4 w4 = __ldg(np + 4);
-        uint32_t imask = w0.w >> 24;
-        uint32_t child_base = w1.x, tri_base = w1.y;
-        uint32_t inner_hits, tri_bits;
-        node_test(r, w0, w2, w3, w4, imask, w1.z, w1.w, best_t, inner_hits, tri_bits);
-        // Triangles of this node's leaf slots.
-        while (tri_bits) {
-            uint32_t j = __ffs(tri_bits) - 1;
-            tri_bits &= tri_bits - 1;
-            const float4* tp = tris + (size_t)(tri_base + j) * bvh8::TRI_VEC4;
-            float4 a = __ldg(tp), b = __ldg(tp + 1), c = __ldg(tp + 2);
-            float t, U, V, W, det;
-            h.tests++;
-            if (tri_test(r, v3(a.x, a.y, a.z), v3(b.x, b.y, b.z), v3(c.x, c.y, c.z), t, U, V, W, det)) {
-                uint32_t gid = __float_as_uint(c.w);
-                bool take = ANY ? t < tmax : (t < best_t || (h.hit && t == best_t && gid < h.gid));
-                if (take) {
-                    h.hit = true;
-                    h.t = t;
-                    best_t = t;
-                    h.gid = gid;
-                    h.inst = __float_as_uint(a.w);
-                    h.prim = __float_as_uint(b.w);
-                    h.b1 = V / det;
-                    h.b2 = W / det;
-                    if (ANY)
-                        return h;
-                }
-            }
-        }
-        // Next node: from this node's hit children, else from the stack.
-        uint32_t hits = inner_hits;
-        uint32_t gbase = child_base, gmask = imask;
-        if (hits == 0) {
-            if (sp == 0)
-                break;
-            --sp;
-            gbase = stack[sp].x;
-            gmask = stack[sp].y & 0xffu;
-            hits = stack[sp].y >> 8;
-        }
-        uint32_t b = __ffs(hits) - 1;
-        hits &= hits - 1;
-        uint32_t slot = b ^ r.oct;
-        node = gbase + __popc(gmask & ((1u << slot) - 1u));
-        if (hits) {
-            if (sp >= (int)bvh8::STACK_SIZE) {
-                atomicOr(err, bvh8::ERR_STACK);
-                break;
-            }
-            stack[sp++] = make_uint2(gbase, gmask | (hits << 8));
-        }
-    }
     return h;
+}
+
+template <bool ANY>
+__device__ __forceinline__ TraceHit trace_bvh(const uint4* __restrict__ nodes, const float4* __restrict__ tris, V3 o,
+                                              V3 d, float tmax, uint32_t* err)
+{
+    uint2 stack[bvh8::STACK_SIZE];
+    Walk w;
+    walk_begin(w, o, d, tmax);
+    while (!walk_step<ANY>(nodes, tris, w, stack, err)) {
+    }
+    return walk_hit(tris, w);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -276,75 +380,6 @@ __device__ __forceinline__ TraceHit trace_bvh(const uint4* __restrict__ nodes, c
 //
 // get(i, r, tmax) loads queue item i into a ray and returns false when it has no ray (it then
 // completes at once with a miss); put(i, hit) stores the result of item i.
-
-struct Walk {
-    TRay r;
-    float tmax;
-    uint32_t item;
-    uint32_t node;
-    int sp;
-    TraceHit h;
-};
-
-// One node visit: box tests, the node's triangles, then the next node. Returns true when the walk
-// has finished (stack empty, or any-hit found).
-template <bool ANY>
-__device__ __forceinline__ bool walk_step(const uint4* __restrict__ nodes, const float4* __restrict__ tris, Walk& w,
-                                          uint2* stack, uint32_t* err)
-{
-    const TRay& r = w.r;
-    const uint4* np = nodes + (size_t)w.node * bvh8::NODE_VEC4;
-    uint4 w0 = __ldg(np), w1 = __ldg(np + 1), w2 = __ldg(np + 2), w3 = __ldg(np + 3), w4 = __ldg(np + 4);
-    w.h.nodes++;
-    uint32_t imask = w0.w >> 24;
-    uint32_t child_base = w1.x, tri_base = w1.y;
-    uint32_t inner_hits, tri_bits;
-    node_test(r, w0, w2, w3, w4, imask, w1.z, w1.w, w.tmax, inner_hits, tri_bits);
-    while (tri_bits) {
-        uint32_t j = __ffs(tri_bits) - 1;
-        tri_bits &= tri_bits - 1;
-        const float4* tp = tris + (size_t)(tri_base + j) * bvh8::TRI_VEC4;
-        float4 a = __ldg(tp), b = __ldg(tp + 1), c = __ldg(tp + 2);
-        float t, U, V, W, det;
-        w.h.tests++;
-        if (tri_test(r, v3(a.x, a.y, a.z), v3(b.x, b.y, b.z), v3(c.x, c.y, c.z), t, U, V, W, det)) {
-            uint32_t gid = __float_as_uint(c.w);
-            bool take = ANY ? t < w.tmax : (t < w.tmax || (w.h.hit && t == w.tmax && gid < w.h.gid));
-            if (take) {
-                w.h.hit = true;
-                w.h.t = t;
-                w.tmax = ANY ? w.tmax : t;
-                w.h.gid = gid;
-                w.h.inst = __float_as_uint(a.w);
-                w.h.prim = __float_as_uint(b.w);
-                w.h.b1 = V / det;
-                w.h.b2 = W / det;
-                if (ANY)
-                    return true;
-            }
-        }
-    }
-    uint32_t hits = inner_hits, gbase = child_base, gmask = imask;
-    if (hits == 0) {
-        if (w.sp == 0)
-            return true;
-        --w.sp;
-        gbase = stack[w.sp].x;
-        gmask = stack[w.sp].y & 0xffu;
-        hits = stack[w.sp].y >> 8;
-    }
-    uint32_t b = __ffs(hits) - 1;
-    hits &= hits - 1;
-    w.node = gbase + __popc(gmask & ((1u << (b ^ r.oct)) - 1u));
-    if (hits) {
-        if (w.sp >= (int)bvh8::STACK_SIZE) {
-            atomicOr(err, bvh8::ERR_STACK);
-            return true;
-        }
-        stack[w.sp++] = make_uint2(gbase, gmask | (hits << 8));
-    }
-    return false;
-}
 
 // ---------------------------------------------------------------------------------------------
 // Warp-cooperative leaf testing. In walk_step every lane tests its node's triangles itself, so a
@@ -362,15 +397,15 @@ __device__ __forceinline__ bool walk_step(const uint4* __restrict__ nodes, const
 // A pair lane reads the owner's ray from shared memory (written once per ray) and reports a hit
 // with a 64-bit shared-memory atomicMin of (t bits << 32 | global triangle index) on the owner's
 // slot: for t > 0 the float bits order like the floats, so the minimum is the closest hit with the
-// lower index on ties, the rule of trace_bvh. The winning lane then leaves the hit's instance,
-// primitive and barycentrics in the owner's slot. Any-hit rays only need a flag.
+// lower index on ties, the rule of trace_bvh. The winning lane then leaves the hit's triangle
+// record and barycentrics in the owner's slot. Any-hit rays only need a flag.
 
 // Shared state of one warp (block size 128: four per block).
 struct CoopWarp {
     float4 ra[32];               // owner ray: origin xyz, watertight axes kx | ky << 2 | kz << 4
     float4 rb[32];               // owner ray: shear sx, sy, sz; tmax (any-hit)
     unsigned long long key[32];  // closest-hit candidates, min-reduced
-    uint4 info[32];              // the winner's instance, primitive, b1, b2 bits; any-hit: x = hit
+    uint4 info[32];              // the winner's triangle record, 0, b1, b2 bits; any-hit: x = hit
 };
 constexpr uint32_t COOP_WARPS = 4; // warps per block of the cooperative kernels (128 threads)
 
@@ -378,49 +413,6 @@ __device__ __forceinline__ void coop_publish_ray(CoopWarp& cw, uint32_t lane, co
 {
     cw.ra[lane] = make_float4(r.o.x, r.o.y, r.o.z, __uint_as_float((uint32_t)(r.kx | (r.ky << 2) | (r.kz << 4))));
     cw.rb[lane] = make_float4(r.sx, r.sy, r.sz, tmax);
-}
-
-// Child-box tests of the walk's current node: the hit internal children (in ray-octant order, as
-// walk_step) and the triangles of the hit leaf slots.
-__device__ __forceinline__ void node_visit(const uint4* __restrict__ nodes, Walk& w, uint32_t& inner_hits,
-                                           uint32_t& tri_bits, uint32_t& tri_base, uint32_t& child_base,
-                                           uint32_t& imask)
-{
-    const TRay& r = w.r;
-    const uint4* np = nodes + (size_t)w.node * bvh8::NODE_VEC4;
-    uint4 w0 = __ldg(np), w1 = __ldg(np + 1), w2 = __ldg(np + 2), w3 = __ldg(np + 3), w4 = __ldg(np + 4);
-    w.h.nodes++;
-    imask = w0.w >> 24;
-    child_base = w1.x;
-    tri_base = w1.y;
-    node_test(r, w0, w2, w3, w4, imask, w1.z, w1.w, w.tmax, inner_hits, tri_bits);
-}
-
-// The next node of the walk after a visit (walk_step's tail). Returns true when the walk has
-// finished (stack empty, or the stack overflowed: the error flag is then set).
-__device__ __forceinline__ bool next_node(Walk& w, uint32_t inner_hits, uint32_t child_base, uint32_t imask,
-                                          uint2* stack, uint32_t* err)
-{
-    uint32_t hits = inner_hits, gbase = child_base, gmask = imask;
-    if (hits == 0) {
-        if (w.sp == 0)
-            return true;
-        --w.sp;
-        gbase = stack[w.sp].x;
-        gmask = stack[w.sp].y & 0xffu;
-        hits = stack[w.sp].y >> 8;
-    }
-    uint32_t b = __ffs(hits) - 1;
-    hits &= hits - 1;
-    w.node = gbase + __popc(gmask & ((1u << (b ^ w.r.oct)) - 1u));
-    if (hits) {
-        if (w.sp >= (int)bvh8::STACK_SIZE) {
-            atomicOr(err, bvh8::ERR_STACK);
-            return true;
-        }
-        stack[w.sp++] = make_uint2(gbase, gmask | (hits << 8));
-    }
-    return false;
 }
 
 // Tests every (ray, triangle) pair the warp's lanes collected in this step: lane i owns the
@@ -447,11 +439,14 @@ __device__ __forceinline__ bool coop_tris(CoopWarp& cw, uint32_t lane, uint32_t 
     uint32_t excl = incl - cnt;
     unsigned long long init = 0;
     if (cnt) {
-        w.h.tests += cnt;
+        w.tests += cnt;
         if (ANY) {
             cw.info[lane].x = 0u;
         } else {
-            init = ((unsigned long long)__float_as_uint(w.tmax) << 32) | (w.h.hit ? w.h.gid : 0u);
+            uint32_t gid = 0;
+            if (w.hit_tri != NO_TRI)
+                gid = __float_as_uint(__ldg(&tris[(size_t)w.hit_tri * bvh8::TRI_VEC4 + 2].w));
+            init = ((unsigned long long)__float_as_uint(w.tmax) << 32) | gid;
             cw.key[lane] = init;
         }
     }
@@ -473,11 +468,12 @@ __device__ __forceinline__ bool coop_tris(CoopWarp& cw, uint32_t lane, uint32_t 
         bool mine = false;
         unsigned long long key = 0;
         float V = 0.0f, Wb = 0.0f, det = 1.0f;
-        uint32_t ainst = 0, bprim = 0;
+        uint32_t ktri = 0;
         if (q < total) {
             for (uint32_t j = q - oexcl; j > 0; j--)
                 obits &= obits - 1;
-            const float4* tp = tris + (size_t)(obase + __ffs(obits) - 1) * bvh8::TRI_VEC4;
+            ktri = obase + __ffs(obits) - 1;
+            const float4* tp = tris + (size_t)ktri * bvh8::TRI_VEC4;
             float4 a = __ldg(tp), b = __ldg(tp + 1), c = __ldg(tp + 2);
             float4 ra = cw.ra[L], rb = cw.rb[L];
             TRay r;
@@ -498,8 +494,6 @@ __device__ __forceinline__ bool coop_tris(CoopWarp& cw, uint32_t lane, uint32_t 
                     key = ((unsigned long long)__float_as_uint(t) << 32) | __float_as_uint(c.w);
                     atomicMin(&cw.key[L], key);
                     mine = true;
-                    ainst = __float_as_uint(a.w);
-                    bprim = __float_as_uint(b.w);
                 }
             }
         }
@@ -507,7 +501,7 @@ __device__ __forceinline__ bool coop_tris(CoopWarp& cw, uint32_t lane, uint32_t 
             __syncwarp();
             // The lane whose candidate is the owner's minimum so far leaves its hit there.
             if (mine && cw.key[L] == key)
-                cw.info[L] = make_uint4(ainst, bprim, __float_as_uint(V / det), __float_as_uint(Wb / det));
+                cw.info[L] = make_uint4(ktri, 0u, __float_as_uint(V / det), __float_as_uint(Wb / det));
         }
         __syncwarp();
     }
@@ -518,14 +512,10 @@ __device__ __forceinline__ bool coop_tris(CoopWarp& cw, uint32_t lane, uint32_t 
     unsigned long long best = cw.key[lane];
     if (best < init) {
         uint4 in = cw.info[lane];
-        w.h.hit = true;
-        w.h.t = __uint_as_float((uint32_t)(best >> 32));
-        w.tmax = w.h.t;
-        w.h.gid = (uint32_t)best;
-        w.h.inst = in.x;
-        w.h.prim = in.y;
-        w.h.b1 = __uint_as_float(in.z);
-        w.h.b2 = __uint_as_float(in.w);
+        w.tmax = __uint_as_float((uint32_t)(best >> 32));
+        w.hit_tri = in.x;
+        w.b1 = __uint_as_float(in.z);
+        w.b2 = __uint_as_float(in.w);
     }
     return false;
 }
@@ -557,23 +547,13 @@ __device__ __forceinline__ void trace_queue_coop(const uint4* __restrict__ nodes
                 if (idx < count) {
                     V3 o, d;
                     float tmax;
-                    w.item = idx;
-                    w.h.hit = false;
-                    w.h.inst = w.h.prim = 0;
-                    w.h.gid = 0xffffffffu;
-                    w.h.b1 = w.h.b2 = 0.0f;
-                    w.h.nodes = w.h.tests = 0;
                     if (get(idx, o, d, tmax)) {
-                        w.r = make_ray(o, d);
-                        w.tmax = tmax;
-                        w.h.t = tmax;
-                        w.node = 0;
-                        w.sp = 0;
+                        walk_begin(w, o, d, tmax);
+                        w.item = idx;
                         active = true;
                         coop_publish_ray(cw, lane, w.r, tmax);
                     } else {
-                        w.h.t = tmax;
-                        put(idx, w.h);
+                        put(idx, no_hit(tmax));
                     }
                 }
             }
@@ -586,17 +566,18 @@ __device__ __forceinline__ void trace_queue_coop(const uint4* __restrict__ nodes
         __syncwarp();
 #pragma unroll 1
         for (uint32_t s = 0; s < steps; s++) {
-            uint32_t inner = 0, bits = 0, tbase = 0, cbase = 0, imask = 0;
-            if (active)
-                node_visit(nodes, w, inner, bits, tbase, cbase, imask);
-            bool hit = coop_tris<ANY>(cw, lane, bits, tbase, w, tris);
+            uint32_t bits = 0;
             if (active) {
-                bool done = (ANY && hit) ? true : next_node(w, inner, cbase, imask, stack, err);
-                if (ANY && hit) {
-                    w.h.hit = true;
-                }
-                if (done) {
-                    put(w.item, w.h);
+                node_visit(nodes, w);
+                bits = w.tri_bits;
+                w.tri_bits = 0;
+            }
+            bool hit = coop_tris<ANY>(cw, lane, bits, w.tri_base, w, tris);
+            if (active) {
+                if (ANY && hit)
+                    w.hit_tri = 0; // any-hit: the flag alone
+                if ((ANY && hit) || next_node(w, stack, err)) {
+                    put(w.item, walk_hit(tris, w));
                     active = false;
                 }
             }
@@ -635,27 +616,17 @@ __device__ __forceinline__ void trace_queue_impl(const uint4* __restrict__ nodes
                 if (idx < count) {
                     V3 o, d;
                     float tmax;
-                    w.item = idx;
-                    w.h.hit = false;
-                    w.h.inst = w.h.prim = 0;
-                    w.h.gid = 0xffffffffu;
-                    w.h.b1 = w.h.b2 = 0.0f;
-                    w.h.nodes = w.h.tests = 0;
                     bool ok;
                     if constexpr (SCENES)
                         ok = get(idx, o, d, tmax, nodes, tris);
                     else
                         ok = get(idx, o, d, tmax);
                     if (ok) {
-                        w.r = make_ray(o, d);
-                        w.tmax = tmax;
-                        w.h.t = tmax;
-                        w.node = 0;
-                        w.sp = 0;
+                        walk_begin(w, o, d, tmax);
+                        w.item = idx;
                         active = true;
                     } else {
-                        w.h.t = tmax;
-                        put(idx, w.h);
+                        put(idx, no_hit(tmax));
                     }
                 }
             }
@@ -669,7 +640,7 @@ __device__ __forceinline__ void trace_queue_impl(const uint4* __restrict__ nodes
 #pragma unroll 1
             for (uint32_t s = 0; s < steps; s++) {
                 if (walk_step<ANY>(nodes, tris, w, stack, err)) {
-                    put(w.item, w.h);
+                    put(w.item, walk_hit(tris, w));
                     active = false;
                     break;
                 }
