@@ -77,6 +77,12 @@ constexpr uint32_t BASE_PLANES = 4;  // 16-byte state planes per path
 constexpr uint32_t SHADE_CLASSES = 4; // material-sorted shading: missed, diffuse, conductor, dielectric
 constexpr uint32_t SPLIT_PLANES = 5; // more planes with the lighting split
 
+// Wave::flags of a path slot.
+constexpr uint32_t SLOT_RAY = 1u;     // its path has a ray to trace and shade
+constexpr uint32_t SLOT_SHADOW = 2u;  // a shadow ray: its contribution goes to the path's radiance
+constexpr uint32_t SLOT_ENDED = 4u;   // the path before the one in SLOT_RAY has ended: pend holds its radiance
+constexpr uint32_t SLOT_BLOCKED = 8u; // the shadow ray was occluded
+
 // Wavefront buffers of one accumulation.
 struct Wave {
     float4* state;
@@ -95,6 +101,13 @@ struct Wave {
     // class k in squeue[k * n ...], counts scount[parity * 4 + k] (null when off).
     uint32_t* squeue;
     uint32_t* scount;
+    // Deferred shadows (flags null without them): what each slot still has in flight (SLOT_* bits), the
+    // radiance of a slot's path that has ended and waits for its last shadow ray, and the slots with a
+    // shadow ray, shcount[parity] of them.
+    uint32_t* flags;
+    float4* pend;
+    uint32_t* shqueue;
+    uint32_t* shcount;
 };
 
 // Radiance-cache frames on the streaming wavefront: the path spread (a0, a) of every slot,

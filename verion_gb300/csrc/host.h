@@ -210,7 +210,6 @@ struct VgRenderer {
     int stream_shade_blocks[8] = {};
     int deferred_blocks[2] = {};
     int deferred_restir_blocks[2] = {};
-    int shadow_blocks[2] = {};
     bool defer_shadows = true; // streaming: shadow rays of the light sample in their own stage
     bool dynamic_fetch = true; // streaming: traversal stages refill idle lanes from the queue
     bool coop_tris = false;    // streaming, dynamic fetch: warp-cooperative leaf testing (measured slower)
@@ -251,7 +250,7 @@ struct VgAccum {
     Restir restir;               // captured at the first sample
     DevBuf re_g[2], re_n[2], re_x[2], re_m[2];
     DevBuf re_gx[2], re_gn[2], re_gl[2], re_s[7]; // ReSTIR GI planes
-    DevBuf state, hits, queue[2], counts, fetch, tstats, meta, sreq, squeue, scount;
+    DevBuf state, hits, queue[2], counts, fetch, tstats, meta, sreq, squeue, scount, flags, pend, shqueue;
     DevBuf mk_next;                  // the megakernel's pixel counter
     uint32_t* host_counts = nullptr; // pinned ring of wave output counts (streaming wavefront)
     uint32_t last_waves = 0;
@@ -440,6 +439,10 @@ vgk::Wave wave_of(const VgRenderer* r, const VgAccum* acc)
     w.shadow_steps = r->shadow_fetch_steps;
     w.squeue = (uint32_t*)acc->squeue.p;
     w.scount = (uint32_t*)acc->scount.p;
+    w.flags = (uint32_t*)acc->flags.p;
+    w.pend = (float4*)acc->pend.p;
+    w.shqueue = (uint32_t*)acc->shqueue.p;
+    w.shcount = w.scount ? w.scount + 2 * vgk::SHADE_CLASSES : nullptr;
     return w;
 }
 

@@ -204,10 +204,32 @@ cudaError_t launch_stream_shade_deferred(bool f64, bool sorted, int blocks, cuda
     return cudaGetLastError();
 }
 
-cudaError_t launch_stream_classify(int blocks, cudaStream_t s, const vgd::Ctx& c, const vgk::Wave& w, uint32_t wave)
+cudaError_t launch_stream_resolve(bool f64, bool sorted, int blocks, cudaStream_t s, const vgd::Ctx& c,
+                                  const vgk::Wave& w, uint32_t wave)
 {
-    vgk::wf_stream_classify<<<blocks, 256, 0, s>>>(c, w, wave);
+    if (f64 && sorted)
+        vgk::wf_stream_resolve<double, false, true><<<blocks, 256, 0, s>>>(c, w, wave);
+    else if (f64)
+        vgk::wf_stream_resolve<double><<<blocks, 256, 0, s>>>(c, w, wave);
+    else if (sorted)
+        vgk::wf_stream_resolve<float, false, true><<<blocks, 256, 0, s>>>(c, w, wave);
+    else
+        vgk::wf_stream_resolve<float><<<blocks, 256, 0, s>>>(c, w, wave);
     return cudaGetLastError();
+}
+
+int stream_resolve_blocks_per_sm(bool f64)
+{
+    static int n[2] = {0, 0};
+    int& k = n[f64 ? 1 : 0];
+    if (k == 0) {
+        if (f64)
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&k, vgk::wf_stream_resolve<double, false, true>, 256, 0);
+        else
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&k, vgk::wf_stream_resolve<float, false, true>, 256, 0);
+        k = k > 0 ? k : 1;
+    }
+    return k;
 }
 
 // Radiance-cache frames (lighting split off): start without the training pixels, shade with the
@@ -260,41 +282,27 @@ cudaError_t launch_stream_cache_tail(bool f64, uint32_t max_slots, cudaStream_t 
     return cudaGetLastError();
 }
 
-cudaError_t launch_stream_shadow(bool f64, int blocks, cudaStream_t s, const vgd::Ctx& c, const vgk::Wave& w,
-                                 uint32_t wave)
+cudaError_t launch_stream_shadow_layers(int blocks, cudaStream_t s, const vgd::Ctx& c, const vgk::Wave& w,
+                                        uint32_t wave)
 {
-    if (f64)
-        vgk::wf_stream_shadow<double><<<blocks, 128, 0, s>>>(c, w, wave);
-    else
-        vgk::wf_stream_shadow<float><<<blocks, 128, 0, s>>>(c, w, wave);
+    vgk::wf_stream_shadow_layers<<<blocks, 128, 0, s>>>(c, w, wave);
     return cudaGetLastError();
 }
 
-int stream_finish_blocks_per_sm(bool f64)
+int stream_shadow_layers_blocks_per_sm()
 {
-    static int n[2] = {0, 0};
-    int& k = n[f64 ? 1 : 0];
-    if (k == 0) {
-        if (f64)
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&k, vgk::wf_stream_finish<double>, 128, 0);
-        else
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&k, vgk::wf_stream_finish<float>, 128, 0);
-        k = k > 0 ? k : 1;
-    }
-    return k;
+    int n = 0;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, vgk::wf_stream_shadow_layers, 128, 0);
+    return n > 0 ? n : 1;
 }
 
-int stream_deferred_blocks_per_sm(bool f64, int* shadow)
+int stream_deferred_blocks_per_sm(bool f64)
 {
-    int n = 0, m = 0;
-    if (f64) {
+    int n = 0;
+    if (f64)
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, vgk::wf_stream_shade_deferred<double>, 128, 0);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&m, vgk::wf_stream_shadow<double>, 128, 0);
-    } else {
+    else
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, vgk::wf_stream_shade_deferred<float>, 128, 0);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&m, vgk::wf_stream_shadow<float>, 128, 0);
-    }
-    *shadow = m > 0 ? m : 1;
     return n > 0 ? n : 1;
 }
 
@@ -313,6 +321,12 @@ cudaError_t launch_stream_extend_dyn(bool stats, bool coop, int blocks, cudaStre
         vgk::wf_stream_extend_dyn<false, true><<<blocks, 128, 0, s>>>(c, w, wave);
     else
         vgk::wf_stream_extend_dyn<false, false><<<blocks, 128, 0, s>>>(c, w, wave);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_stream_trace(int blocks, cudaStream_t s, const vgd::Ctx& c, const vgk::Wave& w, uint32_t wave)
+{
+    vgk::wf_stream_trace<<<blocks, 128, 0, s>>>(c, w, wave);
     return cudaGetLastError();
 }
 
@@ -348,16 +362,6 @@ int stream_trace_blocks_per_sm(bool coop)
     else
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, vgk::wf_stream_extend_dyn<false, false>, 128, 0);
     return n > 0 ? n : 1;
-}
-
-cudaError_t launch_stream_finish(bool f64, int blocks, cudaStream_t s, const vgd::Ctx& c, const vgk::Wave& w,
-                                 uint32_t wave)
-{
-    if (f64)
-        vgk::wf_stream_finish<double><<<blocks, 128, 0, s>>>(c, w, wave);
-    else
-        vgk::wf_stream_finish<float><<<blocks, 128, 0, s>>>(c, w, wave);
-    return cudaGetLastError();
 }
 
 } // namespace vgx

@@ -72,23 +72,17 @@ cudaError_t launch_stream_shade_deferred_restir(bool f64, bool sorted, int block
     return cudaGetLastError();
 }
 
-cudaError_t launch_stream_shadow_restir(bool f64, int blocks, cudaStream_t s, const vgd::Ctx& c, const vgk::Wave& w,
-                                        uint32_t wave)
+cudaError_t launch_stream_resolve_restir(bool f64, bool sorted, int blocks, cudaStream_t s, const vgd::Ctx& c,
+                                         const vgk::Wave& w, uint32_t wave)
 {
-    if (f64)
-        vgk::wf_stream_shadow<double, true><<<blocks, 128, 0, s>>>(c, w, wave);
+    if (f64 && sorted)
+        vgk::wf_stream_resolve<double, true, true><<<blocks, 256, 0, s>>>(c, w, wave);
+    else if (f64)
+        vgk::wf_stream_resolve<double, true><<<blocks, 256, 0, s>>>(c, w, wave);
+    else if (sorted)
+        vgk::wf_stream_resolve<float, true, true><<<blocks, 256, 0, s>>>(c, w, wave);
     else
-        vgk::wf_stream_shadow<float, true><<<blocks, 128, 0, s>>>(c, w, wave);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_stream_finish_restir(bool f64, int blocks, cudaStream_t s, const vgd::Ctx& c, const vgk::Wave& w,
-                                        uint32_t wave)
-{
-    if (f64)
-        vgk::wf_stream_finish<double, true><<<blocks, 128, 0, s>>>(c, w, wave);
-    else
-        vgk::wf_stream_finish<float, true><<<blocks, 128, 0, s>>>(c, w, wave);
+        vgk::wf_stream_resolve<float, true><<<blocks, 256, 0, s>>>(c, w, wave);
     return cudaGetLastError();
 }
 

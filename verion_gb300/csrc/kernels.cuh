@@ -476,20 +476,31 @@ __global__ void __launch_bounds__(256) wf_stream_start(const __grid_constant__ C
         PathState<LIGHT> st = generatePathFor<LIGHT>(c, p % c.p[P_WIDTH], p / c.p[P_WIDTH], c.p[P_SAMPLE]);
         storePath<LIGHT>(w, st, p);
         w.meta[p] = 0;
+        if (w.flags)
+            w.flags[p] = SLOT_RAY;
         live = true;
     }
     block_append<8>(&w.counts[0], w.queue[0], live, p, slot);
 }
 
-template <bool STATS>
-__global__ void __launch_bounds__(128, 8) wf_stream_extend(const __grid_constant__ Ctx c, const __grid_constant__ Wave w, uint32_t wave)
+// The counters that the stages of wave parity `in` use after its first kernel, which calls this: the
+// next queue's length, the work counters of the stages that follow, and the shading class counts.
+static __device__ __forceinline__ void clear_wave_counters(const Wave& w, uint32_t in)
 {
-    uint32_t in = wave & 1u, out = in ^ 1u;
     if (blockIdx.x == 0 && threadIdx.x == 0) {
-        w.counts[out] = 0;
+        w.counts[in ^ 1u] = 0;
         w.fetch[2 + in] = 0;
         w.fetch[4 + in] = 0;
     }
+    if (w.flags && blockIdx.x == 0 && threadIdx.x < SHADE_CLASSES)
+        w.scount[in * SHADE_CLASSES + threadIdx.x] = 0;
+}
+
+template <bool STATS>
+__global__ void __launch_bounds__(128, 8) wf_stream_extend(const __grid_constant__ Ctx c, const __grid_constant__ Wave w, uint32_t wave)
+{
+    uint32_t in = wave & 1u;
+    clear_wave_counters(w, in);
     uint32_t count = w.counts[in];
     const uint32_t* qin = w.queue[in];
     uint32_t n_rays = 0, n_nodes = 0, n_tests = 0, n_later = 0;
@@ -498,8 +509,8 @@ __global__ void __launch_bounds__(128, 8) wf_stream_extend(const __grid_constant
         if (base >= count)
             break;
         uint32_t i = base + lane_id();
-        if (i < count) {
-            uint32_t p = qin[i];
+        uint32_t p = i < count ? qin[i] : 0u;
+        if (i < count && (!w.flags || (w.flags[p] & SLOT_RAY))) {
             float4 a = w.state[p];
             float4 b = w.state[w.n + p];
             vgt::TraceHit q = vgt::trace_bvh<false>(c.s.nodes, c.s.tris, v3(a.x, a.y, a.z), v3(b.x, b.y, b.z), 1.0e30f,
@@ -571,6 +582,42 @@ __global__ void __launch_bounds__(128, VG_SHADE_MIN_BLOCKS) wf_stream_shade(cons
     }
 }
 
+// What a slot's shadow ray (SLOT_SHADOW) decides once it is traced, in the order of the pixel's samples:
+// its contribution is the last add of the vertex that asked for it. Returns whether the slot still has
+// a path to go on with.
+template <typename A, bool RESTIR>
+__device__ __forceinline__ bool resolveSlot(const Ctx& c, const Wave& w, uint32_t p, uint32_t fl, bool blocked)
+{
+    uint32_t n = w.n;
+    bool lit = (fl & SLOT_SHADOW) && !blocked;
+    if (fl & SLOT_ENDED) {
+        float4 t = w.pend[p];
+        V3 total = v3(t.x, t.y, t.z);
+        if (lit) {
+            float4 r = w.sreq[2 * n + p];
+            total += v3(r.x, r.y, r.z);
+        }
+        PathState<false> st;
+        st.parts.zero();
+        st.parts.total = total;
+        st.visLit = st.visTotal = 0.0f;
+        // The deferred stages never carry ReSTIR GI (the host traces the light sample inside shade
+        // when GI is on), so the path's GI flag is false here.
+        st.gi = false;
+        st.chan = -1;
+        finishPath<false, A, RESTIR>(c, st, p);
+        // The next sample was started before this one's radiance was known: it is dropped untouched when
+        // the pixel takes no more.
+        return (fl & SLOT_RAY) && (c.p[P_ADAPTIVE] == 0 || pixelActive<A>(c, p));
+    }
+    if (lit) {
+        float4 t = w.state[3 * n + p], r = w.sreq[2 * n + p];
+        V3 total = v3(t.x, t.y, t.z) + v3(r.x, r.y, r.z);
+        w.state[3 * n + p] = make_float4(total.x, total.y, total.z, t.w);
+    }
+    return (fl & SLOT_RAY) != 0;
+}
+
 // Shading classes of material-sorted shading (SHADE_CLASSES, ctx.h): a missed ray (environment or
 // sky), a diffuse surface, a conductor, a dielectric. Only the order in which slots are shaded
 // changes (each slot adds to its own pixel), so the sums stay bit-identical.
@@ -585,45 +632,101 @@ static __device__ __forceinline__ uint32_t shadeClass(const Ctx& c, uint4 hr)
     return fget(c.s.materials, mi + 6) >= 0.5f ? 2u : 1u;
 }
 
-// Between extend and shade: every slot of the wave's queue goes to the queue of its shading class
-// (one atomic per class present in a warp), so the deferred shade stage's warps mostly run one
-// BSDF's code. Clears the other parity's class counts for the next wave (the shade stage of the
-// previous wave, their last reader, has finished).
-static __global__ void __launch_bounds__(256) wf_stream_classify(const __grid_constant__ Ctx c, const __grid_constant__ Wave w, uint32_t wave)
+// Between trace and shade (lighting split off, deferred shadows): what the wave's rays brought each slot
+// of its queue. A shadow ray that got through adds its contribution, to the slot's path or, when that
+// path ended at the vertex, to its radiance in w.pend, which then goes to the pixel's sums; adaptive
+// sampling decides from them whether the slot's next sample, whose camera ray was traced meanwhile, is
+// kept. Every slot that has a ray goes to the next wave's queue, in the order of this one, and (SORT)
+// to the queue of its hit's shading class, so that the shade stage's warps mostly run one BSDF's code.
+// One pass and one atomic per queue and 256 slots: as two kernels (classify with up to four atomics a
+// warp, 61 us per wave of about a million slots, and finish, 69 us) it was a seventh of the wave.
+template <typename A, bool RESTIR = false, bool SORT = false>
+__global__ void __launch_bounds__(256) wf_stream_resolve(const __grid_constant__ Ctx c, const __grid_constant__ Wave w,
+                                                         uint32_t wave)
 {
+    constexpr uint32_t WARPS = 8, QUEUES = SORT ? SHADE_CLASSES + 1 : 1;
+    __shared__ uint32_t slot[WARPS * QUEUES];
     uint32_t in = wave & 1u, out = in ^ 1u;
-    if (blockIdx.x == 0 && threadIdx.x < SHADE_CLASSES)
-        w.scount[out * SHADE_CLASSES + threadIdx.x] = 0;
-    uint32_t count = w.counts[in];
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        w.fetch[out] = 0;
+        w.shcount[out] = 0;
+    }
+    uint32_t count = w.counts[in], n = w.n;
     const uint32_t* qin = w.queue[in];
+    uint32_t* qout = w.queue[out];
+    uint32_t lane = lane_id(), warp = threadIdx.x >> 5, lt = (1u << lane) - 1u;
     uint32_t stride = gridDim.x * blockDim.x;
     for (uint32_t base = blockIdx.x * blockDim.x; base < count; base += stride) {
         uint32_t i = base + threadIdx.x;
-        bool have = i < count;
-        uint32_t p = have ? qin[i] : 0u;
-        uint32_t k = have ? shadeClass(c, w.hits[p]) : SHADE_CLASSES;
-        for (uint32_t cls = 0; cls < SHADE_CLASSES; cls++)
-            warp_append(&w.scount[in * SHADE_CLASSES + cls], w.squeue + (size_t)cls * w.n, k == cls, p);
+        uint32_t p = 0, cls = SHADE_CLASSES;
+        bool live = false;
+        if (i < count) {
+            p = qin[i];
+            uint32_t fl = w.flags[p];
+            live = resolveSlot<A, RESTIR>(c, w, p, fl, (fl & SLOT_BLOCKED) != 0);
+            if (SORT && live)
+                cls = shadeClass(c, w.hits[p]);
+        }
+        // Queue 0 is the next wave's, queue 1 + k the shading class k's. Warp q's lanes scan queue q's counts.
+        uint32_t mine = __ballot_sync(FULL, live);
+        if (lane == 0)
+            slot[warp] = __popc(mine);
+        uint32_t own = 0;
+        if (SORT) {
+#pragma unroll
+            for (uint32_t k = 0; k < SHADE_CLASSES; k++) {
+                uint32_t b = __ballot_sync(FULL, cls == k);
+                if (lane == 0)
+                    slot[(1 + k) * WARPS + warp] = __popc(b);
+                own = cls == k ? b : own;
+            }
+        }
+        __syncthreads();
+        if (warp < QUEUES) {
+            uint32_t v = lane < WARPS ? slot[warp * WARPS + lane] : 0u;
+            uint32_t incl = v;
+#pragma unroll
+            for (uint32_t o = 1; o < WARPS; o <<= 1) {
+                uint32_t t = __shfl_up_sync(FULL, incl, o);
+                if (lane >= o)
+                    incl += t;
+            }
+            uint32_t total = __shfl_sync(FULL, incl, WARPS - 1);
+            uint32_t first = 0;
+            if (lane == 0 && total)
+                first = atomicAdd(warp == 0 ? &w.counts[out] : &w.scount[in * SHADE_CLASSES + warp - 1], total);
+            first = __shfl_sync(FULL, first, 0);
+            if (lane < WARPS)
+                slot[warp * WARPS + lane] = first + incl - v;
+        }
+        __syncthreads();
+        if (live) {
+            qout[slot[warp] + __popc(mine & lt)] = p;
+            if (SORT)
+                w.squeue[(size_t)cls * n + slot[(1 + cls) * WARPS + warp] + __popc(own & lt)] = p;
+        }
+        __syncthreads();
     }
 }
 
-// Streaming wave in three stages (lighting split off): extend, then shade without any traversal,
-// then shadow. Shade leaves its emitter / environment light sample as a request per slot
-// (w.sreq planes: origin + tmax, direction + flags, contribution); the shadow stage traces it,
-// adds the contribution when unoccluded, and only then finishes, restarts or queues the slot.
-// flags: bit 0 a request is present, bit 1 the path goes on to the next depth.
+// Streaming wave in three stages (lighting split off): trace, resolve, then shade without any traversal.
+// Shade leaves its emitter / environment light sample as a request of the slot (w.sreq planes: origin +
+// tmax, direction, contribution) in the shadow queue; the next wave traces it along with the slot's next
+// ray, and the resolve stage adds the contribution when it is unoccluded. A path that ends leaves its
+// radiance in w.pend and the slot starts the pixel's next sample at once.
 // With CACHE a path also ends where its spread passes the cache threshold (shadePath's cache
 // hook); it then leaves a query record (one atomic per warp) and finishes like any other.
-// With SORTED the wave's slots are taken class by class from the classify stage's queues.
+// With SORTED the wave's slots are taken class by class from the resolve stage's queues.
 template <typename A, bool CACHE = false, bool RESTIR = false, bool SORTED = false>
 __global__ void __launch_bounds__(128, RESTIR ? VG_RESTIR_SHADE_MIN_BLOCKS : VG_SHADE_MIN_BLOCKS) wf_stream_shade_deferred(const __grid_constant__ Ctx c,
                                                                                     const __grid_constant__ Wave w, uint32_t wave,
                                                                                     CacheWave q)
 {
-    uint32_t in = wave & 1u;
-    uint32_t count = w.counts[in];
-    const uint32_t* qin = w.queue[in];
+    uint32_t in = wave & 1u, out = in ^ 1u;
+    uint32_t count = w.counts[out];
+    const uint32_t* qin = w.queue[out];
     uint32_t n = w.n;
+    uint32_t batch = c.p[P_SAMPLES_PER_DISPATCH];
     uint32_t seg[SHADE_CLASSES + 1] = {0, 0, 0, 0, 0};
     if (SORTED)
         for (uint32_t k = 0; k < SHADE_CLASSES; k++)
@@ -633,7 +736,7 @@ __global__ void __launch_bounds__(128, RESTIR ? VG_RESTIR_SHADE_MIN_BLOCKS : VG_
         if (base >= count)
             break;
         uint32_t i = base + lane_id();
-        bool query = false;
+        bool query = false, shadow = false;
         uint32_t p = 0, kq = 0;
         CacheHook hk;
         if (i < count) {
@@ -669,17 +772,31 @@ __global__ void __launch_bounds__(128, RESTIR ? VG_RESTIR_SHADE_MIN_BLOCKS : VG_
                 if (alive)
                     q.st[p] = make_float2(hk.a0, hk.a);
             }
-            if (alive)
+            uint32_t fl = SLOT_RAY;
+            if (alive) {
+                w.meta[p] = (depth + 1) | (kq << 8);
+            } else {
+                w.pend[p] = make_float4(st.parts.total.x, st.parts.total.y, st.parts.total.z, 0.0f);
+                fl = SLOT_ENDED;
+                if (kq + 1 < batch) {
+                    fl |= SLOT_RAY;
+                    st = generatePathFor<false>(c, p % c.p[P_WIDTH], p / c.p[P_WIDTH], c.p[P_SAMPLE] + kq + 1);
+                    w.meta[p] = (kq + 1) << 8;
+                }
+            }
+            if (fl & SLOT_RAY)
                 storePath<false>(w, st, p);
-            else
-                w.state[3 * n + p] = make_float4(st.parts.total.x, st.parts.total.y, st.parts.total.z, st.qPrev);
-            uint32_t flags = (req.valid ? 1u : 0u) | (alive ? 2u : 0u);
-            w.sreq[n + p] = make_float4(req.d.x, req.d.y, req.d.z, __uint_as_float(flags));
-            if (req.valid) {
+            shadow = req.valid;
+            if (shadow) {
+                fl |= SLOT_SHADOW;
                 w.sreq[p] = make_float4(req.o.x, req.o.y, req.o.z, req.tmax);
+                w.sreq[n + p] = make_float4(req.d.x, req.d.y, req.d.z, 0.0f);
                 w.sreq[2 * n + p] = make_float4(req.c.x, req.c.y, req.c.z, 0.0f);
             }
+            w.flags[p] = fl;
         }
+        __syncwarp();
+        warp_append(&w.shcount[out], w.shqueue, shadow, p);
         if (CACHE && __ballot_sync(FULL, query)) {
             // Records of sample kq go to range kq (one atomic per sample present in the warp).
             uint32_t grp = __match_any_sync(FULL, query ? kq : 0xffffffffu);
@@ -696,75 +813,25 @@ __global__ void __launch_bounds__(128, RESTIR ? VG_RESTIR_SHADE_MIN_BLOCKS : VG_
     }
 }
 
-// Finish of one slot after its shadow ray (or with no light sample): add the unoccluded sample,
-// then queue the path for its next depth, or finish it and restart the slot with the batch's next
-// sample. Returns whether the slot goes to the next wave's queue.
-template <typename A, bool RESTIR = false>
-__device__ __forceinline__ bool finishSlot(const Ctx& c, const Wave& w, uint32_t p, bool blocked)
+// Shadow rays of scenes with translucent surfaces (layers, opacity rolls), and of the static-fetch form:
+// one ray per lane, 32 queue entries per fetch.
+static __global__ void __launch_bounds__(128, 8) wf_stream_shadow_layers(const __grid_constant__ Ctx c,
+                                                                         const __grid_constant__ Wave w, uint32_t wave)
 {
-    uint32_t n = w.n;
-    uint32_t meta = w.meta[p];
-    uint32_t depth = meta & 0xffu, k = meta >> 8;
-    uint32_t flags = __float_as_uint(w.sreq[n + p].w);
-    float4 tot = w.state[3 * n + p];
-    V3 total = v3(tot.x, tot.y, tot.z);
-    if ((flags & 1u) && !blocked) {
-        float4 r2 = w.sreq[2 * n + p];
-        total += v3(r2.x, r2.y, r2.z);
-        if (flags & 2u)
-            w.state[3 * n + p] = make_float4(total.x, total.y, total.z, tot.w);
-    }
-    if (flags & 2u) {
-        w.meta[p] = (depth + 1) | (k << 8);
-        return true;
-    }
-    PathState<false> st;
-    st.parts.zero();
-    st.parts.total = total;
-    st.visLit = st.visTotal = 0.0f;
-    // The deferred stages never carry ReSTIR GI (the host traces the light sample inside shade
-    // when GI is on), so the path's GI flag is false here.
-    st.gi = false;
-    st.chan = -1;
-    finishPath<false, A, RESTIR>(c, st, p);
-    if (k + 1 < c.p[P_SAMPLES_PER_DISPATCH] && (c.p[P_ADAPTIVE] == 0 || pixelActive<A>(c, p))) {
-        PathState<false> nx = generatePathFor<false>(c, p % c.p[P_WIDTH], p / c.p[P_WIDTH], c.p[P_SAMPLE] + k + 1);
-        storePath<false>(w, nx, p);
-        w.meta[p] = (k + 1) << 8;
-        return true;
-    }
-    return false;
-}
-
-template <typename A, bool RESTIR = false>
-__global__ void __launch_bounds__(128, 8) wf_stream_shadow(const __grid_constant__ Ctx c, const __grid_constant__ Wave w, uint32_t wave)
-{
-    uint32_t in = wave & 1u, out = in ^ 1u;
-    if (blockIdx.x == 0 && threadIdx.x == 0)
-        w.fetch[out] = 0;
-    uint32_t count = w.counts[in];
-    const uint32_t* qin = w.queue[in];
-    uint32_t* qout = w.queue[out];
-    uint32_t n = w.n;
-    __shared__ uint32_t slot[4], fetched;
+    uint32_t in = wave & 1u, n = w.n;
+    uint32_t count = w.shcount[in];
     for (;;) {
-        uint32_t base = block_fetch(&w.fetch[4 + in], &fetched);
+        uint32_t base = warp_fetch(&w.fetch[4 + in]);
         if (base >= count)
             break;
-        uint32_t i = base + threadIdx.x;
-        bool live = false;
-        uint32_t p = 0;
+        uint32_t i = base + lane_id();
         if (i < count) {
-            p = qin[i];
-            float4 r1 = w.sreq[n + p];
-            bool occ = false;
-            if (__float_as_uint(r1.w) & 1u) {
-                float4 r0 = w.sreq[p];
-                occ = occluded(c, v3(r0.x, r0.y, r0.z), v3(r1.x, r1.y, r1.z), r0.w);
-            }
-            live = finishSlot<A, RESTIR>(c, w, p, occ);
+            uint32_t p = w.shqueue[i];
+            float4 r0 = w.sreq[p], r1 = w.sreq[n + p];
+            if (occluded(c, v3(r0.x, r0.y, r0.z), v3(r1.x, r1.y, r1.z), r0.w))
+                w.flags[p] |= SLOT_BLOCKED;
         }
-        block_append<4>(&w.counts[out], qout, live, p, slot);
+        __syncwarp();
     }
 }
 
@@ -777,17 +844,44 @@ __global__ void __launch_bounds__(128, 8) wf_stream_shadow(const __grid_constant
 
 // Runs trace_queue, or with COOP trace_queue_coop (warp-cooperative leaf testing; blocks of 128
 // threads, the launchers' size): the same hits either way.
-template <bool ANY, bool COOP, typename GetRay, typename PutHit>
+template <vgt::Hits H, bool COOP, typename GetRay, typename PutHit>
 __device__ __forceinline__ void trace_queue_any(const Ctx& c, uint32_t* fetch, uint32_t count, uint32_t refill,
                                                 uint32_t steps, GetRay get, PutHit put)
 {
     if (COOP) {
         __shared__ vgt::CoopWarp coop[vgt::COOP_WARPS];
-        vgt::trace_queue_coop<ANY>(c.s.nodes, c.s.tris, fetch, count, c.err, refill, steps, coop[threadIdx.x >> 5],
-                                   get, put);
+        vgt::trace_queue_coop<H == vgt::HITS_ANY>(c.s.nodes, c.s.tris, fetch, count, c.err, refill, steps,
+                                                  coop[threadIdx.x >> 5], get, put);
     } else {
-        vgt::trace_queue<ANY>(c.s.nodes, c.s.tris, fetch, count, c.err, refill, steps, get, put);
+        vgt::trace_queue<H>(c.s.nodes, c.s.tris, fetch, count, c.err, refill, steps, get, put);
     }
+}
+
+// The path ray of slot p, if it has one (a slot whose last path has ended keeps its place in the queue
+// until its shadow ray is resolved).
+static __device__ __forceinline__ bool slot_ray(const Wave& w, uint32_t p, V3& o, V3& d, float& tmax)
+{
+    tmax = 1.0e30f;
+    if (w.flags && !(w.flags[p] & SLOT_RAY))
+        return false;
+    float4 a = w.state[p];
+    float4 b = w.state[w.n + p];
+    o = v3(a.x, a.y, a.z);
+    d = v3(b.x, b.y, b.z);
+    return true;
+}
+
+static __device__ __forceinline__ void slot_shadow_ray(const Wave& w, uint32_t p, V3& o, V3& d, float& tmax)
+{
+    float4 r0 = w.sreq[p], r1 = w.sreq[w.n + p];
+    o = v3(r0.x, r0.y, r0.z);
+    d = v3(r1.x, r1.y, r1.z);
+    tmax = r0.w;
+}
+
+static __device__ __forceinline__ void put_slot_hit(const Wave& w, uint32_t p, const vgt::TraceHit& q)
+{
+    w.hits[p] = make_uint4(q.hit ? 1u : 0u, q.hit ? q.inst : 0u, q.hit ? q.prim : 0u, __float_as_uint(q.hit ? q.t : 0.0f));
 }
 
 // Minimum resident 128-thread blocks per SM requested for the dynamic-fetch traversal stages (a
@@ -796,39 +890,58 @@ __device__ __forceinline__ void trace_queue_any(const Ctx& c, uint32_t* fetch, u
 #define VG_TRACE_MIN_BLOCKS 8
 #endif
 
-template <bool STATS, bool COOP>
-__global__ void __launch_bounds__(128, VG_TRACE_MIN_BLOCKS) wf_stream_extend_dyn(const __grid_constant__ Ctx c, const __grid_constant__ Wave w, uint32_t wave)
+// A wave's rays in one launch: the path ray of every queued slot (closest hit) and the shadow rays that
+// the last shade stage left (any hit), one after the other in one work counter. As two launches each
+// waits for its longest ray with most of the chip idle: at 960x540 a fifth of both stages' time.
+static __global__ void __launch_bounds__(128, VG_TRACE_MIN_BLOCKS) wf_stream_trace(const __grid_constant__ Ctx c,
+                                                                                  const __grid_constant__ Wave w,
+                                                                                  uint32_t wave)
 {
-    uint32_t in = wave & 1u, out = in ^ 1u;
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        w.counts[out] = 0;
-        w.fetch[2 + in] = 0;
-        w.fetch[4 + in] = 0;
-        w.fetch[6 + in] = 0;
-    }
-    uint32_t count = w.counts[in];
+    uint32_t in = wave & 1u;
+    clear_wave_counters(w, in);
+    uint32_t rays = w.counts[in], count = rays + w.shcount[in];
     const uint32_t* qin = w.queue[in];
-    uint32_t n_rays = 0, n_nodes = 0, n_tests = 0, n_later = 0;
-    trace_queue_any<false, COOP>(
+    trace_queue_any<vgt::HITS_EITHER, false>(
         c, &w.fetch[in], count, w.refill, w.steps,
-        [&](uint32_t i, V3& o, V3& d, float& tmax) {
-            uint32_t p = qin[i];
-            float4 a = w.state[p];
-            float4 b = w.state[w.n + p];
-            o = v3(a.x, a.y, a.z);
-            d = v3(b.x, b.y, b.z);
-            tmax = 1.0e30f;
+        [&](uint32_t i, V3& o, V3& d, float& tmax, bool& any) {
+            any = i >= rays;
+            if (!any)
+                return slot_ray(w, qin[i], o, d, tmax);
+            slot_shadow_ray(w, w.shqueue[i - rays], o, d, tmax);
             return true;
         },
         [&](uint32_t i, const vgt::TraceHit& q) {
-            uint32_t p = qin[i];
-            w.hits[p] = make_uint4(q.hit ? 1u : 0u, q.hit ? q.inst : 0u, q.hit ? q.prim : 0u,
-                                   __float_as_uint(q.hit ? q.t : 0.0f));
-            if (STATS) {
+            if (i < rays)
+                put_slot_hit(w, qin[i], q);
+            else if (q.hit)
+                atomicOr(&w.flags[w.shqueue[i - rays]], SLOT_BLOCKED);
+        });
+}
+
+// The path rays alone. STATS counts rays, nodes and triangle tests (tstats[0..2], rays past depth 0 in [3]).
+template <bool STATS, bool COOP>
+__global__ void __launch_bounds__(128, VG_TRACE_MIN_BLOCKS) wf_stream_extend_dyn(const __grid_constant__ Ctx c, const __grid_constant__ Wave w, uint32_t wave)
+{
+    uint32_t in = wave & 1u;
+    clear_wave_counters(w, in);
+    uint32_t count = w.counts[in];
+    const uint32_t* qin = w.queue[in];
+    uint32_t n_rays = 0, n_nodes = 0, n_tests = 0, n_later = 0;
+    trace_queue_any<vgt::HITS_CLOSEST, COOP>(
+        c, &w.fetch[in], count, w.refill, w.steps,
+        [&](uint32_t i, V3& o, V3& d, float& tmax, bool&) {
+            bool ray = slot_ray(w, qin[i], o, d, tmax);
+            if (STATS && ray)
                 n_rays++;
+            return ray;
+        },
+        [&](uint32_t i, const vgt::TraceHit& q) {
+            uint32_t p = qin[i];
+            put_slot_hit(w, p, q);
+            if (STATS) {
                 n_nodes += q.nodes;
                 n_tests += q.tests;
-                n_later += (w.meta[p] & 0xffu) != 0 ? 1u : 0u;
+                n_later += q.nodes != 0 && (w.meta[p] & 0xffu) != 0 ? 1u : 0u;
             }
         });
     if (STATS) {
@@ -839,76 +952,29 @@ __global__ void __launch_bounds__(128, VG_TRACE_MIN_BLOCKS) wf_stream_extend_dyn
     }
 }
 
-// Shadow rays of the deferred light samples, any hit (opaque scenes: one layer, no opacity roll).
-// The result goes to hits[p].x (1 occluded), which the finish stage reads. STATS: the rays traced
-// are counted into tstats[4].
-// The same for the shadow stage alone (its any-hit rays end at the first occluder; its grid
-// follows). 10 or 12 blocks (48 or 40 registers) make the stage 4% and 9% slower than 8.
-#ifndef VG_SHADOW_MIN_BLOCKS
-#define VG_SHADOW_MIN_BLOCKS VG_TRACE_MIN_BLOCKS
-#endif
-
+// The shadow rays of the deferred light samples alone, any hit (opaque scenes: one layer, no opacity
+// roll). STATS: the rays traced are counted into tstats[4]. (10 or 12 blocks per SM, 48 or 40
+// registers, make the stage 4% and 9% slower than 8.)
 template <bool STATS, bool COOP>
-__global__ void __launch_bounds__(128, VG_SHADOW_MIN_BLOCKS) wf_stream_shadow_trace(const __grid_constant__ Ctx c, const __grid_constant__ Wave w, uint32_t wave)
+__global__ void __launch_bounds__(128, VG_TRACE_MIN_BLOCKS) wf_stream_shadow_trace(const __grid_constant__ Ctx c, const __grid_constant__ Wave w, uint32_t wave)
 {
     uint32_t in = wave & 1u;
-    uint32_t count = w.counts[in];
-    const uint32_t* qin = w.queue[in];
-    uint32_t n = w.n;
+    uint32_t count = w.shcount[in];
     uint32_t n_rays = 0;
-    trace_queue_any<true, COOP>(
+    trace_queue_any<vgt::HITS_ANY, COOP>(
         c, &w.fetch[4 + in], count, w.shadow_refill, w.shadow_steps,
-        [&](uint32_t i, V3& o, V3& d, float& tmax) {
-            uint32_t p = qin[i];
-            float4 r1 = w.sreq[n + p];
-            if (!(__float_as_uint(r1.w) & 1u)) {
-                tmax = 0.0f;
-                return false;
-            }
-            float4 r0 = w.sreq[p];
-            o = v3(r0.x, r0.y, r0.z);
-            d = v3(r1.x, r1.y, r1.z);
-            tmax = r0.w;
+        [&](uint32_t i, V3& o, V3& d, float& tmax, bool&) {
+            slot_shadow_ray(w, w.shqueue[i], o, d, tmax);
             if (STATS)
                 n_rays++;
             return true;
         },
-        [&](uint32_t i, const vgt::TraceHit& q) { ((uint32_t*)w.hits)[4 * (size_t)qin[i]] = q.hit ? 1u : 0u; });
+        [&](uint32_t i, const vgt::TraceHit& q) {
+            if (q.hit)
+                w.flags[w.shqueue[i]] |= SLOT_BLOCKED;
+        });
     if (STATS)
         warp_count(&w.tstats[4], n_rays);
-}
-
-// After the shadow trace: add the unoccluded light sample, then queue, finish or restart each slot
-// (the second half of wf_stream_shadow).
-// Minimum resident 128-thread blocks per SM requested for the finish stage (a register cap; its grid
-// follows). 12 or 16 blocks (40 or 32 registers) are 1.1-1.6% slower per benchmark step than 8.
-#ifndef VG_FINISH_MIN_BLOCKS
-#define VG_FINISH_MIN_BLOCKS 8
-#endif
-
-template <typename A, bool RESTIR = false>
-__global__ void __launch_bounds__(128, VG_FINISH_MIN_BLOCKS) wf_stream_finish(const __grid_constant__ Ctx c, const __grid_constant__ Wave w, uint32_t wave)
-{
-    uint32_t in = wave & 1u, out = in ^ 1u;
-    if (blockIdx.x == 0 && threadIdx.x == 0)
-        w.fetch[out] = 0;
-    uint32_t count = w.counts[in];
-    const uint32_t* qin = w.queue[in];
-    uint32_t* qout = w.queue[out];
-    __shared__ uint32_t slot[4], fetched;
-    for (;;) {
-        uint32_t base = block_fetch(&w.fetch[6 + in], &fetched);
-        if (base >= count)
-            break;
-        uint32_t i = base + threadIdx.x;
-        bool live = false;
-        uint32_t p = 0;
-        if (i < count) {
-            p = qin[i];
-            live = finishSlot<A, RESTIR>(c, w, p, ((const uint32_t*)w.hits)[4 * (size_t)p] != 0u);
-        }
-        block_append<4>(&w.counts[out], qout, live, p, slot);
-    }
 }
 
 // The tail of a streaming batch: once few slots are live, one thread per remaining slot runs its
@@ -925,6 +991,19 @@ __global__ void __launch_bounds__(128, VG_TAIL_MIN_BLOCKS) wf_stream_tail(const 
     if (i >= w.counts[in])
         return;
     uint32_t p = w.queue[in][i];
+    if (!LIGHT && w.flags) {
+        // A wave's shadow ray is still to be traced, and the path before this one may wait for it.
+        uint32_t fl = w.flags[p];
+        bool blocked = false;
+        if (fl & SLOT_SHADOW) {
+            V3 o, d;
+            float tmax;
+            slot_shadow_ray(w, p, o, d, tmax);
+            blocked = occluded(c, o, d, tmax);
+        }
+        if (!resolveSlot<A, RESTIR>(c, w, p, fl, blocked))
+            return;
+    }
     uint32_t meta = w.meta[p];
     uint32_t depth = meta & 0xffu, k = meta >> 8;
     uint32_t batch = c.p[P_SAMPLES_PER_DISPATCH];

@@ -41,26 +41,26 @@ cudaError_t launch_stream_cache_shade(bool f64, bool sorted, int blocks, cudaStr
 int stream_cache_shade_blocks_per_sm(bool f64);
 cudaError_t launch_stream_cache_tail(bool f64, uint32_t max_slots, cudaStream_t s, const vgd::Ctx& c,
                                      const vgk::Wave& w, uint32_t wave, const vgk::CacheWave& q);
-// With `sorted` the shade stage takes the wave's slots class by class (launch_stream_classify first).
+// With `sorted` the resolve stage also fills the class queues and the shade stage takes the wave's slots
+// class by class.
 cudaError_t launch_stream_shade_deferred(bool f64, bool sorted, int blocks, cudaStream_t s, const vgd::Ctx& c,
                                          const vgk::Wave& w, uint32_t wave);
-cudaError_t launch_stream_classify(int blocks, cudaStream_t s, const vgd::Ctx& c, const vgk::Wave& w, uint32_t wave);
-cudaError_t launch_stream_shadow(bool f64, int blocks, cudaStream_t s, const vgd::Ctx& c, const vgk::Wave& w,
-                                 uint32_t wave);
-int stream_deferred_blocks_per_sm(bool f64, int* shadow);
-// Dynamic-fetch traversal stages: extend, the shadow trace of opaque scenes, then finish.
+cudaError_t launch_stream_resolve(bool f64, bool sorted, int blocks, cudaStream_t s, const vgd::Ctx& c,
+                                  const vgk::Wave& w, uint32_t wave);
+int stream_resolve_blocks_per_sm(bool f64);
+cudaError_t launch_stream_shadow_layers(int blocks, cudaStream_t s, const vgd::Ctx& c, const vgk::Wave& w,
+                                        uint32_t wave);
+int stream_shadow_layers_blocks_per_sm();
+int stream_deferred_blocks_per_sm(bool f64);
+// Dynamic-fetch traversal stages: a wave's path and shadow rays in one launch, or each in its own.
 // With `coop` the warp-cooperative leaf testing of traverse.cuh (the same hits).
+cudaError_t launch_stream_trace(int blocks, cudaStream_t s, const vgd::Ctx& c, const vgk::Wave& w, uint32_t wave);
 cudaError_t launch_stream_extend_dyn(bool stats, bool coop, int blocks, cudaStream_t s, const vgd::Ctx& c,
                                      const vgk::Wave& w, uint32_t wave);
 cudaError_t launch_stream_shadow_trace(bool stats, bool coop, int blocks, cudaStream_t s, const vgd::Ctx& c,
                                        const vgk::Wave& w, uint32_t wave);
 int stream_trace_blocks_per_sm(bool coop);
-// Resident 128-thread blocks per SM of the finish stage and of the shadow stage (their grids fill
-// the SMs once).
-int stream_finish_blocks_per_sm(bool f64);
 int stream_shadow_trace_blocks_per_sm();
-cudaError_t launch_stream_finish(bool f64, int blocks, cudaStream_t s, const vgd::Ctx& c, const vgk::Wave& w,
-                                 uint32_t wave);
 // The same streaming stages compiled with ReSTIR (kern_wf_restir.cu); the host runs them one
 // sample per launch sequence.
 cudaError_t launch_stream_shade_restir(Variant v, int blocks, cudaStream_t s, const vgd::Ctx& c, const vgk::Wave& w,
@@ -71,10 +71,8 @@ cudaError_t launch_stream_tail_restir(Variant v, uint32_t max_slots, cudaStream_
 cudaError_t launch_stream_shade_deferred_restir(bool f64, bool sorted, int blocks, cudaStream_t s, const vgd::Ctx& c,
                                                 const vgk::Wave& w, uint32_t wave);
 int stream_deferred_restir_blocks_per_sm(bool f64);
-cudaError_t launch_stream_shadow_restir(bool f64, int blocks, cudaStream_t s, const vgd::Ctx& c, const vgk::Wave& w,
-                                        uint32_t wave);
-cudaError_t launch_stream_finish_restir(bool f64, int blocks, cudaStream_t s, const vgd::Ctx& c, const vgk::Wave& w,
-                                        uint32_t wave);
+cudaError_t launch_stream_resolve_restir(bool f64, bool sorted, int blocks, cudaStream_t s, const vgd::Ctx& c,
+                                         const vgk::Wave& w, uint32_t wave);
 // Finishes every slot still live after `wave` (at most max_slots of them) in one launch.
 cudaError_t launch_stream_tail(Variant v, uint32_t max_slots, cudaStream_t s, const vgd::Ctx& c, const vgk::Wave& w,
                                uint32_t wave);

@@ -232,9 +232,13 @@ struct Walk {
     uint2 group;
     uint32_t tri_base, tri_bits;
     int sp;
+    bool any;               // HITS_EITHER: this ray ends at its first hit
     float b1, b2;           // barycentric weights of vertices 1 and 2 at the hit (dropped unless read)
     uint32_t nodes, tests;  // nodes visited and triangles tested (dropped unless read)
 };
+
+// What a traversal looks for: every ray's closest hit, any hit, or one of the two by the ray (Walk::any).
+enum Hits { HITS_CLOSEST, HITS_ANY, HITS_EITHER };
 
 __device__ __forceinline__ void walk_begin(Walk& w, V3 o, V3 d, float tmax)
 {
@@ -263,7 +267,7 @@ __device__ __forceinline__ void node_visit(const uint4* __restrict__ nodes, Walk
 }
 
 // Tests one pending triangle. Returns true when an any-hit walk has its hit.
-template <bool ANY>
+template <Hits H>
 __device__ __forceinline__ bool test_one(const float4* __restrict__ tris, Walk& w)
 {
     uint32_t j = high_bit(w.tri_bits);
@@ -275,14 +279,14 @@ __device__ __forceinline__ bool test_one(const float4* __restrict__ tris, Walk& 
     w.tests++;
     if (tri_test(w.r, v3(a.x, a.y, a.z), v3(b.x, b.y, b.z), v3(c.x, c.y, c.z), t, U, V, W, det)) {
         bool take = t < w.tmax;
-        if (!ANY && t == w.tmax && w.hit_tri != NO_TRI)
+        if (H != HITS_ANY && t == w.tmax && w.hit_tri != NO_TRI)
             take = __float_as_uint(c.w) < __float_as_uint(__ldg(&tris[(size_t)w.hit_tri * bvh8::TRI_VEC4 + 2].w));
         if (take) {
             w.hit_tri = k;
             w.tmax = t;
             w.b1 = V / det;
             w.b2 = W / det;
-            return ANY;
+            return H == HITS_ANY || (H == HITS_EITHER && w.any);
         }
     }
     return false;
@@ -317,13 +321,13 @@ __device__ __forceinline__ bool next_node(Walk& w, uint2* stack, uint32_t* err)
 // finished (nothing left, or an any-hit walk has its hit). (Tried: one triangle a step, a lane with
 // more of them skipping the node test of the steps that follow, so that the triangle test runs once
 // a step instead of as often as the warp's busiest lane needs: 7% slower on the 1M-triangle workload.)
-template <bool ANY>
+template <Hits H>
 __device__ __forceinline__ bool walk_step(const uint4* __restrict__ nodes, const float4* __restrict__ tris, Walk& w,
                                           uint2* stack, uint32_t* err)
 {
     node_visit(nodes, w);
     while (w.tri_bits)
-        if (test_one<ANY>(tris, w))
+        if (test_one<H>(tris, w))
             return true;
     return next_node(w, stack, err);
 }
@@ -366,7 +370,7 @@ __device__ __forceinline__ TraceHit trace_bvh(const uint4* __restrict__ nodes, c
     uint2 stack[bvh8::STACK_SIZE];
     Walk w;
     walk_begin(w, o, d, tmax);
-    while (!walk_step<ANY>(nodes, tris, w, stack, err)) {
+    while (!walk_step<ANY ? HITS_ANY : HITS_CLOSEST>(nodes, tris, w, stack, err)) {
     }
     return walk_hit(tris, w);
 }
@@ -378,8 +382,9 @@ __device__ __forceinline__ TraceHit trace_bvh(const uint4* __restrict__ nodes, c
 // Efficiency of Ray Traversal on GPUs", HPG 2009). Each lane runs at most `steps` node visits
 // between refills. Results are those of trace_bvh: the hit rule does not depend on the visiting order.
 //
-// get(i, r, tmax) loads queue item i into a ray and returns false when it has no ray (it then
-// completes at once with a miss); put(i, hit) stores the result of item i.
+// get(i, o, d, tmax, any) loads queue item i into a ray (with HITS_EITHER also whether any hit will do)
+// and returns false when it has no ray (it then completes at once with a miss); put(i, hit) stores the
+// result of item i.
 
 // ---------------------------------------------------------------------------------------------
 // Warp-cooperative leaf testing. In walk_step every lane tests its node's triangles itself, so a
@@ -547,7 +552,7 @@ __device__ __forceinline__ void trace_queue_coop(const uint4* __restrict__ nodes
                 if (idx < count) {
                     V3 o, d;
                     float tmax;
-                    if (get(idx, o, d, tmax)) {
+                    if (get(idx, o, d, tmax, w.any)) {
                         walk_begin(w, o, d, tmax);
                         w.item = idx;
                         active = true;
@@ -589,7 +594,7 @@ __device__ __forceinline__ void trace_queue_coop(const uint4* __restrict__ nodes
 
 // The body of trace_queue and trace_queue_scenes: with SCENES, `get` also names the BVH of each ray
 // (its node and triangle arrays), which the lane keeps while it walks that ray.
-template <bool ANY, bool SCENES, typename GetRay, typename PutHit>
+template <Hits H, bool SCENES, typename GetRay, typename PutHit>
 __device__ __forceinline__ void trace_queue_impl(const uint4* __restrict__ nodes0, const float4* __restrict__ tris0,
                                                  uint32_t* fetch, uint32_t count, uint32_t* err, uint32_t refill,
                                                  uint32_t steps, GetRay get, PutHit put)
@@ -620,7 +625,7 @@ __device__ __forceinline__ void trace_queue_impl(const uint4* __restrict__ nodes
                     if constexpr (SCENES)
                         ok = get(idx, o, d, tmax, nodes, tris);
                     else
-                        ok = get(idx, o, d, tmax);
+                        ok = get(idx, o, d, tmax, w.any);
                     if (ok) {
                         walk_begin(w, o, d, tmax);
                         w.item = idx;
@@ -639,7 +644,7 @@ __device__ __forceinline__ void trace_queue_impl(const uint4* __restrict__ nodes
         if (active) {
 #pragma unroll 1
             for (uint32_t s = 0; s < steps; s++) {
-                if (walk_step<ANY>(nodes, tris, w, stack, err)) {
+                if (walk_step<H>(nodes, tris, w, stack, err)) {
                     put(w.item, walk_hit(tris, w));
                     active = false;
                     break;
@@ -649,12 +654,12 @@ __device__ __forceinline__ void trace_queue_impl(const uint4* __restrict__ nodes
     }
 }
 
-template <bool ANY, typename GetRay, typename PutHit>
+template <Hits H, typename GetRay, typename PutHit>
 __device__ __forceinline__ void trace_queue(const uint4* __restrict__ nodes, const float4* __restrict__ tris,
                                             uint32_t* fetch, uint32_t count, uint32_t* err, uint32_t refill,
                                             uint32_t steps, GetRay get, PutHit put)
 {
-    trace_queue_impl<ANY, false>(nodes, tris, fetch, count, err, refill, steps, get, put);
+    trace_queue_impl<H, false>(nodes, tris, fetch, count, err, refill, steps, get, put);
 }
 
 // trace_queue over the rays of several scenes: get(idx, o, d, tmax, nodes, tris) also sets the
@@ -663,7 +668,7 @@ template <bool ANY, typename GetRay, typename PutHit>
 __device__ __forceinline__ void trace_queue_scenes(uint32_t* fetch, uint32_t count, uint32_t* err, uint32_t refill,
                                                    uint32_t steps, GetRay get, PutHit put)
 {
-    trace_queue_impl<ANY, true>(nullptr, nullptr, fetch, count, err, refill, steps, get, put);
+    trace_queue_impl<ANY ? HITS_ANY : HITS_CLOSEST, true>(nullptr, nullptr, fetch, count, err, refill, steps, get, put);
 }
 
 } // namespace vgt

@@ -172,7 +172,7 @@ void bind_tables(VgRenderer* r)
 // until no slot is live (the host reads each wave's live count LAG waves later, so the GPU never
 // idles on the poll) and a tail launch once few slots are live. With `q` the radiance-cache
 // variants run (lighting split off, shadow rays always in their own stage).
-int stream_samples(VgRenderer* r, VgAccum* acc, vgd::Ctx& c, vgx::Variant v, const vgk::Wave& w, uint32_t sample0,
+int stream_samples(VgRenderer* r, VgAccum* acc, vgd::Ctx& c, vgx::Variant v, const vgk::Wave& wave0, uint32_t sample0,
                    uint32_t samples, bool timed, EventPool& pool, StageEvents& stages, const vgk::CacheWave* q)
 {
     cudaStream_t s = r->ctx->stream;
@@ -190,8 +190,7 @@ int stream_samples(VgRenderer* r, VgAccum* acc, vgd::Ctx& c, vgx::Variant v, con
     // sample's shadow ray is traced inside shade.
     bool deferred = (!acc->lighting && r->defer_shadows && !(v.restir && acc->restir.gi)) || q;
     if (deferred && r->deferred_blocks[v.f64 ? 1 : 0] == 0)
-        r->deferred_blocks[v.f64 ? 1 : 0] =
-            vgx::stream_deferred_blocks_per_sm(v.f64, &r->shadow_blocks[v.f64 ? 1 : 0]);
+        r->deferred_blocks[v.f64 ? 1 : 0] = vgx::stream_deferred_blocks_per_sm(v.f64);
     int dsb = blocks_for(r, r->deferred_blocks[v.f64 ? 1 : 0]);
     if (deferred && v.restir) {
         if (r->deferred_restir_blocks[v.f64 ? 1 : 0] == 0)
@@ -204,20 +203,65 @@ int stream_samples(VgRenderer* r, VgAccum* acc, vgd::Ctx& c, vgx::Variant v, con
             r->cache_shade_blocks[v.f64 ? 1 : 0] = vgx::stream_cache_shade_blocks_per_sm(v.f64);
         csb = blocks_for(r, r->cache_shade_blocks[v.f64 ? 1 : 0]);
     }
-    int shb = blocks_for(r, r->shadow_blocks[v.f64 ? 1 : 0]);
-    int fnb = blocks_for(r, vgx::stream_finish_blocks_per_sm(v.f64));
     int stb = blocks_for(r, vgx::stream_shadow_trace_blocks_per_sm());
+    int rvb = blocks_for(r, vgx::stream_resolve_blocks_per_sm(v.f64));
     // Material-sorted shading of the deferred shade stage (plain, ReSTIR and cache waves).
     bool sorted = deferred && r->material_sort && acc->squeue.p != nullptr && acc->scount.p != nullptr &&
-                  acc->squeue.bytes >= (size_t)w.n * 4 * vgk::SHADE_CLASSES;
-    int clb = r->ctx->sms * 4;
+                  acc->squeue.bytes >= (size_t)wave0.n * 4 * vgk::SHADE_CLASSES;
     acc->wave_stages = deferred ? 3 : 2;
+    vgk::Wave w = wave0;
+    if (!deferred)
+        w.flags = nullptr;
+    // Path and shadow rays share a launch where both stages run the same way; timed and counted calls keep
+    // them apart, and translucent scenes' shadow rays have their own kernel.
+    bool dyn = r->dynamic_fetch;
+    bool shadow_dyn = dyn && r->ds.shadow_any;
+    bool merged = deferred && shadow_dyn && !r->coop_tris && !timed && !r->traversal_stats &&
+                  r->fetch_refill == r->shadow_fetch_refill && r->fetch_steps == r->shadow_fetch_steps;
+    int slb = deferred && !shadow_dyn ? blocks_for(r, vgx::stream_shadow_layers_blocks_per_sm()) : 0;
+    // The launches of one wave (their kernels read the queue parity from the wave index only); `mark` is
+    // called after the path rays (0), the shadow rays' and resolve stages (1) and shading (2).
+    auto launch_wave = [&](uint32_t i, auto&& mark) -> cudaError_t {
+        cudaError_t e;
+        if (merged)
+            e = vgx::launch_stream_trace(eb, s, c, w, i);
+        else
+            e = dyn ? vgx::launch_stream_extend_dyn(r->traversal_stats, r->coop_tris, eb, s, c, w, i)
+                    : vgx::launch_stream_extend(r->traversal_stats, eb, s, c, w, i);
+        if (e != cudaSuccess || (e = mark(0)) != cudaSuccess)
+            return e;
+        acc->launches++;
+        if (deferred) {
+            if (!merged) {
+                e = shadow_dyn ? vgx::launch_stream_shadow_trace(r->traversal_stats, r->coop_tris, stb, s, c, w, i)
+                               : vgx::launch_stream_shadow_layers(slb, s, c, w, i);
+                if (e != cudaSuccess)
+                    return e;
+                acc->launches++;
+            }
+            e = (v.restir ? vgx::launch_stream_resolve_restir : vgx::launch_stream_resolve)(v.f64, sorted, rvb, s, c, w, i);
+            if (e != cudaSuccess)
+                return e;
+            acc->launches++;
+        }
+        if ((e = mark(1)) != cudaSuccess)
+            return e;
+        if (!deferred)
+            e = vgx::launch_stream_shade(v, ssb, s, c, w, i);
+        else if (q)
+            e = vgx::launch_stream_cache_shade(v.f64, sorted, csb, s, c, w, i, *q);
+        else
+            e = (v.restir ? vgx::launch_stream_shade_deferred_restir : vgx::launch_stream_shade_deferred)(v.f64, sorted, dsb,
+                                                                                                           s, c, w, i);
+        acc->launches++;
+        return e != cudaSuccess ? e : mark(2);
+    };
     c.p[P_SAMPLE] = sample0;
     c.p[P_SAMPLES_PER_DISPATCH] = samples;
     VG_CHECK(cudaMemsetAsync(acc->counts.p, 0, 2 * 4, s), "counters");
     VG_CHECK(cudaMemsetAsync(acc->fetch.p, 0, 4 * 4, s), "counters");
-    if (sorted)
-        VG_CHECK(cudaMemsetAsync(acc->scount.p, 0, 2 * vgk::SHADE_CLASSES * 4, s), "counters");
+    if (deferred)
+        VG_CHECK(cudaMemsetAsync(w.shcount, 0, 2 * 4, s), "counters");
     VG_CHECK((q ? vgx::launch_stream_cache_start(v.f64, s, c, w, *q) : vgx::launch_stream_start(v, s, c, w)), "stream start launch");
     acc->launches++;
     // Waves until no slot is live. The host reads each wave's output count LAG waves later,
@@ -236,22 +280,11 @@ int stream_samples(VgRenderer* r, VgAccum* acc, vgd::Ctx& c, vgx::Variant v, con
         uint32_t K = r->graph_waves;
         VG_CHECK(cudaStreamBeginCapture(s, cudaStreamCaptureModeRelaxed), "graph capture");
         cudaError_t ce = cudaSuccess;
-        for (uint32_t i = 0; i < K && ce == cudaSuccess; i++) {
-            ce = r->dynamic_fetch ? vgx::launch_stream_extend_dyn(r->traversal_stats, r->coop_tris, eb, s, c, w, i)
-                                  : vgx::launch_stream_extend(r->traversal_stats, eb, s, c, w, i);
-            if (ce == cudaSuccess && sorted)
-                ce = vgx::launch_stream_classify(clb, s, c, w, i);
-            if (ce == cudaSuccess && deferred) {
-                ce = (q ? vgx::launch_stream_cache_shade(v.f64, sorted, csb, s, c, w, i, *q) : (v.restir ? vgx::launch_stream_shade_deferred_restir : vgx::launch_stream_shade_deferred)(v.f64, sorted, dsb, s, c, w, i));
-                if (ce == cudaSuccess && r->dynamic_fetch && r->ds.shadow_any) {
-                    ce = vgx::launch_stream_shadow_trace(r->traversal_stats, r->coop_tris, stb, s, c, w, i);
-                    if (ce == cudaSuccess)
-                        ce = (v.restir ? vgx::launch_stream_finish_restir : vgx::launch_stream_finish)(v.f64, fnb, s, c, w, i);
-                } else if (ce == cudaSuccess)
-                    ce = (v.restir ? vgx::launch_stream_shadow_restir : vgx::launch_stream_shadow)(v.f64, shb, s, c, w, i);
-            } else if (ce == cudaSuccess)
-                ce = vgx::launch_stream_shade(v, ssb, s, c, w, i);
-        }
+        uint64_t launches0 = acc->launches;
+        for (uint32_t i = 0; i < K && ce == cudaSuccess; i++)
+            ce = launch_wave(i, [](int) { return cudaSuccess; });
+        const uint64_t per_replay = acc->launches - launches0;
+        acc->launches = launches0;
         if (ce == cudaSuccess)
             ce = cudaMemcpyAsync(&ring[0], (uint32_t*)acc->counts.p + (K & 1u), 4, cudaMemcpyDeviceToHost, s);
         cudaGraph_t g = nullptr;
@@ -266,7 +299,6 @@ int stream_samples(VgRenderer* r, VgAccum* acc, vgd::Ctx& c, vgx::Variant v, con
         cudaGraphDestroy(g);
         if (ce != cudaSuccess)
             return cuda_fail(ce, "wave graph instantiation");
-        uint32_t per_wave = deferred ? (r->dynamic_fetch && r->ds.shadow_any ? 4 : 3) : 2;
         uint64_t max_rep = (max_waves + K - 1) / K + 2;
         uint64_t rep = 0;
         for (; rep < max_rep && !done; rep++) {
@@ -277,7 +309,7 @@ int stream_samples(VgRenderer* r, VgAccum* acc, vgd::Ctx& c, vgx::Variant v, con
                 cudaGraphExecDestroy(ge);
                 return cuda_fail(ce, "wave graph launch");
             }
-            acc->launches += (uint64_t)K * per_wave;
+            acc->launches += per_replay;
             if (rep >= 1) {
                 if ((st = wait_event(ring_ev[(rep - 1) & 1u])) != VG_OK) {
                     cudaGraphExecDestroy(ge);
@@ -307,54 +339,19 @@ int stream_samples(VgRenderer* r, VgAccum* acc, vgd::Ctx& c, vgx::Variant v, con
         done = true;
     }
     for (; wave < max_waves && !done; wave++) {
-        cudaEvent_t a = nullptr, m = nullptr, b = nullptr;
+        cudaEvent_t ev[4] = {};
         if (timed) {
-            a = pool.get();
-            m = pool.get();
-            b = pool.get();
-            VG_CHECK(cudaEventRecord(a, s), "event");
+            for (auto& e : ev)
+                e = pool.get();
+            VG_CHECK(cudaEventRecord(ev[0], s), "event");
         }
-        if (r->dynamic_fetch)
-            VG_CHECK(vgx::launch_stream_extend_dyn(r->traversal_stats, r->coop_tris, eb, s, c, w, (uint32_t)wave),
-                     "extend launch");
-        else
-            VG_CHECK(vgx::launch_stream_extend(r->traversal_stats, eb, s, c, w, (uint32_t)wave),
-                     "extend launch");
-        if (timed)
-            VG_CHECK(cudaEventRecord(m, s), "event");
-        if (sorted) {
-            VG_CHECK(vgx::launch_stream_classify(clb, s, c, w, (uint32_t)wave), "classify launch");
-            acc->launches++;
-        }
-        if (deferred) {
-            VG_CHECK((q ? vgx::launch_stream_cache_shade(v.f64, sorted, csb, s, c, w, (uint32_t)wave, *q) : (v.restir ? vgx::launch_stream_shade_deferred_restir : vgx::launch_stream_shade_deferred)(v.f64, sorted, dsb, s, c, w, (uint32_t)wave)), "shade launch");
-            cudaEvent_t qe = nullptr;
-            if (timed) {
-                qe = pool.get();
-                VG_CHECK(cudaEventRecord(qe, s), "event");
-            }
-            if (r->dynamic_fetch && r->ds.shadow_any) {
-                VG_CHECK(vgx::launch_stream_shadow_trace(r->traversal_stats, r->coop_tris, stb, s, c, w, (uint32_t)wave), "shadow launch");
-                VG_CHECK((v.restir ? vgx::launch_stream_finish_restir : vgx::launch_stream_finish)(v.f64, fnb, s, c, w, (uint32_t)wave), "finish launch");
-                acc->launches++;
-            } else {
-                VG_CHECK((v.restir ? vgx::launch_stream_shadow_restir : vgx::launch_stream_shadow)(v.f64, shb, s, c, w, (uint32_t)wave), "shadow launch");
-            }
-            if (timed) {
-                VG_CHECK(cudaEventRecord(b, s), "event");
-                stages.push_back({0, {a, m}});
-                stages.push_back({1, {m, qe}});
-                stages.push_back({3, {qe, b}});
-            }
-            acc->launches += 3;
-        } else {
-            VG_CHECK(vgx::launch_stream_shade(v, ssb, s, c, w, (uint32_t)wave), "shade launch");
-            if (timed) {
-                VG_CHECK(cudaEventRecord(b, s), "event");
-                stages.push_back({0, {a, m}});
-                stages.push_back({1, {m, b}});
-            }
-            acc->launches += 2;
+        VG_CHECK(launch_wave((uint32_t)wave, [&](int k) { return timed ? cudaEventRecord(ev[k + 1], s) : cudaSuccess; }),
+                 "wave launch");
+        if (timed) {
+            stages.push_back({0, {ev[0], ev[1]}});
+            stages.push_back({1, {ev[2], ev[3]}});
+            if (deferred)
+                stages.push_back({3, {ev[1], ev[2]}});
         }
         uint32_t slot = (uint32_t)(wave % RING);
         VG_CHECK(cudaMemcpyAsync(&ring[slot], (uint32_t*)acc->counts.p + ((wave + 1) & 1u), 4,
@@ -1043,7 +1040,10 @@ int vg_accumulate(VgRenderer* r, VgAccum* acc, uint32_t samples)
             (st = alloc(acc->meta, px * 4, s, false)) != VG_OK ||
             (st = alloc(acc->sreq, acc->lighting ? 16 : px * 3 * 16, s, false)) != VG_OK ||
             (st = alloc(acc->squeue, acc->lighting ? 16 : px * 4 * vgk::SHADE_CLASSES, s, false)) != VG_OK ||
-            (st = alloc(acc->scount, 2 * vgk::SHADE_CLASSES * 4, s, true)) != VG_OK)
+            (st = alloc(acc->flags, acc->lighting ? 16 : px * 4, s, false)) != VG_OK ||
+            (st = alloc(acc->pend, acc->lighting ? 16 : px * 16, s, false)) != VG_OK ||
+            (st = alloc(acc->shqueue, acc->lighting ? 16 : px * 4, s, false)) != VG_OK ||
+            (st = alloc(acc->scount, (2 * vgk::SHADE_CLASSES + 2) * 4, s, true)) != VG_OK)
             return st;
         if (!acc->host_counts && cudaHostAlloc((void**)&acc->host_counts, 64 * 4, cudaHostAllocDefault) != cudaSuccess) {
             acc->host_counts = nullptr;
