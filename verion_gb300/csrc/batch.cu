@@ -27,7 +27,7 @@ struct WaveGraphs {
 // The batch wavefront's buffers: the wave planes of `slots` path slots, the request table and the
 // completion state, and its captured graph.
 struct WaveBufs {
-    DevBuf state, hits, q0, q1, counts, fetch, sreq, meta, squeue, scount, slot_req, slot_pix;
+    DevBuf state, hits, q0, q1, counts, fetch, sreq, meta, squeue, scount, flags, pend, shqueue, slot_req, slot_pix;
     DevBuf reqs, done, next, err, loop, t0;
     DevBuf spread, tvert, tnv, caches, qrec, qcount; // cached requests
     uint32_t slots = 0, cache_slots = 0;
@@ -322,7 +322,7 @@ int bwave_graphs(VgContext* ctx, const vgb::WaveBatch& b, const vgk::Wave& w,
         if (ce == cudaSuccess)
             ce = cudaMemsetAsync(w.fetch, 0, 16 * 4, s);
         if (ce == cudaSuccess)
-            ce = cudaMemsetAsync(w.scount, 0, 2 * 2 * vgk::SHADE_CLASSES * 4, s);
+            ce = cudaMemsetAsync(w.scount, 0, (2 * 2 * vgk::SHADE_CLASSES + 2) * 4, s); // and w.shcount
         if (ce == cudaSuccess)
             ce = cudaMemsetAsync(b.err, 0, 4, s);
         if (ce == cudaSuccess)
@@ -458,7 +458,8 @@ int batch_wave_run(VgContext* ctx, const VgBatchRequest* reqs, size_t n, int ord
         if ((st = alloc(B.state, S * 16 * vgk::BASE_PLANES, s, false)) != VG_OK ||
             (st = alloc(B.hits, S * 16, s, false)) != VG_OK || (st = alloc(B.q0, S * 4, s, false)) != VG_OK ||
             (st = alloc(B.q1, S * 4, s, false)) != VG_OK || (st = alloc(B.sreq, S * 16 * 3, s, false)) != VG_OK ||
-            (st = alloc(B.meta, S * 4, s, false)) != VG_OK ||
+            (st = alloc(B.meta, S * 4, s, false)) != VG_OK || (st = alloc(B.flags, S * 4, s, false)) != VG_OK ||
+            (st = alloc(B.pend, S * 16, s, false)) != VG_OK || (st = alloc(B.shqueue, S * 4, s, false)) != VG_OK ||
             (st = alloc(B.squeue, S * 4 * 2 * vgk::SHADE_CLASSES, s, false)) != VG_OK ||
             (st = alloc(B.slot_req, S * 4, s, false)) != VG_OK || (st = alloc(B.slot_pix, S * 4, s, false)) != VG_OK) {
             B.slots = 0;
@@ -478,7 +479,7 @@ int batch_wave_run(VgContext* ctx, const VgBatchRequest* reqs, size_t n, int ord
     }
     if ((!B.counts.p && (st = alloc(B.counts, 16, s, true)) != VG_OK) ||
         (!B.fetch.p && (st = alloc(B.fetch, 64, s, true)) != VG_OK) ||
-        (!B.scount.p && (st = alloc(B.scount, 64, s, true)) != VG_OK) ||
+        (!B.scount.p && (st = alloc(B.scount, (2 * 2 * vgk::SHADE_CLASSES + 2) * 4, s, true)) != VG_OK) ||
         (!B.next.p && (st = alloc(B.next, 16, s, true)) != VG_OK) ||
         (!B.err.p && (st = alloc(B.err, 16, s, true)) != VG_OK) ||
         (!B.loop.p && (st = alloc(B.loop, 16, s, true)) != VG_OK) ||
@@ -524,7 +525,7 @@ int batch_wave_run(VgContext* ctx, const VgBatchRequest* reqs, size_t n, int ord
     if (nc && B.ncache < nc) {
         if ((st = alloc(B.caches, nc * sizeof(vgb::WaveCache), s, false)) != VG_OK ||
             (st = alloc(B.qrec, nc * (size_t)B.cache_slots * vgn::REC_WORDS * 4, s, false)) != VG_OK ||
-            (st = alloc(B.qcount, nc * 4, s, true)) != VG_OK) {
+            (st = alloc(B.qcount, nc * 8, s, true)) != VG_OK) {
             B.ncache = 0;
             return st;
         }
@@ -539,7 +540,7 @@ int batch_wave_run(VgContext* ctx, const VgBatchRequest* reqs, size_t n, int ord
         memset(&K, 0, sizeof(K));
         K.cd = k->dev();
         K.qrec = (float*)B.qrec.p + j * (size_t)B.cache_slots * vgn::REC_WORDS;
-        K.qcount = (uint32_t*)B.qcount.p + j;
+        K.qcount = (uint32_t*)B.qcount.p + 2 * j;
         K.trec = (float*)k->batch_rec.p;
         K.tcount = (uint32_t*)k->batch_count.p;
         K.tcap = r->cache_steps * r->cache_batch;
@@ -597,6 +598,10 @@ int batch_wave_run(VgContext* ctx, const VgBatchRequest* reqs, size_t n, int ord
     w.shadow_steps = r0->shadow_fetch_steps;
     w.squeue = (uint32_t*)B.squeue.p;
     w.scount = (uint32_t*)B.scount.p;
+    w.flags = (uint32_t*)B.flags.p;
+    w.pend = (float4*)B.pend.p;
+    w.shqueue = (uint32_t*)B.shqueue.p;
+    w.shcount = w.scount + 2 * 2 * vgk::SHADE_CLASSES;
     vgb::WaveBatch b{};
     b.reqs = (const vgb::WaveReq*)B.reqs.p;
     b.nreq = (uint32_t)n;
@@ -614,9 +619,9 @@ int batch_wave_run(VgContext* ctx, const VgBatchRequest* reqs, size_t n, int ord
     b.spread = nc ? (float2*)B.spread.p : nullptr;
     b.tvert = nc ? (float4*)B.tvert.p : nullptr;
     b.tnv = nc ? (uint32_t*)B.tnv.p : nullptr;
-    // Until the work items run out every slot is live, so each wave takes `slots` bounces; then at
-    // most one pixel's samples remain per slot. Two waves per iteration.
-    uint64_t waves = bounces / slots + chain + 4;
+    // Until the work items run out every slot is live, so each wave takes `slots` bounces, or resolves a
+    // pixel and starts the next; then at most one pixel's samples remain per slot. Two waves per iteration.
+    uint64_t waves = (bounces + items64) / slots + chain + 6;
     b.max_iter = (uint32_t)std::min<uint64_t>(waves / 2 + 2, 1u << 30);
     sig.insert(sig.end(), {(uint64_t)slots, (uint64_t)items, (uint64_t)b.tail, (uint64_t)b.max_iter,
                            (uint64_t)w.refill << 32 | w.steps, (uint64_t)w.shadow_refill << 32 | w.shadow_steps});

@@ -53,7 +53,7 @@ constexpr uint32_t WAVE_VERTEX_VEC4 = 6;         // per vertex: 16 features, thr
 struct alignas(16) WaveCache {
     vgn::CacheDev cd;
     float* qrec;
-    uint32_t* qcount;
+    uint32_t* qcount;    // by wave parity
     float* trec;
     uint32_t* tcount;
     uint32_t tcap;

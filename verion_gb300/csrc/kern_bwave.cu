@@ -11,8 +11,8 @@
 // A request with a radiance cache runs the cache integrator's paths: a query path ends where its
 // spread passes the cache's threshold and leaves a query record; a training pixel of the sample
 // (the pixel test of mk_cache_train) runs its full path and records its vertices, which become
-// training records when the path ends. After each wave's finish stage one kernel evaluates every
-// cache's queries of that wave (encoding and MMA layers per 128-record tile, the cache's weights
+// training records when the path ends. After each wave's resolve stage one kernel evaluates every
+// cache's queries of the wave before (encoding and MMA layers per 128-record tile, the cache's weights
 // in shared memory) and adds each answer times the path throughput to its pixel. So per pixel the
 // sums take path radiance and cache answer of one sample before those of the next, as the
 // megakernel cache integrator adds them, and the sums match it bit for bit while the cache is
@@ -78,6 +78,7 @@ static __device__ __forceinline__ void begin_item(const WaveBatch& b, const Wave
     PathState<false> st = generatePathFor<false>(R.c, pix % width, pix / width, R.c.p[P_SAMPLE]);
     storePath<false>(w, st, p);
     w.meta[p] = 0;
+    w.flags[p] = SLOT_RAY;
     b.slot_req[p] = r;
     b.slot_pix[p] = pix;
     if (b.tnv)
@@ -124,6 +125,8 @@ __global__ void __launch_bounds__(256) bw_start(const __grid_constant__ WaveBatc
         b.loop[0] = 0;
         *b.t0 = now_ns();
     }
+    if (p < b.ncache)
+        b.caches[p].qcount[0] = b.caches[p].qcount[1] = 0;
     if (p < b.nreq) {
         b.done[p].remaining = b.reqs[p].pixels;
         b.done[p].done_ns = 0;
@@ -134,64 +137,148 @@ __global__ void __launch_bounds__(256) bw_start(const __grid_constant__ WaveBatc
     block_append<8>(&w.counts[0], w.queue[0], live, p, slot);
 }
 
-// Closest hits of the wave's rays, each in its request's scene (wf_stream_extend_dyn).
-__global__ void __launch_bounds__(128, VG_TRACE_MIN_BLOCKS) bw_extend(const __grid_constant__ WaveBatch b, const __grid_constant__ Wave w, uint32_t wave)
+// The wave's path rays (closest hit) and the shadow rays the last shade stages left (any hit), each in
+// its request's scene (wf_stream_trace). A scene with translucent surfaces leaves its shadow rays to the
+// resolve stage (occluded(): layers with opacity).
+__global__ void __launch_bounds__(128, VG_TRACE_MIN_BLOCKS) bw_trace(const __grid_constant__ WaveBatch b, const __grid_constant__ Wave w, uint32_t wave)
 {
     uint32_t in = wave & 1u, out = in ^ 1u;
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         w.counts[out] = 0;
         w.fetch[2 + in] = 0;
-        w.fetch[4 + in] = 0;
-        w.fetch[6 + in] = 0;
         w.fetch[8 + in] = 0;
     }
-    // The previous wave's queries are answered: this wave's start empty.
+    if (blockIdx.x == 0 && threadIdx.x < BW_CLASSES)
+        w.scount[in * BW_CLASSES + threadIdx.x] = 0;
+    // This wave's queries start empty (the last wave of this parity has had its answers).
     if (blockIdx.x == 0)
         for (uint32_t j = threadIdx.x; j < b.ncache; j += blockDim.x)
-            *b.caches[j].qcount = 0;
-    uint32_t count = w.counts[in];
+            b.caches[j].qcount[in] = 0;
+    uint32_t rays = w.counts[in], count = rays + w.shcount[in];
     const uint32_t* qin = w.queue[in];
-    vgt::trace_queue_scenes<false>(
+    vgt::trace_queue_scenes<vgt::HITS_EITHER>(
         &w.fetch[in], count, b.err, w.refill, w.steps,
-        [&](uint32_t i, V3& o, V3& d, float& tmax, const uint4*& nodes, const float4*& tris) {
-            uint32_t p = qin[i];
+        [&](uint32_t i, V3& o, V3& d, float& tmax, bool& any, const uint4*& nodes, const float4*& tris) {
+            any = i >= rays;
+            uint32_t p = any ? w.shqueue[i - rays] : qin[i];
             const DeviceScene& s = b.reqs[b.slot_req[p]].c.s;
             nodes = s.nodes;
             tris = s.tris;
-            float4 a = w.state[p];
-            float4 e = w.state[w.n + p];
-            o = v3(a.x, a.y, a.z);
-            d = v3(e.x, e.y, e.z);
-            tmax = 1.0e30f;
-            return true;
+            if (!any)
+                return slot_ray(w, p, o, d, tmax);
+            slot_shadow_ray(w, p, o, d, tmax);
+            return s.shadow_any != 0;
         },
         [&](uint32_t i, const vgt::TraceHit& q) {
-            w.hits[qin[i]] = make_uint4(q.hit ? 1u : 0u, q.hit ? q.inst : 0u, q.hit ? q.prim : 0u,
-                                        __float_as_uint(q.hit ? q.t : 0.0f));
+            if (i < rays)
+                put_slot_hit(w, qin[i], q);
+            else if (q.hit)
+                atomicOr(&w.flags[w.shqueue[i - rays]], SLOT_BLOCKED);
         });
 }
 
-// Material classes of the wave's slots (wf_stream_classify), each from its request's scene; a
-// cached request's slots in classes SHADE_CLASSES and up.
-__global__ void __launch_bounds__(256) bw_classify(const __grid_constant__ WaveBatch b, const __grid_constant__ Wave w, uint32_t wave)
+// The training records of a finished training path (mk_cache_train's): per recorded vertex its
+// features and the radiance the rest of the path brought, over the throughput arriving there.
+// None for a path whose radiance is not finite; records past the cache's capacity are dropped.
+static __device__ __forceinline__ void training_records(const WaveBatch& b, const WaveCache& K, uint32_t p, V3 total)
 {
+    uint32_t nv = bad3(total) ? 0u : b.tnv[p];
+    if (nv == 0)
+        return;
+    uint32_t t0 = atomicAdd(K.tcount, nv);
+    const float4* v = b.tvert + (size_t)p * vgb::WAVE_MAX_TRAIN_VERTICES * vgb::WAVE_VERTEX_VEC4;
+    for (uint32_t k = 0; k < nv && t0 + k < K.tcap; k++, v += vgb::WAVE_VERTEX_VEC4) {
+        float* d = K.trec + (size_t)(t0 + k) * REC_WORDS;
+        for (int j = 0; j < 4; j++) {
+            d[4 * j] = v[j].x;
+            d[4 * j + 1] = v[j].y;
+            d[4 * j + 2] = v[j].z;
+            d[4 * j + 3] = v[j].w;
+        }
+        V3 t = v3(v[4].x, v[4].y, v[4].z);
+        V3 rest = total - v3(v[4].w, v[5].x, v[5].y);
+        d[16] = t.x > 0.0f ? rest.x / t.x : 0.0f;
+        d[17] = t.y > 0.0f ? rest.y / t.y : 0.0f;
+        d[18] = t.z > 0.0f ? rest.z / t.z : 0.0f;
+        d[19] = 0.0f;
+    }
+}
+
+// resolveSlot (kernels.cuh) for a slot of any request: adds the light sample that got through, and a path
+// that has ended to its pixel. Returns whether the slot still has a ray; without one its pixel is done.
+static __device__ __forceinline__ bool resolve_slot(const WaveBatch& b, const Wave& w, uint32_t p)
+{
+    uint32_t n = w.n, r = b.slot_req[p], fl = w.flags[p];
+    const WaveReq& R = b.reqs[r];
+    const Ctx& c = R.c;
+    bool blocked = (fl & SLOT_BLOCKED) != 0;
+    if ((fl & SLOT_SHADOW) && !c.s.shadow_any) {
+        V3 o, d;
+        float tmax;
+        slot_shadow_ray(w, p, o, d, tmax);
+        blocked = occluded(c, o, d, tmax);
+    }
+    bool lit = (fl & SLOT_SHADOW) && !blocked;
+    if (fl & SLOT_ENDED) {
+        float4 t = w.pend[p];
+        V3 total = v3(t.x, t.y, t.z);
+        if (lit) {
+            float4 s = w.sreq[2 * n + p];
+            total += v3(s.x, s.y, s.z);
+        }
+        PathState<false> st;
+        st.parts.zero();
+        st.parts.total = total;
+        st.visLit = st.visTotal = 0.0f;
+        st.gi = false;
+        st.chan = -1;
+        uint32_t pix = b.slot_pix[p];
+        if (R.f64)
+            finishPath<false, double>(c, st, pix);
+        else
+            finishPath<false, float>(c, st, pix);
+        if (R.cache != NO_CACHE && training_pixel(R, pix, c.p[P_SAMPLE] + __float_as_uint(t.w)))
+            training_records(b, b.caches[R.cache], p, total);
+        if (b.tnv)
+            b.tnv[p] = 0;
+        if (!(fl & SLOT_RAY))
+            pixel_done(b, r);
+    } else if (lit) {
+        float4 t = w.state[3 * n + p], s = w.sreq[2 * n + p];
+        V3 total = v3(t.x, t.y, t.z) + v3(s.x, s.y, s.z);
+        w.state[3 * n + p] = make_float4(total.x, total.y, total.z, t.w);
+    }
+    return (fl & SLOT_RAY) != 0;
+}
+
+// wf_stream_resolve over the slots of all requests; a slot whose pixel is done takes the next work item,
+// whose camera ray the next wave traces. Classes SHADE_CLASSES and up are the cached requests' slots.
+__global__ void __launch_bounds__(256) bw_resolve(const __grid_constant__ WaveBatch b, const __grid_constant__ Wave w, uint32_t wave)
+{
+    __shared__ uint32_t slot[8 * (1 + BW_CLASSES)];
     uint32_t in = wave & 1u, out = in ^ 1u;
-    if (blockIdx.x == 0 && threadIdx.x < BW_CLASSES)
-        w.scount[out * BW_CLASSES + threadIdx.x] = 0;
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        w.fetch[out] = 0;
+        w.shcount[out] = 0;
+    }
     uint32_t count = w.counts[in];
     const uint32_t* qin = w.queue[in];
     uint32_t stride = gridDim.x * blockDim.x;
     for (uint32_t base = blockIdx.x * blockDim.x; base < count; base += stride) {
         uint32_t i = base + threadIdx.x;
-        bool have = i < count;
-        uint32_t p = have ? qin[i] : 0u;
-        uint32_t k = BW_CLASSES;
-        if (have) {
-            const WaveReq& R = b.reqs[b.slot_req[p]];
-            k = shadeClass(R.c, w.hits[p]) + (R.cache != NO_CACHE ? SHADE_CLASSES : 0u);
+        bool live = false;
+        uint32_t p = 0, cls = BW_CLASSES;
+        if (i < count) {
+            p = qin[i];
+            live = resolve_slot(b, w, p);
+            if (live) {
+                const WaveReq& R = b.reqs[b.slot_req[p]];
+                cls = shadeClass(R.c, w.hits[p]) + (R.cache != NO_CACHE ? SHADE_CLASSES : 0u);
+            }
         }
-        for (uint32_t cls = 0; cls < BW_CLASSES; cls++)
-            warp_append(&w.scount[in * BW_CLASSES + cls], w.squeue + (size_t)cls * w.n, k == cls, p);
+        live |= take_items(b, w, p, i < count && !live);
+        block_append_classes<8, BW_CLASSES>(&w.counts[out], w.queue[out], live, w.scount + in * BW_CLASSES, w.squeue,
+                                            w.n, cls, p, slot);
     }
 }
 
@@ -202,7 +289,7 @@ __global__ void __launch_bounds__(256) bw_classify(const __grid_constant__ WaveB
 template <bool CACHE>
 __global__ void __launch_bounds__(128, VG_SHADE_MIN_BLOCKS) bw_shade(const __grid_constant__ WaveBatch b, const __grid_constant__ Wave w, uint32_t wave)
 {
-    uint32_t in = wave & 1u;
+    uint32_t in = wave & 1u, out = in ^ 1u;
     uint32_t n = w.n;
     const uint32_t c0 = CACHE ? SHADE_CLASSES : 0u;
     uint32_t seg[SHADE_CLASSES + 1] = {0, 0, 0, 0, 0};
@@ -214,12 +301,12 @@ __global__ void __launch_bounds__(128, VG_SHADE_MIN_BLOCKS) bw_shade(const __gri
         if (base >= count)
             break;
         uint32_t i = base + lane_id();
-        bool query = false;
-        uint32_t r = 0, pix = 0;
+        bool query = false, shadow = false;
+        uint32_t r = 0, pix = 0, p = 0;
         CacheHook hk;
         if (i < count) {
             uint32_t k = i >= seg[1] ? (i >= seg[2] ? (i >= seg[3] ? 3u : 2u) : 1u) : 0u;
-            uint32_t p = w.squeue[(size_t)(c0 + k) * n + (i - seg[k])];
+            p = w.squeue[(size_t)(c0 + k) * n + (i - seg[k])];
             r = b.slot_req[p];
             pix = b.slot_pix[p];
             const WaveReq& R = b.reqs[r];
@@ -264,17 +351,32 @@ __global__ void __launch_bounds__(128, VG_SHADE_MIN_BLOCKS) bw_shade(const __gri
                 if (alive)
                     b.spread[p] = make_float2(hk.a0, hk.a);
             }
-            if (alive)
+            uint32_t fl = SLOT_RAY, sample = meta >> 8;
+            if (alive) {
+                w.meta[p] = (depth + 1) | (sample << 8);
+            } else {
+                w.pend[p] = make_float4(st.parts.total.x, st.parts.total.y, st.parts.total.z, __uint_as_float(sample));
+                fl = SLOT_ENDED;
+                if (sample + 1 < c.p[P_SAMPLES_PER_DISPATCH]) {
+                    fl |= SLOT_RAY;
+                    uint32_t width = c.p[P_WIDTH];
+                    st = generatePathFor<false>(c, pix % width, pix / width, c.p[P_SAMPLE] + sample + 1);
+                    w.meta[p] = (sample + 1) << 8;
+                }
+            }
+            if (fl & SLOT_RAY)
                 storePath<false>(w, st, p);
-            else
-                w.state[3 * n + p] = make_float4(st.parts.total.x, st.parts.total.y, st.parts.total.z, st.qPrev);
-            uint32_t flags = (req.valid ? 1u : 0u) | (alive ? 2u : 0u);
-            w.sreq[n + p] = make_float4(req.d.x, req.d.y, req.d.z, __uint_as_float(flags));
-            if (req.valid) {
+            shadow = req.valid;
+            if (shadow) {
+                fl |= SLOT_SHADOW;
                 w.sreq[p] = make_float4(req.o.x, req.o.y, req.o.z, req.tmax);
+                w.sreq[n + p] = make_float4(req.d.x, req.d.y, req.d.z, 0.0f);
                 w.sreq[2 * n + p] = make_float4(req.c.x, req.c.y, req.c.z, 0.0f);
             }
+            w.flags[p] = fl;
         }
+        __syncwarp();
+        warp_append(&w.shcount[out], w.shqueue, shadow, p);
         if (CACHE && __ballot_sync(FULL, query)) {
             // Records of one cache together: one atomic per cache present in the warp.
             uint32_t j = query ? b.reqs[r].cache : 0xffffffffu;
@@ -282,7 +384,7 @@ __global__ void __launch_bounds__(128, VG_SHADE_MIN_BLOCKS) bw_shade(const __gri
             uint32_t leader = __ffs(grp) - 1u;
             uint32_t first = 0;
             if (query && lane_id() == leader)
-                first = atomicAdd(b.caches[j].qcount, __popc(grp));
+                first = atomicAdd(b.caches[j].qcount + in, __popc(grp));
             first = __shfl_sync(FULL, first, leader);
             if (query) {
                 uint32_t slot = first + __popc(grp & ((1u << lane_id()) - 1u));
@@ -293,157 +395,16 @@ __global__ void __launch_bounds__(128, VG_SHADE_MIN_BLOCKS) bw_shade(const __gri
     }
 }
 
-// Shadow rays of the wave's light samples, any hit, each in its request's scene. A scene with
-// translucent surfaces leaves its rays to the finish stage (occluded(): layers with opacity).
-__global__ void __launch_bounds__(128, VG_TRACE_MIN_BLOCKS) bw_shadow_trace(const __grid_constant__ WaveBatch b, const __grid_constant__ Wave w, uint32_t wave)
-{
-    uint32_t in = wave & 1u;
-    uint32_t count = w.counts[in];
-    const uint32_t* qin = w.queue[in];
-    uint32_t n = w.n;
-    vgt::trace_queue_scenes<true>(
-        &w.fetch[4 + in], count, b.err, w.shadow_refill, w.shadow_steps,
-        [&](uint32_t i, V3& o, V3& d, float& tmax, const uint4*& nodes, const float4*& tris) {
-            uint32_t p = qin[i];
-            float4 r1 = w.sreq[n + p];
-            const DeviceScene& s = b.reqs[b.slot_req[p]].c.s;
-            if (!(__float_as_uint(r1.w) & 1u) || !s.shadow_any) {
-                tmax = 0.0f;
-                return false;
-            }
-            nodes = s.nodes;
-            tris = s.tris;
-            float4 r0 = w.sreq[p];
-            o = v3(r0.x, r0.y, r0.z);
-            d = v3(r1.x, r1.y, r1.z);
-            tmax = r0.w;
-            return true;
-        },
-        [&](uint32_t i, const vgt::TraceHit& q) { ((uint32_t*)w.hits)[4 * (size_t)qin[i]] = q.hit ? 1u : 0u; });
-}
-
-// The training records of a finished training path (mk_cache_train's): per recorded vertex its
-// features and the radiance the rest of the path brought, over the throughput arriving there.
-// None for a path whose radiance is not finite; records past the cache's capacity are dropped.
-static __device__ __forceinline__ void training_records(const WaveBatch& b, const WaveCache& K, uint32_t p, V3 total)
-{
-    uint32_t nv = bad3(total) ? 0u : b.tnv[p];
-    if (nv == 0)
-        return;
-    uint32_t t0 = atomicAdd(K.tcount, nv);
-    const float4* v = b.tvert + (size_t)p * vgb::WAVE_MAX_TRAIN_VERTICES * vgb::WAVE_VERTEX_VEC4;
-    for (uint32_t k = 0; k < nv && t0 + k < K.tcap; k++, v += vgb::WAVE_VERTEX_VEC4) {
-        float* d = K.trec + (size_t)(t0 + k) * REC_WORDS;
-        for (int j = 0; j < 4; j++) {
-            d[4 * j] = v[j].x;
-            d[4 * j + 1] = v[j].y;
-            d[4 * j + 2] = v[j].z;
-            d[4 * j + 3] = v[j].w;
-        }
-        V3 t = v3(v[4].x, v[4].y, v[4].z);
-        V3 rest = total - v3(v[4].w, v[5].x, v[5].y);
-        d[16] = t.x > 0.0f ? rest.x / t.x : 0.0f;
-        d[17] = t.y > 0.0f ? rest.y / t.y : 0.0f;
-        d[18] = t.z > 0.0f ? rest.z / t.z : 0.0f;
-        d[19] = 0.0f;
-    }
-}
-
-// After the shadow rays (finishSlot for a slot of any request): add the unoccluded light sample,
-// then queue the path for its next depth, or add it to its pixel and start the pixel's next sample.
-// Returns 1 when the slot goes on, 0 when its pixel is finished.
-static __device__ __forceinline__ bool finish_slot(const WaveBatch& b, const Wave& w, uint32_t p)
-{
-    uint32_t n = w.n;
-    uint32_t r = b.slot_req[p];
-    const WaveReq& R = b.reqs[r];
-    const Ctx& c = R.c;
-    uint32_t meta = w.meta[p];
-    uint32_t depth = meta & 0xffu, k = meta >> 8;
-    uint32_t flags = __float_as_uint(w.sreq[n + p].w);
-    float4 tot = w.state[3 * n + p];
-    V3 total = v3(tot.x, tot.y, tot.z);
-    if (flags & 1u) {
-        bool blocked;
-        if (c.s.shadow_any) {
-            blocked = ((const uint32_t*)w.hits)[4 * (size_t)p] != 0u;
-        } else {
-            float4 r0 = w.sreq[p], r1 = w.sreq[n + p];
-            blocked = occluded(c, v3(r0.x, r0.y, r0.z), v3(r1.x, r1.y, r1.z), r0.w);
-        }
-        if (!blocked) {
-            float4 r2 = w.sreq[2 * n + p];
-            total += v3(r2.x, r2.y, r2.z);
-            if (flags & 2u)
-                w.state[3 * n + p] = make_float4(total.x, total.y, total.z, tot.w);
-        }
-    }
-    if (flags & 2u) {
-        w.meta[p] = (depth + 1) | (k << 8);
-        return true;
-    }
-    PathState<false> st;
-    st.parts.zero();
-    st.parts.total = total;
-    st.visLit = st.visTotal = 0.0f;
-    st.gi = false;
-    st.chan = -1;
-    uint32_t pix = b.slot_pix[p];
-    if (R.f64)
-        finishPath<false, double>(c, st, pix);
-    else
-        finishPath<false, float>(c, st, pix);
-    if (R.cache != NO_CACHE && training_pixel(R, pix, c.p[P_SAMPLE] + k))
-        training_records(b, b.caches[R.cache], p, total);
-    if (k + 1 < c.p[P_SAMPLES_PER_DISPATCH]) {
-        uint32_t width = c.p[P_WIDTH];
-        PathState<false> nx = generatePathFor<false>(c, pix % width, pix / width, c.p[P_SAMPLE] + k + 1);
-        storePath<false>(w, nx, p);
-        w.meta[p] = (k + 1) << 8;
-        if (b.tnv)
-            b.tnv[p] = 0;
-        return true;
-    }
-    pixel_done(b, r);
-    return false;
-}
-
-__global__ void __launch_bounds__(128, 8) bw_finish(const __grid_constant__ WaveBatch b, const __grid_constant__ Wave w, uint32_t wave)
-{
-    uint32_t in = wave & 1u, out = in ^ 1u;
-    if (blockIdx.x == 0 && threadIdx.x == 0)
-        w.fetch[out] = 0;
-    uint32_t count = w.counts[in];
-    const uint32_t* qin = w.queue[in];
-    uint32_t* qout = w.queue[out];
-    __shared__ uint32_t slot[4], fetched;
-    for (;;) {
-        uint32_t base = block_fetch(&w.fetch[6 + in], &fetched);
-        if (base >= count)
-            break;
-        uint32_t i = base + threadIdx.x;
-        bool live = false, want = false;
-        uint32_t p = 0;
-        if (i < count) {
-            p = qin[i];
-            live = finish_slot(b, w, p);
-            want = !live;
-        }
-        live |= take_items(b, w, p, want);
-        block_append<4>(&w.counts[out], qout, live, p, slot);
-    }
-}
-
-// The wave's cache queries, all caches in one launch: each CTA takes 128-record tiles (the tiles of
+// The last wave's cache queries (`parity`), once its paths are resolved, all caches in one launch: each CTA takes 128-record tiles (the tiles of
 // cache 0, then of cache 1, ...), loads the tile's cache weights into shared memory when they
 // change, encodes its records (hash grid and the other inputs, one row per thread), runs the five
 // MMA layers with TMEM accumulators, and adds each clamped answer times the record's throughput to
 // its request's pixel (the fused form of nrc_encode + nrc_infer of the cache integrator).
-__global__ void __launch_bounds__(128) bw_answer(WaveBatch b)
+__global__ void __launch_bounds__(128) bw_answer(WaveBatch b, uint32_t parity)
 {
     uint32_t total = 0;
     for (uint32_t j = 0; j < b.ncache; j++)
-        total += (*b.caches[j].qcount + TILE - 1) / TILE;
+        total += (b.caches[j].qcount[parity] + TILE - 1) / TILE;
     if (blockIdx.x >= total)
         return;
     extern __shared__ uint8_t smem_raw[];
@@ -472,7 +433,7 @@ __global__ void __launch_bounds__(128) bw_answer(WaveBatch b)
         // The tile's cache and its first record.
         uint32_t j = 0, first = t * TILE, n = 0;
         for (;; j++) {
-            n = *b.caches[j].qcount;
+            n = b.caches[j].qcount[parity];
             uint32_t tiles = (n + TILE - 1) / TILE;
             if (first < tiles * TILE)
                 break;
@@ -565,6 +526,21 @@ __global__ void __launch_bounds__(128, VG_TAIL_MIN_BLOCKS) bw_tail(const __grid_
     uint32_t count = w.counts[0];
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) {
         uint32_t p = w.queue[0][i];
+        if (w.flags[p] & SLOT_SHADOW) {
+            const Ctx& c0 = b.reqs[b.slot_req[p]].c;
+            V3 o, d;
+            float tmax;
+            slot_shadow_ray(w, p, o, d, tmax);
+            // Scenes with translucent surfaces trace it in resolve_slot.
+            if (c0.s.shadow_any && occluded(c0, o, d, tmax))
+                w.flags[p] |= SLOT_BLOCKED;
+        }
+        if (!resolve_slot(b, w, p)) {
+            uint32_t item = atomicAdd(b.next, 1u);
+            if (item >= b.items)
+                continue;
+            begin_item(b, w, p, item);
+        }
         uint32_t meta = w.meta[p];
         uint32_t depth = meta & 0xffu, k = meta >> 8;
         uint32_t r = b.slot_req[p], pix = b.slot_pix[p];
@@ -617,15 +593,13 @@ cudaError_t bwave_capture_body(cudaStream_t s, int trace_blocks, int shade_block
                                const vgk::Wave& w, cudaGraphConditionalHandle loop, bool condition)
 {
     for (uint32_t wave = 0; wave < 2; wave++) {
-        bw_extend<<<trace_blocks, 128, 0, s>>>(b, w, wave);
-        bw_classify<<<sms * 4, 256, 0, s>>>(b, w, wave);
+        bw_trace<<<trace_blocks, 128, 0, s>>>(b, w, wave);
+        bw_resolve<<<sms * 4, 256, 0, s>>>(b, w, wave);
+        if (b.ncache)
+            bw_answer<<<sms * 2, 128, ANSWER_SMEM, s>>>(b, wave ^ 1u);
         bw_shade<false><<<shade_blocks, 128, 0, s>>>(b, w, wave);
         if (b.ncache)
             bw_shade<true><<<shade_blocks, 128, 0, s>>>(b, w, wave);
-        bw_shadow_trace<<<trace_blocks, 128, 0, s>>>(b, w, wave);
-        bw_finish<<<trace_blocks, 128, 0, s>>>(b, w, wave);
-        if (b.ncache)
-            bw_answer<<<sms * 2, 128, ANSWER_SMEM, s>>>(b);
     }
     if (condition)
         bw_condition<<<1, 1, 0, s>>>(b, w, loop);
@@ -644,7 +618,7 @@ void bwave_blocks_per_sm(int* trace, int* shade)
 {
     static int t = -1, sh = -1;
     if (t < 0) {
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&t, bw_extend, 128, 0) != cudaSuccess || t < 1)
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&t, bw_trace, 128, 0) != cudaSuccess || t < 1)
             t = 1;
         if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&sh, bw_shade<true>, 128, 0) != cudaSuccess || sh < 1)
             sh = 1;

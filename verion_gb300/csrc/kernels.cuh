@@ -109,14 +109,50 @@ __device__ __forceinline__ void block_append(uint32_t* count, uint32_t* queue, b
         queue[slot[warp] + __popc(b & ((1u << lane) - 1u))] = value;
 }
 
-// Block-wide work fetch: blockDim.x consecutive items per atomic (thread 0 takes them, a barrier
-// hands them out). `word` is one word of shared memory.
-static __device__ __forceinline__ uint32_t block_fetch(uint32_t* counter, uint32_t* word)
+// block_append to a queue (the `live` threads) and, in the same pass, to one of CLASSES more (threads with
+// cls < CLASSES): queue k at squeue + k n, counter counts[k]. One atomic per queue and block; warp q
+// scans the warps' counts of queues q, q + WARPS, .... `slot` is WARPS (1 + CLASSES) words of shared
+// memory; it may be used again at once after the call.
+template <uint32_t WARPS, uint32_t CLASSES>
+__device__ __forceinline__ void block_append_classes(uint32_t* count, uint32_t* queue, bool live, uint32_t* counts,
+                                                     uint32_t* squeue, uint32_t n, uint32_t cls, uint32_t value,
+                                                     uint32_t* slot)
 {
-    if (threadIdx.x == 0)
-        *word = atomicAdd(counter, blockDim.x);
+    uint32_t lane = lane_id(), warp = threadIdx.x >> 5, lt = (1u << lane) - 1u;
+    uint32_t mine = __ballot_sync(FULL, live), own = 0;
+    if (lane == 0)
+        slot[warp] = __popc(mine);
+#pragma unroll
+    for (uint32_t k = 0; k < CLASSES; k++) {
+        uint32_t b = __ballot_sync(FULL, cls == k);
+        if (lane == 0)
+            slot[(1 + k) * WARPS + warp] = __popc(b);
+        own = cls == k ? b : own;
+    }
     __syncthreads();
-    return *word;
+    for (uint32_t q = warp; q < 1 + CLASSES; q += WARPS) {
+        uint32_t v = lane < WARPS ? slot[q * WARPS + lane] : 0u;
+        uint32_t incl = v;
+#pragma unroll
+        for (uint32_t o = 1; o < WARPS; o <<= 1) {
+            uint32_t t = __shfl_up_sync(FULL, incl, o);
+            if (lane >= o)
+                incl += t;
+        }
+        uint32_t total = __shfl_sync(FULL, incl, WARPS - 1);
+        uint32_t first = 0;
+        if (lane == 0 && total)
+            first = atomicAdd(q == 0 ? count : counts + q - 1, total);
+        first = __shfl_sync(FULL, first, 0);
+        if (lane < WARPS)
+            slot[q * WARPS + lane] = first + incl - v;
+    }
+    __syncthreads();
+    if (live)
+        queue[slot[warp] + __popc(mine & lt)] = value;
+    if (CLASSES > 0 && cls < CLASSES)
+        squeue[(size_t)cls * n + slot[(1 + cls) * WARPS + warp] + __popc(own & lt)] = value;
+    __syncthreads();
 }
 
 template <bool LIGHT>
@@ -644,17 +680,14 @@ template <typename A, bool RESTIR = false, bool SORT = false>
 __global__ void __launch_bounds__(256) wf_stream_resolve(const __grid_constant__ Ctx c, const __grid_constant__ Wave w,
                                                          uint32_t wave)
 {
-    constexpr uint32_t WARPS = 8, QUEUES = SORT ? SHADE_CLASSES + 1 : 1;
-    __shared__ uint32_t slot[WARPS * QUEUES];
+    __shared__ uint32_t slot[8 * (1 + (SORT ? SHADE_CLASSES : 0))];
     uint32_t in = wave & 1u, out = in ^ 1u;
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         w.fetch[out] = 0;
         w.shcount[out] = 0;
     }
-    uint32_t count = w.counts[in], n = w.n;
+    uint32_t count = w.counts[in];
     const uint32_t* qin = w.queue[in];
-    uint32_t* qout = w.queue[out];
-    uint32_t lane = lane_id(), warp = threadIdx.x >> 5, lt = (1u << lane) - 1u;
     uint32_t stride = gridDim.x * blockDim.x;
     for (uint32_t base = blockIdx.x * blockDim.x; base < count; base += stride) {
         uint32_t i = base + threadIdx.x;
@@ -667,45 +700,8 @@ __global__ void __launch_bounds__(256) wf_stream_resolve(const __grid_constant__
             if (SORT && live)
                 cls = shadeClass(c, w.hits[p]);
         }
-        // Queue 0 is the next wave's, queue 1 + k the shading class k's. Warp q's lanes scan queue q's counts.
-        uint32_t mine = __ballot_sync(FULL, live);
-        if (lane == 0)
-            slot[warp] = __popc(mine);
-        uint32_t own = 0;
-        if (SORT) {
-#pragma unroll
-            for (uint32_t k = 0; k < SHADE_CLASSES; k++) {
-                uint32_t b = __ballot_sync(FULL, cls == k);
-                if (lane == 0)
-                    slot[(1 + k) * WARPS + warp] = __popc(b);
-                own = cls == k ? b : own;
-            }
-        }
-        __syncthreads();
-        if (warp < QUEUES) {
-            uint32_t v = lane < WARPS ? slot[warp * WARPS + lane] : 0u;
-            uint32_t incl = v;
-#pragma unroll
-            for (uint32_t o = 1; o < WARPS; o <<= 1) {
-                uint32_t t = __shfl_up_sync(FULL, incl, o);
-                if (lane >= o)
-                    incl += t;
-            }
-            uint32_t total = __shfl_sync(FULL, incl, WARPS - 1);
-            uint32_t first = 0;
-            if (lane == 0 && total)
-                first = atomicAdd(warp == 0 ? &w.counts[out] : &w.scount[in * SHADE_CLASSES + warp - 1], total);
-            first = __shfl_sync(FULL, first, 0);
-            if (lane < WARPS)
-                slot[warp * WARPS + lane] = first + incl - v;
-        }
-        __syncthreads();
-        if (live) {
-            qout[slot[warp] + __popc(mine & lt)] = p;
-            if (SORT)
-                w.squeue[(size_t)cls * n + slot[(1 + cls) * WARPS + warp] + __popc(own & lt)] = p;
-        }
-        __syncthreads();
+        block_append_classes<8, SORT ? SHADE_CLASSES : 0>(&w.counts[out], w.queue[out], live,
+                                                          w.scount + in * SHADE_CLASSES, w.squeue, w.n, cls, p, slot);
     }
 }
 

@@ -623,7 +623,7 @@ __device__ __forceinline__ void trace_queue_impl(const uint4* __restrict__ nodes
                     float tmax;
                     bool ok;
                     if constexpr (SCENES)
-                        ok = get(idx, o, d, tmax, nodes, tris);
+                        ok = get(idx, o, d, tmax, w.any, nodes, tris);
                     else
                         ok = get(idx, o, d, tmax, w.any);
                     if (ok) {
@@ -662,13 +662,13 @@ __device__ __forceinline__ void trace_queue(const uint4* __restrict__ nodes, con
     trace_queue_impl<H, false>(nodes, tris, fetch, count, err, refill, steps, get, put);
 }
 
-// trace_queue over the rays of several scenes: get(idx, o, d, tmax, nodes, tris) also sets the
+// trace_queue over the rays of several scenes: get(idx, o, d, tmax, any, nodes, tris) also sets the
 // ray's BVH arrays.
-template <bool ANY, typename GetRay, typename PutHit>
+template <Hits H, typename GetRay, typename PutHit>
 __device__ __forceinline__ void trace_queue_scenes(uint32_t* fetch, uint32_t count, uint32_t* err, uint32_t refill,
                                                    uint32_t steps, GetRay get, PutHit put)
 {
-    trace_queue_impl<ANY ? HITS_ANY : HITS_CLOSEST, true>(nullptr, nullptr, fetch, count, err, refill, steps, get, put);
+    trace_queue_impl<H, true>(nullptr, nullptr, fetch, count, err, refill, steps, get, put);
 }
 
 } // namespace vgt
