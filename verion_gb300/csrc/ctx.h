@@ -76,6 +76,8 @@ namespace vgk {
 constexpr uint32_t BASE_PLANES = 4;  // 16-byte state planes per path
 constexpr uint32_t SHADE_CLASSES = 4; // material-sorted shading: missed, diffuse, conductor, dielectric
 constexpr uint32_t SPLIT_PLANES = 5; // more planes with the lighting split
+constexpr uint32_t REQ_PLANES = 3;       // shadow request planes per slot (Wave::sreq)
+constexpr uint32_t SPLIT_REQ_PLANES = 5; // ... with the lighting split
 
 // Wave::flags of a path slot.
 constexpr uint32_t SLOT_RAY = 1u;     // its path has a ray to trace and shade
@@ -91,7 +93,7 @@ struct Wave {
     uint32_t* counts;  // live paths per depth, max depth + 1 entries
     uint32_t* fetch;   // work counters: extend of depth d at [d], shade at [(D + 1) + d]
     unsigned long long* tstats; // traversal counters: rays, nodes, triangle tests, rays past depth 0
-    float4* sreq;      // streaming mode, deferred shadow requests: 3 planes of float4 per slot
+    float4* sreq;      // streaming mode, deferred shadow requests: REQ_PLANES planes of float4 per slot
     uint32_t* meta;    // streaming mode: per path slot, depth (bits 0-7) and sample within the batch (8+)
     uint32_t n;        // paths: one per pixel
     uint32_t depth;    // max depth
@@ -102,8 +104,8 @@ struct Wave {
     uint32_t* squeue;
     uint32_t* scount;
     // Deferred shadows (flags null without them): what each slot still has in flight (SLOT_* bits), the
-    // radiance of a slot's path that has ended and waits for its last shadow ray, and the slots with a
-    // shadow ray, shcount[parity] of them.
+    // radiance of a slot's path that has ended and waits for its last shadow ray (with the lighting split
+    // as in the state planes 3 to 8), and the slots with a shadow ray, shcount[parity] of them.
     uint32_t* flags;
     float4* pend;
     uint32_t* shqueue;

@@ -208,8 +208,9 @@ struct VgRenderer {
     int extend_blocks = 0;
     int shade_blocks[8] = {};
     int stream_shade_blocks[8] = {};
-    int deferred_blocks[2] = {};
-    int deferred_restir_blocks[2] = {};
+    int deferred_blocks = 0;
+    int deferred_restir_blocks = 0;
+    int deferred_light_blocks = 0;
     bool defer_shadows = true; // streaming: shadow rays of the light sample in their own stage
     bool dynamic_fetch = true; // streaming: traversal stages refill idle lanes from the queue
     bool coop_tris = false;    // streaming, dynamic fetch: warp-cooperative leaf testing (measured slower)
@@ -227,7 +228,7 @@ struct VgRenderer {
     uint32_t cache_batch = 16384;
     uint32_t cache_frame = 4;     // integrator WAVEFRONT: samples per cache frame (one cache update per frame)
     uint32_t cache_warmup = 0;    // training-only frames before the first sample of an accumulation
-    int cache_shade_blocks[2] = {};
+    int cache_shade_blocks = 0;
 };
 
 struct VgAccum {

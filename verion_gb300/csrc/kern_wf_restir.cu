@@ -41,34 +41,31 @@ int stream_shade_restir_blocks_per_sm(Variant v)
     return rshade_occ<false, float>();
 }
 
-cudaError_t launch_stream_tail_restir(Variant v, uint32_t max_slots, cudaStream_t s, const vgd::Ctx& c,
+cudaError_t launch_stream_tail_restir(Variant v, uint32_t max_slots, int sms, cudaStream_t s, const vgd::Ctx& c,
                                       const vgk::Wave& w, uint32_t wave)
 {
-    unsigned blocks = (max_slots + 127) / 128;
+    uint32_t lanes = 0;
+    unsigned blocks = tail_blocks(max_slots, sms, &lanes);
     if (blocks == 0)
         return cudaSuccess;
     if (v.light && v.f64)
-        vgk::wf_stream_tail<true, double, false, true><<<blocks, 128, 0, s>>>(c, w, wave, vgk::CacheWave{});
+        vgk::wf_stream_tail<true, double, false, true><<<blocks, 128, 0, s>>>(c, w, wave, lanes, vgk::CacheWave{});
     else if (v.light)
-        vgk::wf_stream_tail<true, float, false, true><<<blocks, 128, 0, s>>>(c, w, wave, vgk::CacheWave{});
+        vgk::wf_stream_tail<true, float, false, true><<<blocks, 128, 0, s>>>(c, w, wave, lanes, vgk::CacheWave{});
     else if (v.f64)
-        vgk::wf_stream_tail<false, double, false, true><<<blocks, 128, 0, s>>>(c, w, wave, vgk::CacheWave{});
+        vgk::wf_stream_tail<false, double, false, true><<<blocks, 128, 0, s>>>(c, w, wave, lanes, vgk::CacheWave{});
     else
-        vgk::wf_stream_tail<false, float, false, true><<<blocks, 128, 0, s>>>(c, w, wave, vgk::CacheWave{});
+        vgk::wf_stream_tail<false, float, false, true><<<blocks, 128, 0, s>>>(c, w, wave, lanes, vgk::CacheWave{});
     return cudaGetLastError();
 }
 
-cudaError_t launch_stream_shade_deferred_restir(bool f64, bool sorted, int blocks, cudaStream_t s, const vgd::Ctx& c,
+cudaError_t launch_stream_shade_deferred_restir(bool sorted, int blocks, cudaStream_t s, const vgd::Ctx& c,
                                                 const vgk::Wave& w, uint32_t wave)
 {
-    if (f64 && sorted)
-        vgk::wf_stream_shade_deferred<double, false, true, true><<<blocks, 128, 0, s>>>(c, w, wave, vgk::CacheWave{});
-    else if (f64)
-        vgk::wf_stream_shade_deferred<double, false, true><<<blocks, 128, 0, s>>>(c, w, wave, vgk::CacheWave{});
-    else if (sorted)
-        vgk::wf_stream_shade_deferred<float, false, true, true><<<blocks, 128, 0, s>>>(c, w, wave, vgk::CacheWave{});
+    if (sorted)
+        vgk::wf_stream_shade_deferred<false, true, true><<<blocks, 128, 0, s>>>(c, w, wave, vgk::CacheWave{});
     else
-        vgk::wf_stream_shade_deferred<float, false, true><<<blocks, 128, 0, s>>>(c, w, wave, vgk::CacheWave{});
+        vgk::wf_stream_shade_deferred<false, true><<<blocks, 128, 0, s>>>(c, w, wave, vgk::CacheWave{});
     return cudaGetLastError();
 }
 
@@ -86,13 +83,10 @@ cudaError_t launch_stream_resolve_restir(bool f64, bool sorted, int blocks, cuda
     return cudaGetLastError();
 }
 
-int stream_deferred_restir_blocks_per_sm(bool f64)
+int stream_deferred_restir_blocks_per_sm()
 {
     int n = 0;
-    if (f64)
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, vgk::wf_stream_shade_deferred<double, false, true, true>, 128, 0);
-    else
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, vgk::wf_stream_shade_deferred<float, false, true, true>, 128, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, vgk::wf_stream_shade_deferred<false, true, true>, 128, 0);
     return n > 0 ? n : 1;
 }
 

@@ -155,6 +155,18 @@ __device__ __forceinline__ void block_append_classes(uint32_t* count, uint32_t* 
     __syncthreads();
 }
 
+// The split's five planes of slot p.
+template <bool LIGHT>
+__device__ __forceinline__ void store_split(float4* planes, size_t n, const PathState<LIGHT>& s, uint32_t p)
+{
+    const Parts<LIGHT>& q = s.parts;
+    planes[p] = make_float4(q.directDiffuse.x, q.directDiffuse.y, q.directDiffuse.z, s.visLit);
+    planes[n + p] = make_float4(q.indirectDiffuse.x, q.indirectDiffuse.y, q.indirectDiffuse.z, s.visTotal);
+    planes[2 * n + p] = make_float4(q.specular.x, q.specular.y, q.specular.z, 0.0f);
+    planes[3 * n + p] = make_float4(q.transmission.x, q.transmission.y, q.transmission.z, 0.0f);
+    planes[4 * n + p] = make_float4(q.emission.x, q.emission.y, q.emission.z, 0.0f);
+}
+
 template <bool LIGHT>
 __device__ __forceinline__ void storePath(const Wave& w, const PathState<LIGHT>& s, uint32_t p)
 {
@@ -165,14 +177,8 @@ __device__ __forceinline__ void storePath(const Wave& w, const PathState<LIGHT>&
     w.state[n + p] = make_float4(s.dir.x, s.dir.y, s.dir.z, __uint_as_float(flags));
     w.state[2 * n + p] = make_float4(s.thr.x, s.thr.y, s.thr.z, s.pathLen);
     w.state[3 * n + p] = make_float4(s.parts.total.x, s.parts.total.y, s.parts.total.z, s.qPrev);
-    if (LIGHT) {
-        const Parts<LIGHT>& q = s.parts;
-        w.state[4 * n + p] = make_float4(q.directDiffuse.x, q.directDiffuse.y, q.directDiffuse.z, s.visLit);
-        w.state[5 * n + p] = make_float4(q.indirectDiffuse.x, q.indirectDiffuse.y, q.indirectDiffuse.z, s.visTotal);
-        w.state[6 * n + p] = make_float4(q.specular.x, q.specular.y, q.specular.z, 0.0f);
-        w.state[7 * n + p] = make_float4(q.transmission.x, q.transmission.y, q.transmission.z, 0.0f);
-        w.state[8 * n + p] = make_float4(q.emission.x, q.emission.y, q.emission.z, 0.0f);
-    }
+    if (LIGHT)
+        store_split(w.state + 4 * (size_t)n, n, s, p);
 }
 
 // wf_state.slang:60-92. Depth 0 keeps no state: the camera path is generated again.
@@ -621,10 +627,59 @@ __global__ void __launch_bounds__(128, VG_SHADE_MIN_BLOCKS) wf_stream_shade(cons
 // What a slot's shadow ray (SLOT_SHADOW) decides once it is traced, in the order of the pixel's samples:
 // its contribution is the last add of the vertex that asked for it. Returns whether the slot still has
 // a path to go on with.
-template <typename A, bool RESTIR>
+template <typename A, bool RESTIR, bool LIGHT = false>
 __device__ __forceinline__ bool resolveSlot(const Ctx& c, const Wave& w, uint32_t p, uint32_t fl, bool blocked)
 {
     uint32_t n = w.n;
+    if constexpr (LIGHT) {
+        if (!(fl & (SLOT_ENDED | SLOT_SHADOW)))
+            return (fl & SLOT_RAY) != 0;
+        // The path's parts, in the order of the state planes 3 to 8.
+        float4* P = (fl & SLOT_ENDED) ? w.pend : w.state + 3 * (size_t)n;
+        float4 q[6];
+#pragma unroll
+        for (uint32_t k = 0; k < 6; k++)
+            q[k] = P[k * (size_t)n + p];
+        PathState<true> st;
+        st.parts.total = v3(q[0].x, q[0].y, q[0].z);
+        st.parts.directDiffuse = v3(q[1].x, q[1].y, q[1].z);
+        st.visLit = q[1].w;
+        st.parts.indirectDiffuse = v3(q[2].x, q[2].y, q[2].z);
+        st.visTotal = q[2].w;
+        st.parts.specular = v3(q[3].x, q[3].y, q[3].z);
+        st.parts.transmission = v3(q[4].x, q[4].y, q[4].z);
+        st.parts.emission = v3(q[5].x, q[5].y, q[5].z);
+        if (fl & SLOT_SHADOW) {
+            float4 r1 = w.sreq[n + p], r2 = w.sreq[2 * n + p], r3 = w.sreq[3 * (size_t)n + p],
+                   r4 = w.sreq[4 * (size_t)n + p];
+            V3 cd = v3(r3.x, r3.y, r3.z), cs = v3(r4.x, r4.y, r4.z);
+            float cosi = r3.w;
+            uint32_t bits = __float_as_uint(r4.w);
+            bool first = (bits & 1u) != 0;
+            if (!blocked)
+                st.parts.addLight(first ? 0u : 1u, (bits >> 1) & 3u, v3(r2.x, r2.y, r2.z), cd, cs);
+            if (first) {
+                float vv = lum(cd + cs);
+                st.visTotal += vv;
+                st.visLit += blocked ? 0.0f : vv;
+                if (bits & 8u)
+                    addSlot(c, p, 3u, cd / cosi, cs / cosi, v3(r1.x, r1.y, r1.z), blocked ? 0.0f : 1.0f, blocked ? 0.0f : cosi);
+            }
+        }
+        if (fl & SLOT_ENDED) {
+            st.gi = false;
+            st.chan = -1;
+            finishPath<true, A, RESTIR>(c, st, p);
+            return (fl & SLOT_RAY) && (c.p[P_ADAPTIVE] == 0 || pixelActive<A>(c, p));
+        }
+        const Parts<true>& t = st.parts;
+        P[p] = make_float4(t.total.x, t.total.y, t.total.z, q[0].w);
+        P[n + p] = make_float4(t.directDiffuse.x, t.directDiffuse.y, t.directDiffuse.z, st.visLit);
+        P[2 * (size_t)n + p] = make_float4(t.indirectDiffuse.x, t.indirectDiffuse.y, t.indirectDiffuse.z, st.visTotal);
+        P[3 * (size_t)n + p] = make_float4(t.specular.x, t.specular.y, t.specular.z, 0.0f);
+        P[4 * (size_t)n + p] = make_float4(t.transmission.x, t.transmission.y, t.transmission.z, 0.0f);
+        return (fl & SLOT_RAY) != 0;
+    }
     bool lit = (fl & SLOT_SHADOW) && !blocked;
     if (fl & SLOT_ENDED) {
         float4 t = w.pend[p];
@@ -668,7 +723,7 @@ static __device__ __forceinline__ uint32_t shadeClass(const Ctx& c, uint4 hr)
     return fget(c.s.materials, mi + 6) >= 0.5f ? 2u : 1u;
 }
 
-// Between trace and shade (lighting split off, deferred shadows): what the wave's rays brought each slot
+// Between trace and shade (deferred shadows): what the wave's rays brought each slot
 // of its queue. A shadow ray that got through adds its contribution, to the slot's path or, when that
 // path ended at the vertex, to its radiance in w.pend, which then goes to the pixel's sums; adaptive
 // sampling decides from them whether the slot's next sample, whose camera ray was traced meanwhile, is
@@ -676,7 +731,7 @@ static __device__ __forceinline__ uint32_t shadeClass(const Ctx& c, uint4 hr)
 // to the queue of its hit's shading class, so that the shade stage's warps mostly run one BSDF's code.
 // One pass and one atomic per queue and 256 slots: as two kernels (classify with up to four atomics a
 // warp, 61 us per wave of about a million slots, and finish, 69 us) it was a seventh of the wave.
-template <typename A, bool RESTIR = false, bool SORT = false>
+template <typename A, bool RESTIR = false, bool SORT = false, bool LIGHT = false>
 __global__ void __launch_bounds__(256) wf_stream_resolve(const __grid_constant__ Ctx c, const __grid_constant__ Wave w,
                                                          uint32_t wave)
 {
@@ -696,7 +751,7 @@ __global__ void __launch_bounds__(256) wf_stream_resolve(const __grid_constant__
         if (i < count) {
             p = qin[i];
             uint32_t fl = w.flags[p];
-            live = resolveSlot<A, RESTIR>(c, w, p, fl, (fl & SLOT_BLOCKED) != 0);
+            live = resolveSlot<A, RESTIR, LIGHT>(c, w, p, fl, (fl & SLOT_BLOCKED) != 0);
             if (SORT && live)
                 cls = shadeClass(c, w.hits[p]);
         }
@@ -705,7 +760,7 @@ __global__ void __launch_bounds__(256) wf_stream_resolve(const __grid_constant__
     }
 }
 
-// Streaming wave in three stages (lighting split off): trace, resolve, then shade without any traversal.
+// Streaming wave in three stages: trace, resolve, then shade without any traversal.
 // Shade leaves its emitter / environment light sample as a request of the slot (w.sreq planes: origin +
 // tmax, direction, contribution) in the shadow queue; the next wave traces it along with the slot's next
 // ray, and the resolve stage adds the contribution when it is unoccluded. A path that ends leaves its
@@ -713,7 +768,7 @@ __global__ void __launch_bounds__(256) wf_stream_resolve(const __grid_constant__
 // With CACHE a path also ends where its spread passes the cache threshold (shadePath's cache
 // hook); it then leaves a query record (one atomic per warp) and finishes like any other.
 // With SORTED the wave's slots are taken class by class from the resolve stage's queues.
-template <typename A, bool CACHE = false, bool RESTIR = false, bool SORTED = false>
+template <bool CACHE = false, bool RESTIR = false, bool SORTED = false, bool LIGHT = false>
 __global__ void __launch_bounds__(128, RESTIR ? VG_RESTIR_SHADE_MIN_BLOCKS : VG_SHADE_MIN_BLOCKS) wf_stream_shade_deferred(const __grid_constant__ Ctx c,
                                                                                     const __grid_constant__ Wave w, uint32_t wave,
                                                                                     CacheWave q)
@@ -745,7 +800,7 @@ __global__ void __launch_bounds__(128, RESTIR ? VG_RESTIR_SHADE_MIN_BLOCKS : VG_
             uint32_t meta = w.meta[p];
             uint32_t depth = meta & 0xffu;
             kq = meta >> 8;
-            PathState<false> st = loadState<false>(w, p);
+            PathState<LIGHT> st = loadState<LIGHT>(w, p);
             uint4 hr = w.hits[p];
             Hit h;
             h.hit = hr.x != 0;
@@ -762,7 +817,7 @@ __global__ void __launch_bounds__(128, RESTIR ? VG_RESTIR_SHADE_MIN_BLOCKS : VG_
                 hk.a0 = sp.x;
                 hk.a = sp.y;
             }
-            bool alive = shadePath<false, RESTIR, true, CACHE>(c, st, h, depth, p, &req, &hk) && depth + 1 < w.depth;
+            bool alive = shadePath<LIGHT, RESTIR, true, CACHE>(c, st, h, depth, p, &req, &hk) && depth + 1 < w.depth;
             if (CACHE) {
                 query = hk.query && !bad3(st.parts.total);
                 if (alive)
@@ -773,21 +828,27 @@ __global__ void __launch_bounds__(128, RESTIR ? VG_RESTIR_SHADE_MIN_BLOCKS : VG_
                 w.meta[p] = (depth + 1) | (kq << 8);
             } else {
                 w.pend[p] = make_float4(st.parts.total.x, st.parts.total.y, st.parts.total.z, 0.0f);
+                if (LIGHT)
+                    store_split(w.pend + n, n, st, p);
                 fl = SLOT_ENDED;
                 if (kq + 1 < batch) {
                     fl |= SLOT_RAY;
-                    st = generatePathFor<false>(c, p % c.p[P_WIDTH], p / c.p[P_WIDTH], c.p[P_SAMPLE] + kq + 1);
+                    st = generatePathFor<LIGHT>(c, p % c.p[P_WIDTH], p / c.p[P_WIDTH], c.p[P_SAMPLE] + kq + 1);
                     w.meta[p] = (kq + 1) << 8;
                 }
             }
             if (fl & SLOT_RAY)
-                storePath<false>(w, st, p);
+                storePath<LIGHT>(w, st, p);
             shadow = req.valid;
             if (shadow) {
                 fl |= SLOT_SHADOW;
                 w.sreq[p] = make_float4(req.o.x, req.o.y, req.o.z, req.tmax);
                 w.sreq[n + p] = make_float4(req.d.x, req.d.y, req.d.z, 0.0f);
                 w.sreq[2 * n + p] = make_float4(req.c.x, req.c.y, req.c.z, 0.0f);
+                if (LIGHT) {
+                    w.sreq[3 * (size_t)n + p] = make_float4(req.cd.x, req.cd.y, req.cd.z, req.cosi);
+                    w.sreq[4 * (size_t)n + p] = make_float4(req.cs.x, req.cs.y, req.cs.z, __uint_as_float(req.bits));
+                }
             }
             w.flags[p] = fl;
         }
@@ -979,15 +1040,16 @@ __global__ void __launch_bounds__(128, VG_TRACE_MIN_BLOCKS) wf_stream_shadow_tra
 // With CACHE (lighting split off) paths end at the cache as in wf_stream_shade_deferred.
 template <bool LIGHT, typename A, bool CACHE = false, bool RESTIR = false>
 __global__ void __launch_bounds__(128, VG_TAIL_MIN_BLOCKS) wf_stream_tail(const __grid_constant__ Ctx c, const __grid_constant__ Wave w,
-                                                                          uint32_t wave, CacheWave q)
+                                                                          uint32_t wave, uint32_t lanes,
+                                                                          const __grid_constant__ CacheWave q)
 {
     static_assert(!(CACHE && LIGHT), "the cache runs with the lighting split off");
     uint32_t in = wave & 1u;
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= w.counts[in])
+    uint32_t i = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * lanes + lane_id();
+    if (lane_id() >= lanes || i >= w.counts[in])
         return;
     uint32_t p = w.queue[in][i];
-    if (!LIGHT && w.flags) {
+    if (w.flags) {
         // A wave's shadow ray is still to be traced, and the path before this one may wait for it.
         uint32_t fl = w.flags[p];
         bool blocked = false;
@@ -997,7 +1059,7 @@ __global__ void __launch_bounds__(128, VG_TAIL_MIN_BLOCKS) wf_stream_tail(const 
             slot_shadow_ray(w, p, o, d, tmax);
             blocked = occluded(c, o, d, tmax);
         }
-        if (!resolveSlot<A, RESTIR>(c, w, p, fl, blocked))
+        if (!resolveSlot<A, RESTIR, LIGHT>(c, w, p, fl, blocked))
             return;
     }
     uint32_t meta = w.meta[p];

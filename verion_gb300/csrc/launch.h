@@ -36,14 +36,14 @@ int stream_shade_blocks_per_sm(Variant v);
 // Three-stage wave (lighting split off): shade without traversal, then the shadow stage.
 cudaError_t launch_stream_cache_start(bool f64, cudaStream_t s, const vgd::Ctx& c, const vgk::Wave& w,
                                       const vgk::CacheWave& q);
-cudaError_t launch_stream_cache_shade(bool f64, bool sorted, int blocks, cudaStream_t s, const vgd::Ctx& c,
+cudaError_t launch_stream_cache_shade(bool sorted, int blocks, cudaStream_t s, const vgd::Ctx& c,
                                       const vgk::Wave& w, uint32_t wave, const vgk::CacheWave& q);
-int stream_cache_shade_blocks_per_sm(bool f64);
-cudaError_t launch_stream_cache_tail(bool f64, uint32_t max_slots, cudaStream_t s, const vgd::Ctx& c,
+int stream_cache_shade_blocks_per_sm();
+cudaError_t launch_stream_cache_tail(bool f64, uint32_t max_slots, int sms, cudaStream_t s, const vgd::Ctx& c,
                                      const vgk::Wave& w, uint32_t wave, const vgk::CacheWave& q);
 // With `sorted` the resolve stage also fills the class queues and the shade stage takes the wave's slots
 // class by class.
-cudaError_t launch_stream_shade_deferred(bool f64, bool sorted, int blocks, cudaStream_t s, const vgd::Ctx& c,
+cudaError_t launch_stream_shade_deferred(bool sorted, int blocks, cudaStream_t s, const vgd::Ctx& c,
                                          const vgk::Wave& w, uint32_t wave);
 cudaError_t launch_stream_resolve(bool f64, bool sorted, int blocks, cudaStream_t s, const vgd::Ctx& c,
                                   const vgk::Wave& w, uint32_t wave);
@@ -51,7 +51,7 @@ int stream_resolve_blocks_per_sm(bool f64);
 cudaError_t launch_stream_shadow_layers(int blocks, cudaStream_t s, const vgd::Ctx& c, const vgk::Wave& w,
                                         uint32_t wave);
 int stream_shadow_layers_blocks_per_sm();
-int stream_deferred_blocks_per_sm(bool f64);
+int stream_deferred_blocks_per_sm();
 // Dynamic-fetch traversal stages: a wave's path and shadow rays in one launch, or each in its own.
 // With `coop` the warp-cooperative leaf testing of traverse.cuh (the same hits).
 cudaError_t launch_stream_trace(int blocks, cudaStream_t s, const vgd::Ctx& c, const vgk::Wave& w, uint32_t wave);
@@ -66,15 +66,23 @@ int stream_shadow_trace_blocks_per_sm();
 cudaError_t launch_stream_shade_restir(Variant v, int blocks, cudaStream_t s, const vgd::Ctx& c, const vgk::Wave& w,
                                        uint32_t wave);
 int stream_shade_restir_blocks_per_sm(Variant v);
-cudaError_t launch_stream_tail_restir(Variant v, uint32_t max_slots, cudaStream_t s, const vgd::Ctx& c,
+cudaError_t launch_stream_tail_restir(Variant v, uint32_t max_slots, int sms, cudaStream_t s, const vgd::Ctx& c,
                                       const vgk::Wave& w, uint32_t wave);
-cudaError_t launch_stream_shade_deferred_restir(bool f64, bool sorted, int blocks, cudaStream_t s, const vgd::Ctx& c,
+cudaError_t launch_stream_shade_deferred_restir(bool sorted, int blocks, cudaStream_t s, const vgd::Ctx& c,
                                                 const vgk::Wave& w, uint32_t wave);
-int stream_deferred_restir_blocks_per_sm(bool f64);
+int stream_deferred_restir_blocks_per_sm();
 cudaError_t launch_stream_resolve_restir(bool f64, bool sorted, int blocks, cudaStream_t s, const vgd::Ctx& c,
                                          const vgk::Wave& w, uint32_t wave);
+// Blocks of the tail over at most max_slots slots, and how many slots each of its warps takes.
+unsigned tail_blocks(uint32_t max_slots, int sms, uint32_t* lanes);
+// The deferred stages with the lighting split (kern_wf_light.cu).
+cudaError_t launch_stream_shade_deferred_light(bool sorted, int blocks, cudaStream_t s, const vgd::Ctx& c,
+                                               const vgk::Wave& w, uint32_t wave);
+int stream_deferred_light_blocks_per_sm();
+cudaError_t launch_stream_resolve_light(bool f64, bool sorted, int blocks, cudaStream_t s, const vgd::Ctx& c,
+                                        const vgk::Wave& w, uint32_t wave);
 // Finishes every slot still live after `wave` (at most max_slots of them) in one launch.
-cudaError_t launch_stream_tail(Variant v, uint32_t max_slots, cudaStream_t s, const vgd::Ctx& c, const vgk::Wave& w,
+cudaError_t launch_stream_tail(Variant v, uint32_t max_slots, int sms, cudaStream_t s, const vgd::Ctx& c, const vgk::Wave& w,
                                uint32_t wave);
 // Primary-hit AOVs (normals.slang, aov.slang); camera18 is the reference's camera record.
 cudaError_t launch_aov_normals(cudaStream_t s, const vgd::Ctx& c, const float* camera18, float* out);

@@ -985,12 +985,23 @@ struct ShadowReq {
     V3 o, d;
     float tmax;
     V3 c;
+    // With the lighting split: the diffuse and specular parts of c, the cosine at the vertex, and whether
+    // the sample goes to the first hit's light slot (splitBits).
+    V3 cd, cs;
+    float cosi;
+    uint32_t bits;
 };
 
+// ShadowReq::bits: the sample's vertex is the path's first (bit 0), else the path's class (bits 1-2), and
+// whether its light has a slot (bit 3; a virtual environment light has none).
+static __device__ __forceinline__ uint32_t splitBits(uint32_t depth, uint32_t cls, bool slot)
+{
+    return (depth == 0 ? 1u : 0u) | (cls << 1) | (slot ? 8u : 0u);
+}
+
 // pt_core.slang:992-1543: one bounce at `depth`. Returns false when the path ends here.
-// DEFER (lighting split off only): the emitter / environment sample is not traced here but
-// returned in *req; it is the last contribution of the bounce, so adding it afterwards keeps the
-// order of the sums.
+// DEFER: the emitter / environment sample is not traced here but returned in *req; it is the last
+// contribution of the bounce, so adding it afterwards keeps the order of the sums.
 // Radiance-cache hook of shadePath (no reference counterpart). At every surface vertex the
 // path reaches (after that vertex's emission is added, before its light sampling) the hook
 // records the cache inputs, the throughput and the path radiance so far, and grows the path
@@ -1041,7 +1052,6 @@ template <bool LIGHT, bool RESTIR, bool DEFER = false, bool CACHE = false>
 __device__ __forceinline__ bool shadePath(const Ctx& c, PathState<LIGHT>& st, Hit hq, uint32_t depth, uint32_t pixel,
                           ShadowReq* req = nullptr, CacheHook* hk = nullptr)
 {
-    static_assert(!(DEFER && LIGHT), "deferred shadow rays need the lighting split off");
     if (DEFER)
         req->valid = false;
     if (CACHE) {
@@ -1405,6 +1415,12 @@ __device__ __forceinline__ bool shadePath(const Ctx& c, PathState<LIGHT>& st, Hi
                 req->d = wi;
                 req->tmax = dist * (1.0f - 1.0e-3f);
                 req->c = thr * (l.specular + l.diffuse) * lE / pl * wl;
+                if (LIGHT) {
+                    req->cd = thr * l.diffuse * lE / pl * wl;
+                    req->cs = thr * l.specular * lE / pl * wl;
+                    req->cosi = cosi;
+                    req->bits = splitBits(depth, cls, true);
+                }
             } else if (cosi > 0.0f && cosl > 1.0e-5f && (__float_as_uint(fget(E, e + 14)) & recvHere) != 0) {
                 bool occ = occluded(c, p, wi, dist * (1.0f - 1.0e-3f));
                 bool track = lightingOn && depth == 0;
@@ -1450,6 +1466,12 @@ __device__ __forceinline__ bool shadePath(const Ctx& c, PathState<LIGHT>& st, Hi
                 req->d = wi;
                 req->tmax = 1.0e30f;
                 req->c = thr * (l.specular + l.diffuse) * leE / pl * wl;
+                if (LIGHT) {
+                    req->cd = thr * l.diffuse * leE / pl * wl;
+                    req->cs = thr * l.specular * leE / pl * wl;
+                    req->cosi = cosi;
+                    req->bits = splitBits(depth, cls, c.p[P_VIRTUAL_LIGHT] == 0);
+                }
             } else if (pdfE > 0.0f && cosi > 0.0f) {
                 bool occ = occluded(c, p, wi, 1.0e30f);
                 bool track = lightingOn && depth == 0;

@@ -185,24 +185,22 @@ int stream_samples(VgRenderer* r, VgAccum* acc, vgd::Ctx& c, vgx::Variant v, con
     if (r->stream_shade_blocks[svi] == 0)
         r->stream_shade_blocks[svi] = vgx::stream_shade_blocks_per_sm(v);
     int ssb = blocks_for(r, r->stream_shade_blocks[svi]);
-    // Lighting split off: three-stage waves with the shadow rays in their own kernel.
+    // Three-stage waves, shadow rays traced apart from shading.
     // ReSTIR GI records the second vertex's direct light while shading it, so with GI the light
     // sample's shadow ray is traced inside shade.
-    bool deferred = (!acc->lighting && r->defer_shadows && !(v.restir && acc->restir.gi)) || q;
-    if (deferred && r->deferred_blocks[v.f64 ? 1 : 0] == 0)
-        r->deferred_blocks[v.f64 ? 1 : 0] = vgx::stream_deferred_blocks_per_sm(v.f64);
-    int dsb = blocks_for(r, r->deferred_blocks[v.f64 ? 1 : 0]);
-    if (deferred && v.restir) {
-        if (r->deferred_restir_blocks[v.f64 ? 1 : 0] == 0)
-            r->deferred_restir_blocks[v.f64 ? 1 : 0] = vgx::stream_deferred_restir_blocks_per_sm(v.f64);
-        dsb = blocks_for(r, r->deferred_restir_blocks[v.f64 ? 1 : 0]);
-    }
-    int csb = 0;
-    if (q) {
-        if (r->cache_shade_blocks[v.f64 ? 1 : 0] == 0)
-            r->cache_shade_blocks[v.f64 ? 1 : 0] = vgx::stream_cache_shade_blocks_per_sm(v.f64);
-        csb = blocks_for(r, r->cache_shade_blocks[v.f64 ? 1 : 0]);
-    }
+    // With ReSTIR the lighting split is shaded the same way.
+    bool deferred = (r->defer_shadows && !(v.restir && (acc->restir.gi || acc->lighting))) || q;
+    // Resident blocks of the deferred shade stage's form, asked for once.
+    auto resident = [&](int& n, int (*per_sm)()) {
+        if (n == 0)
+            n = per_sm();
+        return blocks_for(r, n);
+    };
+    int dsb = !deferred ? 0
+              : q       ? resident(r->cache_shade_blocks, vgx::stream_cache_shade_blocks_per_sm)
+              : v.light ? resident(r->deferred_light_blocks, vgx::stream_deferred_light_blocks_per_sm)
+              : v.restir ? resident(r->deferred_restir_blocks, vgx::stream_deferred_restir_blocks_per_sm)
+                         : resident(r->deferred_blocks, vgx::stream_deferred_blocks_per_sm);
     int stb = blocks_for(r, vgx::stream_shadow_trace_blocks_per_sm());
     int rvb = blocks_for(r, vgx::stream_resolve_blocks_per_sm(v.f64));
     // Material-sorted shading of the deferred shade stage (plain, ReSTIR and cache waves).
@@ -239,7 +237,9 @@ int stream_samples(VgRenderer* r, VgAccum* acc, vgd::Ctx& c, vgx::Variant v, con
                     return e;
                 acc->launches++;
             }
-            e = (v.restir ? vgx::launch_stream_resolve_restir : vgx::launch_stream_resolve)(v.f64, sorted, rvb, s, c, w, i);
+            e = (v.light    ? vgx::launch_stream_resolve_light
+                 : v.restir ? vgx::launch_stream_resolve_restir
+                            : vgx::launch_stream_resolve)(v.f64, sorted, rvb, s, c, w, i);
             if (e != cudaSuccess)
                 return e;
             acc->launches++;
@@ -249,10 +249,11 @@ int stream_samples(VgRenderer* r, VgAccum* acc, vgd::Ctx& c, vgx::Variant v, con
         if (!deferred)
             e = vgx::launch_stream_shade(v, ssb, s, c, w, i);
         else if (q)
-            e = vgx::launch_stream_cache_shade(v.f64, sorted, csb, s, c, w, i, *q);
+            e = vgx::launch_stream_cache_shade(sorted, dsb, s, c, w, i, *q);
         else
-            e = (v.restir ? vgx::launch_stream_shade_deferred_restir : vgx::launch_stream_shade_deferred)(v.f64, sorted, dsb,
-                                                                                                           s, c, w, i);
+            e = (v.light    ? vgx::launch_stream_shade_deferred_light
+                 : v.restir ? vgx::launch_stream_shade_deferred_restir
+                            : vgx::launch_stream_shade_deferred)(sorted, dsb, s, c, w, i);
         acc->launches++;
         return e != cudaSuccess ? e : mark(2);
     };
@@ -321,7 +322,7 @@ int stream_samples(VgRenderer* r, VgAccum* acc, vgd::Ctx& c, vgx::Variant v, con
                 acc->wave_live.push_back(live);
                 done = live == 0;
                 if (!done && live <= r->tail_threshold) {
-                    ce = (q ? vgx::launch_stream_cache_tail(v.f64, live, s, c, w, (uint32_t)((rep + 1) * K), *q) : vgx::launch_stream_tail(v, live, s, c, w, (uint32_t)((rep + 1) * K)));
+                    ce = (q ? vgx::launch_stream_cache_tail(v.f64, live, r->ctx->sms, s, c, w, (uint32_t)((rep + 1) * K), *q) : vgx::launch_stream_tail(v, live, r->ctx->sms, s, c, w, (uint32_t)((rep + 1) * K)));
                     if (ce != cudaSuccess) {
                         cudaGraphExecDestroy(ge);
                         return cuda_fail(ce, "tail launch");
@@ -373,7 +374,7 @@ int stream_samples(VgRenderer* r, VgAccum* acc, vgd::Ctx& c, vgx::Variant v, con
                     b = pool.get();
                     VG_CHECK(cudaEventRecord(a, s), "event");
                 }
-                VG_CHECK((q ? vgx::launch_stream_cache_tail(v.f64, live, s, c, w, (uint32_t)(wave + 1), *q) : vgx::launch_stream_tail(v, live, s, c, w, (uint32_t)(wave + 1))), "tail launch");
+                VG_CHECK((q ? vgx::launch_stream_cache_tail(v.f64, live, r->ctx->sms, s, c, w, (uint32_t)(wave + 1), *q) : vgx::launch_stream_tail(v, live, r->ctx->sms, s, c, w, (uint32_t)(wave + 1))), "tail launch");
                 if (timed) {
                     VG_CHECK(cudaEventRecord(b, s), "event");
                     stages.push_back({2, {a, b}});
@@ -1030,6 +1031,10 @@ int vg_accumulate(VgRenderer* r, VgAccum* acc, uint32_t samples)
     const uint32_t max_depth_alloc = 64;
     if (r->integrator == VG_WAVEFRONT && !acc->state.p) {
         uint32_t planes = vgk::BASE_PLANES + (acc->lighting ? vgk::SPLIT_PLANES : 0);
+        // Deferred shadows (stream_samples): per slot the request and the ended path's radiance.
+        const size_t dpx = acc->lighting && acc->restir.on ? 0 : px;
+        const size_t req_planes = acc->lighting ? vgk::SPLIT_REQ_PLANES : vgk::REQ_PLANES;
+        const size_t pend_planes = acc->lighting ? 1 + vgk::SPLIT_PLANES : 1;
         if ((st = alloc(acc->state, px * planes * 16, s, false)) != VG_OK ||
             (st = alloc(acc->hits, px * 16, s, false)) != VG_OK ||
             (st = alloc(acc->queue[0], px * 4, s, false)) != VG_OK ||
@@ -1038,11 +1043,11 @@ int vg_accumulate(VgRenderer* r, VgAccum* acc, uint32_t samples)
             (st = alloc(acc->fetch, 2 * (max_depth_alloc + 1) * 4, s, true)) != VG_OK ||
             (st = alloc(acc->tstats, 8 * 8, s, true)) != VG_OK ||
             (st = alloc(acc->meta, px * 4, s, false)) != VG_OK ||
-            (st = alloc(acc->sreq, acc->lighting ? 16 : px * 3 * 16, s, false)) != VG_OK ||
-            (st = alloc(acc->squeue, acc->lighting ? 16 : px * 4 * vgk::SHADE_CLASSES, s, false)) != VG_OK ||
-            (st = alloc(acc->flags, acc->lighting ? 16 : px * 4, s, false)) != VG_OK ||
-            (st = alloc(acc->pend, acc->lighting ? 16 : px * 16, s, false)) != VG_OK ||
-            (st = alloc(acc->shqueue, acc->lighting ? 16 : px * 4, s, false)) != VG_OK ||
+            (st = alloc(acc->sreq, dpx * req_planes * 16, s, false)) != VG_OK ||
+            (st = alloc(acc->squeue, dpx * 4 * vgk::SHADE_CLASSES, s, false)) != VG_OK ||
+            (st = alloc(acc->flags, dpx * 4, s, false)) != VG_OK ||
+            (st = alloc(acc->pend, dpx * pend_planes * 16, s, false)) != VG_OK ||
+            (st = alloc(acc->shqueue, dpx * 4, s, false)) != VG_OK ||
             (st = alloc(acc->scount, (2 * vgk::SHADE_CLASSES + 2) * 4, s, true)) != VG_OK)
             return st;
         if (!acc->host_counts && cudaHostAlloc((void**)&acc->host_counts, 64 * 4, cudaHostAllocDefault) != cudaSuccess) {
