@@ -94,10 +94,12 @@ static __global__ void __launch_bounds__(128) aov_normals(const __grid_constant_
     out[o + 2] = n.z;
 }
 
-// aov.slang:86-188
+// aov.slang:86-188 but for the coverage (aov_coverage_*). Albedo and depth go to planes of their own or
+// interleaved, by their strides.
 static __global__ void __launch_bounds__(128) aov_main(const __grid_constant__ Ctx c, CameraRecord cam,
-                                                       float* albedo_depth, uint32_t* object_ids,
-                                                       uint32_t* material_ids, float* coverage)
+                                                       float* albedo, uint32_t albedo_stride, float* depths,
+                                                       uint32_t depth_stride, uint32_t* object_ids,
+                                                       uint32_t* material_ids)
 {
     uint32_t w = (uint32_t)cam.v[0], h = (uint32_t)cam.v[1];
     uint32_t x = blockIdx.x * 16 + (threadIdx.x & 15u), y = blockIdx.y * 8 + (threadIdx.x >> 4);
@@ -110,7 +112,7 @@ static __global__ void __launch_bounds__(128) aov_main(const __grid_constant__ C
     V3 d = pixelDir(cam, (float)x + 0.5f, (float)y + 0.5f, w, h, t, aspect, dir);
     dir = normalize(dir);
     Hit hq = traceClosest(c, org, dir);
-    V3 albedo = v3(0.0f);
+    V3 alb = v3(0.0f);
     float depth = 0.0f;
     uint32_t id = 0, matId = 0;
     if (hq.hit) {
@@ -120,7 +122,7 @@ static __global__ void __launch_bounds__(128) aov_main(const __grid_constant__ C
         matId = mat + 1;
         depth = hq.t * -d.z;
         uint32_t mi = mat * 24;
-        albedo = v3(__ldg(c.s.materials + mi), __ldg(c.s.materials + mi + 1), __ldg(c.s.materials + mi + 2));
+        alb = v3(__ldg(c.s.materials + mi), __ldg(c.s.materials + mi + 1), __ldg(c.s.materials + mi + 2));
         uint32_t texBase = (uint32_t)__ldg(c.s.materials + mi + 10);
         if (texBase > 0) {
             V3 p0, p1, p2;
@@ -133,17 +135,42 @@ static __global__ void __launch_bounds__(128) aov_main(const __grid_constant__ C
             float ux = u0x + b1 * (u1x - u0x) + b2 * (u2x - u0x);
             float uy = u0y + b1 * (u1y - u0y) + b2 * (u2y - u0y);
             uint32_t ti = (texBase - 1) * 4;
-            albedo *= bilinear(c, __ldg(c.s.tex_info + ti), __ldg(c.s.tex_info + ti + 1), __ldg(c.s.tex_info + ti + 2),
+            alb *= bilinear(c, __ldg(c.s.tex_info + ti), __ldg(c.s.tex_info + ti + 1), __ldg(c.s.tex_info + ti + 2),
                                ux, uy);
         }
     }
+    size_t pixel = (size_t)y * w + x;
+    albedo[albedo_stride * pixel] = alb.x;
+    albedo[albedo_stride * pixel + 1] = alb.y;
+    albedo[albedo_stride * pixel + 2] = alb.z;
+    depths[depth_stride * pixel] = depth;
+    object_ids[pixel] = id;
+    material_ids[pixel] = matId;
+}
+
+// World direction of coverage sample k (of 4 x 4) of pixel (x, y), as its ray is traced.
+__device__ __forceinline__ V3 sampleDir(const CameraRecord& cam, uint32_t x, uint32_t y, uint32_t k, uint32_t w, uint32_t h,
+                                        float t, float aspect)
+{
+    V3 sdir;
+    pixelDir(cam, (float)x + ((float)(k % 4) + 0.5f) / 4.0f, (float)y + ((float)(k / 4) + 0.5f) / 4.0f, w, h, t, aspect,
+             sdir);
+    return normalize(sdir);
+}
+
+// aov.slang:150-181: the coverage of 16 stratified rays followed through translucent surfaces.
+static __global__ void __launch_bounds__(128) aov_coverage_layers(const __grid_constant__ Ctx c, CameraRecord cam,
+                                                                  float* coverage)
+{
+    uint32_t w = (uint32_t)cam.v[0], h = (uint32_t)cam.v[1];
+    uint32_t x = blockIdx.x * 16 + (threadIdx.x & 15u), y = blockIdx.y * 8 + (threadIdx.x >> 4);
+    if (x >= w || y >= h)
+        return;
+    V3 org = v3(cam.v[7], cam.v[11], cam.v[15]);
     float cover = 0.0f;
     for (uint32_t k = 0; k < 16; k++) {
-        V3 sdir;
-        pixelDir(cam, (float)x + ((float)(k % 4) + 0.5f) / 4.0f, (float)y + ((float)(k / 4) + 0.5f) / 4.0f, w, h, t,
-                 aspect, sdir);
         V3 so = org;
-        V3 sd = normalize(sdir);
+        V3 sd = sampleDir(cam, x, y, k, w, h, cam.v[2], cam.v[0] / cam.v[1]);
         float seen = 0.0f, through = 1.0f;
         for (uint32_t layer = 0; layer < 8 && through > 0.0f; layer++) {
             vgt::TraceHit q = vgt::trace_bvh<false>(c.s.nodes, c.s.tris, so, sd, 1.0e30f, c.err);
@@ -156,14 +183,95 @@ static __global__ void __launch_bounds__(128) aov_main(const __grid_constant__ C
         }
         cover += seen;
     }
-    size_t pixel = (size_t)y * w + x;
-    coverage[pixel] = cover / 16.0f;
-    albedo_depth[4 * pixel] = albedo.x;
-    albedo_depth[4 * pixel + 1] = albedo.y;
-    albedo_depth[4 * pixel + 2] = albedo.z;
-    albedo_depth[4 * pixel + 3] = depth;
-    object_ids[pixel] = id;
-    material_ids[pixel] = matId;
+    coverage[(size_t)y * w + x] = cover / 16.0f;
+}
+
+// The same where every surface is solid (DeviceScene::solid: a sample counts 1 if its ray hits anything):
+// one walk of the tree per pixel. Its box test takes all of the pixel's 16 rays as one beam: they share
+// their origin, and in each axis the near plane is divided by the largest and the far plane by the
+// smallest of their direction components, so a box that any of them meets is visited (a superset of what
+// each ray's own walk visits, and a hit of any triangle is what each ray's walk looks for: the counts
+// are the same). A triangle found is tested against every sample not covered yet, by the rays' own
+// test; the walk ends when all 16 are. Lanes go on to their next leaf before the warp tests triangles,
+// and a pixel whose directions change sign in an axis (a line or two of pixels) traces its rays one by
+// one. Bound by issue: 16 walks of some 13 nodes become one of about 15. With one walk per ray this was
+// most of aov_main's 7.5 ms per 1920x1080 frame of the 1M-triangle scene.
+static __global__ void __launch_bounds__(128, 6) aov_coverage_solid(const __grid_constant__ Ctx c, CameraRecord cam,
+                                                                    float* coverage)
+{
+    __shared__ float4 rays[16][128]; // shear x, y, z and the axis permutation of each thread's samples
+    uint32_t tid = threadIdx.x;
+    uint32_t w = (uint32_t)cam.v[0], h = (uint32_t)cam.v[1];
+    uint32_t x = blockIdx.x * 16 + (tid >> 5) * 4 + (tid & 3u), y = blockIdx.y * 8 + ((tid >> 2) & 7u);
+    if (x >= w || y >= h)
+        return;
+    float t = cam.v[2], aspect = cam.v[0] / cam.v[1];
+    V3 org = v3(cam.v[7], cam.v[11], cam.v[15]);
+    V3 lo = v3(3.0e38f), hi = v3(-3.0e38f);
+    for (uint32_t k = 0; k < 16; k++) {
+        V3 d = sampleDir(cam, x, y, k, w, h, t, aspect);
+        vgt::TRay r = vgt::make_ray(org, d);
+        rays[k][tid] = make_float4(r.sx, r.sy, r.sz, __uint_as_float((uint32_t)(r.kx | (r.ky << 2) | (r.kz << 4))));
+        lo = v3(fminf(lo.x, d.x), fminf(lo.y, d.y), fminf(lo.z, d.z));
+        hi = v3(fmaxf(hi.x, d.x), fmaxf(hi.y, d.y), fmaxf(hi.z, d.z));
+        if (bad3(d))
+            lo = v3(-3.0e38f); // no beam
+    }
+    auto one_sign = [](float a, float b) { return a > bvh8::MIN_DIR || (b < -bvh8::MIN_DIR && a > -2.0f); };
+    uint32_t covered = 0;
+    if (one_sign(lo.x, hi.x) && one_sign(lo.y, hi.y) && one_sign(lo.z, hi.z)) {
+        // Positive components: near / hi, far / lo; negative ones: near / lo, far / hi.
+        vgt::Slabs b;
+        b.o = org;
+        b.nx = 1.0f / (lo.x > 0.0f ? hi.x : lo.x), b.fx = 1.0f / (lo.x > 0.0f ? lo.x : hi.x);
+        b.ny = 1.0f / (lo.y > 0.0f ? hi.y : lo.y), b.fy = 1.0f / (lo.y > 0.0f ? lo.y : hi.y);
+        b.nz = 1.0f / (lo.z > 0.0f ? hi.z : lo.z), b.fz = 1.0f / (lo.z > 0.0f ? lo.z : hi.z);
+        b.oct = (lo.x < 0.0f ? 1u : 0u) | (lo.y < 0.0f ? 2u : 0u) | (lo.z < 0.0f ? 4u : 0u);
+        uint2 stack[bvh8::STACK_SIZE];
+        vgt::Walk k;
+        k.r.oct = b.oct;
+        k.tmax = 1.0e30f;
+        k.node = 0;
+        k.sp = 0;
+        k.nodes = 0;
+        bool done = false;
+        while (!done && covered != 0xffffu) {
+            do {
+                vgt::node_visit(c.s.nodes, k, b);
+                done = vgt::next_node(k, stack, c.err);
+            } while (!done && k.tri_bits == 0);
+            while (k.tri_bits && covered != 0xffffu) {
+                uint32_t j = vgt::high_bit(k.tri_bits);
+                k.tri_bits ^= 1u << j;
+                const float4* tp = c.s.tris + (size_t)(k.tri_base + j) * bvh8::TRI_VEC4;
+                float4 p0 = __ldg(tp), p1 = __ldg(tp + 1), p2 = __ldg(tp + 2);
+#pragma unroll 2
+                for (uint32_t i = 0; i < 16; i++) {
+                    float4 q = rays[i][tid];
+                    uint32_t kk = __float_as_uint(q.w);
+                    vgt::TRay r;
+                    r.o = org;
+                    r.kx = (int)(kk & 3u);
+                    r.ky = (int)((kk >> 2) & 3u);
+                    r.kz = (int)((kk >> 4) & 3u);
+                    r.sx = q.x;
+                    r.sy = q.y;
+                    r.sz = q.z;
+                    float th, U, V, W, det;
+                    if (vgt::tri_test(r, v3(p0.x, p0.y, p0.z), v3(p1.x, p1.y, p1.z), v3(p2.x, p2.y, p2.z), th, U, V, W, det) &&
+                        th < 1.0e30f)
+                        covered |= 1u << i;
+                }
+            }
+        }
+    } else {
+        for (uint32_t k = 0; k < 16; k++) {
+            V3 d = sampleDir(cam, x, y, k, w, h, t, aspect);
+            if (vgt::trace_bvh<true>(c.s.nodes, c.s.tris, org, d, 1.0e30f, c.err).hit)
+                covered |= 1u << k;
+        }
+    }
+    coverage[(size_t)y * w + x] = (float)__popc(covered) / 16.0f;
 }
 
 } // namespace vga

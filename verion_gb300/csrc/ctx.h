@@ -40,6 +40,7 @@ struct DeviceScene {
     const uint4* nodes;
     const float4* tris;
     uint32_t shadow_any; // 1 when every surface is opaque: shadow rays stop at any hit
+    uint32_t solid;      // 1 when every material's opacity is exactly 1: a ray's coverage is hit or miss
 };
 
 // ReSTIR DI reservoirs in structure-of-arrays form, one set per frame parity. The reference keeps

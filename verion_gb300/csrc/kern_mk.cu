@@ -58,15 +58,23 @@ cudaError_t launch_aov_normals(cudaStream_t s, const vgd::Ctx& c, const float* c
     return cudaGetLastError();
 }
 
-cudaError_t launch_aov_main(cudaStream_t s, const vgd::Ctx& c, const float* camera18, float* albedo_depth,
-                            uint32_t* object_ids, uint32_t* material_ids, float* coverage)
+cudaError_t launch_aov_main(cudaStream_t s, const vgd::Ctx& c, const float* camera18, float* albedo,
+                            uint32_t albedo_stride, float* depth, uint32_t depth_stride, uint32_t* object_ids,
+                            uint32_t* material_ids, float* coverage)
 {
     vga::CameraRecord cam;
     for (int i = 0; i < 18; i++)
         cam.v[i] = camera18[i];
     uint32_t w = (uint32_t)cam.v[0], h = (uint32_t)cam.v[1];
     dim3 grid((w + 15) / 16, (h + 7) / 8);
-    vga::aov_main<<<grid, 128, 0, s>>>(c, cam, albedo_depth, object_ids, material_ids, coverage);
+    vga::aov_main<<<grid, 128, 0, s>>>(c, cam, albedo, albedo_stride, depth, depth_stride, object_ids, material_ids);
+    cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess)
+        return e;
+    if (c.s.solid)
+        vga::aov_coverage_solid<<<grid, 128, 0, s>>>(c, cam, coverage);
+    else
+        vga::aov_coverage_layers<<<grid, 128, 0, s>>>(c, cam, coverage);
     return cudaGetLastError();
 }
 

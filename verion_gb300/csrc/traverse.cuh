@@ -150,7 +150,21 @@ __device__ __forceinline__ uint32_t high_bit(uint32_t x) { return 31u - (uint32_
 // x << (s mod 32): the shift count's upper bits are ignored, so a packed byte needs no mask.
 __device__ __forceinline__ uint32_t shl_wrap(uint32_t x, uint32_t s) { return __funnelshift_l(0u, x, s); }
 
-// Child-box tests of one BVH8 node (words w0, w1.zw = meta, w2..w4, bvh8.h) for ray r with the
+// What the box test reads of a ray: its origin, and per axis the reciprocal direction that its near and
+// its far plane are divided by (one and the same for a single ray; the ends of an interval of directions
+// for a beam of rays from one origin, whose components must not change sign within it).
+struct Slabs {
+    V3 o;
+    float nx, ny, nz, fx, fy, fz;
+    uint32_t oct;
+};
+
+__device__ __forceinline__ Slabs slabs_of(const TRay& r)
+{
+    return Slabs{r.o, r.ix, r.iy, r.iz, r.ix, r.iy, r.iz, r.oct};
+}
+
+// Child-box tests of one BVH8 node (words w0, w1.zw = meta, w2..w4, bvh8.h) for a ray with the
 // closest hit so far at best_t. Returns the hit children in one word: bits 24-31 the internal ones
 // (bit 24 + (slot XOR octant XOR 7): the highest set bit is the child to visit first), bits 0-23 the
 // triangles of the hit leaf slots, from the node's triangle base.
@@ -164,7 +178,7 @@ __device__ __forceinline__ uint32_t shl_wrap(uint32_t x, uint32_t s) { return __
 // node visits; the byte's exact value (a subtraction per plane, 48 per node) needed 2^-13 of a step.
 //
 // Each child ends in one predicated OR of its meta byte's bits: no branch, whatever the lanes hit.
-__device__ __forceinline__ uint32_t node_test(const TRay& r, uint4 w0, uint32_t meta_lo, uint32_t meta_hi, uint4 w2,
+__device__ __forceinline__ uint32_t node_test(const Slabs& r, uint4 w0, uint32_t meta_lo, uint32_t meta_hi, uint4 w2,
                                               uint4 w3, uint4 w4, float best_t)
 {
     float px = __uint_as_float(w0.x), py = __uint_as_float(w0.y), pz = __uint_as_float(w0.z);
@@ -172,7 +186,7 @@ __device__ __forceinline__ uint32_t node_test(const TRay& r, uint4 w0, uint32_t 
     float scx = __uint_as_float((em & 0xffu) << 23);
     float scy = __uint_as_float(((em >> 8) & 0xffu) << 23);
     float scz = __uint_as_float(((em >> 16) & 0xffu) << 23);
-    bool px_pos = r.ix >= 0.0f, py_pos = r.iy >= 0.0f, pz_pos = r.iz >= 0.0f;
+    bool px_pos = r.nx >= 0.0f, py_pos = r.ny >= 0.0f, pz_pos = r.nz >= 0.0f;
     // Near and far quantised planes per axis (low words at w2.x .. high words at w4.w).
     uint32_t nxl = px_pos ? w2.x : w3.z, nxh = px_pos ? w2.y : w3.w;
     uint32_t fxl = px_pos ? w3.z : w2.x, fxh = px_pos ? w3.w : w2.y;
@@ -180,16 +194,18 @@ __device__ __forceinline__ uint32_t node_test(const TRay& r, uint4 w0, uint32_t 
     uint32_t fyl = py_pos ? w4.x : w2.z, fyh = py_pos ? w4.y : w2.w;
     uint32_t nzl = pz_pos ? w3.x : w4.z, nzh = pz_pos ? w3.y : w4.w;
     uint32_t fzl = pz_pos ? w4.z : w3.x, fzh = pz_pos ? w4.w : w3.y;
-    float ax = (px - r.o.x) * r.ix, sx = scx * r.ix;
-    float ay = (py - r.o.y) * r.iy, sy = scy * r.iy;
-    float az = (pz - r.o.z) * r.iz, sz = scz * r.iz;
+    float dx = px - r.o.x, dy = py - r.o.y, dz = pz - r.o.z;
+    float snx = scx * r.nx, sny = scy * r.ny, snz = scz * r.nz;
+    float sfx = scx * r.fx, sfy = scy * r.fy, sfz = scz * r.fz;
+    float anx = dx * r.nx, any_ = dy * r.ny, anz = dz * r.nz;
+    float afx = dx * r.fx, afy = dy * r.fy, afz = dz * r.fz;
     constexpr float EA = 4.76837158e-7f, ES = 3.90625e-3f; // 2^-21, 2^-8
-    float ex = fmaf(EA, fabsf(ax), ES * fabsf(sx));
-    float ey = fmaf(EA, fabsf(ay), ES * fabsf(sy));
-    float ez = fmaf(EA, fabsf(az), ES * fabsf(sz));
-    float anx = fmaf(-32768.0f, sx, ax - ex), afx = fmaf(-32768.0f, sx, ax + ex);
-    float any_ = fmaf(-32768.0f, sy, ay - ey), afy = fmaf(-32768.0f, sy, ay + ey);
-    float anz = fmaf(-32768.0f, sz, az - ez), afz = fmaf(-32768.0f, sz, az + ez);
+    anx = fmaf(-32768.0f, snx, anx - fmaf(EA, fabsf(anx), ES * fabsf(snx)));
+    any_ = fmaf(-32768.0f, sny, any_ - fmaf(EA, fabsf(any_), ES * fabsf(sny)));
+    anz = fmaf(-32768.0f, snz, anz - fmaf(EA, fabsf(anz), ES * fabsf(snz)));
+    afx = fmaf(-32768.0f, sfx, afx + fmaf(EA, fabsf(afx), ES * fabsf(sfx)));
+    afy = fmaf(-32768.0f, sfy, afy + fmaf(EA, fabsf(afy), ES * fabsf(sfy)));
+    afz = fmaf(-32768.0f, sfz, afz + fmaf(EA, fabsf(afz), ES * fabsf(sfz)));
     uint32_t flip = (r.oct ^ 7u) * 0x01010101u;
     uint32_t found = 0;
 #pragma unroll
@@ -202,12 +218,12 @@ __device__ __forceinline__ uint32_t node_test(const TRay& r, uint4 w0, uint32_t 
 #pragma unroll
         for (int j = 0; j < 4; j++) {
             int i = 4 * half + j;
-            float tnx = fmaf(byte_f15(nxl, nxh, i), sx, anx);
-            float tny = fmaf(byte_f15(nyl, nyh, i), sy, any_);
-            float tnz = fmaf(byte_f15(nzl, nzh, i), sz, anz);
-            float tfx = fmaf(byte_f15(fxl, fxh, i), sx, afx);
-            float tfy = fmaf(byte_f15(fyl, fyh, i), sy, afy);
-            float tfz = fmaf(byte_f15(fzl, fzh, i), sz, afz);
+            float tnx = fmaf(byte_f15(nxl, nxh, i), snx, anx);
+            float tny = fmaf(byte_f15(nyl, nyh, i), sny, any_);
+            float tnz = fmaf(byte_f15(nzl, nzh, i), snz, anz);
+            float tfx = fmaf(byte_f15(fxl, fxh, i), sfx, afx);
+            float tfy = fmaf(byte_f15(fyl, fyh, i), sfy, afy);
+            float tfz = fmaf(byte_f15(fzl, fzh, i), sfz, afz);
             float tn = fmaxf(max3(tnx, tny, tnz), 0.0f);
             float tf = fminf(min3(tfx, tfy, tfz), best_t);
             uint32_t b = shl_wrap((bits >> (8 * j)) & 0xffu, at >> (8 * j));
@@ -255,12 +271,12 @@ __device__ __forceinline__ void walk_begin(Walk& w, V3 o, V3 d, float tmax)
 
 // Visits w.node: its hit internal children become the walk's node group, what the group before it
 // had left goes to the stack (next_node), its hit leaf slots' triangles become the pending ones.
-__device__ __forceinline__ void node_visit(const uint4* __restrict__ nodes, Walk& w)
+__device__ __forceinline__ void node_visit(const uint4* __restrict__ nodes, Walk& w, const Slabs& slabs)
 {
     const uint4* np = nodes + (size_t)w.node * bvh8::NODE_VEC4;
     uint4 w0 = __ldg(np), w1 = __ldg(np + 1), w2 = __ldg(np + 2), w3 = __ldg(np + 3), w4 = __ldg(np + 4);
     w.nodes++;
-    uint32_t found = node_test(w.r, w0, w1.z, w1.w, w2, w3, w4, w.tmax);
+    uint32_t found = node_test(slabs, w0, w1.z, w1.w, w2, w3, w4, w.tmax);
     w.group = make_uint2(w1.x, (found & 0xff000000u) | (w0.w >> 24));
     w.tri_base = w1.y;
     w.tri_bits = found & 0x00ffffffu;
@@ -325,7 +341,7 @@ template <Hits H>
 __device__ __forceinline__ bool walk_step(const uint4* __restrict__ nodes, const float4* __restrict__ tris, Walk& w,
                                           uint2* stack, uint32_t* err)
 {
-    node_visit(nodes, w);
+    node_visit(nodes, w, slabs_of(w.r));
     while (w.tri_bits)
         if (test_one<H>(tris, w))
             return true;
@@ -573,7 +589,7 @@ __device__ __forceinline__ void trace_queue_coop(const uint4* __restrict__ nodes
         for (uint32_t s = 0; s < steps; s++) {
             uint32_t bits = 0;
             if (active) {
-                node_visit(nodes, w);
+                node_visit(nodes, w, slabs_of(w.r));
                 bits = w.tri_bits;
                 w.tri_bits = 0;
             }

@@ -96,6 +96,15 @@ bool translucent_materials(const VgPacked* pk)
     return false;
 }
 
+// Every material's opacity is exactly 1 (DeviceScene::solid).
+bool solid_materials(const VgPacked* pk)
+{
+    for (size_t m = 0; m < pk->materials_len / MATERIAL_WORDS; m++)
+        if (pk->materials[m * MATERIAL_WORDS + 22] != 1.0f || pk->materials[m * MATERIAL_WORDS + 23] > 0.0f)
+            return false;
+    return true;
+}
+
 // Guide tables of the environment's CDF searches (cdf_guide.h; sizes vgd::ENV_GUIDE_M / ENV_GUIDE_C):
 // the marginal's, then one per row of the conditional.
 std::vector<uint32_t> env_guide(const VgPacked* pk)
@@ -516,7 +525,7 @@ int vg_renderer_create(VgContext* ctx, const VgPacked* pk, VgRenderer** out)
         delete r;
         return st;
     }
-    bool translucent = translucent_materials(pk);
+    bool translucent = translucent_materials(pk), solid = solid_materials(pk);
 
 #define UP(buf, src, n)                                                                                             \
     do {                                                                                                            \
@@ -565,6 +574,7 @@ int vg_renderer_create(VgContext* ctx, const VgPacked* pk, VgRenderer** out)
     r->env_key = table_key(pk->env_pixels, pk->env_pixels_len, pk->env_conditional, pk->env_conditional_len);
     bind_tables(r);
     r->ds.shadow_any = translucent ? 0u : 1u;
+    r->ds.solid = solid ? 1u : 0u;
     r->extend_blocks = vgx::wf_extend_blocks_per_sm();
     *out = r;
     return VG_OK;
@@ -617,6 +627,7 @@ int vg_renderer_update(VgRenderer* r, const VgPacked* pk, const VgUpdatePlan* pl
         uint32_t shadow_any = f->ds.shadow_any;
         bind_tables(r);
         r->ds.shadow_any = shadow_any;
+        r->ds.solid = f->ds.solid;
         vg_renderer_destroy(f); // frees the old tables
         out->blases_built = pk->mesh_count;
         out->tlas_built = 1;
@@ -663,6 +674,7 @@ int vg_renderer_update(VgRenderer* r, const VgPacked* pk, const VgUpdatePlan* pl
             r->texel_key = key;
         }
         r->ds.shadow_any = translucent_materials(pk) ? 0u : 1u;
+        r->ds.solid = solid_materials(pk) ? 1u : 0u;
     }
     if (plan->lights) {
         if ((st = upload(ctx, r->lights, pk->lights, pk->lights_len * 4)) != VG_OK)
@@ -1541,7 +1553,8 @@ int vg_render_aovs(VgRenderer* r, uint32_t width, uint32_t height, float* albedo
     camera_record(r, width, height, rec);
     vgd::Ctx c = make_ctx(r, nullptr);
     VG_CHECK(cudaMemsetAsync(r->err.p, 0, 4, s), "error flag");
-    VG_CHECK(vgx::launch_aov_main(s, c, rec, (float*)ad.p, (uint32_t*)oi.p, (uint32_t*)mi.p, (float*)cv.p),
+    VG_CHECK(vgx::launch_aov_main(s, c, rec, (float*)ad.p, 4, (float*)ad.p + 3, 4, (uint32_t*)oi.p, (uint32_t*)mi.p,
+                                  (float*)cv.p),
              "aov launch");
     VG_CHECK(cudaMemcpyAsync(albedo_depth, ad.p, px * 16, cudaMemcpyDeviceToHost, s), "readback");
     VG_CHECK(cudaMemcpyAsync(object_id, oi.p, px * 4, cudaMemcpyDeviceToHost, s), "readback");
