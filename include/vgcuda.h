@@ -329,6 +329,10 @@ int vg_render_normals(VgRenderer* r, uint32_t width, uint32_t height, float* out
  * material + 1 (0 on a miss), and coverage of 16 stratified rays through translucent surfaces. */
 int vg_render_aovs(VgRenderer* r, uint32_t width, uint32_t height, float* albedo_depth, uint32_t* object_id,
                    uint32_t* material_id, float* coverage);
+/* The same with albedo (3 floats a pixel) and depth each in an array of its own. */
+int vg_render_aov_planes(VgRenderer* renderer, uint32_t width, uint32_t height, float* albedo, float* depth,
+                         uint32_t* object_id, uint32_t* material_id, float* coverage);
+
 
 /* Traversal entry points (no reference counterpart; the reference's traversal is the driver's).
  * Closest hits of n rays (6 floats each: origin xyz, direction xyz, host memory) into 4 words per

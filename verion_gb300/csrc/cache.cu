@@ -112,10 +112,11 @@ int cache_train_step(VgCache* k, const float* rec, const uint32_t* count, uint32
     return VG_OK;
 }
 
-int stage_records(VgCache* k, DevBuf& b, const float* records, size_t n)
+// The records on the device, and `more` bytes behind them.
+int stage_records(VgCache* k, TempBuf& b, const float* records, size_t n, size_t more = 0)
 {
     int st;
-    if ((st = alloc(b, n * vgn::REC_WORDS * 4, k->ctx->stream, false)) != VG_OK)
+    if ((st = b.get(k->ctx, n * vgn::REC_WORDS * 4 + more)) != VG_OK)
         return st;
     if (n > 0)
         VG_CHECK(cudaMemcpyAsync(b.p, records, n * vgn::REC_WORDS * 4, cudaMemcpyHostToDevice, k->ctx->stream),
@@ -451,11 +452,11 @@ int vg_cache_infer(VgCache* k, const float* records, size_t n, float* out)
         return fail(VG_ERR_INVALID, "too many records");
     if (n == 0)
         return VG_OK;
-    DevBuf rec, o;
+    TempBuf rec;
     int st;
-    if ((st = stage_records(k, rec, records, n)) != VG_OK || (st = alloc(o, n * 12, k->ctx->stream, false)) != VG_OK ||
-        (st = ensure_work(k, n)) != VG_OK)
+    if ((st = stage_records(k, rec, records, n, n * 12)) != VG_OK || (st = ensure_work(k, n)) != VG_OK)
         return st;
+    float* o = (float*)rec.at(n * vgn::REC_WORDS * 4);
     cudaStream_t s = k->ctx->stream;
     vgn::CacheDev d = k->dev();
     const uint32_t* cnt = (const uint32_t*)k->count.p;
@@ -464,9 +465,9 @@ int vg_cache_infer(VgCache* k, const float* records, size_t n, float* out)
                                     (uint8_t*)k->X.p),
              "encode launch");
     VG_CHECK(vgx::nrc_launch_infer(3 * k->ctx->sms, s, d, (const uint8_t*)k->X.p, (const float*)rec.p, cnt,
-                                   (uint32_t)n, (float*)o.p, nullptr, 32),
+                                   (uint32_t)n, o, nullptr, 32),
              "inference launch");
-    VG_CHECK(cudaMemcpyAsync(out, o.p, n * 12, cudaMemcpyDeviceToHost, s), "readback");
+    VG_CHECK(cudaMemcpyAsync(out, o, n * 12, cudaMemcpyDeviceToHost, s), "readback");
     return cache_check(k);
 }
 
@@ -477,7 +478,7 @@ int vg_cache_gradients(VgCache* k, const float* records, size_t n, float* mlp_gr
         return fail(VG_ERR_INVALID, "null argument");
     if (n > 0x7fffffffull)
         return fail(VG_ERR_INVALID, "too many records");
-    DevBuf rec;
+    TempBuf rec;
     int st;
     if ((st = stage_records(k, rec, records, n)) != VG_OK || (st = ensure_work(k, n)) != VG_OK)
         return st;
@@ -512,7 +513,7 @@ int vg_cache_train(VgCache* k, const float* records, size_t n, uint32_t batch, d
         return fail(VG_ERR_INVALID, "null argument");
     if (batch == 0 || n > 0x7fffffffull)
         return fail(VG_ERR_INVALID, "batch must be non-zero");
-    DevBuf rec;
+    TempBuf rec;
     int st;
     if ((st = stage_records(k, rec, records, n)) != VG_OK || (st = ensure_work(k, std::min<size_t>(n, batch))) != VG_OK)
         return st;
@@ -541,11 +542,11 @@ int vg_cache_time(VgCache* k, const float* records, size_t n, uint32_t reps, dou
         return fail(VG_ERR_INVALID, "null argument or empty input");
     if (n > 0x7fffffffull)
         return fail(VG_ERR_INVALID, "too many records");
-    DevBuf rec, o;
+    TempBuf rec;
     int st;
-    if ((st = stage_records(k, rec, records, n)) != VG_OK || (st = ensure_work(k, n)) != VG_OK ||
-        (st = alloc(o, n * 12, k->ctx->stream, false)) != VG_OK)
+    if ((st = stage_records(k, rec, records, n, n * 12)) != VG_OK || (st = ensure_work(k, n)) != VG_OK)
         return st;
+    float* o = (float*)rec.at(n * vgn::REC_WORDS * 4);
     cudaStream_t s = k->ctx->stream;
     vgn::CacheDev d = k->dev();
     const uint32_t* cnt = (const uint32_t*)k->count.p;
@@ -566,7 +567,7 @@ int vg_cache_time(VgCache* k, const float* records, size_t n, uint32_t reps, dou
         if (round == 1)
             VG_CHECK(cudaEventRecord(ev[1], s), "event");
         for (uint32_t i = 0; i < m; i++)
-            VG_CHECK(vgx::nrc_launch_infer(3 * k->ctx->sms, s, d, (const uint8_t*)k->X.p, rp, cnt, n32, (float*)o.p,
+            VG_CHECK(vgx::nrc_launch_infer(3 * k->ctx->sms, s, d, (const uint8_t*)k->X.p, rp, cnt, n32, o,
                                            nullptr, 32),
                      "infer");
         if (round == 1)

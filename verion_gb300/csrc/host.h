@@ -87,7 +87,9 @@ int wait_event(cudaEvent_t ev)
         double dt = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
         if (dt > limit)
             return fail(VG_ERR_TIMEOUT, "the GPU did not finish within " + std::to_string(limit) + " s");
-        std::this_thread::sleep_for(std::chrono::microseconds(dt < 0.01 ? 20 : 200));
+        // The shortest sleep takes some 70 us, longer than a small wave: the first 2 ms are polled.
+        if (dt > 0.002)
+            std::this_thread::sleep_for(std::chrono::microseconds(dt < 0.02 ? 20 : 200));
     }
 }
 
@@ -104,18 +106,110 @@ namespace {
 struct DevBuf {
     void* p = nullptr;
     size_t bytes = 0;
+    bool part = false; // a piece of another DevBuf's memory, which frees it
     DevBuf() = default;
     DevBuf(const DevBuf&) = delete;
     DevBuf& operator=(const DevBuf&) = delete;
     ~DevBuf() { release(); }
     void release()
     {
-        if (p) {
+        if (p && !part) {
             cudaFree(p);
             vgh::g_frees++;
         }
         p = nullptr;
         bytes = 0;
+        part = false;
+    }
+};
+
+// Device buffers that entry points use for the length of a call (rays and hits, records, AOV planes), kept
+// for the next call: a cudaMalloc and cudaFree of some tens of MB cost more than most of those calls'
+// kernels. A buffer has one owner at a time (TempBuf), whichever thread that is on; it is given back when
+// the context's stream is done with it. At most KEEP bytes wait here, and they go with the context.
+struct TempPool {
+    static constexpr size_t KEEP = 256u << 20;
+    std::mutex mu;
+    std::vector<std::pair<void*, size_t>> idle;
+    size_t idle_bytes = 0;
+    // The smallest idle buffer of at least n bytes and at most four times that.
+    void* take(size_t n, size_t* bytes)
+    {
+        std::lock_guard<std::mutex> lock(mu);
+        size_t best = idle.size();
+        for (size_t i = 0; i < idle.size(); i++)
+            if (idle[i].second >= n && idle[i].second / 4 <= n && (best == idle.size() || idle[i].second < idle[best].second))
+                best = i;
+        if (best == idle.size())
+            return nullptr;
+        void* p = idle[best].first;
+        *bytes = idle[best].second;
+        idle_bytes -= idle[best].second;
+        idle.erase(idle.begin() + (long)best);
+        return p;
+    }
+    void give(void* p, size_t bytes)
+    {
+        std::vector<void*> drop;
+        {
+            std::lock_guard<std::mutex> lock(mu);
+            if (bytes <= KEEP) {
+                while (idle_bytes + bytes > KEEP) { // the oldest first
+                    drop.push_back(idle.front().first);
+                    idle_bytes -= idle.front().second;
+                    idle.erase(idle.begin());
+                }
+                idle.emplace_back(p, bytes);
+                idle_bytes += bytes;
+            } else {
+                drop.push_back(p);
+            }
+        }
+        for (void* q : drop) {
+            cudaFree(q);
+            vgh::g_frees++;
+        }
+    }
+    ~TempPool()
+    {
+        for (auto& b : idle) {
+            cudaFree(b.first);
+            vgh::g_frees++;
+        }
+    }
+};
+
+// Pinned words that the GPU writes its wave counts and status to: a ring per accumulate call in flight.
+// The rings of finished calls are used again; they go with the context.
+struct RingPool {
+    static constexpr size_t WORDS = 16;
+    std::mutex mu;
+    std::vector<uint32_t*> idle, all;
+    uint32_t* take()
+    {
+        std::lock_guard<std::mutex> lock(mu);
+        if (idle.empty()) {
+            void* p = nullptr;
+            if (cudaHostAlloc(&p, WORDS * 4, cudaHostAllocPortable) != cudaSuccess) {
+                cudaGetLastError();
+                return nullptr;
+            }
+            idle.push_back((uint32_t*)p);
+            all.push_back((uint32_t*)p);
+        }
+        uint32_t* r = idle.back();
+        idle.pop_back();
+        return r;
+    }
+    void give(uint32_t* r)
+    {
+        std::lock_guard<std::mutex> lock(mu);
+        idle.push_back(r);
+    }
+    ~RingPool()
+    {
+        for (uint32_t* p : all)
+            cudaFreeHost(p);
     }
 };
 
@@ -167,6 +261,8 @@ struct VgContext {
     bool batch_device_loop = true;                // batch wavefront: bounce loop in the graph (else the host's)
     cudaStream_t side = nullptr;                 // second stream (created on first use): cache training paths
     cudaEvent_t fork = nullptr, join = nullptr;  // ordering between `stream` and `side`
+    TempPool temps;
+    RingPool rings;
     ~VgContext();
 };
 
@@ -251,19 +347,14 @@ struct VgAccum {
     Restir restir;               // captured at the first sample
     DevBuf re_g[2], re_n[2], re_x[2], re_m[2];
     DevBuf re_gx[2], re_gn[2], re_gl[2], re_s[7]; // ReSTIR GI planes
+    DevBuf wave; // the wavefront buffers' memory: the DevBufs of the next line are parts of it
     DevBuf state, hits, queue[2], counts, fetch, tstats, meta, sreq, squeue, scount, flags, pend, shqueue;
     DevBuf mk_next;                  // the megakernel's pixel counter
-    uint32_t* host_counts = nullptr; // pinned ring of wave output counts (streaming wavefront)
     uint32_t last_waves = 0;
     std::vector<uint32_t> wave_live; // last streaming accumulate: live slots after each wave
     std::vector<float> wave_ms;      // with stage timing: extend, shade milliseconds per wave
     float tail_ms = 0.0f;            // with stage timing: the tail launch of the last call
     size_t wave_stages = 2;          // kernels per wave in wave_ms (2, or 3 with deferred shadows)
-    ~VgAccum()
-    {
-        if (host_counts)
-            cudaFreeHost(host_counts);
-    }
     size_t wavefront_bytes = 0;
     size_t restir_bytes = 0;
     uint32_t last_depth = 0; // max depth of the last wavefront sample
@@ -316,6 +407,91 @@ int alloc(DevBuf& b, size_t bytes, cudaStream_t s, bool zero)
     }
     return VG_OK;
 }
+
+// One allocation for several buffers (256-byte aligned parts of `whole`); those asked to be zero come
+// first and are cleared together.
+struct Part {
+    DevBuf* buf;
+    size_t bytes;
+    bool zero;
+};
+int alloc_parts(DevBuf& whole, std::vector<Part> parts, cudaStream_t s)
+{
+    std::stable_sort(parts.begin(), parts.end(), [](const Part& a, const Part& b) { return a.zero > b.zero; });
+    size_t total = 0, zero = 0;
+    auto padded = [](size_t n) { return (std::max<size_t>(n, 16) + 255) / 256 * 256; };
+    for (auto& p : parts) {
+        total += padded(p.bytes);
+        zero += p.zero ? padded(p.bytes) : 0;
+    }
+    int st = alloc(whole, total, s, false);
+    if (st != VG_OK)
+        return st;
+    if (zero)
+        VG_CHECK(cudaMemsetAsync(whole.p, 0, zero, s), "cudaMemsetAsync");
+    char* at = (char*)whole.p;
+    for (auto& p : parts) {
+        p.buf->release();
+        p.buf->p = at;
+        p.buf->bytes = std::max<size_t>(p.bytes, 16);
+        p.buf->part = true;
+        at += padded(p.bytes);
+    }
+    return VG_OK;
+}
+
+// A buffer of the context's TempPool for the length of a call: at(offset) of up to the bytes asked for.
+struct TempBuf {
+    VgContext* ctx = nullptr;
+    void* p = nullptr;
+    size_t bytes = 0;
+    TempBuf() = default;
+    TempBuf(const TempBuf&) = delete;
+    TempBuf& operator=(const TempBuf&) = delete;
+    int get(VgContext* c, size_t n)
+    {
+        n = std::max<size_t>(n, 256);
+        ctx = c;
+        p = c->temps.take(n, &bytes);
+        if (p)
+            return VG_OK;
+        int st = check_fits(n);
+        if (st != VG_OK)
+            return st;
+        cudaError_t e = cudaMalloc(&p, n);
+        if (e != cudaSuccess) {
+            p = nullptr;
+            return cuda_fail(e, "cudaMalloc");
+        }
+        vgh::g_mallocs++;
+        bytes = n;
+        return VG_OK;
+    }
+    char* at(size_t offset) const { return (char*)p + offset; }
+    ~TempBuf()
+    {
+        if (p) {
+            cudaStreamSynchronize(ctx->stream); // the call may have failed with work in flight
+            ctx->temps.give(p, bytes);
+        }
+    }
+};
+
+// The same for a ring of pinned words.
+struct Ring {
+    VgContext* ctx;
+    uint32_t* words;
+    explicit Ring(VgContext* c) : ctx(c), words(c->rings.take()) {}
+    Ring(const Ring&) = delete;
+    Ring& operator=(const Ring&) = delete;
+    ~Ring()
+    {
+        if (words) {
+            cudaStreamSynchronize(ctx->stream);
+            ctx->rings.give(words);
+        }
+    }
+};
 
 int upload(VgContext* ctx, DevBuf& b, const void* src, size_t bytes)
 {
@@ -520,16 +696,21 @@ vgd::Ctx make_ctx(VgRenderer* r, VgAccum* acc)
     return c;
 }
 
-int read_err(VgRenderer* r)
+int err_status(uint32_t e)
 {
-    uint32_t e = 0;
-    VG_CHECK(cudaMemcpyAsync(&e, r->err.p, 4, cudaMemcpyDeviceToHost, r->ctx->stream), "error flag");
-    VG_CHECK(cudaStreamSynchronize(r->ctx->stream), "error flag");
     if (e & bvh8::ERR_STACK)
         return fail(VG_ERR_KERNEL, "BVH traversal stack overflow");
     if (e)
         return fail(VG_ERR_KERNEL, "kernel reported error status " + std::to_string(e));
     return VG_OK;
+}
+
+int read_err(VgRenderer* r)
+{
+    uint32_t e = 0;
+    VG_CHECK(cudaMemcpyAsync(&e, r->err.p, 4, cudaMemcpyDeviceToHost, r->ctx->stream), "error flag");
+    VG_CHECK(cudaStreamSynchronize(r->ctx->stream), "error flag");
+    return err_status(e);
 }
 
 } // namespace

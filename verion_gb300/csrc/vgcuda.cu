@@ -276,9 +276,13 @@ int stream_samples(VgRenderer* r, VgAccum* acc, vgd::Ctx& c, vgx::Variant v, con
     acc->launches++;
     // Waves until no slot is live. The host reads each wave's output count LAG waves later,
     // so the GPU never idles on the poll; extra waves on an empty queue exit at once.
-    const uint32_t LAG = 2, RING = 64;
+    const uint32_t LAG = 2, RING = 8;
+    static_assert(RING <= RingPool::WORDS, "wave counts per ring");
     uint64_t max_waves = (uint64_t)samples * r->max_depth + LAG + 1;
-    uint32_t* ring = acc->host_counts;
+    Ring pinned(r->ctx);
+    uint32_t* ring = pinned.words;
+    if (!ring)
+        return fail(VG_ERR_RESOURCE, "pinned host buffer");
     std::vector<cudaEvent_t> ring_ev(RING);
     for (auto& e : ring_ev)
         e = pool.get();
@@ -959,12 +963,7 @@ int vg_accum_create(VgRenderer* r, uint32_t width, uint32_t height, int lighting
     int st = alloc(acc->accum, px * 3 * es, r->ctx->stream, true);
     if (st == VG_OK && acc->lighting)
         st = alloc(acc->light, px * LIGHTING_STRIDE * 4, r->ctx->stream, true);
-    if (st == VG_OK) {
-        cudaError_t e = cudaStreamSynchronize(r->ctx->stream);
-        if (e != cudaSuccess)
-            st = cuda_fail(e, "accumulation clear");
-    }
-    if (st != VG_OK) {
+    if (st != VG_OK) { // (the clears are in the order of the context's stream, as every use of the sums)
         delete acc;
         return st;
     }
@@ -1047,25 +1046,23 @@ int vg_accumulate(VgRenderer* r, VgAccum* acc, uint32_t samples)
         const size_t dpx = acc->lighting && acc->restir.on ? 0 : px;
         const size_t req_planes = acc->lighting ? vgk::SPLIT_REQ_PLANES : vgk::REQ_PLANES;
         const size_t pend_planes = acc->lighting ? 1 + vgk::SPLIT_PLANES : 1;
-        if ((st = alloc(acc->state, px * planes * 16, s, false)) != VG_OK ||
-            (st = alloc(acc->hits, px * 16, s, false)) != VG_OK ||
-            (st = alloc(acc->queue[0], px * 4, s, false)) != VG_OK ||
-            (st = alloc(acc->queue[1], px * 4, s, false)) != VG_OK ||
-            (st = alloc(acc->counts, (max_depth_alloc + 1) * 4, s, true)) != VG_OK ||
-            (st = alloc(acc->fetch, 2 * (max_depth_alloc + 1) * 4, s, true)) != VG_OK ||
-            (st = alloc(acc->tstats, 8 * 8, s, true)) != VG_OK ||
-            (st = alloc(acc->meta, px * 4, s, false)) != VG_OK ||
-            (st = alloc(acc->sreq, dpx * req_planes * 16, s, false)) != VG_OK ||
-            (st = alloc(acc->squeue, dpx * 4 * vgk::SHADE_CLASSES, s, false)) != VG_OK ||
-            (st = alloc(acc->flags, dpx * 4, s, false)) != VG_OK ||
-            (st = alloc(acc->pend, dpx * pend_planes * 16, s, false)) != VG_OK ||
-            (st = alloc(acc->shqueue, dpx * 4, s, false)) != VG_OK ||
-            (st = alloc(acc->scount, (2 * vgk::SHADE_CLASSES + 2) * 4, s, true)) != VG_OK)
+        if ((st = alloc_parts(acc->wave,
+                              {{&acc->state, px * planes * 16, false},
+                               {&acc->hits, px * 16, false},
+                               {&acc->queue[0], px * 4, false},
+                               {&acc->queue[1], px * 4, false},
+                               {&acc->counts, (max_depth_alloc + 1) * 4, true},
+                               {&acc->fetch, 2 * (max_depth_alloc + 1) * 4, true},
+                               {&acc->tstats, 8 * 8, true},
+                               {&acc->meta, px * 4, false},
+                               {&acc->sreq, dpx * req_planes * 16, false},
+                               {&acc->squeue, dpx * 4 * vgk::SHADE_CLASSES, false},
+                               {&acc->flags, dpx * 4, false},
+                               {&acc->pend, dpx * pend_planes * 16, false},
+                               {&acc->shqueue, dpx * 4, false},
+                               {&acc->scount, (2 * vgk::SHADE_CLASSES + 2) * 4, true}},
+                              s)) != VG_OK)
             return st;
-        if (!acc->host_counts && cudaHostAlloc((void**)&acc->host_counts, 64 * 4, cudaHostAllocDefault) != cudaSuccess) {
-            acc->host_counts = nullptr;
-            return fail(VG_ERR_RESOURCE, "pinned host buffer");
-        }
         acc->wavefront_bytes = acc->state.bytes + acc->hits.bytes + acc->queue[0].bytes + acc->queue[1].bytes +
                                acc->counts.bytes + acc->fetch.bytes;
     }
@@ -1145,7 +1142,13 @@ int vg_accumulate(VgRenderer* r, VgAccum* acc, uint32_t samples)
         }
     }
     VG_CHECK(cudaEventRecord(t1, s), "event");
-    st = wait_event(t1);
+    Ring status(r->ctx);
+    if (!status.words)
+        return fail(VG_ERR_RESOURCE, "pinned host buffer");
+    VG_CHECK(cudaMemcpyAsync(status.words, r->err.p, 4, cudaMemcpyDeviceToHost, s), "error flag");
+    cudaEvent_t t2 = pool.get();
+    VG_CHECK(cudaEventRecord(t2, s), "event");
+    st = wait_event(t2);
     if (st != VG_OK)
         return st;
     float ms = 0.0f;
@@ -1165,7 +1168,7 @@ int vg_accumulate(VgRenderer* r, VgAccum* acc, uint32_t samples)
                 acc->extend_launches_timed++;
         }
     }
-    st = read_err(r);
+    st = err_status(status.words[0]);
     if (st != VG_OK)
         return st;
     if ((st = cache_status(r)) != VG_OK)
@@ -1520,9 +1523,9 @@ int vg_render_normals(VgRenderer* r, uint32_t width, uint32_t height, float* out
         return fail(VG_ERR_SCENE, "image size must be non-zero");
     size_t px = (size_t)width * height;
     cudaStream_t s = r->ctx->stream;
-    DevBuf d;
+    TempBuf d;
     int st;
-    if ((st = alloc(d, px * 12, s, false)) != VG_OK)
+    if ((st = d.get(r->ctx, px * 12)) != VG_OK)
         return st;
     float rec[18];
     camera_record(r, width, height, rec);
@@ -1534,34 +1537,53 @@ int vg_render_normals(VgRenderer* r, uint32_t width, uint32_t height, float* out
     return read_err(r);
 }
 
+// Albedo and depth interleaved (depth null) or each in a plane of its own.
+static int render_aovs(VgRenderer* r, uint32_t width, uint32_t height, float* albedo, float* depth, uint32_t* object_id,
+                       uint32_t* material_id, float* coverage)
+{
+    if (width == 0 || height == 0)
+        return fail(VG_ERR_SCENE, "image size must be non-zero");
+    size_t px = (size_t)width * height;
+    cudaStream_t s = r->ctx->stream;
+    TempBuf d;
+    int st;
+    if ((st = d.get(r->ctx, px * 28)) != VG_OK)
+        return st;
+    float* ad = (float*)d.p;
+    float* dp = depth ? ad + 3 * px : ad + 3;
+    uint32_t *oi = (uint32_t*)d.at(px * 16), *mi = (uint32_t*)d.at(px * 20);
+    float* cv = (float*)d.at(px * 24);
+    float rec[18];
+    camera_record(r, width, height, rec);
+    vgd::Ctx c = make_ctx(r, nullptr);
+    VG_CHECK(cudaMemsetAsync(r->err.p, 0, 4, s), "error flag");
+    VG_CHECK(vgx::launch_aov_main(s, c, rec, ad, depth ? 3 : 4, dp, depth ? 1 : 4, oi, mi, cv), "aov launch");
+    VG_CHECK(cudaMemcpyAsync(albedo, ad, px * (depth ? 12 : 16), cudaMemcpyDeviceToHost, s), "readback");
+    if (depth)
+        VG_CHECK(cudaMemcpyAsync(depth, dp, px * 4, cudaMemcpyDeviceToHost, s), "readback");
+    VG_CHECK(cudaMemcpyAsync(object_id, oi, px * 4, cudaMemcpyDeviceToHost, s), "readback");
+    VG_CHECK(cudaMemcpyAsync(material_id, mi, px * 4, cudaMemcpyDeviceToHost, s), "readback");
+    VG_CHECK(cudaMemcpyAsync(coverage, cv, px * 4, cudaMemcpyDeviceToHost, s), "readback");
+    VG_CHECK(cudaStreamSynchronize(s), "aovs");
+    return read_err(r);
+}
+
 int vg_render_aovs(VgRenderer* r, uint32_t width, uint32_t height, float* albedo_depth, uint32_t* object_id,
                    uint32_t* material_id, float* coverage)
 {
     DevGuard device_guard(dev_of(r));
     if (!r || !albedo_depth || !object_id || !material_id || !coverage)
         return fail(VG_ERR_INVALID, "null argument");
-    if (width == 0 || height == 0)
-        return fail(VG_ERR_SCENE, "image size must be non-zero");
-    size_t px = (size_t)width * height;
-    cudaStream_t s = r->ctx->stream;
-    DevBuf ad, oi, mi, cv;
-    int st;
-    if ((st = alloc(ad, px * 16, s, false)) != VG_OK || (st = alloc(oi, px * 4, s, false)) != VG_OK ||
-        (st = alloc(mi, px * 4, s, false)) != VG_OK || (st = alloc(cv, px * 4, s, false)) != VG_OK)
-        return st;
-    float rec[18];
-    camera_record(r, width, height, rec);
-    vgd::Ctx c = make_ctx(r, nullptr);
-    VG_CHECK(cudaMemsetAsync(r->err.p, 0, 4, s), "error flag");
-    VG_CHECK(vgx::launch_aov_main(s, c, rec, (float*)ad.p, 4, (float*)ad.p + 3, 4, (uint32_t*)oi.p, (uint32_t*)mi.p,
-                                  (float*)cv.p),
-             "aov launch");
-    VG_CHECK(cudaMemcpyAsync(albedo_depth, ad.p, px * 16, cudaMemcpyDeviceToHost, s), "readback");
-    VG_CHECK(cudaMemcpyAsync(object_id, oi.p, px * 4, cudaMemcpyDeviceToHost, s), "readback");
-    VG_CHECK(cudaMemcpyAsync(material_id, mi.p, px * 4, cudaMemcpyDeviceToHost, s), "readback");
-    VG_CHECK(cudaMemcpyAsync(coverage, cv.p, px * 4, cudaMemcpyDeviceToHost, s), "readback");
-    VG_CHECK(cudaStreamSynchronize(s), "aovs");
-    return read_err(r);
+    return render_aovs(r, width, height, albedo_depth, nullptr, object_id, material_id, coverage);
+}
+
+int vg_render_aov_planes(VgRenderer* r, uint32_t width, uint32_t height, float* albedo, float* depth, uint32_t* object_id,
+                         uint32_t* material_id, float* coverage)
+{
+    DevGuard device_guard(dev_of(r));
+    if (!r || !albedo || !depth || !object_id || !material_id || !coverage)
+        return fail(VG_ERR_INVALID, "null argument");
+    return render_aovs(r, width, height, albedo, depth, object_id, material_id, coverage);
 }
 
 int vg_trace_closest_device(VgRenderer* r, const float* d_rays, size_t n, uint32_t* d_hits, double* seconds)
@@ -1600,17 +1622,18 @@ int vg_trace_closest(VgRenderer* r, const float* rays, size_t n, uint32_t* hits)
     DevGuard device_guard(dev_of(r));
     if (!r || (n > 0 && (!rays || !hits)))
         return fail(VG_ERR_INVALID, "null argument");
-    DevBuf dr, dh;
+    TempBuf d; // hits, then rays
     cudaStream_t s = r->ctx->stream;
     int st;
-    if ((st = alloc(dr, n * 24, s, false)) != VG_OK || (st = alloc(dh, n * 16, s, false)) != VG_OK)
+    if ((st = d.get(r->ctx, n * 40)) != VG_OK)
         return st;
+    float* dr = (float*)d.at(n * 16);
     if (n > 0)
-        VG_CHECK(cudaMemcpyAsync(dr.p, rays, n * 24, cudaMemcpyHostToDevice, s), "ray upload");
-    if ((st = vg_trace_closest_device(r, (const float*)dr.p, n, (uint32_t*)dh.p, nullptr)) != VG_OK)
+        VG_CHECK(cudaMemcpyAsync(dr, rays, n * 24, cudaMemcpyHostToDevice, s), "ray upload");
+    if ((st = vg_trace_closest_device(r, dr, n, (uint32_t*)d.p, nullptr)) != VG_OK)
         return st;
     if (n > 0) {
-        VG_CHECK(cudaMemcpyAsync(hits, dh.p, n * 16, cudaMemcpyDeviceToHost, s), "hit readback");
+        VG_CHECK(cudaMemcpyAsync(hits, d.p, n * 16, cudaMemcpyDeviceToHost, s), "hit readback");
         VG_CHECK(cudaStreamSynchronize(s), "hit readback");
     }
     return VG_OK;
@@ -1693,17 +1716,18 @@ int vg_trace_occluded(VgRenderer* r, const float* rays, size_t n, uint32_t* out)
         return fail(VG_ERR_INVALID, "null argument");
     if (n > 0xffffffffull)
         return fail(VG_ERR_INVALID, "too many rays");
-    DevBuf dr, dh;
+    TempBuf d; // results, then rays
     cudaStream_t s = r->ctx->stream;
     int st;
-    if ((st = alloc(dr, n * 28, s, false)) != VG_OK || (st = alloc(dh, n * 4, s, false)) != VG_OK)
+    if ((st = d.get(r->ctx, n * 32)) != VG_OK)
         return st;
+    float* dr = (float*)d.at(n * 4);
     vgd::Ctx c = make_ctx(r, nullptr);
     VG_CHECK(cudaMemsetAsync(r->err.p, 0, 4, s), "error flag");
     if (n > 0) {
-        VG_CHECK(cudaMemcpyAsync(dr.p, rays, n * 28, cudaMemcpyHostToDevice, s), "ray upload");
-        VG_CHECK(vgx::launch_occlusion_rays(s, c, (const float*)dr.p, (uint32_t*)dh.p, (uint32_t)n), "occlusion launch");
-        VG_CHECK(cudaMemcpyAsync(out, dh.p, n * 4, cudaMemcpyDeviceToHost, s), "readback");
+        VG_CHECK(cudaMemcpyAsync(dr, rays, n * 28, cudaMemcpyHostToDevice, s), "ray upload");
+        VG_CHECK(vgx::launch_occlusion_rays(s, c, dr, (uint32_t*)d.p, (uint32_t)n), "occlusion launch");
+        VG_CHECK(cudaMemcpyAsync(out, d.p, n * 4, cudaMemcpyDeviceToHost, s), "readback");
     }
     VG_CHECK(cudaStreamSynchronize(s), "occlusion");
     return read_err(r);
