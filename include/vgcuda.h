@@ -202,12 +202,14 @@ int vg_set_max_depth(VgRenderer* r, uint32_t depth);
  * still added in order, and the sums are identical. ReSTIR always runs per sample. */
 typedef enum VgWavefrontMode { VG_WAVEFRONT_PER_SAMPLE = 0, VG_WAVEFRONT_STREAMING = 1 } VgWavefrontMode;
 int vg_set_wavefront_mode(VgRenderer* r, int mode);
-/* Streaming mode: when at most `threshold` slots are live after a wave, the rest of the batch
- * (those paths and their remaining samples) runs in one launch, trace and shade in a loop per slot,
- * instead of one wave per bounce. 0 disables it. Default 32768. */
+/* Streaming mode: when at most `threshold` slots are live after a wave, or the frame has no more pixels
+ * than that, the rest of the batch (those paths and their remaining samples) runs in one launch instead of
+ * one wave per bounce: with deferred shadows as block wavefronts, without them a path per thread. 0
+ * disables it. Default 262144 (32768 without deferred shadows). */
 int vg_set_stream_tail(VgRenderer* r, uint32_t threshold);
-/* Streaming mode without the lighting split: trace the bounce's emitter / environment shadow ray
- * in a separate stage after shade (default on) or inline in shade (off). Same sums either way. */
+/* Streaming mode: trace the bounce's emitter / environment shadow ray after shade, with the next wave's rays
+ * (default on), or inline in shade (off, and always with ReSTIR GI or ReSTIR with the lighting split). Same sums
+ * either way. */
 int vg_set_deferred_shadows(VgRenderer* r, int on);
 /* Streaming mode: the extend and shadow stages refill a warp's idle lanes with queued rays
  * (default on) or give each warp 32 rays at a time (off). Same results either way. */

@@ -613,7 +613,7 @@ int batch_wave_run(VgContext* ctx, const VgBatchRequest* reqs, size_t n, int ord
     b.err = (uint32_t*)B.err.p;
     b.loop = (uint32_t*)B.loop.p;
     b.t0 = (unsigned long long*)B.t0.p;
-    b.tail = nc ? 0u : std::min(r0->tail_threshold, slots);
+    b.tail = nc ? 0u : std::min(r0->inline_tail_threshold, slots);
     b.caches = nc ? (const vgb::WaveCache*)B.caches.p : nullptr;
     b.ncache = (uint32_t)nc;
     b.spread = nc ? (float2*)B.spread.p : nullptr;

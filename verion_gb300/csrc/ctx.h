@@ -80,6 +80,8 @@ constexpr uint32_t SPLIT_PLANES = 5; // more planes with the lighting split
 constexpr uint32_t REQ_PLANES = 3;       // shadow request planes per slot (Wave::sreq)
 constexpr uint32_t SPLIT_REQ_PLANES = 5; // ... with the lighting split
 
+constexpr uint32_t FINISH_FETCH = 8; // word of Wave::fetch: the finish kernel's place in the queue
+
 // Wave::flags of a path slot.
 constexpr uint32_t SLOT_RAY = 1u;     // its path has a ray to trace and shade
 constexpr uint32_t SLOT_SHADOW = 2u;  // a shadow ray: its contribution goes to the path's radiance

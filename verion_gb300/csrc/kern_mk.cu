@@ -1,44 +1,53 @@
 // Megakernel variants (shaders/pathtrace.slang).
-#include "kernels.cuh"
+#include <algorithm>
+
 #include "launch.h"
+#include "megakernel.cuh"
 
 namespace vgx {
 
-// Persistent form: resident blocks per SM times the SMs, the work counter cleared first; else one
-// 16 x 8 tile per block.
-template <bool L, bool R, typename A>
-static cudaError_t mk(int sms, uint32_t w, uint32_t h, cudaStream_t s, const vgd::Ctx& c, uint32_t* next)
+template <bool L, typename A>
+static cudaError_t mk_tiles(uint32_t w, uint32_t h, cudaStream_t s, const vgd::Ctx& c)
 {
-    if constexpr (vgk::mk_persistent(R)) {
-        static int per_sm = 0;
-        if (per_sm == 0) {
-            if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, vgk::mk_pathtrace<L, R, A>, 128, 0) != cudaSuccess ||
-                per_sm < 1)
-                per_sm = 1;
-        }
-        cudaError_t e = cudaMemsetAsync(next, 0, 4, s);
-        if (e != cudaSuccess)
-            return e;
-        vgk::mk_pathtrace<L, R, A><<<per_sm * sms, 128, 0, s>>>(c, next);
-    } else {
-        vgk::mk_pathtrace<L, R, A><<<dim3((w + 15) / 16, (h + 7) / 8), 128, 0, s>>>(c, next);
-    }
+    vgk::mk_pathtrace_restir<L, A><<<dim3((w + 15) / 16, (h + 7) / 8), 128, 0, s>>>(c);
     return cudaGetLastError();
 }
 
-cudaError_t launch_megakernel(Variant v, int sms, uint32_t w, uint32_t h, cudaStream_t s, const vgd::Ctx& c,
-                              uint32_t* next)
+// A small frame is spread over all SMs, eight paths to a block at least.
+BlockGrid block_grid(int sms, uint64_t items)
 {
-    switch (v.index()) {
-    case 0: return mk<false, false, float>(sms, w, h, s, c, next);
-    case 1: return mk<true, false, float>(sms, w, h, s, c, next);
-    case 2: return mk<false, true, float>(sms, w, h, s, c, next);
-    case 3: return mk<true, true, float>(sms, w, h, s, c, next);
-    case 4: return mk<false, false, double>(sms, w, h, s, c, next);
-    case 5: return mk<true, false, double>(sms, w, h, s, c, next);
-    case 6: return mk<false, true, double>(sms, w, h, s, c, next);
-    default: return mk<true, true, double>(sms, w, h, s, c, next);
-    }
+    uint64_t per = (items + (uint64_t)sms - 1) / (uint64_t)sms;
+    BlockGrid g;
+    g.slots = (uint32_t)std::min<uint64_t>((per + 7) / 8 * 8, vgk::BLOCK_SLOTS);
+    g.blocks = g.slots == 0 ? 0 : (uint32_t)std::min<uint64_t>((uint64_t)sms, (items + g.slots - 1) / g.slots);
+    return g;
+}
+
+bool megakernel_blocks(Variant v, bool gi) { return !v.restir || !(v.light || gi); }
+
+uint64_t megakernel_items(uint32_t w, uint32_t h) { return (uint64_t)((w + 15) / 16) * ((h + 7) / 8) * 128; }
+
+cudaError_t launch_megakernel(Variant v, const BlockGrid& g, cudaStream_t s, const vgd::Ctx& c, const vgk::Wave& w,
+                              uint32_t* pixels, uint32_t* next)
+{
+    cudaError_t e = cudaMemsetAsync(next, 0, 4, s);
+    if (e != cudaSuccess)
+        return e;
+    uint32_t f64 = v.f64 ? 1u : 0u;
+    if (v.restir)
+        vgk::mk_pathtrace<false, true><<<g.blocks, vgk::MK_THREADS, 0, s>>>(c, w, g.slots, f64, pixels, next);
+    else if (v.light)
+        vgk::mk_pathtrace<true, false><<<g.blocks, vgk::MK_THREADS, 0, s>>>(c, w, g.slots, f64, pixels, next);
+    else
+        vgk::mk_pathtrace<false, false><<<g.blocks, vgk::MK_THREADS, 0, s>>>(c, w, g.slots, f64, pixels, next);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_megakernel_restir(Variant v, uint32_t w, uint32_t h, cudaStream_t s, const vgd::Ctx& c)
+{
+    if (v.light)
+        return v.f64 ? mk_tiles<true, double>(w, h, s, c) : mk_tiles<true, float>(w, h, s, c);
+    return v.f64 ? mk_tiles<false, double>(w, h, s, c) : mk_tiles<false, float>(w, h, s, c);
 }
 
 } // namespace vgx

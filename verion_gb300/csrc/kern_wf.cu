@@ -167,36 +167,22 @@ int stream_shade_blocks_per_sm(Variant v)
 
 namespace vgx {
 
-// Few slots go one, two, four or eight to a warp, as many warps as the tail keeps resident (four blocks
-// per SM): a warp then waits for fewer paths' branches and longest walks (Cornell 64x48, 1 sample: 350 ->
-// 336 us a call). From nine on the warps are as many as before and the idle lanes only cost issue slots
-// (sixteen of 32 on 30,000 slots of a 110k-triangle scene: 1.94 ms a call against 1.69).
-unsigned tail_blocks(uint32_t max_slots, int sms, uint32_t* lanes)
-{
-    uint32_t l = 1;
-    while (l < 32 && (uint64_t)l * sms * 16 < max_slots)
-        l = l < 8 ? 2 * l : 32;
-    *lanes = l;
-    return (unsigned)(((uint64_t)max_slots + 4 * l - 1) / (4 * l));
-}
-
-cudaError_t launch_stream_tail(Variant v, uint32_t max_slots, int sms, cudaStream_t s, const vgd::Ctx& c, const vgk::Wave& w,
+cudaError_t launch_stream_tail(Variant v, uint32_t max_slots, cudaStream_t s, const vgd::Ctx& c, const vgk::Wave& w,
                                uint32_t wave)
 {
     if (v.restir)
-        return launch_stream_tail_restir(v, max_slots, sms, s, c, w, wave);
-    uint32_t lanes = 0;
-    unsigned blocks = tail_blocks(max_slots, sms, &lanes);
+        return launch_stream_tail_restir(v, max_slots, s, c, w, wave);
+    unsigned blocks = (max_slots + 127) / 128;
     if (blocks == 0)
         return cudaSuccess;
     if (v.light && v.f64)
-        vgk::wf_stream_tail<true, double><<<blocks, 128, 0, s>>>(c, w, wave, lanes, vgk::CacheWave{});
+        vgk::wf_stream_tail<true, double><<<blocks, 128, 0, s>>>(c, w, wave);
     else if (v.light)
-        vgk::wf_stream_tail<true, float><<<blocks, 128, 0, s>>>(c, w, wave, lanes, vgk::CacheWave{});
+        vgk::wf_stream_tail<true, float><<<blocks, 128, 0, s>>>(c, w, wave);
     else if (v.f64)
-        vgk::wf_stream_tail<false, double><<<blocks, 128, 0, s>>>(c, w, wave, lanes, vgk::CacheWave{});
+        vgk::wf_stream_tail<false, double><<<blocks, 128, 0, s>>>(c, w, wave);
     else
-        vgk::wf_stream_tail<false, float><<<blocks, 128, 0, s>>>(c, w, wave, lanes, vgk::CacheWave{});
+        vgk::wf_stream_tail<false, float><<<blocks, 128, 0, s>>>(c, w, wave);
     return cudaGetLastError();
 }
 
@@ -270,20 +256,6 @@ int stream_cache_shade_blocks_per_sm()
     int n = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, vgk::wf_stream_shade_deferred<true>, 128, 0);
     return n > 0 ? n : 1;
-}
-
-cudaError_t launch_stream_cache_tail(bool f64, uint32_t max_slots, int sms, cudaStream_t s, const vgd::Ctx& c,
-                                     const vgk::Wave& w, uint32_t wave, const vgk::CacheWave& q)
-{
-    uint32_t lanes = 0;
-    unsigned blocks = tail_blocks(max_slots, sms, &lanes);
-    if (blocks == 0)
-        return cudaSuccess;
-    if (f64)
-        vgk::wf_stream_tail<false, double, true><<<blocks, 128, 0, s>>>(c, w, wave, lanes, q);
-    else
-        vgk::wf_stream_tail<false, float, true><<<blocks, 128, 0, s>>>(c, w, wave, lanes, q);
-    return cudaGetLastError();
 }
 
 cudaError_t launch_stream_shadow_layers(int blocks, cudaStream_t s, const vgd::Ctx& c, const vgk::Wave& w,

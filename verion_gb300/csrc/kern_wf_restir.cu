@@ -41,21 +41,20 @@ int stream_shade_restir_blocks_per_sm(Variant v)
     return rshade_occ<false, float>();
 }
 
-cudaError_t launch_stream_tail_restir(Variant v, uint32_t max_slots, int sms, cudaStream_t s, const vgd::Ctx& c,
+cudaError_t launch_stream_tail_restir(Variant v, uint32_t max_slots, cudaStream_t s, const vgd::Ctx& c,
                                       const vgk::Wave& w, uint32_t wave)
 {
-    uint32_t lanes = 0;
-    unsigned blocks = tail_blocks(max_slots, sms, &lanes);
+    unsigned blocks = (max_slots + 127) / 128;
     if (blocks == 0)
         return cudaSuccess;
     if (v.light && v.f64)
-        vgk::wf_stream_tail<true, double, false, true><<<blocks, 128, 0, s>>>(c, w, wave, lanes, vgk::CacheWave{});
+        vgk::wf_stream_tail<true, double, true><<<blocks, 128, 0, s>>>(c, w, wave);
     else if (v.light)
-        vgk::wf_stream_tail<true, float, false, true><<<blocks, 128, 0, s>>>(c, w, wave, lanes, vgk::CacheWave{});
+        vgk::wf_stream_tail<true, float, true><<<blocks, 128, 0, s>>>(c, w, wave);
     else if (v.f64)
-        vgk::wf_stream_tail<false, double, false, true><<<blocks, 128, 0, s>>>(c, w, wave, lanes, vgk::CacheWave{});
+        vgk::wf_stream_tail<false, double, true><<<blocks, 128, 0, s>>>(c, w, wave);
     else
-        vgk::wf_stream_tail<false, float, false, true><<<blocks, 128, 0, s>>>(c, w, wave, lanes, vgk::CacheWave{});
+        vgk::wf_stream_tail<false, float, true><<<blocks, 128, 0, s>>>(c, w, wave);
     return cudaGetLastError();
 }
 

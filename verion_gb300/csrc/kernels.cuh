@@ -224,122 +224,6 @@ __device__ __forceinline__ PathState<LIGHT> loadPath(const Ctx& c, const Wave& w
     return s;
 }
 
-// Minimum resident 128-thread blocks per SM requested for the megakernel (a register cap; 0: none).
-// Its threads spend most of their time waiting on dependent node loads in the traversal, so
-// occupancy pays more than registers: on the 1M-triangle workload at 1080p, 72.8 Mpaths/s with no
-// cap (168 registers, 3 blocks per SM), 88.9 at 8 blocks (64 registers), 102.4 at 12, 114.1 at 16
-// (32 registers, every warp slot of the SM; the spills mostly stay in L1 and L2).
-#ifndef VG_MK_MIN_BLOCKS
-#define VG_MK_MIN_BLOCKS 16
-#endif
-#if VG_MK_MIN_BLOCKS > 0
-#define VG_MK_BOUNDS __launch_bounds__(128, VG_MK_MIN_BLOCKS)
-#else
-#define VG_MK_BOUNDS __launch_bounds__(128)
-#endif
-
-// Idle lanes at or above which a megakernel warp takes new pixels (VG_MK_PERSISTENT).
-#ifndef VG_MK_REFILL
-#define VG_MK_REFILL 4
-#endif
-#ifndef VG_MK_PERSISTENT
-#define VG_MK_PERSISTENT 1
-#endif
-
-// Whether a megakernel instantiation is the persistent form. ReSTIR frames keep one tile per block:
-// with one sample per launch the refills cost more than they save (the many-light ReSTIR frame
-// 15.6 ms persistent against 13.0 ms; plain frames 119.9 against 113.9 Mpaths/s on the
-// 1M-triangle workload, 5.9 against 6.7 ms per many-light frame).
-__host__ __device__ constexpr bool mk_persistent(bool restir) { return VG_MK_PERSISTENT && !restir; }
-
-// pathtrace.slang:9-26: params[35] samples from params[6] for every pixel, each pixel's samples in
-// order in one thread. One loop over bounces: a lane whose path ends adds it and starts its
-// pixel's next sample in the same iteration. Persistent (mk_persistent: frames without ReSTIR): a
-// grid that fills the SMs once, whose warps take pixels from the work counter `next` (one atomic per
-// refill) whenever at least VG_MK_REFILL lanes have finished theirs, so a warp does not idle on its
-// longest pixel; else one 16 x 8 tile per block. Same samples, same order per pixel, same sums.
-template <bool LIGHT, bool RESTIR, typename A>
-__global__ void VG_MK_BOUNDS mk_pathtrace(const __grid_constant__ Ctx c, uint32_t* next)
-{
-    uint32_t width = c.p[P_WIDTH];
-    uint32_t n = c.p[P_SAMPLES_PER_DISPATCH];
-    bool adaptive = c.p[P_ADAPTIVE] != 0;
-    if constexpr (mk_persistent(RESTIR)) {
-        // Work items in 16 x 8 tiles (128 consecutive items per tile), so a warp's 32 pixels are a
-        // 16 x 2 block as in the one-tile-per-block form; items outside the frame are skipped.
-        uint32_t height = c.p[P_HEIGHT];
-        uint32_t tiles_x = (width + 15) / 16;
-        uint32_t nitems = tiles_x * ((height + 7) / 8) * 128u;
-        uint32_t lane = lane_id(), lt = (1u << lane) - 1u;
-        bool active = false, exhausted = n == 0;
-        uint32_t pixel = 0, k = 0, depth = 0;
-        PathState<LIGHT> st;
-        for (;;) {
-            uint32_t idle = __ballot_sync(FULL, !active);
-            if (!exhausted && (idle == FULL || (uint32_t)__popc(idle) >= VG_MK_REFILL)) {
-                uint32_t cnt = __popc(idle), base = 0;
-                if (lane == 0)
-                    base = atomicAdd(next, cnt);
-                base = __shfl_sync(FULL, base, 0);
-                exhausted = base + cnt >= nitems;
-                if (!active) {
-                    uint32_t idx = base + __popc(idle & lt);
-                    uint32_t t = idx >> 7, r = idx & 127u;
-                    uint32_t x = (t % tiles_x) * 16 + (r & 15u), y = (t / tiles_x) * 8 + (r >> 4);
-                    if (idx < nitems && x < width && y < height && !(adaptive && !pixelActive<A>(c, y * width + x))) {
-                        pixel = y * width + x;
-                        k = 0;
-                        depth = 0;
-                        st = generatePathFor<LIGHT>(c, x, y, c.p[P_SAMPLE]);
-                        active = true;
-                    }
-                }
-            }
-            if (__ballot_sync(FULL, active) == 0) {
-                if (exhausted)
-                    break;
-                continue;
-            }
-            if (active) {
-                if (shadePathCall<LIGHT, RESTIR>(c, st, traceClosest(c, st.org, st.dir), depth, pixel) &&
-                    depth + 1 < c.p[P_MAX_DEPTH]) {
-                    depth++;
-                } else {
-                    finishPath<LIGHT, A, RESTIR>(c, st, pixel);
-                    if (++k < n && !(adaptive && !pixelActive<A>(c, pixel))) {
-                        depth = 0;
-                        st = generatePathFor<LIGHT>(c, pixel % width, pixel / width, c.p[P_SAMPLE] + k);
-                    } else {
-                        active = false;
-                    }
-                }
-            }
-        }
-    } else {
-        uint32_t x = blockIdx.x * 16 + (threadIdx.x & 15u);
-        uint32_t y = blockIdx.y * 8 + (threadIdx.x >> 4);
-        if (x >= width || y >= c.p[P_HEIGHT])
-            return;
-        uint32_t pixel = y * width + x;
-        if (n == 0 || (adaptive && !pixelActive<A>(c, pixel)))
-            return;
-        uint32_t k = 0, depth = 0;
-        PathState<LIGHT> st = generatePathFor<LIGHT>(c, x, y, c.p[P_SAMPLE]);
-        for (;;) {
-            if (shadePathCall<LIGHT, RESTIR>(c, st, traceClosest(c, st.org, st.dir), depth, pixel) &&
-                depth + 1 < c.p[P_MAX_DEPTH]) {
-                depth++;
-                continue;
-            }
-            finishPath<LIGHT, A, RESTIR>(c, st, pixel);
-            if (++k >= n || (adaptive && !pixelActive<A>(c, pixel)))
-                break;
-            depth = 0;
-            st = generatePathFor<LIGHT>(c, x, y, c.p[P_SAMPLE] + k);
-        }
-    }
-}
-
 // wf_args.slang:9-24 at depth 0: starts a sample. Every pixel's path is live unless adaptive
 // sampling fills the depth-0 queue (wf_select); the later queues and all work counters restart.
 static __global__ void wf_begin(const __grid_constant__ Ctx c, const __grid_constant__ Wave w)
@@ -513,6 +397,8 @@ __global__ void __launch_bounds__(256) wf_stream_start(const __grid_constant__ C
     __shared__ uint32_t slot[8];
     uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
     bool live = false;
+    if (p == 0)
+        w.fetch[FINISH_FETCH] = 0;
     if (p < w.n && c.p[P_SAMPLES_PER_DISPATCH] > 0 && (c.p[P_ADAPTIVE] == 0 || pixelActive<A>(c, p)) &&
         !(CACHE && (p + q.train_offset) % q.train_stride == 0)) {
         PathState<LIGHT> st = generatePathFor<LIGHT>(c, p % c.p[P_WIDTH], p / c.p[P_WIDTH], c.p[P_SAMPLE]);
@@ -624,11 +510,11 @@ __global__ void __launch_bounds__(128, VG_SHADE_MIN_BLOCKS) wf_stream_shade(cons
     }
 }
 
-// What a slot's shadow ray (SLOT_SHADOW) decides once it is traced, in the order of the pixel's samples:
+// What the shadow ray (SLOT_SHADOW) of slot p, of pixel `pixel`, decides once it is traced, in the order of the pixel's samples:
 // its contribution is the last add of the vertex that asked for it. Returns whether the slot still has
 // a path to go on with.
 template <typename A, bool RESTIR, bool LIGHT = false>
-__device__ __forceinline__ bool resolveSlot(const Ctx& c, const Wave& w, uint32_t p, uint32_t fl, bool blocked)
+__device__ __forceinline__ bool resolveSlot(const Ctx& c, const Wave& w, uint32_t p, uint32_t pixel, uint32_t fl, bool blocked)
 {
     uint32_t n = w.n;
     if constexpr (LIGHT) {
@@ -663,14 +549,14 @@ __device__ __forceinline__ bool resolveSlot(const Ctx& c, const Wave& w, uint32_
                 st.visTotal += vv;
                 st.visLit += blocked ? 0.0f : vv;
                 if (bits & 8u)
-                    addSlot(c, p, 3u, cd / cosi, cs / cosi, v3(r1.x, r1.y, r1.z), blocked ? 0.0f : 1.0f, blocked ? 0.0f : cosi);
+                    addSlot(c, pixel, 3u, cd / cosi, cs / cosi, v3(r1.x, r1.y, r1.z), blocked ? 0.0f : 1.0f, blocked ? 0.0f : cosi);
             }
         }
         if (fl & SLOT_ENDED) {
             st.gi = false;
             st.chan = -1;
-            finishPath<true, A, RESTIR>(c, st, p);
-            return (fl & SLOT_RAY) && (c.p[P_ADAPTIVE] == 0 || pixelActive<A>(c, p));
+            finishPath<true, A, RESTIR>(c, st, pixel);
+            return (fl & SLOT_RAY) && (c.p[P_ADAPTIVE] == 0 || pixelActive<A>(c, pixel));
         }
         const Parts<true>& t = st.parts;
         P[p] = make_float4(t.total.x, t.total.y, t.total.z, q[0].w);
@@ -696,10 +582,10 @@ __device__ __forceinline__ bool resolveSlot(const Ctx& c, const Wave& w, uint32_
         // when GI is on), so the path's GI flag is false here.
         st.gi = false;
         st.chan = -1;
-        finishPath<false, A, RESTIR>(c, st, p);
+        finishPath<false, A, RESTIR>(c, st, pixel);
         // The next sample was started before this one's radiance was known: it is dropped untouched when
         // the pixel takes no more.
-        return (fl & SLOT_RAY) && (c.p[P_ADAPTIVE] == 0 || pixelActive<A>(c, p));
+        return (fl & SLOT_RAY) && (c.p[P_ADAPTIVE] == 0 || pixelActive<A>(c, pixel));
     }
     if (lit) {
         float4 t = w.state[3 * n + p], r = w.sreq[2 * n + p];
@@ -751,13 +637,93 @@ __global__ void __launch_bounds__(256) wf_stream_resolve(const __grid_constant__
         if (i < count) {
             p = qin[i];
             uint32_t fl = w.flags[p];
-            live = resolveSlot<A, RESTIR, LIGHT>(c, w, p, fl, (fl & SLOT_BLOCKED) != 0);
+            live = resolveSlot<A, RESTIR, LIGHT>(c, w, p, p, fl, (fl & SLOT_BLOCKED) != 0);
             if (SORT && live)
                 cls = shadeClass(c, w.hits[p]);
         }
         block_append_classes<8, SORT ? SHADE_CLASSES : 0>(&w.counts[out], w.queue[out], live,
                                                           w.scount + in * SHADE_CLASSES, w.squeue, w.n, cls, p, slot);
     }
+}
+
+// Shades the hit of slot p, of pixel `pixel`, without any traversal: its path goes on, or ends and the
+// pixel's next sample starts in its place (a path that ends leaves its radiance in w.pend). Returns
+// whether the vertex's light sample needs a shadow ray, left in w.sreq. With CACHE: the hook, the path's sample within the batch and whether it ended at the cache.
+template <bool CACHE, bool RESTIR, bool LIGHT>
+__device__ __forceinline__ bool shadeSlot(const Ctx& c, const Wave& w, uint32_t p, uint32_t pixel, const CacheWave& q,
+                                          CacheHook& hk, uint32_t& kq, bool& query)
+{
+    uint32_t n = w.n, meta = w.meta[p], depth = meta & 0xffu;
+    kq = meta >> 8;
+    PathState<LIGHT> st = loadState<LIGHT>(w, p);
+    uint4 hr = w.hits[p];
+    Hit h;
+    h.hit = hr.x != 0;
+    h.inst = hr.y;
+    h.prim = hr.z;
+    h.t = __uint_as_float(hr.w);
+    ShadowReq req;
+    if (CACHE) {
+        // The spread starts at zero with each sample (a path may pass a cut-out surface at
+        // depth 0 without meeting the hook).
+        float2 sp = depth > 0 ? q.st[p] : make_float2(0.0f, 0.0f);
+        hk.c = q.spread;
+        hk.train = false;
+        hk.a0 = sp.x;
+        hk.a = sp.y;
+    }
+    bool alive = shadePath<LIGHT, RESTIR, true, CACHE>(c, st, h, depth, pixel, &req, &hk) && depth + 1 < w.depth;
+    if (CACHE) {
+        query = hk.query && !bad3(st.parts.total);
+        if (alive)
+            q.st[p] = make_float2(hk.a0, hk.a);
+    }
+    uint32_t fl = SLOT_RAY;
+    if (alive) {
+        w.meta[p] = (depth + 1) | (kq << 8);
+    } else {
+        w.pend[p] = make_float4(st.parts.total.x, st.parts.total.y, st.parts.total.z, 0.0f);
+        if (LIGHT)
+            store_split(w.pend + n, n, st, p);
+        fl = SLOT_ENDED;
+        if (kq + 1 < c.p[P_SAMPLES_PER_DISPATCH]) {
+            fl |= SLOT_RAY;
+            st = generatePathFor<LIGHT>(c, pixel % c.p[P_WIDTH], pixel / c.p[P_WIDTH], c.p[P_SAMPLE] + kq + 1);
+            w.meta[p] = (kq + 1) << 8;
+        }
+    }
+    if (fl & SLOT_RAY)
+        storePath<LIGHT>(w, st, p);
+    if (req.valid) {
+        fl |= SLOT_SHADOW;
+        w.sreq[p] = make_float4(req.o.x, req.o.y, req.o.z, req.tmax);
+        w.sreq[n + p] = make_float4(req.d.x, req.d.y, req.d.z, 0.0f);
+        w.sreq[2 * (size_t)n + p] = make_float4(req.c.x, req.c.y, req.c.z, 0.0f);
+        if (LIGHT) {
+            w.sreq[3 * (size_t)n + p] = make_float4(req.cd.x, req.cd.y, req.cd.z, req.cosi);
+            w.sreq[4 * (size_t)n + p] = make_float4(req.cs.x, req.cs.y, req.cs.z, __uint_as_float(req.bits));
+        }
+    }
+    w.flags[p] = fl;
+    return req.valid;
+}
+
+// The `query` lanes of a converged warp leave their paths' query records: those of sample kq go to range kq
+// (one atomic per sample present in the warp).
+static __device__ __forceinline__ void append_queries(const CacheWave& q, bool query, uint32_t kq, const CacheHook& hk,
+                                                      uint32_t pixel)
+{
+    if (!__ballot_sync(FULL, query))
+        return;
+    uint32_t grp = __match_any_sync(FULL, query ? kq : 0xffffffffu);
+    uint32_t leader = __ffs(grp) - 1u;
+    uint32_t first = 0;
+    if (query && lane_id() == leader)
+        first = atomicAdd(q.qcount + kq, __popc(grp));
+    first = __shfl_sync(FULL, first, leader);
+    uint32_t slot = first + __popc(grp & ((1u << lane_id()) - 1u));
+    if (query && slot < q.qcap)
+        cacheQueryRecord(q.qrec + ((size_t)kq * q.qcap + slot) * CACHE_REC_WORDS, hk, pixel);
 }
 
 // Streaming wave in three stages: trace, resolve, then shade without any traversal.
@@ -777,7 +743,6 @@ __global__ void __launch_bounds__(128, RESTIR ? VG_RESTIR_SHADE_MIN_BLOCKS : VG_
     uint32_t count = w.counts[out];
     const uint32_t* qin = w.queue[out];
     uint32_t n = w.n;
-    uint32_t batch = c.p[P_SAMPLES_PER_DISPATCH];
     uint32_t seg[SHADE_CLASSES + 1] = {0, 0, 0, 0, 0};
     if (SORTED)
         for (uint32_t k = 0; k < SHADE_CLASSES; k++)
@@ -797,75 +762,12 @@ __global__ void __launch_bounds__(128, RESTIR ? VG_RESTIR_SHADE_MIN_BLOCKS : VG_
             } else {
                 p = qin[i];
             }
-            uint32_t meta = w.meta[p];
-            uint32_t depth = meta & 0xffu;
-            kq = meta >> 8;
-            PathState<LIGHT> st = loadState<LIGHT>(w, p);
-            uint4 hr = w.hits[p];
-            Hit h;
-            h.hit = hr.x != 0;
-            h.inst = hr.y;
-            h.prim = hr.z;
-            h.t = __uint_as_float(hr.w);
-            ShadowReq req;
-            if (CACHE) {
-                // The spread starts at zero with each sample (a path may pass a cut-out surface at
-                // depth 0 without meeting the hook).
-                float2 sp = depth > 0 ? q.st[p] : make_float2(0.0f, 0.0f);
-                hk.c = q.spread;
-                hk.train = false;
-                hk.a0 = sp.x;
-                hk.a = sp.y;
-            }
-            bool alive = shadePath<LIGHT, RESTIR, true, CACHE>(c, st, h, depth, p, &req, &hk) && depth + 1 < w.depth;
-            if (CACHE) {
-                query = hk.query && !bad3(st.parts.total);
-                if (alive)
-                    q.st[p] = make_float2(hk.a0, hk.a);
-            }
-            uint32_t fl = SLOT_RAY;
-            if (alive) {
-                w.meta[p] = (depth + 1) | (kq << 8);
-            } else {
-                w.pend[p] = make_float4(st.parts.total.x, st.parts.total.y, st.parts.total.z, 0.0f);
-                if (LIGHT)
-                    store_split(w.pend + n, n, st, p);
-                fl = SLOT_ENDED;
-                if (kq + 1 < batch) {
-                    fl |= SLOT_RAY;
-                    st = generatePathFor<LIGHT>(c, p % c.p[P_WIDTH], p / c.p[P_WIDTH], c.p[P_SAMPLE] + kq + 1);
-                    w.meta[p] = (kq + 1) << 8;
-                }
-            }
-            if (fl & SLOT_RAY)
-                storePath<LIGHT>(w, st, p);
-            shadow = req.valid;
-            if (shadow) {
-                fl |= SLOT_SHADOW;
-                w.sreq[p] = make_float4(req.o.x, req.o.y, req.o.z, req.tmax);
-                w.sreq[n + p] = make_float4(req.d.x, req.d.y, req.d.z, 0.0f);
-                w.sreq[2 * n + p] = make_float4(req.c.x, req.c.y, req.c.z, 0.0f);
-                if (LIGHT) {
-                    w.sreq[3 * (size_t)n + p] = make_float4(req.cd.x, req.cd.y, req.cd.z, req.cosi);
-                    w.sreq[4 * (size_t)n + p] = make_float4(req.cs.x, req.cs.y, req.cs.z, __uint_as_float(req.bits));
-                }
-            }
-            w.flags[p] = fl;
+            shadow = shadeSlot<CACHE, RESTIR, LIGHT>(c, w, p, p, q, hk, kq, query);
         }
         __syncwarp();
         warp_append(&w.shcount[out], w.shqueue, shadow, p);
-        if (CACHE && __ballot_sync(FULL, query)) {
-            // Records of sample kq go to range kq (one atomic per sample present in the warp).
-            uint32_t grp = __match_any_sync(FULL, query ? kq : 0xffffffffu);
-            uint32_t leader = __ffs(grp) - 1u;
-            uint32_t first = 0;
-            if (query && lane_id() == leader)
-                first = atomicAdd(q.qcount + kq, __popc(grp));
-            first = __shfl_sync(FULL, first, leader);
-            uint32_t slot = first + __popc(grp & ((1u << lane_id()) - 1u));
-            if (query && slot < q.qcap)
-                cacheQueryRecord(q.qrec + ((size_t)kq * q.qcap + slot) * CACHE_REC_WORDS, hk, p);
-        }
+        if (CACHE)
+            append_queries(q, query, kq, hk, p);
         __syncwarp();
     }
 }
@@ -1034,64 +936,33 @@ __global__ void __launch_bounds__(128, VG_TRACE_MIN_BLOCKS) wf_stream_shadow_tra
         warp_count(&w.tstats[4], n_rays);
 }
 
-// The tail of a streaming batch: once few slots are live, one thread per remaining slot runs its
-// path and the rest of its samples to the end, trace and shade in a loop as the megakernel does,
-// instead of one half-empty wave per bounce. Same functions, same order per pixel, same sums.
-// With CACHE (lighting split off) paths end at the cache as in wf_stream_shade_deferred.
-template <bool LIGHT, typename A, bool CACHE = false, bool RESTIR = false>
+// The tail of a streaming batch whose shade stage traces the light samples itself: once few slots are live,
+// one thread per remaining slot runs its path and the rest of its samples to the end, trace and shade in a
+// loop, instead of one half-empty wave per bounce. Same functions, same order per pixel, same sums.
+// (With deferred shadows: wf_stream_finish.)
+template <bool LIGHT, typename A, bool RESTIR = false>
 __global__ void __launch_bounds__(128, VG_TAIL_MIN_BLOCKS) wf_stream_tail(const __grid_constant__ Ctx c, const __grid_constant__ Wave w,
-                                                                          uint32_t wave, uint32_t lanes,
-                                                                          const __grid_constant__ CacheWave q)
+                                                                          uint32_t wave)
 {
-    static_assert(!(CACHE && LIGHT), "the cache runs with the lighting split off");
     uint32_t in = wave & 1u;
-    uint32_t i = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * lanes + lane_id();
-    if (lane_id() >= lanes || i >= w.counts[in])
+    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= w.counts[in])
         return;
     uint32_t p = w.queue[in][i];
-    if (w.flags) {
-        // A wave's shadow ray is still to be traced, and the path before this one may wait for it.
-        uint32_t fl = w.flags[p];
-        bool blocked = false;
-        if (fl & SLOT_SHADOW) {
-            V3 o, d;
-            float tmax;
-            slot_shadow_ray(w, p, o, d, tmax);
-            blocked = occluded(c, o, d, tmax);
-        }
-        if (!resolveSlot<A, RESTIR, LIGHT>(c, w, p, fl, blocked))
-            return;
-    }
     uint32_t meta = w.meta[p];
     uint32_t depth = meta & 0xffu, k = meta >> 8;
     uint32_t batch = c.p[P_SAMPLES_PER_DISPATCH];
     PathState<LIGHT> st = loadState<LIGHT>(w, p);
-    CacheHook hk;
-    if (CACHE) {
-        float2 sp = depth > 0 ? q.st[p] : make_float2(0.0f, 0.0f);
-        hk.c = q.spread;
-        hk.train = false;
-        hk.a0 = sp.x;
-        hk.a = sp.y;
-    }
     for (;;) {
-        if (shadePathCall<LIGHT, RESTIR, false, CACHE>(c, st, traceClosest(c, st.org, st.dir), depth, p, nullptr, &hk) &&
-            depth + 1 < w.depth) {
+        if (shadePathCall<LIGHT, RESTIR>(c, st, traceClosest(c, st.org, st.dir), depth, p) && depth + 1 < w.depth) {
             depth++;
             continue;
-        }
-        if (CACHE && hk.query && !bad3(st.parts.total)) {
-            uint32_t slot = atomicAdd(q.qcount + k, 1u);
-            if (slot < q.qcap)
-                cacheQueryRecord(q.qrec + ((size_t)k * q.qcap + slot) * CACHE_REC_WORDS, hk, p);
         }
         finishPath<LIGHT, A, RESTIR>(c, st, p);
         if (k + 1 < batch && (c.p[P_ADAPTIVE] == 0 || pixelActive<A>(c, p))) {
             k++;
             depth = 0;
             st = generatePathFor<LIGHT>(c, p % c.p[P_WIDTH], p / c.p[P_WIDTH], c.p[P_SAMPLE] + k);
-            if (CACHE)
-                hk.a0 = hk.a = 0.0f;
             continue;
         }
         break;

@@ -16,9 +16,21 @@ struct Variant {
     int index() const { return (light ? 1 : 0) | (restir ? 2 : 0) | (f64 ? 4 : 0); }
 };
 
-// The megakernel over a w x h frame; `next` is a device word (its pixel counter).
-cudaError_t launch_megakernel(Variant v, int sms, uint32_t w, uint32_t h, cudaStream_t s, const vgd::Ctx& c,
-                              uint32_t* next);
+// The block wavefront (megakernel.cuh) over `items` pixels or slots: one block per SM, `slots` paths to a block.
+struct BlockGrid {
+    uint32_t blocks, slots;
+};
+BlockGrid block_grid(int sms, uint64_t items);
+// The megakernel over a frame. w's planes hold blocks x slots paths, as many words are at `pixels`; `next` is a
+// device word, its pixel counter. Without megakernel_blocks: one path per thread, launch_megakernel_restir.
+bool megakernel_blocks(Variant v, bool gi);
+uint64_t megakernel_items(uint32_t w, uint32_t h);
+cudaError_t launch_megakernel(Variant v, const BlockGrid& g, cudaStream_t s, const vgd::Ctx& c, const vgk::Wave& w,
+                              uint32_t* pixels, uint32_t* next);
+cudaError_t launch_megakernel_restir(Variant v, uint32_t w, uint32_t h, cudaStream_t s, const vgd::Ctx& c);
+// With deferred shadows: finishes every slot live after `wave`; with `q` the radiance cache's paths.
+cudaError_t launch_stream_finish(Variant v, const BlockGrid& g, cudaStream_t s, const vgd::Ctx& c, const vgk::Wave& w,
+                                 uint32_t wave, const vgk::CacheWave* q);
 cudaError_t launch_wf_shade(Variant v, int blocks, cudaStream_t s, const vgd::Ctx& c, const vgk::Wave& w, uint32_t d);
 int wf_shade_blocks_per_sm(Variant v);
 
@@ -39,8 +51,6 @@ cudaError_t launch_stream_cache_start(bool f64, cudaStream_t s, const vgd::Ctx& 
 cudaError_t launch_stream_cache_shade(bool sorted, int blocks, cudaStream_t s, const vgd::Ctx& c,
                                       const vgk::Wave& w, uint32_t wave, const vgk::CacheWave& q);
 int stream_cache_shade_blocks_per_sm();
-cudaError_t launch_stream_cache_tail(bool f64, uint32_t max_slots, int sms, cudaStream_t s, const vgd::Ctx& c,
-                                     const vgk::Wave& w, uint32_t wave, const vgk::CacheWave& q);
 // With `sorted` the resolve stage also fills the class queues and the shade stage takes the wave's slots
 // class by class.
 cudaError_t launch_stream_shade_deferred(bool sorted, int blocks, cudaStream_t s, const vgd::Ctx& c,
@@ -66,23 +76,21 @@ int stream_shadow_trace_blocks_per_sm();
 cudaError_t launch_stream_shade_restir(Variant v, int blocks, cudaStream_t s, const vgd::Ctx& c, const vgk::Wave& w,
                                        uint32_t wave);
 int stream_shade_restir_blocks_per_sm(Variant v);
-cudaError_t launch_stream_tail_restir(Variant v, uint32_t max_slots, int sms, cudaStream_t s, const vgd::Ctx& c,
+cudaError_t launch_stream_tail_restir(Variant v, uint32_t max_slots, cudaStream_t s, const vgd::Ctx& c,
                                       const vgk::Wave& w, uint32_t wave);
 cudaError_t launch_stream_shade_deferred_restir(bool sorted, int blocks, cudaStream_t s, const vgd::Ctx& c,
                                                 const vgk::Wave& w, uint32_t wave);
 int stream_deferred_restir_blocks_per_sm();
 cudaError_t launch_stream_resolve_restir(bool f64, bool sorted, int blocks, cudaStream_t s, const vgd::Ctx& c,
                                          const vgk::Wave& w, uint32_t wave);
-// Blocks of the tail over at most max_slots slots, and how many slots each of its warps takes.
-unsigned tail_blocks(uint32_t max_slots, int sms, uint32_t* lanes);
 // The deferred stages with the lighting split (kern_wf_light.cu).
 cudaError_t launch_stream_shade_deferred_light(bool sorted, int blocks, cudaStream_t s, const vgd::Ctx& c,
                                                const vgk::Wave& w, uint32_t wave);
 int stream_deferred_light_blocks_per_sm();
 cudaError_t launch_stream_resolve_light(bool f64, bool sorted, int blocks, cudaStream_t s, const vgd::Ctx& c,
                                         const vgk::Wave& w, uint32_t wave);
-// Finishes every slot still live after `wave` (at most max_slots of them) in one launch.
-cudaError_t launch_stream_tail(Variant v, uint32_t max_slots, int sms, cudaStream_t s, const vgd::Ctx& c, const vgk::Wave& w,
+// Without deferred shadows: finishes every slot still live after `wave` (at most max_slots of them) in one launch.
+cudaError_t launch_stream_tail(Variant v, uint32_t max_slots, cudaStream_t s, const vgd::Ctx& c, const vgk::Wave& w,
                                uint32_t wave);
 // Primary-hit AOVs (normals.slang, aov.slang); camera18 is the reference's camera record.
 cudaError_t launch_aov_normals(cudaStream_t s, const vgd::Ctx& c, const float* camera18, float* out);

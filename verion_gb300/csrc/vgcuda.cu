@@ -266,6 +266,15 @@ int stream_samples(VgRenderer* r, VgAccum* acc, vgd::Ctx& c, vgx::Variant v, con
         acc->launches++;
         return e != cudaSuccess ? e : mark(2);
     };
+    // All that is left, at most `slots` live slots, in one launch after the waves before `i`.
+    auto launch_tail = [&](uint32_t slots, uint32_t i) {
+        return deferred ? vgx::launch_stream_finish(v, vgx::block_grid(r->ctx->sms, slots), s, c, w, i, q)
+                        : vgx::launch_stream_tail(v, slots, s, c, w, i);
+    };
+    // Counted calls keep to the waves, whose kernels count, for as long as they did with the inline tail.
+    const uint32_t tail = !deferred ? r->inline_tail_threshold
+                          : r->traversal_stats ? std::min(r->tail_threshold, r->inline_tail_threshold)
+                                               : r->tail_threshold;
     c.p[P_SAMPLE] = sample0;
     c.p[P_SAMPLES_PER_DISPATCH] = samples;
     VG_CHECK(cudaMemsetAsync(acc->counts.p, 0, 2 * 4, s), "counters");
@@ -288,6 +297,12 @@ int stream_samples(VgRenderer* r, VgAccum* acc, vgd::Ctx& c, vgx::Variant v, con
         e = pool.get();
     bool done = false;
     uint64_t wave = 0;
+    if (deferred && w.n <= tail && !timed && !r->traversal_stats && r->graph_waves == 0) {
+        // A small frame: no waves at all, from the camera rays on.
+        VG_CHECK(launch_tail(w.n, 0), "tail launch");
+        acc->launches++;
+        done = true;
+    }
     if (r->graph_waves > 0 && !timed) {
         // Captured chunks of graph_waves waves (even, so the queue parity of every wave in a
         // replay matches its place in the sequence), each ending with the live count.
@@ -334,8 +349,8 @@ int stream_samples(VgRenderer* r, VgAccum* acc, vgd::Ctx& c, vgx::Variant v, con
                 uint32_t live = ring[0];
                 acc->wave_live.push_back(live);
                 done = live == 0;
-                if (!done && live <= r->tail_threshold) {
-                    ce = (q ? vgx::launch_stream_cache_tail(v.f64, live, r->ctx->sms, s, c, w, (uint32_t)((rep + 1) * K), *q) : vgx::launch_stream_tail(v, live, r->ctx->sms, s, c, w, (uint32_t)((rep + 1) * K)));
+                if (!done && live <= tail) {
+                    ce = launch_tail(live, (uint32_t)((rep + 1) * K));
                     if (ce != cudaSuccess) {
                         cudaGraphExecDestroy(ge);
                         return cuda_fail(ce, "tail launch");
@@ -379,7 +394,7 @@ int stream_samples(VgRenderer* r, VgAccum* acc, vgd::Ctx& c, vgx::Variant v, con
             uint32_t live = ring[old];
             done = live == 0;
             acc->wave_live.push_back(live);
-            if (!done && live <= r->tail_threshold) {
+            if (!done && live <= tail) {
                 // Few slots left: finish them in one launch (the queue after this wave).
                 cudaEvent_t a = nullptr, b = nullptr;
                 if (timed) {
@@ -387,7 +402,7 @@ int stream_samples(VgRenderer* r, VgAccum* acc, vgd::Ctx& c, vgx::Variant v, con
                     b = pool.get();
                     VG_CHECK(cudaEventRecord(a, s), "event");
                 }
-                VG_CHECK((q ? vgx::launch_stream_cache_tail(v.f64, live, r->ctx->sms, s, c, w, (uint32_t)(wave + 1), *q) : vgx::launch_stream_tail(v, live, r->ctx->sms, s, c, w, (uint32_t)(wave + 1))), "tail launch");
+                VG_CHECK(launch_tail(live, (uint32_t)(wave + 1)), "tail launch");
                 if (timed) {
                     VG_CHECK(cudaEventRecord(b, s), "event");
                     stages.push_back({2, {a, b}});
@@ -397,7 +412,7 @@ int stream_samples(VgRenderer* r, VgAccum* acc, vgd::Ctx& c, vgx::Variant v, con
             }
         }
     }
-    acc->last_waves = (uint32_t)wave;
+    acc->last_waves = (uint32_t)std::max<uint64_t>(wave, 1);
     VG_CHECK(cudaStreamSynchronize(s), "waves");
     for (uint64_t k = wave > LAG ? wave - LAG + 1 : 0; k < wave; k++)
         acc->wave_live.push_back(ring[k % RING]);
@@ -820,7 +835,7 @@ int vg_set_stream_tail(VgRenderer* r, uint32_t threshold)
 {
     if (!r)
         return fail(VG_ERR_INVALID, "null renderer");
-    r->tail_threshold = threshold;
+    r->tail_threshold = r->inline_tail_threshold = threshold;
     return VG_OK;
 }
 
@@ -1082,14 +1097,36 @@ int vg_accumulate(VgRenderer* r, VgAccum* acc, uint32_t samples)
                                    r->integrator == VG_WAVEFRONT ? &w : nullptr)) != VG_OK)
             return st;
     } else if (!wavefront) {
-        if (!acc->mk_next.p && (st = alloc(acc->mk_next, 16, s, true)) != VG_OK)
-            return st;
+        bool blocks = vgx::megakernel_blocks(v, acc->restir.gi);
+        vgx::BlockGrid grid{};
+        vgk::Wave w = wave_of(r, acc);
+        TempBuf scratch;
+        uint32_t *pixels = nullptr, *next = nullptr;
+        if (blocks) {
+            grid = vgx::block_grid(r->ctx->sms, vgx::megakernel_items(acc->width, acc->height));
+            size_t n = (size_t)grid.blocks * grid.slots;
+            const size_t state = vgk::BASE_PLANES + (v.light ? vgk::SPLIT_PLANES : 0);
+            const size_t req = v.light ? vgk::SPLIT_REQ_PLANES : vgk::REQ_PLANES;
+            const size_t pend = 1 + (v.light ? vgk::SPLIT_PLANES : 0);
+            if ((st = scratch.get(r->ctx, n * 16 * (state + 1 + req + pend) + n * 12 + 16)) != VG_OK)
+                return st;
+            w.n = (uint32_t)n;
+            w.state = (float4*)scratch.p;
+            w.hits = (uint4*)(w.state + state * n);
+            w.sreq = (float4*)(w.hits + n);
+            w.pend = w.sreq + req * n;
+            w.meta = (uint32_t*)(w.pend + pend * n);
+            w.flags = w.meta + n;
+            pixels = w.flags + n;
+            next = pixels + n;
+        }
         uint32_t k = 0;
         while (k < samples) {
             c.p[P_SAMPLE] = sample0 + k;
-            c.p[P_SAMPLES_PER_DISPATCH] = std::min<uint32_t>(samples - k, acc->restir.on ? 1u : 8u);
+            c.p[P_SAMPLES_PER_DISPATCH] = std::min<uint32_t>(samples - k, acc->restir.on ? 1u : 64u);
             k += c.p[P_SAMPLES_PER_DISPATCH];
-            VG_CHECK(vgx::launch_megakernel(v, r->ctx->sms, acc->width, acc->height, s, c, (uint32_t*)acc->mk_next.p),
+            VG_CHECK((blocks ? vgx::launch_megakernel(v, grid, s, c, w, pixels, next)
+                             : vgx::launch_megakernel_restir(v, acc->width, acc->height, s, c)),
                      "megakernel launch");
             acc->launches++;
         }
@@ -1416,7 +1453,7 @@ int vg_autotune(VgRenderer* r, const VgPacked* pk, uint32_t width, uint32_t heig
         },
         std::vector<bool>{!r->defer_shadows});
     std::vector<uint32_t> tails;
-    for (uint32_t t : {0u, 8192u, 32768u, 131072u})
+    for (uint32_t t : {0u, 32768u, 131072u, 262144u})
         if (t != r->tail_threshold)
             tails.push_back(t);
     try_setting(
