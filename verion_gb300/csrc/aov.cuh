@@ -15,12 +15,20 @@ struct CameraRecord {
     float v[18];
 };
 
-// aov.slang:79-86: camera-space unit direction through pixel position (px, py), world direction in dir.
-__device__ __forceinline__ V3 pixelDir(const CameraRecord& cam, float px, float py, uint32_t w, uint32_t h, float t,
-                                       float aspect, V3& dir)
+// aov.slang:79-86: camera-space position on the plane z = -1 of pixel position (px, py).
+__device__ __forceinline__ float planeU(const CameraRecord& cam, float px, uint32_t w, float t, float aspect)
 {
-    float u = (2.0f * px / (float)w - 1.0f + cam.v[16]) * aspect * t;
-    float v = (1.0f - 2.0f * py / (float)h + cam.v[17]) * t;
+    return (2.0f * px / (float)w - 1.0f + cam.v[16]) * aspect * t;
+}
+
+__device__ __forceinline__ float planeV(const CameraRecord& cam, float py, uint32_t h, float t)
+{
+    return (1.0f - 2.0f * py / (float)h + cam.v[17]) * t;
+}
+
+// Camera-space unit direction through (u, v) on that plane, world direction in dir.
+__device__ __forceinline__ V3 planeDir(const CameraRecord& cam, float u, float v, V3& dir)
+{
     V3 d = normalize(v3(u, v, -1.0f));
     float r[3];
 #pragma unroll
@@ -28,6 +36,13 @@ __device__ __forceinline__ V3 pixelDir(const CameraRecord& cam, float px, float 
         r[k] = cam.v[4 + 4 * k] * d.x + cam.v[5 + 4 * k] * d.y + cam.v[6 + 4 * k] * d.z;
     dir = v3(r[0], r[1], r[2]);
     return d;
+}
+
+// The same through pixel position (px, py).
+__device__ __forceinline__ V3 pixelDir(const CameraRecord& cam, float px, float py, uint32_t w, uint32_t h, float t,
+                                       float aspect, V3& dir)
+{
+    return planeDir(cam, planeU(cam, px, w, t, aspect), planeV(cam, py, h, t), dir);
 }
 
 // The hit triangle's world vertices and the barycentric weights of vertices 1 and 2 at distance t.
@@ -158,6 +173,42 @@ __device__ __forceinline__ V3 sampleDir(const CameraRecord& cam, uint32_t x, uin
     return normalize(sdir);
 }
 
+// How a triangle covers the samples of a pixel, whose shears lie in a box (centre m, half size h): the edge
+// functions of the watertight test are linear in the shear, so over the box each stays within its centre value
+// +- r, r with an allowance for both computations' rounding (2^-19 of the terms' magnitudes). COVER_NONE: one is
+// surely positive and another surely negative. COVER_ALL: all are surely of one sign, and every vertex is in
+// front of the origin, so the distance is positive. COVER_SOME: to be tested sample by sample.
+enum Cover { COVER_NONE, COVER_ALL, COVER_SOME };
+
+__device__ __forceinline__ Cover cover_box(const vgt::TriRel& v, float mx, float my, float hx, float hy, float sz_lo, float sz_hi)
+{
+    float ex = fabsf(mx) + hx, ey = fabsf(my) + hy;
+    float pa = fmaf(ex, fabsf(v.az), fabsf(v.ax)), qa = fmaf(ey, fabsf(v.az), fabsf(v.ay));
+    float pb = fmaf(ex, fabsf(v.bz), fabsf(v.bx)), qb = fmaf(ey, fabsf(v.bz), fabsf(v.by));
+    float pc = fmaf(ex, fabsf(v.cz), fabsf(v.cx)), qc = fmaf(ey, fabsf(v.cz), fabsf(v.cy));
+    auto edge = [&](float px, float py, float pz, float qx, float qy, float qz, float mag, float& lo, float& hi) {
+        // (p - s pz) x (q - s qz) = p x q + sx (py qz - pz qy) + sy (pz qx - px qz)
+        float gx = fmaf(py, qz, -(pz * qy)), gy = fmaf(pz, qx, -(px * qz));
+        float at = fmaf(mx, gx, fmaf(my, gy, fmaf(px, qy, -(py * qx))));
+        float r = fmaf(hx, fabsf(gx), fmaf(hy, fabsf(gy), 1.9073486e-6f * mag));
+        lo = at - r;
+        hi = at + r;
+    };
+    float ulo, uhi, vlo, vhi, wlo, whi;
+    edge(v.cx, v.cy, v.cz, v.bx, v.by, v.bz, fmaf(pc, qb, qc * pb), ulo, uhi);
+    edge(v.ax, v.ay, v.az, v.cx, v.cy, v.cz, fmaf(pa, qc, qa * pc), vlo, vhi);
+    edge(v.bx, v.by, v.bz, v.ax, v.ay, v.az, fmaf(pb, qa, qb * pa), wlo, whi);
+    bool pos = ulo > 0.0f || vlo > 0.0f || wlo > 0.0f, neg = uhi < 0.0f || vhi < 0.0f || whi < 0.0f;
+    if (pos && neg)
+        return COVER_NONE;
+    // (1e-30: far above where their products with a distance could vanish.)
+    bool all = (ulo > 1.0e-30f && vlo > 1.0e-30f && wlo > 1.0e-30f) || (uhi < -1.0e-30f && vhi < -1.0e-30f && whi < -1.0e-30f);
+    // Distances of the vertices along the ray, at the ends of the samples' scales.
+    float near = fminf(fminf(fminf(v.az * sz_lo, v.az * sz_hi), fminf(v.bz * sz_lo, v.bz * sz_hi)), fminf(v.cz * sz_lo, v.cz * sz_hi));
+    float far = fmaxf(fmaxf(fmaxf(v.az * sz_lo, v.az * sz_hi), fmaxf(v.bz * sz_lo, v.bz * sz_hi)), fmaxf(v.cz * sz_lo, v.cz * sz_hi));
+    return all && near > 1.0e-6f && far < 1.0e20f ? COVER_ALL : COVER_SOME;
+}
+
 // aov.slang:150-181: the coverage of 16 stratified rays followed through translucent surfaces.
 static __global__ void __launch_bounds__(128) aov_coverage_layers(const __grid_constant__ Ctx c, CameraRecord cam,
                                                                   float* coverage)
@@ -191,11 +242,12 @@ static __global__ void __launch_bounds__(128) aov_coverage_layers(const __grid_c
 // their origin, and in each axis the near plane is divided by the largest and the far plane by the
 // smallest of their direction components, so a box that any of them meets is visited (a superset of what
 // each ray's own walk visits, and a hit of any triangle is what each ray's walk looks for: the counts
-// are the same). A triangle found is tested against every sample not covered yet, by the rays' own
-// test; the walk ends when all 16 are. Lanes go on to their next leaf before the warp tests triangles,
+// are the same). A triangle found is classified against the samples' box first (cover_box); one that covers
+// some of it is tested sample by sample, by the rays' own test. The walk ends when all 16 are covered. Lanes go on to their next leaf before the warp tests triangles,
 // and a pixel whose directions change sign in an axis (a line or two of pixels) traces its rays one by
 // one. Bound by issue: 16 walks of some 13 nodes become one of about 15. With one walk per ray this was
-// most of aov_main's 7.5 ms per 1920x1080 frame of the 1M-triangle scene.
+// most of aov_main's 7.5 ms per 1920x1080 frame of the 1M-triangle scene, with every triangle found tested
+// against all samples 2.8 ms.
 static __global__ void __launch_bounds__(128, 6) aov_coverage_solid(const __grid_constant__ Ctx c, CameraRecord cam,
                                                                     float* coverage)
 {
@@ -208,10 +260,28 @@ static __global__ void __launch_bounds__(128, 6) aov_coverage_solid(const __grid
     float t = cam.v[2], aspect = cam.v[0] / cam.v[1];
     V3 org = v3(cam.v[7], cam.v[11], cam.v[15]);
     V3 lo = v3(3.0e38f), hi = v3(-3.0e38f);
+    float us[4], vs[4];
+#pragma unroll
+    for (uint32_t k = 0; k < 4; k++) {
+        us[k] = planeU(cam, (float)x + ((float)k + 0.5f) / 4.0f, w, t, aspect);
+        vs[k] = planeV(cam, (float)y + ((float)k + 0.5f) / 4.0f, h, t);
+    }
+    // The samples' shears, their box, and the axis permutation when all have the same.
+    V3 slo = v3(3.0e38f), shi = v3(-3.0e38f);
+    int kx = 0, ky = 0, kz = 0;
+    bool same = true;
+#pragma unroll
     for (uint32_t k = 0; k < 16; k++) {
-        V3 d = sampleDir(cam, x, y, k, w, h, t, aspect);
+        V3 d;
+        planeDir(cam, us[k % 4], vs[k / 4], d);
+        d = normalize(d);
         vgt::TRay r = vgt::make_ray(org, d);
-        rays[k][tid] = make_float4(r.sx, r.sy, r.sz, __uint_as_float((uint32_t)(r.kx | (r.ky << 2) | (r.kz << 4))));
+        rays[k][tid] = make_float4(r.sx, r.sy, r.sz, 0.0f);
+        if (k == 0)
+            kx = r.kx, ky = r.ky, kz = r.kz;
+        same = same && kx == r.kx && ky == r.ky && kz == r.kz;
+        slo = v3(fminf(slo.x, r.sx), fminf(slo.y, r.sy), fminf(slo.z, r.sz));
+        shi = v3(fmaxf(shi.x, r.sx), fmaxf(shi.y, r.sy), fmaxf(shi.z, r.sz));
         lo = v3(fminf(lo.x, d.x), fminf(lo.y, d.y), fminf(lo.z, d.z));
         hi = v3(fmaxf(hi.x, d.x), fmaxf(hi.y, d.y), fmaxf(hi.z, d.z));
         if (bad3(d))
@@ -219,7 +289,10 @@ static __global__ void __launch_bounds__(128, 6) aov_coverage_solid(const __grid
     }
     auto one_sign = [](float a, float b) { return a > bvh8::MIN_DIR || (b < -bvh8::MIN_DIR && a > -2.0f); };
     uint32_t covered = 0;
-    if (one_sign(lo.x, hi.x) && one_sign(lo.y, hi.y) && one_sign(lo.z, hi.z)) {
+    if (same && one_sign(lo.x, hi.x) && one_sign(lo.y, hi.y) && one_sign(lo.z, hi.z)) {
+        float mx = 0.5f * (slo.x + shi.x), my = 0.5f * (slo.y + shi.y);
+        float hx = 1.000001f * (0.5f * (shi.x - slo.x)) + 1.0e-6f * fabsf(mx);
+        float hy = 1.000001f * (0.5f * (shi.y - slo.y)) + 1.0e-6f * fabsf(my);
         // Positive components: near / hi, far / lo; negative ones: near / lo, far / hi.
         vgt::Slabs b;
         b.o = org;
@@ -245,23 +318,17 @@ static __global__ void __launch_bounds__(128, 6) aov_coverage_solid(const __grid
                 k.tri_bits ^= 1u << j;
                 const float4* tp = c.s.tris + (size_t)(k.tri_base + j) * bvh8::TRI_VEC4;
                 float4 p0 = __ldg(tp), p1 = __ldg(tp + 1), p2 = __ldg(tp + 2);
-#pragma unroll 2
-                for (uint32_t i = 0; i < 16; i++) {
-                    float4 q = rays[i][tid];
-                    uint32_t kk = __float_as_uint(q.w);
-                    vgt::TRay r;
-                    r.o = org;
-                    r.kx = (int)(kk & 3u);
-                    r.ky = (int)((kk >> 2) & 3u);
-                    r.kz = (int)((kk >> 4) & 3u);
-                    r.sx = q.x;
-                    r.sy = q.y;
-                    r.sz = q.z;
-                    float th, U, V, W, det;
-                    if (vgt::tri_test(r, v3(p0.x, p0.y, p0.z), v3(p1.x, p1.y, p1.z), v3(p2.x, p2.y, p2.z), th, U, V, W, det) &&
-                        th < 1.0e30f)
-                        covered |= 1u << i;
-                }
+                vgt::TriRel v = vgt::tri_relative(org, kx, ky, kz, v3(p0.x, p0.y, p0.z), v3(p1.x, p1.y, p1.z), v3(p2.x, p2.y, p2.z));
+                Cover cv = cover_box(v, mx, my, hx, hy, slo.z, shi.z);
+                if (cv == COVER_ALL)
+                    covered = 0xffffu;
+                if (cv == COVER_SOME)
+                    for (uint32_t i = 0; i < 16; i++) {
+                        float4 q = rays[i][tid];
+                        float th, U, V, W, det;
+                        if (vgt::tri_test(v, q.x, q.y, q.z, th, U, V, W, det) && th < 1.0e30f)
+                            covered |= 1u << i;
+                    }
             }
         }
     } else {

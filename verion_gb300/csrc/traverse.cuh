@@ -65,23 +65,31 @@ __device__ __forceinline__ TRay make_ray(V3 o, V3 d)
     return r;
 }
 
-// Watertight test. On success returns true with the distance t = T / det and the edge functions
-// (U, V, W weigh vertices 0, 1, 2; divided by det they are the barycentrics). (Tried: a sign and
+// A triangle's vertices relative to a ray's origin, in the ray's axis permutation.
+struct TriRel {
+    float ax, ay, az, bx, by, bz, cx, cy, cz;
+};
+
+__device__ __forceinline__ TriRel tri_relative(V3 o, int kx, int ky, int kz, V3 v0, V3 v1, V3 v2)
+{
+    V3 A = v0 - o, B = v1 - o, C = v2 - o;
+    return TriRel{comp(A, kx), comp(A, ky), comp(A, kz), comp(B, kx), comp(B, ky),
+                  comp(B, kz), comp(C, kx), comp(C, ky), comp(C, kz)};
+}
+
+// Watertight test of a ray of shear (sx, sy, sz). On success returns true with the distance t = T / det and the
+// edge functions (U, V, W weigh vertices 0, 1, 2; divided by det they are the barycentrics). (Tried: a sign and
 // magnitude test ahead of the division, rejecting where the quotient could only be rejected
 // against the closest hit so far; it measured 1.5% slower per extend launch.)
-__device__ __forceinline__ bool tri_test(const TRay& r, V3 v0, V3 v1, V3 v2, float& t, float& U, float& V, float& W,
-                                         float& det)
+__device__ __forceinline__ bool tri_test(const TriRel& v, float sx, float sy, float sz, float& t, float& U, float& V,
+                                         float& W, float& det)
 {
-    V3 A = v0 - r.o;
-    V3 B = v1 - r.o;
-    V3 C = v2 - r.o;
-    float Akz = comp(A, r.kz), Bkz = comp(B, r.kz), Ckz = comp(C, r.kz);
-    float Ax = comp(A, r.kx) - r.sx * Akz;
-    float Ay = comp(A, r.ky) - r.sy * Akz;
-    float Bx = comp(B, r.kx) - r.sx * Bkz;
-    float By = comp(B, r.ky) - r.sy * Bkz;
-    float Cx = comp(C, r.kx) - r.sx * Ckz;
-    float Cy = comp(C, r.ky) - r.sy * Ckz;
+    float Ax = v.ax - sx * v.az;
+    float Ay = v.ay - sy * v.az;
+    float Bx = v.bx - sx * v.bz;
+    float By = v.by - sy * v.bz;
+    float Cx = v.cx - sx * v.cz;
+    float Cy = v.cy - sy * v.cz;
     U = Cx * By - Cy * Bx;
     V = Ax * Cy - Ay * Cx;
     W = Bx * Ay - By * Ax;
@@ -99,12 +107,18 @@ __device__ __forceinline__ bool tri_test(const TRay& r, V3 v0, V3 v1, V3 v2, flo
     det = U + V + W;
     if (det == 0.0f)
         return false;
-    float Az = r.sz * Akz;
-    float Bz = r.sz * Bkz;
-    float Cz = r.sz * Ckz;
+    float Az = sz * v.az;
+    float Bz = sz * v.bz;
+    float Cz = sz * v.cz;
     float T = U * Az + V * Bz + W * Cz;
     t = T / det;
     return t > 0.0f;
+}
+
+__device__ __forceinline__ bool tri_test(const TRay& r, V3 v0, V3 v1, V3 v2, float& t, float& U, float& V, float& W,
+                                         float& det)
+{
+    return tri_test(tri_relative(r.o, r.kx, r.ky, r.kz, v0, v1, v2), r.sx, r.sy, r.sz, t, U, V, W, det);
 }
 
 struct TraceHit {
