@@ -317,6 +317,9 @@ int bwave_graphs(VgContext* ctx, const vgb::WaveBatch& b, const vgk::Wave& w,
     cudaStream_t s = ctx->stream;
     int tb = 1, sb = 1;
     vgx::bwave_blocks_per_sm(&tb, &sb);
+    int side = side_stream(ctx);
+    if (side != VG_OK)
+        return side;
     auto pro = [&]() -> int {
         cudaError_t ce = cudaMemsetAsync(w.counts, 0, 2 * 4, s);
         if (ce == cudaSuccess)
@@ -359,7 +362,7 @@ int bwave_graphs(VgContext* ctx, const vgb::WaveBatch& b, const vgk::Wave& w,
     if (!device_loop) {
         cudaGraph_t gb = nullptr;
         auto body = [&]() -> int {
-            cudaError_t ce = vgx::bwave_capture_body(s, tb * ctx->sms, sb * ctx->sms, ctx->sms, b, w, 0, false);
+            cudaError_t ce = vgx::bwave_capture_body(s, ctx->side, ctx->fork, ctx->join, tb * ctx->sms, sb * ctx->sms, ctx->sms, b, w, 0, false);
             return ce == cudaSuccess ? VG_OK : cuda_fail(ce, "graph capture (loop body)");
         };
         if ((st = capture_part(s, &gb, body, "graph capture")) != VG_OK) {
@@ -407,7 +410,7 @@ int bwave_graphs(VgContext* ctx, const vgb::WaveBatch& b, const vgk::Wave& w,
     cudaGraph_t body = cp.conditional.phGraph_out[0];
     if ((e = cudaStreamBeginCaptureToGraph(s, body, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed)) != cudaSuccess)
         return done(e, "graph capture");
-    cudaError_t ce = vgx::bwave_capture_body(s, tb * ctx->sms, sb * ctx->sms, ctx->sms, b, w, loop, true);
+    cudaError_t ce = vgx::bwave_capture_body(s, ctx->side, ctx->fork, ctx->join, tb * ctx->sms, sb * ctx->sms, ctx->sms, b, w, loop, true);
     e = cudaStreamEndCapture(s, &body);
     if (ce != cudaSuccess || e != cudaSuccess)
         return done(ce != cudaSuccess ? ce : e, "graph capture (loop body)");
@@ -524,7 +527,7 @@ int batch_wave_run(VgContext* ctx, const VgBatchRequest* reqs, size_t n, int ord
     }
     if (nc && B.ncache < nc) {
         if ((st = alloc(B.caches, nc * sizeof(vgb::WaveCache), s, false)) != VG_OK ||
-            (st = alloc(B.qrec, nc * (size_t)B.cache_slots * vgn::REC_WORDS * 4, s, false)) != VG_OK ||
+            (st = alloc(B.qrec, 2 * nc * (size_t)B.cache_slots * vgn::REC_WORDS * 4, s, false)) != VG_OK ||
             (st = alloc(B.qcount, nc * 8, s, true)) != VG_OK) {
             B.ncache = 0;
             return st;
@@ -539,7 +542,8 @@ int batch_wave_run(VgContext* ctx, const VgBatchRequest* reqs, size_t n, int ord
         vgb::WaveCache& K = ktab[j];
         memset(&K, 0, sizeof(K));
         K.cd = k->dev();
-        K.qrec = (float*)B.qrec.p + j * (size_t)B.cache_slots * vgn::REC_WORDS;
+        for (size_t h = 0; h < 2; h++)
+            K.qrec[h] = (float*)B.qrec.p + (2 * j + h) * (size_t)B.cache_slots * vgn::REC_WORDS;
         K.qcount = (uint32_t*)B.qcount.p + 2 * j;
         K.trec = (float*)k->batch_rec.p;
         K.tcount = (uint32_t*)k->batch_count.p;

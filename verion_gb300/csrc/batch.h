@@ -52,12 +52,12 @@ constexpr uint32_t WAVE_VERTEX_VEC4 = 6;         // per vertex: 16 features, thr
 // last word; the batch's training records.
 struct alignas(16) WaveCache {
     vgn::CacheDev cd;
-    float* qrec;
-    uint32_t* qcount;    // by wave parity
+    float* qrec[2];      // by wave parity, as the counts
+    uint32_t* qcount;
     float* trec;
     uint32_t* tcount;
     uint32_t tcap;
-    uint32_t pad[3];
+    uint32_t pad;
 };
 
 // The batch wavefront's work and completion state besides the wave buffers (vgk::Wave, whose

@@ -159,11 +159,8 @@ int cache_accumulate(VgRenderer* r, VgAccum* acc, vgd::Ctx& c, uint32_t samples,
         return st;
     if (w && !acc->cache_spread.p && (st = alloc(acc->cache_spread, px * 8, s, false)) != VG_OK)
         return st;
-    if (!r->ctx->side) {
-        VG_CHECK(cudaStreamCreateWithFlags(&r->ctx->side, cudaStreamNonBlocking), "side stream");
-        VG_CHECK(cudaEventCreateWithFlags(&r->ctx->fork, cudaEventDisableTiming), "event");
-        VG_CHECK(cudaEventCreateWithFlags(&r->ctx->join, cudaEventDisableTiming), "event");
-    }
+    if ((st = side_stream(r->ctx)) != VG_OK)
+        return st;
     VG_CHECK(cudaMemsetAsync(k->err.p, 0, 4, s), "error flag");
     uint32_t* ctr = (uint32_t*)acc->cache_ctr.p;
     NrcPathArgs a;

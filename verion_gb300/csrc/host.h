@@ -634,6 +634,17 @@ vgx::Variant variant_of(const VgRenderer*, const VgAccum* acc)
     return v;
 }
 
+// The context's second stream and the events that order it, made on first use.
+int side_stream(VgContext* ctx)
+{
+    if (ctx->side)
+        return VG_OK;
+    VG_CHECK(cudaEventCreateWithFlags(&ctx->fork, cudaEventDisableTiming), "event");
+    VG_CHECK(cudaEventCreateWithFlags(&ctx->join, cudaEventDisableTiming), "event");
+    VG_CHECK(cudaStreamCreateWithFlags(&ctx->side, cudaStreamNonBlocking), "side stream");
+    return VG_OK;
+}
+
 // pack.rs:828-874, with the renderer's depth in word 7.
 void base_params(const VgRenderer* r, const VgAccum* acc, uint32_t* p)
 {

@@ -146,7 +146,6 @@ __global__ void __launch_bounds__(128, VG_TRACE_MIN_BLOCKS) bw_trace(const __gri
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         w.counts[out] = 0;
         w.fetch[2 + in] = 0;
-        w.fetch[8 + in] = 0;
     }
     if (blockIdx.x == 0 && threadIdx.x < BW_CLASSES)
         w.scount[in * BW_CLASSES + threadIdx.x] = 0;
@@ -283,21 +282,25 @@ __global__ void __launch_bounds__(256) bw_resolve(const __grid_constant__ WaveBa
 }
 
 // Shading of the wave's hits, class by class, with the light sample left as a shadow request
-// (wf_stream_shade_deferred with material sorting): the plain requests' slots, or with CACHE the
-// cached requests' slots, whose paths may end at the cache (a query record for the wave's answer
-// stage) or, on a training pixel, record their vertices.
+// (wf_stream_shade_deferred with material sorting). With CACHE (a batch with cached requests) the cached
+// requests' slots are classes of their own behind the plain ones': their paths may end at the cache (a query
+// record for the next wave's answers) or, on a training pixel, record their vertices; a plain request's
+// paths pass the hook with an infinite threshold. (One launch each for plain and cached slots: 35 us or more
+// a wave each, most of it ramp-down, when few slots are live.)
 template <bool CACHE>
 __global__ void __launch_bounds__(128, VG_SHADE_MIN_BLOCKS) bw_shade(const __grid_constant__ WaveBatch b, const __grid_constant__ Wave w, uint32_t wave)
 {
+    constexpr uint32_t CLASSES = CACHE ? BW_CLASSES : SHADE_CLASSES;
     uint32_t in = wave & 1u, out = in ^ 1u;
     uint32_t n = w.n;
-    const uint32_t c0 = CACHE ? SHADE_CLASSES : 0u;
-    uint32_t seg[SHADE_CLASSES + 1] = {0, 0, 0, 0, 0};
-    for (uint32_t k = 0; k < SHADE_CLASSES; k++)
-        seg[k + 1] = seg[k] + w.scount[in * BW_CLASSES + c0 + k];
-    uint32_t count = seg[SHADE_CLASSES];
+    uint32_t seg[CLASSES + 1];
+    seg[0] = 0;
+#pragma unroll
+    for (uint32_t k = 0; k < CLASSES; k++)
+        seg[k + 1] = seg[k] + w.scount[in * BW_CLASSES + k];
+    uint32_t count = seg[CLASSES];
     for (;;) {
-        uint32_t base = warp_fetch(&w.fetch[(CACHE ? 8 : 2) + in]);
+        uint32_t base = warp_fetch(&w.fetch[2 + in]);
         if (base >= count)
             break;
         uint32_t i = base + lane_id();
@@ -305,8 +308,12 @@ __global__ void __launch_bounds__(128, VG_SHADE_MIN_BLOCKS) bw_shade(const __gri
         uint32_t r = 0, pix = 0, p = 0;
         CacheHook hk;
         if (i < count) {
-            uint32_t k = i >= seg[1] ? (i >= seg[2] ? (i >= seg[3] ? 3u : 2u) : 1u) : 0u;
-            p = w.squeue[(size_t)(c0 + k) * n + (i - seg[k])];
+            uint32_t k = 0, k0 = 0;
+#pragma unroll
+            for (uint32_t j = 1; j < CLASSES; j++)
+                if (i >= seg[j])
+                    k = j, k0 = seg[j];
+            p = w.squeue[(size_t)k * n + (i - k0)];
             r = b.slot_req[p];
             pix = b.slot_pix[p];
             const WaveReq& R = b.reqs[r];
@@ -321,8 +328,11 @@ __global__ void __launch_bounds__(128, VG_SHADE_MIN_BLOCKS) bw_shade(const __gri
             h.prim = hr.z;
             h.t = __uint_as_float(hr.w);
             ShadowReq req;
-            bool train = false;
-            if (CACHE) {
+            bool train = false, cached = CACHE && R.cache != NO_CACHE;
+            hk.c = INFINITY;
+            hk.train = false;
+            hk.a0 = hk.a = 0.0f;
+            if (cached) {
                 // The spread starts at zero with each sample.
                 float2 sp = depth > 0 ? b.spread[p] : make_float2(0.0f, 0.0f);
                 train = training_pixel(R, pix, c.p[P_SAMPLE] + (meta >> 8));
@@ -333,7 +343,7 @@ __global__ void __launch_bounds__(128, VG_SHADE_MIN_BLOCKS) bw_shade(const __gri
             }
             bool alive = shadePath<false, false, true, CACHE>(c, st, h, depth, pix, &req, CACHE ? &hk : nullptr) &&
                          depth + 1 < c.p[P_MAX_DEPTH];
-            if (CACHE) {
+            if (cached) {
                 if (hk.vertex && train) {
                     uint32_t nv = b.tnv[p];
                     if (nv < vgb::WAVE_MAX_TRAIN_VERTICES) {
@@ -388,7 +398,7 @@ __global__ void __launch_bounds__(128, VG_SHADE_MIN_BLOCKS) bw_shade(const __gri
             first = __shfl_sync(FULL, first, leader);
             if (query) {
                 uint32_t slot = first + __popc(grp & ((1u << lane_id()) - 1u));
-                cacheQueryRecord(b.caches[j].qrec + (size_t)slot * CACHE_REC_WORDS, hk, (r << 22) | pix);
+                cacheQueryRecord(b.caches[j].qrec[in] + (size_t)slot * CACHE_REC_WORDS, hk, (r << 22) | pix);
             }
         }
         __syncwarp();
@@ -450,7 +460,7 @@ __global__ void __launch_bounds__(128) bw_answer(WaveBatch b, uint32_t parity)
         }
         uint32_t i = first + tid;
         bool has = i < n;
-        const float* q = K.qrec + (size_t)i * CACHE_REC_WORDS;
+        const float* q = K.qrec[parity] + (size_t)i * CACHE_REC_WORDS;
         float v[64];
         if (has) {
             input_row(K.cd, q, v);
@@ -589,17 +599,30 @@ cudaError_t bwave_capture_start(cudaStream_t s, const vgb::WaveBatch& b, const v
     return cudaGetLastError();
 }
 
-cudaError_t bwave_capture_body(cudaStream_t s, int trace_blocks, int shade_blocks, int sms, const vgb::WaveBatch& b,
-                               const vgk::Wave& w, cudaGraphConditionalHandle loop, bool condition)
+cudaError_t bwave_capture_body(cudaStream_t s, cudaStream_t side, cudaEvent_t fork, cudaEvent_t join, int trace_blocks,
+                               int shade_blocks, int sms, const vgb::WaveBatch& b, const vgk::Wave& w,
+                               cudaGraphConditionalHandle loop, bool condition)
 {
     for (uint32_t wave = 0; wave < 2; wave++) {
         bw_trace<<<trace_blocks, 128, 0, s>>>(b, w, wave);
         bw_resolve<<<sms * 4, 256, 0, s>>>(b, w, wave);
-        if (b.ncache)
-            bw_answer<<<sms * 2, 128, ANSWER_SMEM, s>>>(b, wave ^ 1u);
-        bw_shade<false><<<shade_blocks, 128, 0, s>>>(b, w, wave);
-        if (b.ncache)
+        if (b.ncache) {
+            // The last wave's answers, beside this wave's shading (its queries go to the other records); the next
+            // wave's paths are added to their pixels after them.
+            cudaError_t e = cudaEventRecord(fork, s);
+            if (e == cudaSuccess)
+                e = cudaStreamWaitEvent(side, fork, 0);
+            if (e != cudaSuccess)
+                return e;
+            bw_answer<<<sms * 2, 128, ANSWER_SMEM, side>>>(b, wave ^ 1u);
+            if ((e = cudaEventRecord(join, side)) != cudaSuccess)
+                return e;
             bw_shade<true><<<shade_blocks, 128, 0, s>>>(b, w, wave);
+            if ((e = cudaStreamWaitEvent(s, join, 0)) != cudaSuccess)
+                return e;
+        } else {
+            bw_shade<false><<<shade_blocks, 128, 0, s>>>(b, w, wave);
+        }
     }
     if (condition)
         bw_condition<<<1, 1, 0, s>>>(b, w, loop);
