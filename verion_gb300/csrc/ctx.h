@@ -26,6 +26,7 @@ struct DeviceScene {
     const float* materials;
     const uint32_t* lights;
     const float* emitters;
+    const float4* emit_aux;    // per emitter: unit normal, area density of its choice (emitterAux)
     const float* emit_cdf;
     const float* env_pixels;
     const float* env_marginal;

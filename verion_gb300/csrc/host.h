@@ -282,7 +282,7 @@ constexpr uint32_t CACHE_WARMUP_SAMPLE = 0x40000000u; // first sample index of c
 struct VgRenderer {
     VgContext* ctx = nullptr;
     int device = -1; // the context's device, kept here so no call dereferences a destroyed context
-    DevBuf positions, indices, uvs, vnormals, instances, materials, lights, emitters, emit_cdf, emit_guide, env_pixels,
+    DevBuf positions, indices, uvs, vnormals, instances, materials, lights, emitters, emit_aux, emit_cdf, emit_guide, env_pixels,
         env_marginal, env_cond, env_guide, texels, tex_info, nodes, tris, err, scratch;
     vgd::DeviceScene ds{};
     VgSceneInfo info{};

@@ -87,6 +87,19 @@ cudaError_t launch_trace_rays(int blocks, cudaStream_t s, const vgd::Ctx& c, con
     return cudaGetLastError();
 }
 
+static __global__ void emitter_aux(const float* emitters, uint32_t n, float4* out)
+{
+    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n)
+        out[i] = vgd::emitterAux(emitters + 16 * (size_t)i);
+}
+
+cudaError_t launch_emitter_aux(cudaStream_t s, const float* emitters, uint32_t n, float4* out)
+{
+    emitter_aux<<<(n + 255) / 256, 256, 0, s>>>(emitters, n, out);
+    return cudaGetLastError();
+}
+
 cudaError_t launch_occlusion_rays(cudaStream_t s, const vgd::Ctx& c, const float* rays, uint32_t* out, uint32_t n)
 {
     vgk::occlusion_rays<<<(n + 127) / 128, 128, 0, s>>>(c, rays, out, n);
@@ -194,9 +207,9 @@ cudaError_t launch_stream_shade_deferred(bool sorted, int blocks, cudaStream_t s
                                          const vgk::Wave& w, uint32_t wave)
 {
     if (sorted)
-        vgk::wf_stream_shade_deferred<false, false, true><<<blocks, 128, 0, s>>>(c, w, wave, vgk::CacheWave{});
+        vgk::wf_stream_shade_deferred<false, false, true><<<blocks, vgk::SHADE_THREADS, 0, s>>>(c, w, wave, vgk::CacheWave{});
     else
-        vgk::wf_stream_shade_deferred<><<<blocks, 128, 0, s>>>(c, w, wave, vgk::CacheWave{});
+        vgk::wf_stream_shade_deferred<><<<blocks, vgk::SHADE_THREADS, 0, s>>>(c, w, wave, vgk::CacheWave{});
     return cudaGetLastError();
 }
 
@@ -245,16 +258,16 @@ cudaError_t launch_stream_cache_shade(bool sorted, int blocks, cudaStream_t s, c
                                       const vgk::Wave& w, uint32_t wave, const vgk::CacheWave& q)
 {
     if (sorted)
-        vgk::wf_stream_shade_deferred<true, false, true><<<blocks, 128, 0, s>>>(c, w, wave, q);
+        vgk::wf_stream_shade_deferred<true, false, true><<<blocks, vgk::SHADE_THREADS, 0, s>>>(c, w, wave, q);
     else
-        vgk::wf_stream_shade_deferred<true><<<blocks, 128, 0, s>>>(c, w, wave, q);
+        vgk::wf_stream_shade_deferred<true><<<blocks, vgk::SHADE_THREADS, 0, s>>>(c, w, wave, q);
     return cudaGetLastError();
 }
 
 int stream_cache_shade_blocks_per_sm()
 {
     int n = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, vgk::wf_stream_shade_deferred<true>, 128, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, vgk::wf_stream_shade_deferred<true>, vgk::SHADE_THREADS, 0);
     return n > 0 ? n : 1;
 }
 
@@ -275,7 +288,7 @@ int stream_shadow_layers_blocks_per_sm()
 int stream_deferred_blocks_per_sm()
 {
     int n = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, vgk::wf_stream_shade_deferred<>, 128, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, vgk::wf_stream_shade_deferred<>, vgk::SHADE_THREADS, 0);
     return n > 0 ? n : 1;
 }
 

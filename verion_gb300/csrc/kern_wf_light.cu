@@ -10,16 +10,16 @@ cudaError_t launch_stream_shade_deferred_light(bool sorted, int blocks, cudaStre
                                                const vgk::Wave& w, uint32_t wave)
 {
     if (sorted)
-        vgk::wf_stream_shade_deferred<false, false, true, true><<<blocks, 128, 0, s>>>(c, w, wave, vgk::CacheWave{});
+        vgk::wf_stream_shade_deferred<false, false, true, true><<<blocks, vgk::SHADE_THREADS, 0, s>>>(c, w, wave, vgk::CacheWave{});
     else
-        vgk::wf_stream_shade_deferred<false, false, false, true><<<blocks, 128, 0, s>>>(c, w, wave, vgk::CacheWave{});
+        vgk::wf_stream_shade_deferred<false, false, false, true><<<blocks, vgk::SHADE_THREADS, 0, s>>>(c, w, wave, vgk::CacheWave{});
     return cudaGetLastError();
 }
 
 int stream_deferred_light_blocks_per_sm()
 {
     int n = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, vgk::wf_stream_shade_deferred<false, false, true, true>, 128, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, vgk::wf_stream_shade_deferred<false, false, true, true>, vgk::SHADE_THREADS, 0);
     return n > 0 ? n : 1;
 }
 

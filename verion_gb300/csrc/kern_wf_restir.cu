@@ -62,9 +62,9 @@ cudaError_t launch_stream_shade_deferred_restir(bool sorted, int blocks, cudaStr
                                                 const vgk::Wave& w, uint32_t wave)
 {
     if (sorted)
-        vgk::wf_stream_shade_deferred<false, true, true><<<blocks, 128, 0, s>>>(c, w, wave, vgk::CacheWave{});
+        vgk::wf_stream_shade_deferred<false, true, true><<<blocks, vgk::RESTIR_SHADE_THREADS, 0, s>>>(c, w, wave, vgk::CacheWave{});
     else
-        vgk::wf_stream_shade_deferred<false, true><<<blocks, 128, 0, s>>>(c, w, wave, vgk::CacheWave{});
+        vgk::wf_stream_shade_deferred<false, true><<<blocks, vgk::RESTIR_SHADE_THREADS, 0, s>>>(c, w, wave, vgk::CacheWave{});
     return cudaGetLastError();
 }
 
@@ -85,7 +85,7 @@ cudaError_t launch_stream_resolve_restir(bool f64, bool sorted, int blocks, cuda
 int stream_deferred_restir_blocks_per_sm()
 {
     int n = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, vgk::wf_stream_shade_deferred<false, true, true>, 128, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, vgk::wf_stream_shade_deferred<false, true, true>, vgk::RESTIR_SHADE_THREADS, 0);
     return n > 0 ? n : 1;
 }
 

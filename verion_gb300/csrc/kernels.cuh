@@ -22,19 +22,20 @@ using namespace vgd;
 
 constexpr uint32_t FULL = 0xffffffffu;
 
-// Minimum resident 128-thread blocks per SM requested for the shade kernels (a register cap), and
-// for the deferred shade stage's ReSTIR instantiations, whose candidate loop waits on memory: on
-// the many-light ReSTIR frame 4 blocks gave 7.89 ms, 6 blocks 7.43 (then 7.01 with the shared
-// candidate target terms), 10 blocks 6.76, 12 blocks 6.72, 16 blocks 6.90. The plain stage keeps
-// 4: 5, 6, 8 or 16 blocks are slower (its inlined shadePath spills heavily below 128 registers),
-// and so is calling the out-of-line shadePathCall from it (8.99 ms of shading per benchmark step
-// inline at 4 blocks; out of line 9.67 at 4 blocks, 10.5 at 8, 10.9 at 12, 11.4 at 16).
+// Minimum resident 128-thread blocks per SM requested for the shade kernels (a register cap): 5, 6, 8 or 16
+// blocks are slower than 4 (the inlined shadePath spills heavily below 128 registers), and so is calling the
+// out-of-line shadePathCall (8.99 ms of shading per benchmark step inline at 4 blocks; out of line 9.67 at 4
+// blocks, 10.5 at 8, 10.9 at 12, 11.4 at 16).
 #ifndef VG_SHADE_MIN_BLOCKS
 #define VG_SHADE_MIN_BLOCKS 4
 #endif
-#ifndef VG_RESTIR_SHADE_MIN_BLOCKS
-#define VG_RESTIR_SHADE_MIN_BLOCKS 12
-#endif
+// The deferred shade stage's ReSTIR instantiations wait on the candidate loop's memory and, with many small
+// blocks, on instructions: their warps run a loop and a shade each of which fills the instruction cache.
+// One block per SM takes its slots together (one fetch and two barriers a round), so that its warps run the
+// same part: the many-light 1080p frame takes 5.15 ms with 128 threads at 12 blocks per SM, each warp
+// fetching for itself (10 blocks 5.33, 8 5.59, 6 5.79); together 4.93, with 256 threads at 6 blocks 4.77, 512 at
+// 3 4.63, 768 at 2 4.58, 1024 at 1 (64 registers) 4.49. The plain stage is 1-3% slower that way.
+constexpr uint32_t SHADE_THREADS = 128, RESTIR_SHADE_THREADS = 1024;
 // The same for the kernels that run whole paths per thread through the out-of-line shadePathCall
 // (the streaming tail, the batch wavefront's tail).
 #ifndef VG_TAIL_MIN_BLOCKS
@@ -735,7 +736,7 @@ static __device__ __forceinline__ void append_queries(const CacheWave& q, bool q
 // hook); it then leaves a query record (one atomic per warp) and finishes like any other.
 // With SORTED the wave's slots are taken class by class from the resolve stage's queues.
 template <bool CACHE = false, bool RESTIR = false, bool SORTED = false, bool LIGHT = false>
-__global__ void __launch_bounds__(128, RESTIR ? VG_RESTIR_SHADE_MIN_BLOCKS : VG_SHADE_MIN_BLOCKS) wf_stream_shade_deferred(const __grid_constant__ Ctx c,
+__global__ void __launch_bounds__(RESTIR ? RESTIR_SHADE_THREADS : SHADE_THREADS, RESTIR ? 1 : VG_SHADE_MIN_BLOCKS) wf_stream_shade_deferred(const __grid_constant__ Ctx c,
                                                                                     const __grid_constant__ Wave w, uint32_t wave,
                                                                                     CacheWave q)
 {
@@ -747,10 +748,23 @@ __global__ void __launch_bounds__(128, RESTIR ? VG_RESTIR_SHADE_MIN_BLOCKS : VG_
     if (SORTED)
         for (uint32_t k = 0; k < SHADE_CLASSES; k++)
             seg[k + 1] = seg[k] + w.scount[in * SHADE_CLASSES + k];
+    __shared__ uint32_t fetched;
     for (;;) {
-        uint32_t base = warp_fetch(&w.fetch[2 + in]);
-        if (base >= count)
-            break;
+        uint32_t base;
+        if (RESTIR) {
+            __syncthreads();
+            if (threadIdx.x == 0)
+                fetched = atomicAdd(&w.fetch[2 + in], blockDim.x);
+            __syncthreads();
+            base = fetched;
+            if (base >= count)
+                break;
+            base += threadIdx.x & ~31u;
+        } else {
+            base = warp_fetch(&w.fetch[2 + in]);
+            if (base >= count)
+                break;
+        }
         uint32_t i = base + lane_id();
         bool query = false, shadow = false;
         uint32_t p = 0, kq = 0;

@@ -633,24 +633,44 @@ static __device__ __forceinline__ Hit traceClosest(const Ctx& c, V3 org, V3 dir)
 // ---------------------------------------------------------------------------------------------
 // ReSTIR DI (pt_core.slang:702-895), reservoirs in the structure-of-arrays form above.
 
-// pt_core.slang:718-736
-static __device__ bool restirLight(const Ctx& c, uint32_t e, uint32_t recv, V3 x, V3 p, V3 n, V3& wi, float& dist, float& cosi,
-                            V3& g, float& plsa)
+// An emitter's table row (four 16-byte loads) and what emitterAux made of it.
+struct EmitterRow {
+    V3 a, b, c, le, n;
+    float area, pdf, q;
+    uint32_t mask;
+};
+
+static __device__ __forceinline__ EmitterRow emitterRow(const Ctx& c, uint32_t e)
 {
-    uint32_t o = e * 16;
-    const float* E = c.s.emitters;
-    V3 a = v3(fget(E, o), fget(E, o + 1), fget(E, o + 2));
-    V3 b = v3(fget(E, o + 3), fget(E, o + 4), fget(E, o + 5));
-    V3 cc = v3(fget(E, o + 6), fget(E, o + 7), fget(E, o + 8));
+    const float4* E = (const float4*)c.s.emitters + 4 * (size_t)e;
+    float4 r0 = __ldg(E), r1 = __ldg(E + 1), r2 = __ldg(E + 2), r3 = __ldg(E + 3), x = __ldg(c.s.emit_aux + e);
+    return EmitterRow{v3(r0.x, r0.y, r0.z), v3(r0.w, r1.x, r1.y), v3(r1.z, r1.w, r2.x), v3(r2.y, r2.z, r2.w),
+                      v3(x.x, x.y, x.z), r3.x, r3.y, x.w, __float_as_uint(r3.z)};
+}
+
+// What every sample of an emitter needs and depends on its row alone, computed once when the table is uploaded,
+// by the operations a sample would: the triangle's unit normal, and the area density of choosing it (0 for one
+// without area).
+static __device__ __forceinline__ float4 emitterAux(const float* row)
+{
+    V3 a = v3(row[0], row[1], row[2]), b = v3(row[3], row[4], row[5]), c = v3(row[6], row[7], row[8]);
+    V3 n = normalize(cross(b - a, c - a));
+    return make_float4(n.x, n.y, n.z, row[12] > 0.0f ? row[13] / row[12] : 0.0f);
+}
+
+// pt_core.slang:718-736
+static __device__ __forceinline__ bool restirLight(const EmitterRow& E, uint32_t recv, V3 x, V3 p, V3 n, V3& wi, float& dist,
+                                                   float& cosi, V3& g, float& plsa)
+{
     V3 toL = x - p;
     float d2 = dot(toL, toL);
     dist = sqrtf(d2);
     wi = toL / fmaxf(dist, 1.0e-6f);
-    float cosl = fabsf(dot(normalize(cross(b - a, cc - a)), wi));
+    float cosl = fabsf(dot(E.n, wi));
     cosi = dot(n, wi);
-    g = v3(fget(E, o + 9), fget(E, o + 10), fget(E, o + 11)) * (cosl / fmaxf(d2, 1.0e-12f));
-    plsa = fget(E, o + 13) * d2 / (fmaxf(fget(E, o + 12), 1.0e-30f) * fmaxf(cosl, 1.0e-5f));
-    return cosi > 0.0f && cosl > 1.0e-5f && d2 > 1.0e-12f && (__float_as_uint(fget(E, o + 14)) & recv) != 0;
+    g = E.le * (cosl / fmaxf(d2, 1.0e-12f));
+    plsa = E.pdf * d2 / (fmaxf(E.area, 1.0e-30f) * fmaxf(cosl, 1.0e-5f));
+    return cosi > 0.0f && cosl > 1.0e-5f && d2 > 1.0e-12f && (E.mask & recv) != 0;
 }
 
 // pt_core.slang:739-743
@@ -669,6 +689,7 @@ static __device__ __forceinline__ float restirMis(const Surface& surf, V3 woL, V
 struct RestirTargetPoint {
     float g1o, g1oCoat, den;
     V3 msf;
+    bool opaque; // no transmission, with an eta and a compensation whose products with its zero are zero
 };
 
 static __device__ __forceinline__ RestirTargetPoint restirTargetPoint(const Ctx& c, const Surface& s, V3 woL)
@@ -678,6 +699,7 @@ static __device__ __forceinline__ RestirTargetPoint restirTargetPoint(const Ctx&
     e.g1oCoat = s.coat > 0.0f ? G1(woL.z, s.coatAlpha) : 0.0f;
     e.den = 4.0f * woL.z;
     e.msf = multiscatterFactor(c, s, woL.z);
+    e.opaque = s.transmission == 0.0f && s.eta > 1.0e-3f && s.eta < 1.0e3f && fabsf(s.tComp) < 1.0e30f;
     return e;
 }
 
@@ -688,7 +710,7 @@ static __device__ __forceinline__ float restirTarget(const Surface& s, const Res
     float woh = fmaxf(dot(woL, hh), 0.0f);
     float t = s.transmission;
     float dg = Dggx(hh.z, s.alpha) * e.g1o;
-    float fEta = fresnelDielectric(woh, s.eta);
+    float fEta = e.opaque ? 0.0f : fresnelDielectric(woh, s.eta); // (weighed by the transmission everywhere)
     // evalLobes
     float core = dg * G1(wiL.z, s.alpha) / e.den;
     V3 spec = s.metallic * schlick(s.albedo, woh) * e.msf * core +
@@ -735,25 +757,20 @@ static __device__ __noinline__ RestirPick restirDI(const Ctx& c, uint32_t pixel,
     uint32_t selE = 0;
     V3 selX = v3(0.0f);
     float selPhat = 0.0f;
-    const float* E = c.s.emitters;
     RestirTargetPoint tp = restirTargetPoint(c, surf, woL);
     for (uint32_t k = 0; k < max(c.p[P_RESTIR_CANDIDATES], 1u); k++) {
         float ue = rng.next();
         float ua = rng.next();
         float ub = rng.next();
         uint32_t lo = guidedCdf(c.s.emit_cdf, emitterCount, c.s.emit_guide, c.s.emit_guide_k, ue);
-        uint32_t o = lo * 16;
-        V3 a = v3(fget(E, o), fget(E, o + 1), fget(E, o + 2));
-        V3 b = v3(fget(E, o + 3), fget(E, o + 4), fget(E, o + 5));
-        V3 cc = v3(fget(E, o + 6), fget(E, o + 7), fget(E, o + 8));
+        EmitterRow E = emitterRow(c, lo);
         float su = sqrtf(ua);
-        V3 x = a * (1.0f - su) + b * (su * (1.0f - ub)) + cc * (su * ub);
-        float area = fget(E, o + 12);
-        float q = area > 0.0f ? fget(E, o + 13) / area : 0.0f;
+        V3 x = E.a * (1.0f - su) + E.b * (su * (1.0f - ub)) + E.c * (su * ub);
+        float q = E.q;
         V3 wi, g;
         float dist, cosi, plsa;
         float phat = 0.0f;
-        if (q > 0.0f && restirLight(c, lo, recv, x, p, n, wi, dist, cosi, g, plsa)) {
+        if (q > 0.0f && restirLight(E, recv, x, p, n, wi, dist, cosi, g, plsa)) {
             V3 wiL = v3(dot(wi, T), dot(wi, B), cosi);
             phat = restirTarget(surf, tp, woL, wiL, g, plsa);
         }
@@ -796,7 +813,7 @@ static __device__ __noinline__ RestirPick restirDI(const Ctx& c, uint32_t pixel,
             V3 wi, g;
             float dist, cosi, plsa;
             float phat = 0.0f;
-            if (restirLight(c, ei - 1, recv, xc, p, n, wi, dist, cosi, g, plsa)) {
+            if (restirLight(emitterRow(c, ei - 1), recv, xc, p, n, wi, dist, cosi, g, plsa)) {
                 V3 wiL = v3(dot(wi, T), dot(wi, B), cosi);
                 phat = restirTarget(surf, tp, woL, wiL, g, plsa);
             }
@@ -821,7 +838,7 @@ static __device__ __noinline__ RestirPick restirDI(const Ctx& c, uint32_t pixel,
     if (r.valid) {
         V3 wi, g;
         float dist, cosi, plsa;
-        restirLight(c, selE - 1, recv, selX, p, n, wi, dist, cosi, g, plsa);
+        restirLight(emitterRow(c, selE - 1), recv, selX, p, n, wi, dist, cosi, g, plsa);
         r.occ = occluded(c, p, wi, dist * (1.0f - 1.0e-3f));
     }
     float4 nn = c.re.n[cur][pixel];
@@ -1360,7 +1377,7 @@ __device__ __forceinline__ bool shadePath(const Ctx& c, PathState<LIGHT>& st, Hi
             if (pick.valid) {
                 V3 wi, g;
                 float dist, cosi, plsa;
-                restirLight(c, pick.e - 1, recvHere, pick.x, p, n, wi, dist, cosi, g, plsa);
+                restirLight(emitterRow(c, pick.e - 1), recvHere, pick.x, p, n, wi, dist, cosi, g, plsa);
                 bool track = lightingOn;
                 if (!pick.occ || track) {
                     V3 wiL = v3(dot(wi, T), dot(wi, B), cosi);
@@ -1400,7 +1417,8 @@ __device__ __forceinline__ bool shadePath(const Ctx& c, PathState<LIGHT>& st, Hi
             float d2 = dot(toL, toL);
             float dist = sqrtf(d2);
             V3 wi = toL / dist;
-            float cosl = fabsf(dot(normalize(cross(b - a, cc - a)), wi));
+            float4 aux = __ldg(c.s.emit_aux + lo);
+            float cosl = fabsf(dot(v3(aux.x, aux.y, aux.z), wi));
             float cosi = dot(n, wi);
             if (DEFER && cosi > 0.0f && cosl > 1.0e-5f && (__float_as_uint(fget(E, e + 14)) & recvHere) != 0) {
                 // Deferred: the shadow stage tests visibility and adds c, as the last add of this bounce.

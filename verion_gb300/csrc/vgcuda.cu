@@ -132,6 +132,17 @@ std::vector<uint32_t> emitter_guide(const VgPacked* pk)
     return g;
 }
 
+// DeviceScene::emit_aux of the uploaded emitters.
+int emitter_aux(VgRenderer* r, uint32_t n)
+{
+    cudaStream_t s = r->ctx->stream;
+    int st = alloc(r->emit_aux, (size_t)n * 16, s, n == 0);
+    if (st != VG_OK || n == 0)
+        return st;
+    VG_CHECK(vgx::launch_emitter_aux(s, (const float*)r->emitters.p, n, (float4*)r->emit_aux.p), "emitter table launch");
+    return VG_OK;
+}
+
 // FNV-1a over two tables: whether a re-packed table differs from the uploaded one.
 uint64_t table_key(const void* a, size_t a_len, const void* b, size_t b_len)
 {
@@ -160,6 +171,7 @@ void bind_tables(VgRenderer* r)
     r->ds.materials = (const float*)r->materials.p;
     r->ds.lights = (const uint32_t*)r->lights.p;
     r->ds.emitters = (const float*)r->emitters.p;
+    r->ds.emit_aux = (const float4*)r->emit_aux.p;
     r->ds.emit_cdf = (const float*)r->emit_cdf.p;
     r->ds.env_pixels = (const float*)r->env_pixels.p;
     r->ds.env_marginal = (const float*)r->env_marginal.p;
@@ -567,6 +579,10 @@ int vg_renderer_create(VgContext* ctx, const VgPacked* pk, VgRenderer** out)
         std::vector<uint32_t> guide = emitter_guide(pk);
         UP(emit_guide, guide.data(), guide.size() * 4);
     }
+    if ((st = emitter_aux(r, pk->info.emitter_count)) != VG_OK) {
+        vg_renderer_destroy(r);
+        return st;
+    }
     UP(env_pixels, pk->env_pixels, pk->env_pixels_len * 4);
     UP(env_marginal, pk->env_marginal, pk->env_marginal_len * 4);
     UP(env_cond, pk->env_conditional, pk->env_conditional_len * 4);
@@ -634,6 +650,8 @@ int vg_renderer_update(VgRenderer* r, const VgPacked* pk, const VgUpdatePlan* pl
             std::swap(mine[i]->bytes, theirs[i]->bytes);
             bytes += mine[i]->bytes;
         }
+        std::swap(r->emit_aux.p, f->emit_aux.p); // made here, not uploaded
+        std::swap(r->emit_aux.bytes, f->emit_aux.bytes);
         r->info = f->info;
         r->bvh = f->bvh;
         r->instance_count = f->instance_count;
@@ -729,6 +747,8 @@ int vg_renderer_update(VgRenderer* r, const VgPacked* pk, const VgUpdatePlan* pl
             return st;
         bytes += (pk->emitters_len + pk->emit_cdf_len + guide.size()) * 4;
         r->info.emitter_count = pk->info.emitter_count;
+        if ((st = emitter_aux(r, pk->info.emitter_count)) != VG_OK)
+            return st;
     }
     if (plan->instances) {
         if ((st = upload(ctx, r->instances, pk->instances, pk->instances_len * 4)) != VG_OK)
