@@ -603,9 +603,13 @@ cudaError_t bwave_capture_body(cudaStream_t s, cudaStream_t side, cudaEvent_t fo
                                int shade_blocks, int sms, const vgb::WaveBatch& b, const vgk::Wave& w,
                                cudaGraphConditionalHandle loop, bool condition)
 {
+    int resolve_blocks = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resolve_blocks, bw_resolve, 256, 0) != cudaSuccess || resolve_blocks < 1)
+        resolve_blocks = 1;
+    resolve_blocks *= sms;
     for (uint32_t wave = 0; wave < 2; wave++) {
         bw_trace<<<trace_blocks, 128, 0, s>>>(b, w, wave);
-        bw_resolve<<<sms * 4, 256, 0, s>>>(b, w, wave);
+        bw_resolve<<<resolve_blocks, 256, 0, s>>>(b, w, wave);
         if (b.ncache) {
             // The last wave's answers, beside this wave's shading (its queries go to the other records); the next
             // wave's paths are added to their pixels after them.

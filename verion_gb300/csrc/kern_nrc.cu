@@ -23,8 +23,9 @@ using namespace vgnd;
 // encoded as the network's input tiles: tile t holds rows offset + 128 t ... in the MMA operand
 // layout (128 x 64 bf16, 128-byte swizzle), so a tile moves to shared memory in one bulk copy.
 // The padding rows of the last tile are zero.
-__global__ void __launch_bounds__(256) nrc_encode(CacheDev cd, const float* __restrict__ rec, const uint32_t* count,
-                                                  uint32_t cap, uint32_t offset, uint32_t limit, uint8_t* X)
+__global__ void __launch_bounds__(256) nrc_encode(CacheDev cd, const float* __restrict__ rec,
+                                                  const uint32_t* count, uint32_t cap, uint32_t offset, uint32_t limit,
+                                                  uint8_t* X)
 {
     uint32_t n = min(*count, cap);
     uint32_t end = offset < n ? min(n, offset + limit) : offset;
@@ -43,24 +44,69 @@ __global__ void __launch_bounds__(256) nrc_encode(CacheDev cd, const float* __re
     }
 }
 
+// The same for few records, four threads a record: each gathers four levels' corners (32 loads) and writes its
+// 16 bytes of the grid columns and 16 of the others. A few records' gathers are bound by their latency, many by
+// the L2's bandwidth: 1,000 / 16,384 / 65,536 / 131,000 records take 8.4 / 12.4 / 27 / 50 us this way, 16.5 / 16.5 /
+// 37 / 55 with one thread a record; 262,147 take 95 against 87 (ENCODE_SMALL, launch_nrc.h).
+static_assert(MAX_LEVELS == 16, "four threads of four levels");
+__global__ void __launch_bounds__(256) nrc_encode_small(const __grid_constant__ CacheDev cd, const float* __restrict__ rec,
+                                                        const uint32_t* count, uint32_t cap, uint32_t offset,
+                                                        uint32_t limit, uint8_t* X)
+{
+    uint32_t n = min(*count, cap);
+    uint32_t end = offset < n ? min(n, offset + limit) : offset;
+    uint32_t rows = end - offset;
+    uint32_t items = (rows + TILE - 1) / TILE * TILE * 4;
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < items; i += gridDim.x * blockDim.x) {
+        uint32_t r = i >> 2, t = i & 3u;
+        float g[8], v[8];
+#pragma unroll
+        for (int k = 0; k < 8; k++)
+            g[k] = v[k] = 0.0f;
+        if (r < rows) {
+            const float* p = rec + (size_t)(offset + r) * REC_WORDS;
+#pragma unroll
+            for (uint32_t k = 0; k < 4; k++)
+                level_features(cd, p, 4 * t + k, g[2 * k], g[2 * k + 1]);
+            // Columns 32 + 8 t ... of the row (input_row).
+            if (t == 0) {
+#pragma unroll
+                for (int k = 0; k < 6; k++)
+                    v[k] = p[3 + k] * 0.5f + 0.5f;
+                v[6] = p[9];
+                v[7] = p[10];
+            } else if (t == 1) {
+#pragma unroll
+                for (int k = 0; k < 4; k++)
+                    v[k] = p[11 + k];
+                v[4] = 1.0f;
+            }
+        }
+        uint8_t* tile = X + (size_t)(r / TILE) * 16384u;
+        store_chunk(tile, r % TILE, t, g);
+        store_chunk(tile, r % TILE, 4 + t, v);
+    }
+}
+
 // Scatters the input-gradient grid columns of rows [offset, end) (GX: 32 floats per row, row r of
-// the batch at GX + 32 r) to the table gradient.
-__global__ void __launch_bounds__(256) nrc_grid_scatter(CacheDev cd, const float* __restrict__ rec,
+// the batch at GX + 32 r) to the table gradient. Four threads a record, four levels each: 16,384 / 65,536 /
+// 262,147 records take 18.5 / 49 / 181 us, 22.6 / 68 / 208 with one thread a record.
+__global__ void __launch_bounds__(256) nrc_grid_scatter(const __grid_constant__ CacheDev cd, const float* __restrict__ rec,
                                                         const uint32_t* count, uint32_t cap, uint32_t offset,
                                                         uint32_t limit, const float* __restrict__ GX)
 {
     uint32_t n = min(*count, cap);
     uint32_t end = offset < n ? min(n, offset + limit) : offset;
-    uint32_t rows = end - offset;
-    for (uint32_t r = blockIdx.x * blockDim.x + threadIdx.x; r < rows; r += gridDim.x * blockDim.x) {
-        float g[32];
-        const float4* src = reinterpret_cast<const float4*>(GX + (size_t)r * 32);
-#pragma unroll
-        for (int k = 0; k < 8; k++) {
-            float4 q = src[k];
-            g[4 * k] = q.x, g[4 * k + 1] = q.y, g[4 * k + 2] = q.z, g[4 * k + 3] = q.w;
-        }
-        grid_backward(cd, rec + (size_t)(offset + r) * REC_WORDS, g);
+    uint64_t items = (uint64_t)(end - offset) * 4;
+    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < items; i += (uint64_t)gridDim.x * blockDim.x) {
+        uint32_t r = (uint32_t)(i >> 2), t = (uint32_t)i & 3u;
+        const float4* src = reinterpret_cast<const float4*>(GX + (size_t)r * 32) + 2 * t;
+        float4 a = src[0], b = src[1];
+        const float* p = rec + (size_t)(offset + r) * REC_WORDS;
+        level_backward(cd, p, 4 * t, a.x, a.y);
+        level_backward(cd, p, 4 * t + 1, a.z, a.w);
+        level_backward(cd, p, 4 * t + 2, b.x, b.y);
+        level_backward(cd, p, 4 * t + 3, b.z, b.w);
     }
 }
 
@@ -626,7 +672,10 @@ void nrc_prepare()
 cudaError_t nrc_launch_encode(int blocks, cudaStream_t s, const vgn::CacheDev& cd, const float* rec,
                               const uint32_t* count, uint32_t cap, uint32_t offset, uint32_t limit, uint8_t* X)
 {
-    nrc_encode<<<blocks, 256, 0, s>>>(cd, rec, count, cap, offset, limit, X);
+    if (std::min(cap, limit) <= ENCODE_SMALL) // (an upper bound of the records: their count is on the device)
+        nrc_encode_small<<<blocks, 256, 0, s>>>(cd, rec, count, cap, offset, limit, X);
+    else
+        nrc_encode<<<blocks, 256, 0, s>>>(cd, rec, count, cap, offset, limit, X);
     return cudaGetLastError();
 }
 

@@ -1,4 +1,6 @@
 // Wavefront kernel variants (shaders/wf_*.slang) and the traversal-only kernels.
+#include <algorithm>
+
 #include "kernels.cuh"
 #include "launch.h"
 
@@ -80,10 +82,18 @@ int wf_extend_blocks_per_sm()
     return n > 0 ? n : 1;
 }
 
-cudaError_t launch_trace_rays(int blocks, cudaStream_t s, const vgd::Ctx& c, const float* rays, uint4* out, uint32_t n,
+static int query_blocks(int sms, uint64_t n, const void* kernel)
+{
+    int per_sm = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, 128, 0) != cudaSuccess || per_sm < 1)
+        per_sm = 1;
+    return (int)std::min<uint64_t>((uint64_t)per_sm * sms, (n + 31) / 32);
+}
+
+cudaError_t launch_trace_rays(int sms, cudaStream_t s, const vgd::Ctx& c, const float* rays, uint4* out, uint32_t n,
                               uint32_t* fetch)
 {
-    vgk::trace_rays<<<blocks, 128, 0, s>>>(c, rays, out, n, fetch);
+    vgk::trace_rays<<<query_blocks(sms, n, (const void*)vgk::trace_rays), 128, 0, s>>>(c, rays, out, n, fetch);
     return cudaGetLastError();
 }
 
@@ -100,9 +110,13 @@ cudaError_t launch_emitter_aux(cudaStream_t s, const float* emitters, uint32_t n
     return cudaGetLastError();
 }
 
-cudaError_t launch_occlusion_rays(cudaStream_t s, const vgd::Ctx& c, const float* rays, uint32_t* out, uint32_t n)
+cudaError_t launch_occlusion_rays(int sms, cudaStream_t s, const vgd::Ctx& c, const float* rays, uint32_t* out, uint32_t n,
+                                  uint32_t* fetch)
 {
-    vgk::occlusion_rays<<<(n + 127) / 128, 128, 0, s>>>(c, rays, out, n);
+    if (c.s.solid)
+        vgk::occlusion_rays_any<<<query_blocks(sms, n, (const void*)vgk::occlusion_rays_any), 128, 0, s>>>(c, rays, out, n, fetch);
+    else
+        vgk::occlusion_rays<<<(n + 127) / 128, 128, 0, s>>>(c, rays, out, n);
     return cudaGetLastError();
 }
 

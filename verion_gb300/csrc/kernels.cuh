@@ -815,6 +815,9 @@ static __global__ void __launch_bounds__(128, 8) wf_stream_shadow_layers(const _
 // of 4 to 10 lanes are within 0.5% of one another and 2% faster than 16; 24 is 3% slower; 2 or 8
 // steps are slower than 4.
 
+// The defaults of the dynamic fetch, for the ray queries.
+constexpr uint32_t TRACE_REFILL = 8, TRACE_STEPS = 4;
+
 // Runs trace_queue, or with COOP trace_queue_coop (warp-cooperative leaf testing; blocks of 128
 // threads, the launchers' size): the same hits either way.
 template <vgt::Hits H, bool COOP, typename GetRay, typename PutHit>
@@ -858,9 +861,10 @@ static __device__ __forceinline__ void put_slot_hit(const Wave& w, uint32_t p, c
 }
 
 // Minimum resident 128-thread blocks per SM requested for the dynamic-fetch traversal stages (a
-// register cap: 8 blocks leave 64 registers per thread).
+// register cap: 9 blocks leave 56 registers per thread; the 1080p frame of the 1M-triangle scene, 32 samples,
+// takes 131.2 ms with 8, 129.9 with 9; before the merged launch 10 made it 3% slower and 7 2%).
 #ifndef VG_TRACE_MIN_BLOCKS
-#define VG_TRACE_MIN_BLOCKS 8
+#define VG_TRACE_MIN_BLOCKS 9
 #endif
 
 // A wave's rays in one launch: the path ray of every queued slot (closest hit) and the shadow rays that
@@ -983,23 +987,24 @@ __global__ void __launch_bounds__(128, VG_TAIL_MIN_BLOCKS) wf_stream_tail(const 
     }
 }
 
-// Closest hits of caller-given rays (6 floats each: origin, direction): the traversal alone, for
-// checking it against an independent implementation and for timing it.
-static __global__ void __launch_bounds__(128) trace_rays(const __grid_constant__ Ctx c, const float* rays, uint4* out,
-                                                   uint32_t n, uint32_t* fetch)
+// Closest hits of caller-given rays (6 floats each: origin, direction): the traversal alone, for tools, for
+// checking it against an independent implementation and for timing it. Dynamic fetch, as the wavefront's: a
+// million random rays over the 12k-triangle scene took 344 us with 32 rays to a warp at a time.
+static __global__ void __launch_bounds__(128, VG_TRACE_MIN_BLOCKS) trace_rays(const __grid_constant__ Ctx c, const float* rays,
+                                                                             uint4* out, uint32_t n, uint32_t* fetch)
 {
-    for (;;) {
-        uint32_t base = warp_fetch(fetch);
-        if (base >= n)
-            break;
-        uint32_t i = base + lane_id();
-        if (i < n) {
-            const float* r = rays + 6 * (size_t)i;
-            Hit h = traceClosest(c, v3(r[0], r[1], r[2]), v3(r[3], r[4], r[5]));
-            out[i] = make_uint4(h.hit ? 1u : 0u, h.inst, h.prim, __float_as_uint(h.t));
-        }
-        __syncwarp();
-    }
+    trace_queue_any<vgt::HITS_CLOSEST, false>(
+        c, fetch, n, TRACE_REFILL, TRACE_STEPS,
+        [&](uint32_t i, V3& o, V3& d, float& tmax, bool&) {
+            const float* r = rays + 6 * (size_t)i; // (a caller's device pointer need be no more than float-aligned)
+            o = v3(r[0], r[1], r[2]);
+            d = v3(r[3], r[4], r[5]);
+            tmax = 1.0e30f;
+            return true;
+        },
+        [&](uint32_t i, const vgt::TraceHit& q) {
+            out[i] = make_uint4(q.hit ? 1u : 0u, q.hit ? q.inst : 0u, q.hit ? q.prim : 0u, __float_as_uint(q.hit ? q.t : 0.0f));
+        });
 }
 
 // Any-hit queries of caller-given rays (7 floats each: origin, direction, tmax) through the
@@ -1012,6 +1017,23 @@ static __global__ void __launch_bounds__(128) occlusion_rays(const __grid_consta
         return;
     const float* r = rays + 7 * (size_t)i;
     out[i] = occluded(c, v3(r[0], r[1], r[2]), v3(r[3], r[4], r[5]), r[6]) ? 1u : 0u;
+}
+
+// The same where every surface is solid: any hit, with dynamic fetch (262 us a million rays with one to a thread).
+static __global__ void __launch_bounds__(128, VG_TRACE_MIN_BLOCKS) occlusion_rays_any(const __grid_constant__ Ctx c,
+                                                                                     const float* rays, uint32_t* out,
+                                                                                     uint32_t n, uint32_t* fetch)
+{
+    trace_queue_any<vgt::HITS_ANY, false>(
+        c, fetch, n, TRACE_REFILL, TRACE_STEPS,
+        [&](uint32_t i, V3& o, V3& d, float& tmax, bool&) {
+            const float* r = rays + 7 * (size_t)i;
+            o = v3(r[0], r[1], r[2]);
+            d = v3(r[3], r[4], r[5]);
+            tmax = r[6];
+            return true;
+        },
+        [&](uint32_t i, const vgt::TraceHit& q) { out[i] = q.hit ? 1u : 0u; });
 }
 
 } // namespace vgk

@@ -98,8 +98,10 @@ cudaError_t launch_aov_main(cudaStream_t s, const vgd::Ctx& c, const float* came
                             uint32_t albedo_stride, float* depth, uint32_t depth_stride, uint32_t* object_ids,
                             uint32_t* material_ids, float* coverage);
 cudaError_t launch_emitter_aux(cudaStream_t s, const float* emitters, uint32_t n, float4* out);
-cudaError_t launch_trace_rays(int blocks, cudaStream_t s, const vgd::Ctx& c, const float* rays, uint4* out, uint32_t n,
+// `fetch`: a cleared device word.
+cudaError_t launch_trace_rays(int sms, cudaStream_t s, const vgd::Ctx& c, const float* rays, uint4* out, uint32_t n,
                               uint32_t* fetch);
-cudaError_t launch_occlusion_rays(cudaStream_t s, const vgd::Ctx& c, const float* rays, uint32_t* out, uint32_t n);
+cudaError_t launch_occlusion_rays(int sms, cudaStream_t s, const vgd::Ctx& c, const float* rays, uint32_t* out, uint32_t n,
+                                  uint32_t* fetch);
 
 } // namespace vgx

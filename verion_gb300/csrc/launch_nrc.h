@@ -38,6 +38,8 @@ inline uint32_t nrc_train_pixels(uint64_t px, uint32_t stride, uint32_t offset, 
 void nrc_prepare();
 
 // Input tiles of records [offset, offset + limit) of the first min(*count, cap) (kern_nrc.cu).
+// At most this many records are encoded with four threads each (nrc_encode_small).
+constexpr uint32_t ENCODE_SMALL = 131072;
 cudaError_t nrc_launch_encode(int blocks, cudaStream_t s, const vgn::CacheDev& cd, const float* rec,
                               const uint32_t* count, uint32_t cap, uint32_t offset, uint32_t limit, uint8_t* X);
 cudaError_t nrc_launch_scatter(int blocks, cudaStream_t s, const vgn::CacheDev& cd, const float* rec,

@@ -1661,7 +1661,7 @@ int vg_trace_closest_device(VgRenderer* r, const float* d_rays, size_t n, uint32
     VG_CHECK(cudaMemsetAsync(r->scratch.p, 0, 4, s), "fetch counter");
     VG_CHECK(cudaEventRecord(a, s), "event");
     if (n > 0)
-        VG_CHECK(vgx::launch_trace_rays(blocks_for(r, r->extend_blocks), s, c, d_rays, (uint4*)d_hits, (uint32_t)n,
+        VG_CHECK(vgx::launch_trace_rays(r->ctx->sms, s, c, d_rays, (uint4*)d_hits, (uint32_t)n,
                                         (uint32_t*)r->scratch.p),
                  "trace launch");
     VG_CHECK(cudaEventRecord(b, s), "event");
@@ -1751,7 +1751,7 @@ int vg_trace_closest_noalloc(VgRenderer* r, const float* rays, size_t n, uint32_
     VG_CHECK(cudaMemsetAsync(base, 0, 8, s), "scratch clear");
     if (n > 0) {
         VG_CHECK(cudaMemcpyAsync(base + NA_RAYS_OFF, rays, n * 24, cudaMemcpyHostToDevice, s), "ray upload");
-        VG_CHECK(vgx::launch_trace_rays(blocks_for(r, r->extend_blocks), s, c, (const float*)(base + NA_RAYS_OFF),
+        VG_CHECK(vgx::launch_trace_rays(r->ctx->sms, s, c, (const float*)(base + NA_RAYS_OFF),
                                         (uint4*)(base + NA_HITS_OFF), (uint32_t)n, (uint32_t*)base),
                  "trace launch");
         VG_CHECK(cudaMemcpyAsync(hits, base + NA_HITS_OFF, n * 16, cudaMemcpyDeviceToHost, s), "hit readback");
@@ -1776,14 +1776,16 @@ int vg_trace_occluded(VgRenderer* r, const float* rays, size_t n, uint32_t* out)
     TempBuf d; // results, then rays
     cudaStream_t s = r->ctx->stream;
     int st;
-    if ((st = d.get(r->ctx, n * 32)) != VG_OK)
+    if ((st = d.get(r->ctx, n * 32 + 4)) != VG_OK)
         return st;
     float* dr = (float*)d.at(n * 4);
+    uint32_t* fetch = (uint32_t*)d.at(n * 32);
     vgd::Ctx c = make_ctx(r, nullptr);
     VG_CHECK(cudaMemsetAsync(r->err.p, 0, 4, s), "error flag");
     if (n > 0) {
         VG_CHECK(cudaMemcpyAsync(dr, rays, n * 28, cudaMemcpyHostToDevice, s), "ray upload");
-        VG_CHECK(vgx::launch_occlusion_rays(s, c, dr, (uint32_t*)d.p, (uint32_t)n), "occlusion launch");
+        VG_CHECK(cudaMemsetAsync(fetch, 0, 4, s), "fetch counter");
+        VG_CHECK(vgx::launch_occlusion_rays(r->ctx->sms, s, c, dr, (uint32_t*)d.p, (uint32_t)n, fetch), "occlusion launch");
         VG_CHECK(cudaMemcpyAsync(out, d.p, n * 4, cudaMemcpyDeviceToHost, s), "readback");
     }
     VG_CHECK(cudaStreamSynchronize(s), "occlusion");
