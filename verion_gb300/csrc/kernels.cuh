@@ -345,12 +345,16 @@ __global__ void __launch_bounds__(128, VG_SHADE_MIN_BLOCKS) wf_shade(const __gri
 // depth by depth (renderer/wavefront.rs:93-177): 2 x depth launches per sample, most of them on a
 // small tail of long paths. Here each pixel's slot runs the batch's params[35] samples back to
 // back: when its path ends, the same thread adds it to the pixel's sums and starts the pixel's next
-// sample in the same slot. A wave is one extend plus one shade over every live slot, whatever the
-// depth of its path. Per pixel the samples are still added in order, one at a time, and adaptive
-// sampling still decides before each sample from the statistics of the samples before it, so the
-// sums are those of the sample-by-sample loop, bit for bit.
-// Counters: queue lengths counts[wave & 1] (in) / counts[~wave & 1] (out), extend work counters
-// fetch[0..1], shade work counters fetch[2..3]; each kernel clears the ones the next kernel uses.
+// sample in the same slot. A wave covers every live slot, whatever the depth of its path: with
+// deferred shadows it is trace (the slots' path rays and the shadow rays that the last wave's shade
+// asked for, one kernel), resolve (shadow results and ended paths into the sums, the next queue and the
+// class queues) and shade; without, extend and a shade that traces its own light samples. Per pixel the
+// samples are still added in order, one at a time, and adaptive sampling still decides before each
+// sample from the statistics of the samples before it, so the sums are those of the sample-by-sample
+// loop, bit for bit.
+// Counters: queue lengths counts[wave & 1] (in) / counts[~wave & 1] (out), trace work counters
+// fetch[0..1], shade work counters fetch[2..3], the separate shadow stage's fetch[4..5]; the kernel that
+// calls clear_wave_counters resets the ones that the stages after it use.
 
 // Path state as stored, for any depth (depth 0 included: it was stored when the sample started).
 template <bool LIGHT>

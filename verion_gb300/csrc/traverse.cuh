@@ -129,12 +129,6 @@ struct TraceHit {
     uint32_t nodes, tests;  // nodes visited and triangles tested (dropped by the compiler unless read)
 };
 
-__device__ __forceinline__ uint32_t byte_of(uint32_t lo, uint32_t hi, int i)
-{
-    uint32_t w = i < 4 ? lo : hi;
-    return (w >> ((i & 3) * 8)) & 0xffu;
-}
-
 // The byte as a float plus 2^15, exactly: the byte placed in bits 8-15 of the mantissa of 2^15 (one
 // byte permute; the last place of the float there is 2^-8). The node test folds the 2^15 into the
 // constant of its FMA, so a plane costs a permute and an FMA, with no subtraction.
