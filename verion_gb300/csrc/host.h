@@ -304,7 +304,8 @@ struct VgRenderer {
     Restir restir;
     uint32_t max_depth = DEFAULT_MAX_DEPTH;
     int precision = 64;
-    int extend_blocks = 0;
+    int extend_blocks = 0, extend_most = 0;
+    int trace_blocks = 0;
     int shade_blocks[8] = {};
     int stream_shade_blocks[8] = {};
     int deferred_blocks = 0;

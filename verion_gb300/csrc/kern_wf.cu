@@ -354,13 +354,10 @@ int stream_shadow_trace_blocks_per_sm()
     return n;
 }
 
-int stream_trace_blocks_per_sm(bool coop)
+int stream_trace_blocks_per_sm()
 {
     int n = 0;
-    if (coop)
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, vgk::wf_stream_extend_dyn<false, true>, 128, 0);
-    else
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, vgk::wf_stream_extend_dyn<false, false>, 128, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, vgk::wf_stream_trace, 128, 0);
     return n > 0 ? n : 1;
 }
 

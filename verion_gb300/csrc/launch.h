@@ -69,7 +69,7 @@ cudaError_t launch_stream_extend_dyn(bool stats, bool coop, int blocks, cudaStre
                                      const vgk::Wave& w, uint32_t wave);
 cudaError_t launch_stream_shadow_trace(bool stats, bool coop, int blocks, cudaStream_t s, const vgd::Ctx& c,
                                        const vgk::Wave& w, uint32_t wave);
-int stream_trace_blocks_per_sm(bool coop);
+int stream_trace_blocks_per_sm();
 int stream_shadow_trace_blocks_per_sm();
 // The same streaming stages compiled with ReSTIR (kern_wf_restir.cu); the host runs them one
 // sample per launch sequence.

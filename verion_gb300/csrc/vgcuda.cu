@@ -199,6 +199,10 @@ int stream_samples(VgRenderer* r, VgAccum* acc, vgd::Ctx& c, vgx::Variant v, con
     cudaStream_t s = r->ctx->stream;
     int st;
     int eb = blocks_for(r, r->extend_blocks);
+    // The merged trace kernel has fewer registers than the per-sample extend kernel that extend_blocks
+    // counts (8 blocks per SM): with that setting at its most it fills the SMs by its own count (9; the 1080p
+    // frame of the 1M-triangle scene, 32 samples: 129.3 against 126.5 ms, smaller frames the same).
+    int tb = r->extend_blocks < r->extend_most ? eb : blocks_for(r, r->trace_blocks);
     acc->wave_live.clear();
     acc->wave_ms.clear();
     acc->tail_ms = 0.0f;
@@ -243,7 +247,7 @@ int stream_samples(VgRenderer* r, VgAccum* acc, vgd::Ctx& c, vgx::Variant v, con
     auto launch_wave = [&](uint32_t i, auto&& mark) -> cudaError_t {
         cudaError_t e;
         if (merged)
-            e = vgx::launch_stream_trace(eb, s, c, w, i);
+            e = vgx::launch_stream_trace(tb, s, c, w, i);
         else
             e = dyn ? vgx::launch_stream_extend_dyn(r->traversal_stats, r->coop_tris, eb, s, c, w, i)
                     : vgx::launch_stream_extend(r->traversal_stats, eb, s, c, w, i);
@@ -610,7 +614,8 @@ int vg_renderer_create(VgContext* ctx, const VgPacked* pk, VgRenderer** out)
     bind_tables(r);
     r->ds.shadow_any = translucent ? 0u : 1u;
     r->ds.solid = solid ? 1u : 0u;
-    r->extend_blocks = vgx::wf_extend_blocks_per_sm();
+    r->extend_blocks = r->extend_most = vgx::wf_extend_blocks_per_sm();
+    r->trace_blocks = vgx::stream_trace_blocks_per_sm();
     *out = r;
     return VG_OK;
 }
