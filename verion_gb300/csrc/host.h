@@ -427,6 +427,8 @@ int alloc_parts(DevBuf& whole, std::vector<Part> parts, cudaStream_t s)
         total += padded(p.bytes);
         zero += p.zero ? padded(p.bytes) : 0;
     }
+    for (auto& p : parts) // (no part outlives the memory it was cut from, should this allocation fail)
+        p.buf->release();
     int st = alloc(whole, total, s, false);
     if (st != VG_OK)
         return st;
@@ -434,7 +436,6 @@ int alloc_parts(DevBuf& whole, std::vector<Part> parts, cudaStream_t s)
         VG_CHECK(cudaMemsetAsync(whole.p, 0, zero, s), "cudaMemsetAsync");
     char* at = (char*)whole.p;
     for (auto& p : parts) {
-        p.buf->release();
         p.buf->p = at;
         p.buf->bytes = std::max<size_t>(p.bytes, 16);
         p.buf->part = true;

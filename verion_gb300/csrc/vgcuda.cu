@@ -1080,10 +1080,12 @@ int vg_accumulate(VgRenderer* r, VgAccum* acc, uint32_t samples)
     const uint32_t sample0 = acc->first_sample + acc->samples; // index of this call's first sample
     bool wavefront = r->integrator == VG_WAVEFRONT && !r->cache;
     const uint32_t max_depth_alloc = 64;
-    if (r->integrator == VG_WAVEFRONT && !acc->state.p) {
+    // Deferred shadows (stream_samples) keep per slot the request and the ended path's radiance; ReSTIR with the
+    // lighting split never defers. ReSTIR is captured anew by each call before the first sample (after a call of
+    // no samples or one that failed), so buffers made for one setting may be too small for the next.
+    const size_t dpx = acc->lighting && acc->restir.on ? 0 : px;
+    if (r->integrator == VG_WAVEFRONT && (!acc->state.p || acc->flags.bytes < dpx * 4)) {
         uint32_t planes = vgk::BASE_PLANES + (acc->lighting ? vgk::SPLIT_PLANES : 0);
-        // Deferred shadows (stream_samples): per slot the request and the ended path's radiance.
-        const size_t dpx = acc->lighting && acc->restir.on ? 0 : px;
         const size_t req_planes = acc->lighting ? vgk::SPLIT_REQ_PLANES : vgk::REQ_PLANES;
         const size_t pend_planes = acc->lighting ? 1 + vgk::SPLIT_PLANES : 1;
         if ((st = alloc_parts(acc->wave,
