@@ -3,6 +3,7 @@
 
 #include "kernels.cuh"
 #include "launch.h"
+#include "ray_chunks.h"
 
 namespace vgx {
 
@@ -87,14 +88,23 @@ static int query_blocks(int sms, uint64_t n, const void* kernel)
     int per_sm = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, 128, 0) != cudaSuccess || per_sm < 1)
         per_sm = 1;
-    return (int)std::min<uint64_t>((uint64_t)per_sm * sms, (n + 31) / 32);
+    return (int)std::min<uint64_t>({(uint64_t)per_sm * sms, (n + 31) / 32, RAY_QUERY_WARPS / 4});
 }
 
 cudaError_t launch_trace_rays(int sms, cudaStream_t s, const vgd::Ctx& c, const float* rays, uint4* out, uint32_t n,
                               uint32_t* fetch)
 {
-    vgk::trace_rays<<<query_blocks(sms, n, (const void*)vgk::trace_rays), 128, 0, s>>>(c, rays, out, n, fetch);
-    return cudaGetLastError();
+    for (uint32_t k = 0; k < ray_chunks(n); k++) {
+        RayChunk q = ray_chunk(n, k);
+        cudaError_t e = k ? cudaMemsetAsync(fetch, 0, 4, s) : cudaSuccess;
+        if (e != cudaSuccess)
+            return e;
+        vgk::trace_rays<<<query_blocks(sms, q.n, (const void*)vgk::trace_rays), 128, 0, s>>>(
+            c, rays + 6 * (size_t)q.at, out + q.at, q.n, fetch);
+        if ((e = cudaGetLastError()) != cudaSuccess)
+            return e;
+    }
+    return cudaSuccess;
 }
 
 static __global__ void emitter_aux(const float* emitters, uint32_t n, float4* out)
@@ -113,11 +123,20 @@ cudaError_t launch_emitter_aux(cudaStream_t s, const float* emitters, uint32_t n
 cudaError_t launch_occlusion_rays(int sms, cudaStream_t s, const vgd::Ctx& c, const float* rays, uint32_t* out, uint32_t n,
                                   uint32_t* fetch)
 {
-    if (c.s.solid)
-        vgk::occlusion_rays_any<<<query_blocks(sms, n, (const void*)vgk::occlusion_rays_any), 128, 0, s>>>(c, rays, out, n, fetch);
-    else
-        vgk::occlusion_rays<<<(n + 127) / 128, 128, 0, s>>>(c, rays, out, n);
-    return cudaGetLastError();
+    for (uint32_t k = 0; k < ray_chunks(n); k++) {
+        RayChunk q = ray_chunk(n, k);
+        const float* r = rays + 7 * (size_t)q.at;
+        cudaError_t e = k ? cudaMemsetAsync(fetch, 0, 4, s) : cudaSuccess;
+        if (e != cudaSuccess)
+            return e;
+        if (c.s.solid)
+            vgk::occlusion_rays_any<<<query_blocks(sms, q.n, (const void*)vgk::occlusion_rays_any), 128, 0, s>>>(c, r, out + q.at, q.n, fetch);
+        else
+            vgk::occlusion_rays<<<(q.n + 127) / 128, 128, 0, s>>>(c, r, out + q.at, q.n);
+        if ((e = cudaGetLastError()) != cudaSuccess)
+            return e;
+    }
+    return cudaSuccess;
 }
 
 } // namespace vgx
