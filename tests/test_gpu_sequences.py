@@ -1,10 +1,12 @@
 """Sequences of calls that the entry points accept before an accumulation's first sample: options changed after a call
 that added no sample, or that failed, give what a fresh accumulation with the later options gives, bit for bit."""
+import time
+
 import numpy as np
 import pytest
 
 from verion_gb300 import pack, scenes
-from verion_gb300.backend import Cache, Error, Integrator, Renderer
+from verion_gb300.backend import VG_ERR_TIMEOUT, Cache, Error, Integrator, Renderer
 from verion_gb300.readback import Restir
 
 from .test_gpu_parity import assert_same, oracle_render
@@ -37,3 +39,38 @@ def test_restir_switched_off_before_the_first_sample_of_a_split(gpu_ctx, first, 
     ref = oracle_render(p, w, h, spp, lighting=True)
     assert_same(acc.sums(), ref.sums, "sums")
     assert_same(acc.raw_lighting(), ref.lighting, "lighting split")
+
+
+@pytest.mark.parametrize("form", ["megakernel", "one launch", "waves"])
+def test_a_deadline_passed_returns_at_once_and_leaves_the_context_usable(gpu_ctx, form, monkeypatch):
+    # The limit is far below what the call's GPU work takes, which ends by itself afterwards.
+    p = pack.pack(scenes.many_spheres(spheres=16, sphere_n=21, grid=160, hdri=(64, 32)))
+    r = Renderer(gpu_ctx, p)
+    r.set_integrator(Integrator.MEGAKERNEL if form == "megakernel" else Integrator.WAVEFRONT)
+    r.set_accum_precision(32)
+    r.set_max_depth(16)
+    w, h, spp = (960, 540, 64) if form == "waves" else (512, 512, 192)
+    r.set_stream_tail(0 if form == "waves" else 1 << 18)
+    small = r.new_accumulation(33, 31)
+    r.accumulate(small, 2)
+    want = small.sums()
+
+    full = r.new_accumulation(w, h)
+    r.accumulate(full, 1)
+    t = time.perf_counter()
+    r.accumulate(full, spp)
+    ordinary = time.perf_counter() - t
+    assert ordinary > 0.02
+    monkeypatch.setenv("VG_TIMEOUT_S", "0.0001")
+    t = time.perf_counter()
+    with pytest.raises(Error) as e:
+        r.accumulate(full, spp)
+    passed = time.perf_counter() - t
+    monkeypatch.delenv("VG_TIMEOUT_S")
+    assert e.value.status == VG_ERR_TIMEOUT
+    assert passed < ordinary / 2
+    # With the abandoned work still in flight, calls that take the same pools give what they gave.
+    for _ in range(3):
+        acc = r.new_accumulation(33, 31)
+        r.accumulate(acc, 2)
+        assert np.array_equal(acc.sums(), want)

@@ -87,9 +87,9 @@ int wait_event(cudaEvent_t ev)
         double dt = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
         if (dt > limit)
             return fail(VG_ERR_TIMEOUT, "the GPU did not finish within " + std::to_string(limit) + " s");
-        // The shortest sleep takes some 70 us, longer than a small wave: the first 2 ms are polled.
-        if (dt > 0.002)
-            std::this_thread::sleep_for(std::chrono::microseconds(dt < 0.02 ? 20 : 200));
+        // The shortest sleep takes some 70 us, longer than a small wave: the first 20 ms are polled.
+        if (dt > 0.02)
+            std::this_thread::sleep_for(std::chrono::microseconds(dt < 0.2 ? 20 : 200));
     }
 }
 
@@ -125,8 +125,9 @@ struct DevBuf {
 
 // Device buffers that entry points use for the length of a call (rays and hits, records, AOV planes), kept
 // for the next call: a cudaMalloc and cudaFree of some tens of MB cost more than most of those calls'
-// kernels. A buffer has one owner at a time (TempBuf), whichever thread that is on; it is given back when
-// the context's stream is done with it. At most KEEP bytes wait here, and they go with the context.
+// kernels. A buffer has one owner at a time (TempBuf), whichever thread that is on. All of its uses are in the
+// order of the context's stream, so that the next owner's work comes after the last one's. At most KEEP bytes
+// wait here (twice that while the stream is busy: freeing waits for the GPU); they go with the context.
 struct TempPool {
     static constexpr size_t KEEP = 256u << 20;
     std::mutex mu;
@@ -148,13 +149,14 @@ struct TempPool {
         idle.erase(idle.begin() + (long)best);
         return p;
     }
-    void give(void* p, size_t bytes)
+    void give(void* p, size_t bytes, cudaStream_t s)
     {
         std::vector<void*> drop;
+        size_t keep = cudaStreamQuery(s) == cudaErrorNotReady ? 2 * KEEP : KEEP;
         {
             std::lock_guard<std::mutex> lock(mu);
-            if (bytes <= KEEP) {
-                while (idle_bytes + bytes > KEEP) { // the oldest first
+            if (bytes <= keep) {
+                while (idle_bytes + bytes > keep) { // the oldest first
                     drop.push_back(idle.front().first);
                     idle_bytes -= idle.front().second;
                     idle.erase(idle.begin());
@@ -179,37 +181,57 @@ struct TempPool {
     }
 };
 
-// Pinned words that the GPU writes its wave counts and status to: a ring per accumulate call in flight.
-// The rings of finished calls are used again; they go with the context.
+// Pinned words that the GPU writes its wave counts and status to: a ring per accumulate call in flight. A ring
+// is used again once the stream has passed the point where its call ended; they go with the context.
 struct RingPool {
     static constexpr size_t WORDS = 16;
+    struct Entry {
+        uint32_t* words;
+        cudaEvent_t passed;
+        bool taken, given;
+    };
     std::mutex mu;
-    std::vector<uint32_t*> idle, all;
+    std::vector<Entry> all;
     uint32_t* take()
     {
         std::lock_guard<std::mutex> lock(mu);
-        if (idle.empty()) {
-            void* p = nullptr;
-            if (cudaHostAlloc(&p, WORDS * 4, cudaHostAllocPortable) != cudaSuccess) {
-                cudaGetLastError();
-                return nullptr;
+        for (Entry& e : all)
+            if (!e.taken && (!e.given || cudaEventQuery(e.passed) == cudaSuccess)) {
+                e.taken = true;
+                return e.words;
             }
-            idle.push_back((uint32_t*)p);
-            all.push_back((uint32_t*)p);
+        void* p = nullptr;
+        Entry e{};
+        if (cudaHostAlloc(&p, WORDS * 4, cudaHostAllocPortable) != cudaSuccess) {
+            cudaGetLastError();
+            return nullptr;
         }
-        uint32_t* r = idle.back();
-        idle.pop_back();
-        return r;
+        if (cudaEventCreateWithFlags(&e.passed, cudaEventDisableTiming) != cudaSuccess) {
+            cudaGetLastError();
+            cudaFreeHost(p);
+            return nullptr;
+        }
+        e.words = (uint32_t*)p;
+        e.taken = true;
+        all.push_back(e);
+        return e.words;
     }
-    void give(uint32_t* r)
+    void give(uint32_t* words, cudaStream_t s)
     {
         std::lock_guard<std::mutex> lock(mu);
-        idle.push_back(r);
+        for (Entry& e : all)
+            if (e.words == words) {
+                // (Not recorded: the words stay taken, and go with the context.)
+                e.taken = cudaEventRecord(e.passed, s) != cudaSuccess;
+                e.given = true;
+            }
     }
     ~RingPool()
     {
-        for (uint32_t* p : all)
-            cudaFreeHost(p);
+        for (Entry& e : all) {
+            cudaEventDestroy(e.passed);
+            cudaFreeHost(e.words);
+        }
     }
 };
 
@@ -449,6 +471,8 @@ struct TempBuf {
     VgContext* ctx = nullptr;
     void* p = nullptr;
     size_t bytes = 0;
+    // The call copies between the buffer and the caller's memory: however it ends, its end waits for the copies.
+    bool host_copies = true;
     TempBuf() = default;
     TempBuf(const TempBuf&) = delete;
     TempBuf& operator=(const TempBuf&) = delete;
@@ -474,10 +498,11 @@ struct TempBuf {
     char* at(size_t offset) const { return (char*)p + offset; }
     ~TempBuf()
     {
-        if (p) {
-            cudaStreamSynchronize(ctx->stream); // the call may have failed with work in flight
-            ctx->temps.give(p, bytes);
-        }
+        if (!p)
+            return;
+        if (host_copies)
+            cudaStreamSynchronize(ctx->stream);
+        ctx->temps.give(p, bytes, ctx->stream);
     }
 };
 
@@ -490,10 +515,8 @@ struct Ring {
     Ring& operator=(const Ring&) = delete;
     ~Ring()
     {
-        if (words) {
-            cudaStreamSynchronize(ctx->stream);
-            ctx->rings.give(words);
-        }
+        if (words)
+            ctx->rings.give(words, ctx->stream);
     }
 };
 

@@ -299,6 +299,13 @@ int stream_samples(VgRenderer* r, VgAccum* acc, vgd::Ctx& c, vgx::Variant v, con
         VG_CHECK(cudaMemsetAsync(w.shcount, 0, 2 * 4, s), "counters");
     VG_CHECK((q ? vgx::launch_stream_cache_start(v.f64, s, c, w, *q) : vgx::launch_stream_start(v, s, c, w)), "stream start launch");
     acc->launches++;
+    if (deferred && w.n <= tail && !timed && !r->traversal_stats && r->graph_waves == 0) {
+        // A small frame: no waves at all, from the camera rays on, and nothing for the host to read.
+        VG_CHECK(launch_tail(w.n, 0), "tail launch");
+        acc->launches++;
+        acc->last_waves = 1;
+        return VG_OK;
+    }
     // Waves until no slot is live. The host reads each wave's output count LAG waves later,
     // so the GPU never idles on the poll; extra waves on an empty queue exit at once.
     const uint32_t LAG = 2, RING = 8;
@@ -313,12 +320,6 @@ int stream_samples(VgRenderer* r, VgAccum* acc, vgd::Ctx& c, vgx::Variant v, con
         e = pool.get();
     bool done = false;
     uint64_t wave = 0;
-    if (deferred && w.n <= tail && !timed && !r->traversal_stats && r->graph_waves == 0) {
-        // A small frame: no waves at all, from the camera rays on.
-        VG_CHECK(launch_tail(w.n, 0), "tail launch");
-        acc->launches++;
-        done = true;
-    }
     if (r->graph_waves > 0 && !timed) {
         // Captured chunks of graph_waves waves (even, so the queue parity of every wave in a
         // replay matches its place in the sequence), each ending with the live count.
@@ -377,8 +378,14 @@ int stream_samples(VgRenderer* r, VgAccum* acc, vgd::Ctx& c, vgx::Variant v, con
             }
         }
         wave = rep * K;
-        VG_CHECK(cudaStreamSynchronize(s), "waves");
+        cudaEvent_t last = pool.get();
+        if ((ce = cudaEventRecord(last, s)) != cudaSuccess)
+            st = cuda_fail(ce, "event");
+        else
+            st = wait_event(last);
         cudaGraphExecDestroy(ge);
+        if (st != VG_OK)
+            return st;
         if (!done && ring[0] != 0)
             return fail(VG_ERR_KERNEL, "streaming wavefront did not drain within its wave bound");
         done = true;
@@ -428,15 +435,15 @@ int stream_samples(VgRenderer* r, VgAccum* acc, vgd::Ctx& c, vgx::Variant v, con
             }
         }
     }
-    acc->last_waves = (uint32_t)std::max<uint64_t>(wave, 1);
-    VG_CHECK(cudaStreamSynchronize(s), "waves");
+    acc->last_waves = (uint32_t)wave;
+    cudaEvent_t last = pool.get();
+    VG_CHECK(cudaEventRecord(last, s), "event");
+    if ((st = wait_event(last)) != VG_OK)
+        return st;
     for (uint64_t k = wave > LAG ? wave - LAG + 1 : 0; k < wave; k++)
         acc->wave_live.push_back(ring[k % RING]);
-    if (!done) {
-        VG_CHECK(cudaStreamSynchronize(s), "waves");
-        if (ring[(wave - 1) % RING] != 0)
-            return fail(VG_ERR_KERNEL, "streaming wavefront did not drain within its wave bound");
-    }
+    if (!done && ring[(wave - 1) % RING] != 0)
+        return fail(VG_ERR_KERNEL, "streaming wavefront did not drain within its wave bound");
     return VG_OK;
 }
 
@@ -1128,6 +1135,7 @@ int vg_accumulate(VgRenderer* r, VgAccum* acc, uint32_t samples)
         vgx::BlockGrid grid{};
         vgk::Wave w = wave_of(r, acc);
         TempBuf scratch;
+        scratch.host_copies = false; // given back with the launches in flight: the call's deadline is waited for below
         uint32_t *pixels = nullptr, *next = nullptr;
         if (blocks) {
             grid = vgx::block_grid(r->ctx->sms, vgx::megakernel_items(acc->width, acc->height));
