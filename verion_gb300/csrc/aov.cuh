@@ -110,12 +110,14 @@ static __global__ void __launch_bounds__(128) aov_normals(const __grid_constant_
 }
 
 // aov.slang:86-188 but for the coverage (aov_coverage_*). Albedo and depth go to planes of their own or
-// interleaved, by their strides.
+// interleaved, by their strides. Also clears the counters of the coverage's rest (two words).
 static __global__ void __launch_bounds__(128) aov_main(const __grid_constant__ Ctx c, CameraRecord cam,
                                                        float* albedo, uint32_t albedo_stride, float* depths,
                                                        uint32_t depth_stride, uint32_t* object_ids,
-                                                       uint32_t* material_ids)
+                                                       uint32_t* material_ids, uint32_t* rest_counters)
 {
+    if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x < 2)
+        rest_counters[threadIdx.x] = 0;
     uint32_t w = (uint32_t)cam.v[0], h = (uint32_t)cam.v[1];
     uint32_t x = blockIdx.x * 16 + (threadIdx.x & 15u), y = blockIdx.y * 8 + (threadIdx.x >> 4);
     if (x >= w || y >= h)
@@ -243,20 +245,46 @@ static __global__ void __launch_bounds__(128) aov_coverage_layers(const __grid_c
 // smallest of their direction components, so a box that any of them meets is visited (a superset of what
 // each ray's own walk visits, and a hit of any triangle is what each ray's walk looks for: the counts
 // are the same). A triangle found is classified against the samples' box first (cover_box); one that covers
-// some of it is tested sample by sample, by the rays' own test. The walk ends when all 16 are covered. Lanes go on to their next leaf before the warp tests triangles,
-// and a pixel whose directions change sign in an axis (a line or two of pixels) traces its rays one by
-// one. Bound by issue: 16 walks of some 13 nodes become one of about 15. With one walk per ray this was
-// most of aov_main's 7.5 ms per 1920x1080 frame of the 1M-triangle scene, with every triangle found tested
-// against all samples 2.8 ms.
+// some of it is tested against the samples still open, by the rays' own test. The walk ends when all 16 are
+// covered. Lanes go on to their next leaf before the warp tests triangles. Bound by issue: where the pixel is
+// no larger than a few triangles, 16 walks of some 13 nodes become one of about 15.
+//
+// Where it is larger the beam meets every box in the pixel, and the warp waits for its worst one. So a walk that
+// has cost COVER_WORK (node visits, and COVER_SOME_WORK for each triangle tested sample by sample) is given up, and
+// the pixel goes to `rest` with its open samples, as does one whose directions change sign in an axis (a line or two of
+// pixels): aov_coverage_rest traces those rays one by one. A block is a tile of 16 x 8 pixels, the launch's from
+// first_tile on, row by row of tiles.
+// Whole calls in us with COVER_WORK 16 / 64 / 256 (COVER_SOME_WORK 4, at 16: 2), and with 16 closest-hit walks a pixel and
+// no beam: the 1M-triangle scene at 16x16 336 / 502 / 1004, 818; 64x48 386 / 572 / 1044, 1021; 641x359 884 / 852 / 1027,
+// 3194; 1920x1080 3627 / 2680 / 2632, 19,673; the 110k-triangle scene at 16x16 300 / 433 / 783, 680; 1920x1080 1762 / 1614 /
+// 1576, 18,033. Without a bound the 1M scene took 35.3 ms at 16x16 and 7.3 at 64x48.
+constexpr uint32_t COVER_WORK = 64, COVER_SOME_WORK = 4;
+constexpr uint32_t COVER_TILES = 1u << 16; // most tiles of one launch: at most 2^23 pixels and 2^27 rays in `rest`
+
+// A pixel of the launch (the tile's number in it x 128 + the thread) and its samples still open.
+struct CoverRest {
+    uint2* pixels;
+    uint32_t* count;
+    uint32_t* fetch;
+};
+
+// Pixel of thread `tid` of tile `tile`: a warp's are 4 x 8.
+static __device__ __forceinline__ void coverPixel(uint32_t w, uint32_t tile, uint32_t tid, uint32_t& x, uint32_t& y)
+{
+    uint32_t tiles_x = (w + 15u) / 16u;
+    x = tile % tiles_x * 16 + (tid >> 5) * 4 + (tid & 3u);
+    y = tile / tiles_x * 8 + ((tid >> 2) & 7u);
+}
+
 static __global__ void __launch_bounds__(128, 6) aov_coverage_solid(const __grid_constant__ Ctx c, CameraRecord cam,
-                                                                    float* coverage)
+                                                                    float* coverage, uint32_t first_tile, CoverRest rest)
 {
     __shared__ float4 rays[16][128]; // shear x, y, z and the axis permutation of each thread's samples
     uint32_t tid = threadIdx.x;
-    uint32_t w = (uint32_t)cam.v[0], h = (uint32_t)cam.v[1];
-    uint32_t x = blockIdx.x * 16 + (tid >> 5) * 4 + (tid & 3u), y = blockIdx.y * 8 + ((tid >> 2) & 7u);
-    if (x >= w || y >= h)
-        return;
+    uint32_t w = (uint32_t)cam.v[0], h = (uint32_t)cam.v[1], x, y;
+    coverPixel(w, first_tile + blockIdx.x, tid, x, y);
+    bool inside = x < w && y < h, open = inside;
+    uint32_t covered = 0;
     float t = cam.v[2], aspect = cam.v[0] / cam.v[1];
     V3 org = v3(cam.v[7], cam.v[11], cam.v[15]);
     V3 lo = v3(3.0e38f), hi = v3(-3.0e38f);
@@ -269,7 +297,7 @@ static __global__ void __launch_bounds__(128, 6) aov_coverage_solid(const __grid
     // The samples' shears, their box, and the axis permutation when all have the same.
     V3 slo = v3(3.0e38f), shi = v3(-3.0e38f);
     int kx = 0, ky = 0, kz = 0;
-    bool same = true;
+    bool same = inside;
 #pragma unroll
     for (uint32_t k = 0; k < 16; k++) {
         V3 d;
@@ -288,7 +316,6 @@ static __global__ void __launch_bounds__(128, 6) aov_coverage_solid(const __grid
             lo = v3(-3.0e38f); // no beam
     }
     auto one_sign = [](float a, float b) { return a > bvh8::MIN_DIR || (b < -bvh8::MIN_DIR && a > -2.0f); };
-    uint32_t covered = 0;
     if (same && one_sign(lo.x, hi.x) && one_sign(lo.y, hi.y) && one_sign(lo.z, hi.z)) {
         float mx = 0.5f * (slo.x + shi.x), my = 0.5f * (slo.y + shi.y);
         float hx = 1.000001f * (0.5f * (shi.x - slo.x)) + 1.0e-6f * fabsf(mx);
@@ -307,12 +334,14 @@ static __global__ void __launch_bounds__(128, 6) aov_coverage_solid(const __grid
         k.node = 0;
         k.sp = 0;
         k.nodes = 0;
+        uint32_t work = 0;
         bool done = false;
-        while (!done && covered != 0xffffu) {
+        while (!done && covered != 0xffffu && work < COVER_WORK) {
             do {
                 vgt::node_visit(c.s.nodes, k, b);
+                work++;
                 done = vgt::next_node(k, stack, c.err);
-            } while (!done && k.tri_bits == 0);
+            } while (!done && k.tri_bits == 0 && work < COVER_WORK);
             while (k.tri_bits && covered != 0xffffu) {
                 uint32_t j = vgt::high_bit(k.tri_bits);
                 k.tri_bits ^= 1u << j;
@@ -322,23 +351,61 @@ static __global__ void __launch_bounds__(128, 6) aov_coverage_solid(const __grid
                 Cover cv = cover_box(v, mx, my, hx, hy, slo.z, shi.z);
                 if (cv == COVER_ALL)
                     covered = 0xffffu;
-                if (cv == COVER_SOME)
-                    for (uint32_t i = 0; i < 16; i++) {
+                if (cv == COVER_SOME) {
+                    work += COVER_SOME_WORK;
+                    for (uint32_t left = covered ^ 0xffffu; left; left &= left - 1) {
+                        uint32_t i = (uint32_t)__ffs((int)left) - 1u;
                         float4 q = rays[i][tid];
                         float th, U, V, W, det;
                         if (vgt::tri_test(v, q.x, q.y, q.z, th, U, V, W, det) && th < 1.0e30f)
                             covered |= 1u << i;
                     }
+                }
             }
         }
-    } else {
-        for (uint32_t k = 0; k < 16; k++) {
-            V3 d = sampleDir(cam, x, y, k, w, h, t, aspect);
-            if (vgt::trace_bvh<true>(c.s.nodes, c.s.tris, org, d, 1.0e30f, c.err).hit)
-                covered |= 1u << k;
-        }
+        open = !done && covered != 0xffffu;
     }
-    coverage[(size_t)y * w + x] = (float)__popc(covered) / 16.0f;
+    if (inside)
+        coverage[(size_t)y * w + x] = (float)__popc(covered) / 16.0f;
+    __syncwarp();
+    uint32_t b = __ballot_sync(vgk::FULL, open), base = 0, lane = tid & 31u;
+    if (b == 0)
+        return;
+    if (lane == 0)
+        base = atomicAdd(rest.count, __popc(b));
+    base = __shfl_sync(vgk::FULL, base, 0);
+    if (open)
+        rest.pixels[base + __popc(b & ((1u << lane) - 1u))] = make_uint2(blockIdx.x * 128 + tid, covered ^ 0xffffu);
+}
+
+// The rays that aov_coverage_solid left, any hit with dynamic fetch: an image of few pixels fills the chip with them
+// too. A hit adds its sixteenth, exactly and in any order.
+static __global__ void __launch_bounds__(128, VG_TRACE_MIN_BLOCKS) aov_coverage_rest(const __grid_constant__ Ctx c, CameraRecord cam,
+                                                                                    float* coverage, uint32_t first_tile,
+                                                                                    CoverRest rest)
+{
+    uint32_t w = (uint32_t)cam.v[0], h = (uint32_t)cam.v[1];
+    auto pixel = [&](uint32_t i, uint32_t& x, uint32_t& y) {
+        uint2 e = rest.pixels[i >> 4];
+        coverPixel(w, first_tile + (e.x >> 7), e.x & 127u, x, y);
+        return ((e.y >> (i & 15u)) & 1u) != 0;
+    };
+    vgk::trace_queue_any<vgt::HITS_ANY, false>(
+        c, rest.fetch, *rest.count * 16u, vgk::TRACE_REFILL, vgk::TRACE_STEPS,
+        [&](uint32_t i, V3& o, V3& d, float& tmax, bool&) {
+            uint32_t x, y;
+            o = v3(cam.v[7], cam.v[11], cam.v[15]);
+            tmax = 1.0e30f;
+            if (!pixel(i, x, y))
+                return false;
+            d = sampleDir(cam, x, y, i & 15u, w, h, cam.v[2], cam.v[0] / cam.v[1]);
+            return true;
+        },
+        [&](uint32_t i, const vgt::TraceHit& q) {
+            uint32_t x, y;
+            if (q.hit && pixel(i, x, y))
+                atomicAdd(coverage + (size_t)y * w + x, 0.0625f);
+        });
 }
 
 } // namespace vga

@@ -67,24 +67,47 @@ cudaError_t launch_aov_normals(cudaStream_t s, const vgd::Ctx& c, const float* c
     return cudaGetLastError();
 }
 
-cudaError_t launch_aov_main(cudaStream_t s, const vgd::Ctx& c, const float* camera18, float* albedo,
+// The launches that cover the frame's tiles, and the bytes of their scratch (two counters, then the pixels left).
+size_t aov_scratch_bytes(uint32_t w, uint32_t h)
+{
+    uint64_t tiles = (uint64_t)((w + 15) / 16) * ((h + 7) / 8);
+    return 256 + std::min<uint64_t>(tiles, vga::COVER_TILES) * 128 * sizeof(uint2);
+}
+
+cudaError_t launch_aov_main(int sms, cudaStream_t s, const vgd::Ctx& c, const float* camera18, float* albedo,
                             uint32_t albedo_stride, float* depth, uint32_t depth_stride, uint32_t* object_ids,
-                            uint32_t* material_ids, float* coverage)
+                            uint32_t* material_ids, float* coverage, void* scratch)
 {
     vga::CameraRecord cam;
     for (int i = 0; i < 18; i++)
         cam.v[i] = camera18[i];
     uint32_t w = (uint32_t)cam.v[0], h = (uint32_t)cam.v[1];
     dim3 grid((w + 15) / 16, (h + 7) / 8);
-    vga::aov_main<<<grid, 128, 0, s>>>(c, cam, albedo, albedo_stride, depth, depth_stride, object_ids, material_ids);
+    uint32_t* counters = (uint32_t*)scratch;
+    vga::aov_main<<<grid, 128, 0, s>>>(c, cam, albedo, albedo_stride, depth, depth_stride, object_ids, material_ids, counters);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess)
         return e;
-    if (c.s.solid)
-        vga::aov_coverage_solid<<<grid, 128, 0, s>>>(c, cam, coverage);
-    else
+    if (!c.s.solid) {
         vga::aov_coverage_layers<<<grid, 128, 0, s>>>(c, cam, coverage);
-    return cudaGetLastError();
+        return cudaGetLastError();
+    }
+    vga::CoverRest rest{(uint2*)(counters + 64), counters, counters + 1};
+    int per_sm = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, vga::aov_coverage_rest, 128, 0) != cudaSuccess || per_sm < 1)
+        per_sm = 1;
+    uint64_t tiles = (uint64_t)grid.x * grid.y;
+    for (uint64_t at = 0; at < tiles; at += vga::COVER_TILES) {
+        uint32_t n = (uint32_t)std::min<uint64_t>(tiles - at, vga::COVER_TILES);
+        if (at && (e = cudaMemsetAsync(counters, 0, 8, s)) != cudaSuccess)
+            return e;
+        vga::aov_coverage_solid<<<n, 128, 0, s>>>(c, cam, coverage, (uint32_t)at, rest);
+        // (A tile's pixels are at most 64 warps of rays: 16 blocks.)
+        vga::aov_coverage_rest<<<(unsigned)std::min<uint64_t>((uint64_t)per_sm * sms, 16ull * n), 128, 0, s>>>(c, cam, coverage, (uint32_t)at, rest);
+        if ((e = cudaGetLastError()) != cudaSuccess)
+            return e;
+    }
+    return cudaSuccess;
 }
 
 } // namespace vgx

@@ -94,9 +94,10 @@ cudaError_t launch_stream_tail(Variant v, uint32_t max_slots, cudaStream_t s, co
                                uint32_t wave);
 // Primary-hit AOVs (normals.slang, aov.slang); camera18 is the reference's camera record.
 cudaError_t launch_aov_normals(cudaStream_t s, const vgd::Ctx& c, const float* camera18, float* out);
-cudaError_t launch_aov_main(cudaStream_t s, const vgd::Ctx& c, const float* camera18, float* albedo,
+size_t aov_scratch_bytes(uint32_t w, uint32_t h); // device memory for launch_aov_main's `scratch`, 256-byte aligned
+cudaError_t launch_aov_main(int sms, cudaStream_t s, const vgd::Ctx& c, const float* camera18, float* albedo,
                             uint32_t albedo_stride, float* depth, uint32_t depth_stride, uint32_t* object_ids,
-                            uint32_t* material_ids, float* coverage);
+                            uint32_t* material_ids, float* coverage, void* scratch);
 cudaError_t launch_emitter_aux(cudaStream_t s, const float* emitters, uint32_t n, float4* out);
 // `fetch`: a cleared device word.
 cudaError_t launch_trace_rays(int sms, cudaStream_t s, const vgd::Ctx& c, const float* rays, uint4* out, uint32_t n,

@@ -1619,7 +1619,8 @@ static int render_aovs(VgRenderer* r, uint32_t width, uint32_t height, float* al
     cudaStream_t s = r->ctx->stream;
     TempBuf d;
     int st;
-    if ((st = d.get(r->ctx, px * 28)) != VG_OK)
+    const size_t planes = (px * 28 + 255) / 256 * 256;
+    if ((st = d.get(r->ctx, planes + vgx::aov_scratch_bytes(width, height))) != VG_OK)
         return st;
     float* ad = (float*)d.p;
     float* dp = depth ? ad + 3 * px : ad + 3;
@@ -1629,7 +1630,8 @@ static int render_aovs(VgRenderer* r, uint32_t width, uint32_t height, float* al
     camera_record(r, width, height, rec);
     vgd::Ctx c = make_ctx(r, nullptr);
     VG_CHECK(cudaMemsetAsync(r->err.p, 0, 4, s), "error flag");
-    VG_CHECK(vgx::launch_aov_main(s, c, rec, ad, depth ? 3 : 4, dp, depth ? 1 : 4, oi, mi, cv), "aov launch");
+    VG_CHECK(vgx::launch_aov_main(r->ctx->sms, s, c, rec, ad, depth ? 3 : 4, dp, depth ? 1 : 4, oi, mi, cv, d.at(planes)),
+             "aov launch");
     VG_CHECK(cudaMemcpyAsync(albedo, ad, px * (depth ? 12 : 16), cudaMemcpyDeviceToHost, s), "readback");
     if (depth)
         VG_CHECK(cudaMemcpyAsync(depth, dp, px * 4, cudaMemcpyDeviceToHost, s), "readback");
