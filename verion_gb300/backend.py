@@ -11,6 +11,7 @@ import mmap
 import os
 import threading
 import weakref
+from collections import deque
 from dataclasses import dataclass
 from enum import IntEnum
 from pathlib import Path
@@ -295,11 +296,16 @@ class _HostPages:
     the GPU's copy writes them (64 MB: 2.5 to 3.9 ms, against 0.36 ms into mapped pages), so the memory
     of arrays that the caller has dropped is kept for the next ones. An array owns its block until the
     last view of it is gone; at most KEEP bytes wait here, the oldest go first. New blocks are mapped when
-    they are made. Safe from several threads, and from a collection inside its own calls."""
+    they are made.
+
+    Safe from several threads, and from a collection at any point, which may drop arrays or ask for new ones: a dropped
+    block goes to a deque, and only the lock's holder touches the idle list. Whoever finds the lock taken leaves
+    its blocks to the holder, who looks again after letting go."""
     LEAST, KEEP = 1 << 18, 256 << 20
 
     def __init__(self):
-        self._lock = threading.RLock()
+        self._lock = threading.Lock()
+        self._returned = deque()  # (size, mmap) of dropped arrays, not yet among the idle
         self._idle = []  # (size, mmap), oldest first
 
     @staticmethod
@@ -312,12 +318,7 @@ class _HostPages:
         if n < self.LEAST or not hasattr(mmap, "MAP_POPULATE"):
             return np.empty(count, dtype)
         size = self._size(n)
-        block = None
-        with self._lock:
-            for i in range(len(self._idle) - 1, -1, -1):
-                if self._idle[i][0] == size:
-                    block = self._idle.pop(i)[1]
-                    break
+        block = self._take(size)
         if block is None:
             block = mmap.mmap(-1, size, flags=mmap.MAP_PRIVATE | mmap.MAP_ANONYMOUS | mmap.MAP_POPULATE)
         # The arrays hold this object through the buffer protocol: its end is the end of all of them.
@@ -325,11 +326,39 @@ class _HostPages:
         weakref.finalize(owner, self._give, size, block).atexit = False
         return np.frombuffer(owner, dtype, count)
 
+    def _take(self, size: int):
+        block = None
+        # (A finalizer that asks for an array inside this very section waits its millisecond and maps a new one.)
+        if self._lock.acquire(timeout=0.001):
+            try:
+                self._sweep()
+                for i in range(len(self._idle) - 1, -1, -1):
+                    if self._idle[i][0] == size:
+                        block = self._idle.pop(i)[1]
+                        break
+            finally:
+                self._lock.release()
+            self._settle()
+        return block
+
     def _give(self, size: int, block) -> None:
-        with self._lock:
-            self._idle.append((size, block))
-            while sum(b for b, _ in self._idle) > self.KEEP:
-                self._idle.pop(0)
+        self._returned.append((size, block))
+        self._settle()
+
+    def _settle(self) -> None:
+        while self._returned and self._lock.acquire(blocking=False):
+            try:
+                self._sweep()
+            finally:
+                self._lock.release()
+
+    def _sweep(self) -> None:
+        """With the lock: the dropped blocks join the idle ones, of which the oldest go."""
+        while self._returned:
+            self._idle.append(self._returned.popleft())
+        held = sum(b for b, _ in self._idle)
+        while held > self.KEEP:
+            held -= self._idle.pop(0)[0]
 
 
 _pages = _HostPages()
