@@ -14,6 +14,7 @@
 #include "../../include/vgcuda.h"
 #include "bvh_build.h"
 #include "launch.h"
+#include "temp_pool.h"
 
 namespace vgh {
 // Error text and out-of-memory figures of the last failing call on this thread (one instance
@@ -26,6 +27,7 @@ using vgh::g_oom_needed;
 using vgh::g_oom_available;
 
 using namespace vgl;
+using vgh::TempPool;
 
 struct VgCache;
 
@@ -95,12 +97,6 @@ int wait_event(cudaEvent_t ev)
 
 } // namespace
 
-namespace vgh {
-// Device allocations and frees made by this library since it was loaded (all of them go through
-// alloc() and DevBuf), readable through vg_debug_allocations.
-inline std::atomic<uint64_t> g_mallocs{0}, g_frees{0};
-} // namespace vgh
-
 namespace {
 
 struct DevBuf {
@@ -120,64 +116,6 @@ struct DevBuf {
         p = nullptr;
         bytes = 0;
         part = false;
-    }
-};
-
-// Device buffers that entry points use for the length of a call (rays and hits, records, AOV planes), kept
-// for the next call: a cudaMalloc and cudaFree of some tens of MB cost more than most of those calls'
-// kernels. A buffer has one owner at a time (TempBuf), whichever thread that is on. All of its uses are in the
-// order of the context's stream, so that the next owner's work comes after the last one's. At most KEEP bytes
-// wait here (twice that while the stream is busy: freeing waits for the GPU); they go with the context.
-struct TempPool {
-    static constexpr size_t KEEP = 256u << 20;
-    std::mutex mu;
-    std::vector<std::pair<void*, size_t>> idle;
-    size_t idle_bytes = 0;
-    // The smallest idle buffer of at least n bytes and at most four times that.
-    void* take(size_t n, size_t* bytes)
-    {
-        std::lock_guard<std::mutex> lock(mu);
-        size_t best = idle.size();
-        for (size_t i = 0; i < idle.size(); i++)
-            if (idle[i].second >= n && idle[i].second / 4 <= n && (best == idle.size() || idle[i].second < idle[best].second))
-                best = i;
-        if (best == idle.size())
-            return nullptr;
-        void* p = idle[best].first;
-        *bytes = idle[best].second;
-        idle_bytes -= idle[best].second;
-        idle.erase(idle.begin() + (long)best);
-        return p;
-    }
-    void give(void* p, size_t bytes, cudaStream_t s)
-    {
-        std::vector<void*> drop;
-        size_t keep = cudaStreamQuery(s) == cudaErrorNotReady ? 2 * KEEP : KEEP;
-        {
-            std::lock_guard<std::mutex> lock(mu);
-            if (bytes <= keep) {
-                while (idle_bytes + bytes > keep) { // the oldest first
-                    drop.push_back(idle.front().first);
-                    idle_bytes -= idle.front().second;
-                    idle.erase(idle.begin());
-                }
-                idle.emplace_back(p, bytes);
-                idle_bytes += bytes;
-            } else {
-                drop.push_back(p);
-            }
-        }
-        for (void* q : drop) {
-            cudaFree(q);
-            vgh::g_frees++;
-        }
-    }
-    ~TempPool()
-    {
-        for (auto& b : idle) {
-            cudaFree(b.first);
-            vgh::g_frees++;
-        }
     }
 };
 
@@ -271,7 +209,7 @@ struct DevGuard {
 struct BatchState; // vg_batch_render's device buffers and captured graph (batch.cu)
 
 struct VgContext {
-    int device = 0;
+    const int device;
     cudaStream_t stream = nullptr;
     int sms = 0;
     uint64_t uploaded = 0;
@@ -285,6 +223,7 @@ struct VgContext {
     cudaEvent_t fork = nullptr, join = nullptr;  // ordering between `stream` and `side`
     TempPool temps;
     RingPool rings;
+    explicit VgContext(int dev) : device(dev), temps(dev) {}
     ~VgContext();
 };
 
@@ -396,37 +335,30 @@ int dev_of(const VgContext* ctx) { return ctx ? ctx->device : -1; }
 int dev_of(const VgRenderer* r) { return r ? r->device : -1; }
 int dev_of(const VgAccum* acc) { return acc ? acc->device : -1; }
 
-int check_fits(size_t bytes)
+// Device memory of n bytes. Does not fit: VG_ERR_OOM with what was asked for and what there was.
+int device_memory(void** p, size_t n)
 {
-    size_t free_b = 0, total_b = 0;
-    cudaError_t e = cudaMemGetInfo(&free_b, &total_b);
-    if (e != cudaSuccess)
-        return cuda_fail(e, "cudaMemGetInfo");
-    if (bytes > free_b) {
-        g_oom_needed = bytes;
-        g_oom_available = free_b;
-        return fail(VG_ERR_OOM, "out of GPU memory: needed " + std::to_string(bytes) + " bytes, available " +
-                                    std::to_string(free_b));
+    size_t available = 0;
+    cudaError_t e = vgh::device_alloc(p, n, &available);
+    if (e == cudaErrorMemoryAllocation && n > available) {
+        g_oom_needed = n;
+        g_oom_available = available;
+        return fail(VG_ERR_OOM, "out of GPU memory: needed " + std::to_string(n) + " bytes, available " +
+                                    std::to_string(available));
     }
-    return VG_OK;
+    return e == cudaSuccess ? VG_OK : cuda_fail(e, "cudaMalloc");
 }
 
 int alloc(DevBuf& b, size_t bytes, cudaStream_t s, bool zero)
 {
     b.release();
     size_t n = std::max<size_t>(bytes, 16);
-    int st = check_fits(n);
+    int st = device_memory(&b.p, n);
     if (st != VG_OK)
         return st;
-    cudaError_t e = cudaMalloc(&b.p, n);
-    if (e != cudaSuccess) {
-        b.p = nullptr;
-        return cuda_fail(e, "cudaMalloc");
-    }
-    vgh::g_mallocs++;
     b.bytes = n;
     if (zero) {
-        e = cudaMemsetAsync(b.p, 0, n, s);
+        cudaError_t e = cudaMemsetAsync(b.p, 0, n, s);
         if (e != cudaSuccess)
             return cuda_fail(e, "cudaMemsetAsync");
     }
@@ -483,15 +415,9 @@ struct TempBuf {
         p = c->temps.take(n, &bytes);
         if (p)
             return VG_OK;
-        int st = check_fits(n);
+        int st = device_memory(&p, n);
         if (st != VG_OK)
             return st;
-        cudaError_t e = cudaMalloc(&p, n);
-        if (e != cudaSuccess) {
-            p = nullptr;
-            return cuda_fail(e, "cudaMalloc");
-        }
-        vgh::g_mallocs++;
         bytes = n;
         return VG_OK;
     }

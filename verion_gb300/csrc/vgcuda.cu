@@ -486,8 +486,7 @@ int vg_context_create_on(int device, VgContext** out)
     if (prop.major != 10 || prop.minor != 3)
         return fail(VG_ERR_UNSUPPORTED, std::string("device ") + prop.name + " is not sm_103 (GB300)");
     DevGuard device_guard(device);
-    VgContext* ctx = new VgContext();
-    ctx->device = device;
+    VgContext* ctx = new VgContext(device);
     ctx->sms = prop.multiProcessorCount;
     cudaError_t e = cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking);
     if (e != cudaSuccess) {
