@@ -331,14 +331,16 @@ class _HostPages:
         # (A finalizer that asks for an array inside this very section waits its millisecond and maps a new one.)
         if self._lock.acquire(timeout=0.001):
             try:
-                self._sweep()
+                if self._returned:
+                    self._sweep()
                 for i in range(len(self._idle) - 1, -1, -1):
                     if self._idle[i][0] == size:
                         block = self._idle.pop(i)[1]
                         break
             finally:
                 self._lock.release()
-            self._settle()
+            if self._returned:
+                self._settle()
         return block
 
     def _give(self, size: int, block) -> None:
