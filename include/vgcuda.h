@@ -204,8 +204,8 @@ typedef enum VgWavefrontMode { VG_WAVEFRONT_PER_SAMPLE = 0, VG_WAVEFRONT_STREAMI
 int vg_set_wavefront_mode(VgRenderer* r, int mode);
 /* Streaming mode: when at most `threshold` slots are live after a wave, or the frame has no more pixels
  * than that, the rest of the batch (those paths and their remaining samples) runs in one launch instead of
- * one wave per bounce: with deferred shadows as block wavefronts, without them a path per thread. 0
- * disables it. Default 262144 (32768 without deferred shadows). */
+ * one wave per bounce: with deferred shadows as block wavefronts, without them (and in vg_batch_render's
+ * wavefront) a path per thread. 0 disables it. Default 262144; a path per thread from at most 32768 slots. */
 int vg_set_stream_tail(VgRenderer* r, uint32_t threshold);
 /* Streaming mode: trace the bounce's emitter / environment shadow ray after shade, with the next wave's rays
  * (default on), or inline in shade (off, and always with ReSTIR GI or ReSTIR with the lighting split). Same sums

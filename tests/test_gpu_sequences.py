@@ -74,3 +74,34 @@ def test_a_deadline_passed_returns_at_once_and_leaves_the_context_usable(gpu_ctx
         acc = r.new_accumulation(33, 31)
         r.accumulate(acc, 2)
         assert np.array_equal(acc.sums(), want)
+
+
+def test_tail_threshold_of_the_inline_form_stays_at_its_own_most(gpu_ctx):
+    # A path per thread from at most 32,768 slots, whatever the block wavefront's threshold is set to.
+    p = pack.pack(scenes.many_spheres(spheres=4, sphere_n=15, grid=48, hdri=(64, 32)))
+
+    def waves(threshold):
+        r = Renderer(gpu_ctx, p)
+        r.set_integrator(Integrator.WAVEFRONT)
+        r.set_deferred_shadows(False)
+        if threshold is not None:
+            r.set_stream_tail(threshold)
+        acc = r.new_accumulation(320, 300)
+        r.accumulate(acc, 2)
+        return acc.last_waves()
+
+    assert waves(1 << 18) == waves(None)
+
+
+def test_autotune_tries_what_its_frame_reaches(gpu_ctx):
+    p = pack.pack(scenes.many_spheres(spheres=4, sphere_n=15, grid=48, hdri=(64, 32)))
+    r = Renderer(gpu_ctx, p)
+    t = r.autotune(96, 54, 1, bvh=False)
+    if t["deferred_shadows"] and t["stream_tail"] >= 96 * 54 and not t["graph_waves"]:
+        # One launch: itself, shadows, three tails, the graph, two refills, two step counts.
+        assert t["trials"] == 10
+        assert t["dynamic_fetch"] and t["material_sort"] and not t["coop_triangles"]
+    # ReSTIR GI traces its light samples inside shade: the threshold tried and reported is that form's.
+    r = Renderer(gpu_ctx, p)
+    r.set_restir(Restir(di=True, gi=True))
+    assert r.autotune(96, 54, 1, bvh=False)["stream_tail"] in (0, 8192, 32768)

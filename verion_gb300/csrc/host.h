@@ -240,6 +240,8 @@ struct Restir {
 constexpr uint32_t MAX_CACHE_FRAME = 16;           // samples per radiance-cache frame at most
 constexpr uint32_t CACHE_WARMUP_SAMPLE = 0x40000000u; // first sample index of cache warm-up frames
 
+constexpr uint32_t INLINE_TAIL = 32768;
+
 struct VgRenderer {
     VgContext* ctx = nullptr;
     int device = -1; // the context's device, kept here so no call dereferences a destroyed context
@@ -257,8 +259,9 @@ struct VgRenderer {
     int wavefront_mode = VG_WAVEFRONT_STREAMING;
     // Live slots at or below which the streaming tail runs in one launch: a block wavefront (deferred shadows;
     // 640x360 of the 1M-triangle scene, 8 samples, tail at 0 / 32768 / 262144: 9.3 / 7.4 / 7.1 ms, 1920x1080:
-    // 30.6 / 29.1 / 28.8), or a path per thread.
-    uint32_t tail_threshold = 262144, inline_tail_threshold = 32768;
+    // 30.6 / 29.1 / 28.8), or a path per thread (shadow rays in shade, and the batch wavefront), for which
+    // INLINE_TAIL is the most.
+    uint32_t tail_threshold = 262144, inline_tail_threshold = INLINE_TAIL;
     bool adaptive = false;
     float adaptive_threshold = 0.02f;
     uint32_t adaptive_min_spp = 16;

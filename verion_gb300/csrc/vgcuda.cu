@@ -866,7 +866,8 @@ int vg_set_stream_tail(VgRenderer* r, uint32_t threshold)
 {
     if (!r)
         return fail(VG_ERR_INVALID, "null renderer");
-    r->tail_threshold = r->inline_tail_threshold = threshold;
+    r->tail_threshold = threshold;
+    r->inline_tail_threshold = std::min(threshold, INLINE_TAIL);
     return VG_OK;
 }
 
@@ -1474,26 +1475,22 @@ int vg_autotune(VgRenderer* r, const VgPacked* pk, uint32_t width, uint32_t heig
     };
     try_setting(
         [&](bool v, bool) {
-            bool o = r->dynamic_fetch;
-            r->dynamic_fetch = v;
-            return o;
-        },
-        std::vector<bool>{!r->dynamic_fetch});
-    try_setting(
-        [&](bool v, bool) {
             bool o = r->defer_shadows;
             r->defer_shadows = v;
             return o;
         },
         std::vector<bool>{!r->defer_shadows});
+    // The tail of the form that runs: block wavefronts, or a path per thread where shade traces the light samples.
+    const bool inlined = !r->defer_shadows || (r->restir.on && r->restir.gi);
+    uint32_t& tail = inlined ? r->inline_tail_threshold : r->tail_threshold;
     std::vector<uint32_t> tails;
-    for (uint32_t t : {0u, 32768u, 131072u, 262144u})
-        if (t != r->tail_threshold)
+    for (uint32_t t : inlined ? std::vector<uint32_t>{0u, 8192u, INLINE_TAIL} : std::vector<uint32_t>{0u, 32768u, 131072u, 262144u})
+        if (t != tail)
             tails.push_back(t);
     try_setting(
         [&](uint32_t v, bool) {
-            uint32_t o = r->tail_threshold;
-            r->tail_threshold = v;
+            uint32_t o = tail;
+            tail = v;
             return o;
         },
         tails);
@@ -1504,20 +1501,31 @@ int vg_autotune(VgRenderer* r, const VgPacked* pk, uint32_t width, uint32_t heig
             return o;
         },
         std::vector<uint32_t>{r->graph_waves == 0 ? 8u : 0u});
-    try_setting(
-        [&](bool v, bool) {
-            bool o = r->coop_tris;
-            r->coop_tris = v;
-            return o;
-        },
-        std::vector<bool>{!r->coop_tris});
-    try_setting(
-        [&](bool v, bool) {
-            bool o = r->material_sort;
-            r->material_sort = v;
-            return o;
-        },
-        std::vector<bool>{!r->material_sort});
+    // A trial frame that runs in one launch reaches none of the waves' settings: a trial of them would be decided by noise.
+    const bool waves = inlined || (uint64_t)width * height > r->tail_threshold || r->graph_waves > 0 || r->traversal_stats;
+    if (waves) {
+        try_setting(
+            [&](bool v, bool) {
+                bool o = r->dynamic_fetch;
+                r->dynamic_fetch = v;
+                return o;
+            },
+            std::vector<bool>{!r->dynamic_fetch});
+        try_setting(
+            [&](bool v, bool) {
+                bool o = r->coop_tris;
+                r->coop_tris = v;
+                return o;
+            },
+            std::vector<bool>{!r->coop_tris});
+        try_setting(
+            [&](bool v, bool) {
+                bool o = r->material_sort;
+                r->material_sort = v;
+                return o;
+            },
+            std::vector<bool>{!r->material_sort});
+    }
     std::vector<uint32_t> refills, steps;
     for (uint32_t v : {4u, 8u, 16u})
         if (v != r->fetch_refill)
@@ -1542,7 +1550,7 @@ int vg_autotune(VgRenderer* r, const VgPacked* pk, uint32_t width, uint32_t heig
     int most = vgx::wf_extend_blocks_per_sm();
     std::vector<int> extend_blocks;
     for (int b : {most, (3 * most) / 4, most / 2})
-        if (b >= 1 && b != r->extend_blocks)
+        if (waves && b >= 1 && b != r->extend_blocks)
             extend_blocks.push_back(b);
     try_setting(
         [&](int v, bool) {
@@ -1572,7 +1580,7 @@ int vg_autotune(VgRenderer* r, const VgPacked* pk, uint32_t width, uint32_t heig
         return st;
     out->dynamic_fetch = r->dynamic_fetch;
     out->deferred_shadows = r->defer_shadows;
-    out->stream_tail = r->tail_threshold;
+    out->stream_tail = tail;
     out->graph_waves = r->graph_waves;
     out->bvh_traversal_cost = r->bvh_traversal_cost;
     out->extend_blocks_per_sm = r->extend_blocks;
