@@ -31,7 +31,7 @@ CXX_FLAGS = ["-O2", "-std=c++17", "-fPIC", "-ffp-contract=off", "-I", str(CSRC)]
 
 CU_SOURCES = ["kern_mk.cu", "kern_wf.cu", "kern_wf_light.cu", "kern_wf_finish.cu", "kern_wf_restir.cu", "kern_nrc.cu", "kern_batch.cu", "kern_bwave.cu", "vgcuda.cu", "cache.cu", "batch.cu"]
 CXX_SOURCES = ["bvh_build.cpp", "exr.cpp"]
-DEPS = ["vg_math.h", "host.h", "temp_pool.h", "cdf_guide.h", "tc.cuh", "nrc.cuh", "nrc_device.cuh", "vg_layout.h", "vec3.h", "bvh8.h", "traverse.cuh", "pt_device.cuh", "kernels.cuh", "megakernel.cuh", "aov.cuh",
+DEPS = ["vg_math.h", "host.h", "temp_pool.h", "cdf_guide.h", "tc.cuh", "nrc.cuh", "nrc_device.cuh", "vg_layout.h", "vec3.h", "bvh8.h", "traverse.cuh", "adaptive_test.h", "pt_device.cuh", "kernels.cuh", "megakernel.cuh", "aov.cuh",
         "launch.h", "ray_chunks.h", "launch_nrc.h", "launch_batch.h", "batch.h", "cache_host.h", "bvh_build.h"]
 
 

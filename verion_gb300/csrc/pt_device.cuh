@@ -10,6 +10,7 @@
 #pragma once
 #include <stdint.h>
 
+#include "adaptive_test.h"
 #include "ctx.h"
 #include "traverse.cuh"
 #include "vg_layout.h"
@@ -1636,21 +1637,9 @@ __device__ __forceinline__ bool pixelActive(const Ctx& c, uint32_t p)
     if (n < (A)c.p[P_ADAPTIVE_MIN_SPP])
         return true;
     if (sizeof(A) == 8) {
-        // Most pixels are far from the threshold: variance of the mean against its square,
-        // (s2 / n - mean^2) / (n - 1) > (threshold m)^2, in single precision. `e` bounds the left side's
-        // rounding (2^-19 of its terms, some 30 ulps), the factors the right side's; only in between does
-        // the test below run in double, whose own rounding is far inside that margin. Not finite, or a
-        // negative threshold: no comparison holds, or none is made. (GB300 has few FP64 units: four
-        // divisions and a root per finished path kept them 61% busy in the resolve stage.)
-        float thr = pf(c, P_ADAPTIVE_THRESHOLD);
-        float nf = (float)n, mf = (float)st[3 * p + 1] / nf, q = (float)st[3 * p + 2] / nf, m2 = mf * mf;
-        float left = q - m2, e = 1.9073486e-6f * (q + m2);
-        float right = thr * fmaxf(mf, 0.05f);
-        right = right * right * (nf - 1.0f);
-        if (thr >= 0.0f && left - e > right * 1.00001f)
-            return true;
-        if (thr >= 0.0f && left + e < right * 0.99999f)
-            return false;
+        int sure = adaptive_certain((double)n, (double)st[3 * p + 1], (double)st[3 * p + 2], pf(c, P_ADAPTIVE_THRESHOLD));
+        if (sure >= 0)
+            return sure != 0;
     }
     A mean = st[3 * p + 1] / n;
     A var = (st[3 * p + 2] / n - mean * mean);
