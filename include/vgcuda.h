@@ -264,11 +264,12 @@ int vg_autotune(VgRenderer* r, const VgPacked* packed, uint32_t width, uint32_t 
                 VgTuneResult* out);
 /* With stage timing: seconds of the last call's tail launch (0 if none ran). */
 double vg_accum_tail_seconds(const VgAccum* acc);
-/* Streaming mode: waves (extend + shade pairs) issued by the last vg_accumulate. */
+/* Streaming mode: waves issued by the last vg_accumulate (with ReSTIR by its last sample). A frame that went into one
+ * launch instead (vg_set_stream_tail) counts as one. */
 uint32_t vg_accum_last_waves(const VgAccum* acc);
 /* Streaming mode, last vg_accumulate: per wave, the live slots after it and (with stage timing)
  * the extend, shade and shadow-stage milliseconds (shadow 0 when shade traced inline), 4 floats
- * per wave for up to `waves` waves. Returns the number of waves recorded. */
+ * per wave for up to `waves` waves. Returns the number of waves recorded: none of a frame in one launch. */
 size_t vg_accum_wave_profile(const VgAccum* acc, float* out, size_t waves);
 /* Wavefront only: count rays, BVH nodes visited and triangles tested in the extend stage of
  * later accumulate calls (read with vg_accum_traversal_stats). */
