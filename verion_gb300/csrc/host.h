@@ -257,10 +257,13 @@ struct VgRenderer {
     bool stage_timing = false;
     bool traversal_stats = false;
     int wavefront_mode = VG_WAVEFRONT_STREAMING;
-    // Live slots at or below which the streaming tail runs in one launch: a block wavefront (deferred shadows;
-    // 640x360 of the 1M-triangle scene, 8 samples, tail at 0 / 32768 / 262144: 9.3 / 7.4 / 7.1 ms, 1920x1080:
-    // 30.6 / 29.1 / 28.8), or a path per thread (shadow rays in shade, and the batch wavefront), for which
-    // INLINE_TAIL is the most.
+    // Live slots at or below which the streaming tail runs in one launch: a block wavefront (deferred shadows), or a
+    // path per thread (shadow rays in shade, and the batch wavefront), for which INLINE_TAIL is the most. Calls of
+    // 8 samples in ms with the tail at 0 / 32768 / 262144: 256x144 Cornell 2.24 / 1.18 / 0.86, 110k triangles 3.39 / 2.24 /
+    // 1.95, 1M 6.8 / 4.3 / 3.6; 512x512 3.84 / 3.19 / 2.94, 5.05 / 4.29 / 4.25, 9.8 / 8.0 / 8.0; 960x540 4.41 / 3.89 / 3.71, 6.79 /
+    // 6.05 / 5.78, 12.8 / 11.1 / 10.8. Whole frames above the line lose in one launch: 1024x1024 Cornell 11.3 against 9.4,
+    // 1M 23.3 against 17.1. With cut-outs, whose shadow rays the block's resolve stage follows, 512x512 takes 14.2 / 11.6 /
+    // 13.1 (11.1 at 131072).
     uint32_t tail_threshold = 262144, inline_tail_threshold = INLINE_TAIL;
     bool adaptive = false;
     float adaptive_threshold = 0.02f;

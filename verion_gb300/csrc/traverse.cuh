@@ -374,7 +374,6 @@ __device__ __forceinline__ TraceHit walk_hit(const float4* __restrict__ tris, co
     return h;
 }
 
-// Closest hit (ANY = false) or any hit (ANY = true) with 0 < t < tmax.
 // The answer of a queue item without a ray.
 __device__ __forceinline__ TraceHit no_hit(float tmax)
 {
@@ -387,6 +386,7 @@ __device__ __forceinline__ TraceHit no_hit(float tmax)
     return h;
 }
 
+// Closest hit (ANY = false) or any hit (ANY = true) with 0 < t < tmax.
 template <bool ANY>
 __device__ __forceinline__ TraceHit trace_bvh(const uint4* __restrict__ nodes, const float4* __restrict__ tris, V3 o,
                                               V3 d, float tmax, uint32_t* err)
@@ -400,17 +400,6 @@ __device__ __forceinline__ TraceHit trace_bvh(const uint4* __restrict__ nodes, c
 }
 
 // ---------------------------------------------------------------------------------------------
-// Queue traversal with dynamic ray fetch: a warp keeps one ray per lane and, whenever at least
-// `refill` lanes have finished theirs, hands those lanes the next rays of the queue (one atomic per
-// refill), so the warp does not idle on its longest ray (Aila and Laine, "Understanding the
-// Efficiency of Ray Traversal on GPUs", HPG 2009). Each lane runs at most `steps` node visits
-// between refills. Results are those of trace_bvh: the hit rule does not depend on the visiting order.
-//
-// get(i, o, d, tmax, any) loads queue item i into a ray (with HITS_EITHER also whether any hit will do)
-// and returns false when it has no ray (it then completes at once with a miss); put(i, hit) stores the
-// result of item i.
-
-// ---------------------------------------------------------------------------------------------
 // Warp-cooperative leaf testing. In walk_step every lane tests its node's triangles itself, so a
 // warp runs its triangle loop as often as its busiest lane needs while the other lanes idle: on the
 // 1M-triangle workload about a third of the lanes are active per instruction. Here a step is split
@@ -418,10 +407,10 @@ __device__ __forceinline__ TraceHit trace_bvh(const uint4* __restrict__ nodes, c
 // (ray, triangle) pairs its lanes collected, one pair per lane (coop_tris), and then every lane
 // picks its next node (next_node). The visiting order per ray is walk_step's, and the hit rule does
 // not depend on which lane tests a triangle, so the results and the counters are the same.
-// Measured on the 1M-triangle workload (1080p, depth 16): the extend stage takes 0.447 ms per launch
-// this way against 0.407 ms with each lane testing its own triangles, so it is off by default: the
-// per-step scan, owner search and shared-memory reductions cost more issue slots than the divergent
-// triangle loop they replace.
+// Measured on the 1M-triangle workload (1080p, depth 16, before the node test lost its branches): the extend
+// stage took 0.447 ms per launch this way against 0.407 ms with each lane testing its own triangles, so it is
+// off by default: the per-step scan, owner search and shared-memory reductions cost more issue slots than the
+// divergent triangle loop they replace.
 //
 // A pair lane reads the owner's ray from shared memory (written once per ray) and reports a hit
 // with a 64-bit shared-memory atomicMin of (t bits << 32 | global triangle index) on the owner's
@@ -549,7 +538,7 @@ __device__ __forceinline__ bool coop_tris(CoopWarp& cw, uint32_t lane, uint32_t 
     return false;
 }
 
-// trace_queue with warp-cooperative leaf testing (same dynamic fetch, same results). `cw` is this
+// trace_queue (below) with warp-cooperative leaf testing (same dynamic fetch, same results). `cw` is this
 // warp's shared state.
 template <bool ANY, typename GetRay, typename PutHit>
 __device__ __forceinline__ void trace_queue_coop(const uint4* __restrict__ nodes, const float4* __restrict__ tris,
@@ -615,6 +604,17 @@ __device__ __forceinline__ void trace_queue_coop(const uint4* __restrict__ nodes
         }
     }
 }
+
+// ---------------------------------------------------------------------------------------------
+// Queue traversal with dynamic ray fetch: a warp keeps one ray per lane and, whenever at least
+// `refill` lanes have finished theirs, hands those lanes the next rays of the queue (one atomic per
+// refill), so the warp does not idle on its longest ray (Aila and Laine, "Understanding the
+// Efficiency of Ray Traversal on GPUs", HPG 2009). Each lane runs at most `steps` node visits
+// between refills. Results are those of trace_bvh: the hit rule does not depend on the visiting order.
+//
+// get(i, o, d, tmax, any) loads queue item i into a ray (with HITS_EITHER also whether any hit will do)
+// and returns false when it has no ray (it then completes at once with a miss); put(i, hit) stores the
+// result of item i.
 
 // The body of trace_queue and trace_queue_scenes: with SCENES, `get` also names the BVH of each ray
 // (its node and triangle arrays), which the lane keeps while it walks that ray.
